@@ -1416,6 +1416,49 @@ Tensor upsample_backward(const GridPtr &coarse, const GridPtr &fine, const std::
     return dx.narrow(1, 0, C).reshape(x.sizes());
 }
 
+// Group normalisation of jagged rows: (y, mean, rstd); weight / bias in the accumulation type.
+std::vector<Tensor> group_norm_forward(const Tensor &x_in, const Tensor &joff, int64_t groups,
+                                       const std::optional<Tensor> &weight, const std::optional<Tensor> &bias,
+                                       double eps) {
+    c10::cuda::CUDAGuard guard(x_in.device());
+    Tensor x = x_in.contiguous();
+    const int64_t n = x.size(0), C = x.size(1), B = joff.size(0) - 1;
+    const auto acc = x.scalar_type() == torch::kFloat64 ? torch::kFloat64 : torch::kFloat32;
+    Tensor y = torch::empty_like(x), mean = torch::zeros({B, groups}, x.options().dtype(acc)),
+           rstd = torch::zeros({B, groups}, x.options().dtype(acc));
+    size_t wsb = 0;
+    check_status(fvgb_group_norm_workspace(fvgb_dtype(x), n, (int32_t)C, (int32_t)groups, (int32_t)B, 0, &wsb),
+                 "group norm (workspace)");
+    Tensor ws = workspace(wsb, x.device());
+    check_status(fvgb_group_norm_forward(fvgb_dtype(x), x.data_ptr(), n, (int32_t)C, (int32_t)groups,
+                                         joff.data_ptr<int64_t>(), (int32_t)B, weight ? weight->data_ptr() : nullptr,
+                                         bias ? bias->data_ptr() : nullptr, eps, y.data_ptr(), mean.data_ptr(),
+                                         rstd.data_ptr(), ws.data_ptr(), ws.numel(), cur_stream()),
+                 "group norm");
+    return {y, mean, rstd};
+}
+
+// (dx, dweight, dbias) of that forward; dx undefined where it is not needed
+std::vector<Tensor> group_norm_backward(const Tensor &dy_in, const Tensor &x_in, const Tensor &joff, int64_t groups,
+                                        const std::optional<Tensor> &weight, const Tensor &mean, const Tensor &rstd,
+                                        bool need_dx) {
+    c10::cuda::CUDAGuard guard(x_in.device());
+    Tensor x = x_in.contiguous(), dy = dy_in.contiguous();
+    const int64_t n = x.size(0), C = x.size(1), B = joff.size(0) - 1;
+    Tensor dx = need_dx ? torch::empty_like(x) : Tensor();
+    Tensor dw = torch::zeros({C}, mean.options()), db = torch::zeros({C}, mean.options());
+    size_t wsb = 0;
+    check_status(fvgb_group_norm_workspace(fvgb_dtype(x), n, (int32_t)C, (int32_t)groups, (int32_t)B, 1, &wsb),
+                 "group norm backward (workspace)");
+    Tensor ws = workspace(wsb, x.device());
+    check_status(fvgb_group_norm_backward(fvgb_dtype(x), x.data_ptr(), dy.data_ptr(), n, (int32_t)C, (int32_t)groups,
+                                          joff.data_ptr<int64_t>(), (int32_t)B, weight ? weight->data_ptr() : nullptr,
+                                          mean.data_ptr(), rstd.data_ptr(), need_dx ? dx.data_ptr() : nullptr,
+                                          dw.data_ptr(), db.data_ptr(), ws.data_ptr(), ws.numel(), cur_stream()),
+                 "group norm backward");
+    return {dx, dw, db};
+}
+
 std::optional<Tensor> opt(const std::optional<Tensor> &t) { return t; }
 
 }  // namespace fvgbh
@@ -1492,6 +1535,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("conv_backward", &conv_backward, py::call_guard<py::gil_scoped_release>());
     m.def("halo_conv", &halo_conv, py::call_guard<py::gil_scoped_release>());
     m.def("halo_wgrad", &halo_wgrad, py::call_guard<py::gil_scoped_release>());
+    m.def("group_norm_forward", &group_norm_forward, py::call_guard<py::gil_scoped_release>());
+    m.def("group_norm_backward", &group_norm_backward, py::call_guard<py::gil_scoped_release>());
     m.def("pool_forward", &pool_forward);
     m.def("pool_backward", &pool_backward);
     m.def("upsample_forward", &upsample_forward);

@@ -16,6 +16,7 @@ from typing import Optional, Sequence, Union
 import torch
 import torch.nn as nn
 
+from .._norm import GroupNormFunction, group_norm_composed, group_norm_kernel_takes
 from ..grid_batch import GridBatch
 from ..sparse_conv_pack_info import ConvPackBackend, SparseConvPackInfo
 from .vdbtensor import VDBTensor
@@ -248,30 +249,29 @@ class GroupNorm(nn.GroupNorm):
     """Group normalisation of a VDBTensor's features, per grid of the batch (reference:
     fvdb/nn/modules.py:408-432, which loops over the grids): each (grid, group) is normalised
     over its voxels and the group's channels, with the biased variance and eps of
-    torch.nn.GroupNorm.  One vectorised pass over all grids: the per-(grid, group) sums are
-    segment sums keyed by the voxels' grid index, the variance is taken about the mean (two
-    passes, FP32 or wider), and empty grids contribute nothing.  The segment sums accumulate with
-    atomics on CUDA, so results agree with the per-grid loop to rounding but are not bitwise
-    reproducible from run to run."""
+    torch.nn.GroupNorm; empty grids contribute nothing.  CUDA features run on the kernels of
+    csrc/norm.cu (statistics about chunk means, merged in FP64 in a fixed order: reproducible);
+    group_norm_composed, plain torch operations over all grids at once, serves what the kernels
+    do not take (function transforms, forward-mode differentiation, tracing, features whose
+    lists are not the grid's)."""
 
     def forward(self, input: VDBTensor) -> VDBTensor:
         x = input.data.jdata
-        n, c = x.shape[0], x.shape[1] if x.dim() == 2 else -1
+        c = x.shape[1] if x.dim() == 2 else -1
         if x.dim() != 2 or c != self.num_channels:
             raise ValueError("Input feature should have the same number of channels as GroupNorm")
-        g, b = self.num_groups, input.grid.grid_count
-        acc = torch.float64 if x.dtype == torch.float64 else torch.float32
-        jidx = input.data.jidx.long()
-        xg = x.to(acc).reshape(n, g, c // g)
-        counts = torch.bincount(jidx, minlength=b).to(acc) * (c // g)
-        denom = counts.clamp(min=1)[:, None]
-        mean = torch.zeros(b, g, dtype=acc, device=x.device).index_add_(0, jidx, xg.sum(2)) / denom
-        d = xg - mean[jidx][:, :, None]
-        var = torch.zeros(b, g, dtype=acc, device=x.device).index_add_(0, jidx, (d * d).sum(2)) / denom
-        y = (d * torch.rsqrt(var + self.eps)[jidx][:, :, None]).reshape(n, c)
-        if self.affine:
-            y = y * self.weight.to(acc) + self.bias.to(acc)
-        return VDBTensor(input.grid, input.grid.jagged_like(y.to(x.dtype)), input.kmap)
+        grid = input.grid
+        if group_norm_kernel_takes(x, self.weight, self.bias) and _same_lists(input.data.joffsets, grid.joffsets):
+            y = GroupNormFunction.apply(x, self.weight, self.bias, grid.joffsets, self.num_groups, self.eps)
+        else:
+            y = group_norm_composed(x, input.data.jidx.long(), grid.grid_count, self.num_groups, self.eps, self.weight,
+                                    self.bias)
+        return VDBTensor(grid, grid.jagged_like(y), input.kmap)
+
+
+def _same_lists(a: torch.Tensor, b: torch.Tensor) -> bool:
+    return a is b or (a.shape == b.shape and a.device == b.device and
+                      (a.data_ptr() == b.data_ptr() or torch.equal(a, b)))
 
 
 class Sequential(nn.Sequential):

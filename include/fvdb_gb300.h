@@ -536,6 +536,29 @@ int fvgb_halo_wgrad(int32_t dtype, const FvgbGrid *grid, const void *x, int64_t 
                     int64_t lddy, int32_t c_out, void *dw, void *workspace, size_t workspace_bytes,
                     fvgb_stream_t stream);
 
+/* ------------------------------------------------------------------------------------------
+ * Group normalisation of jagged features: x [n, channels] contiguous rows, grid b's voxels are
+ * rows joffsets[b] .. joffsets[b+1]-1 (device int64 [num_grids + 1], covering [0, n)); each
+ * (grid, group of channels / groups consecutive channels) is normalised over its rows and
+ * channels with the biased variance.  dtype FVGB_F32 / FVGB_F64 / FVGB_BF16 / FVGB_F16; weight,
+ * bias, mean, rstd and the parameter gradients are FP32 (FP64 for FP64).  Statistics are merged in
+ * FP64 in a fixed order (deterministic).  Replaces the per-grid loop of fvdb/nn/modules.py:408-432.
+ * ------------------------------------------------------------------------------------------ */
+/* Workspace bytes of the forward (backward = 0) or the backward (1). */
+int fvgb_group_norm_workspace(int32_t dtype, int64_t n, int32_t channels, int32_t groups, int32_t num_grids,
+                              int32_t backward, size_t *bytes);
+/* y = (x - mean) * rstd * weight + bias (weight, bias may be null); mean and rstd
+ * [num_grids, groups] are written for the backward. */
+int fvgb_group_norm_forward(int32_t dtype, const void *x, int64_t n, int32_t channels, int32_t groups,
+                            const int64_t *joffsets, int32_t num_grids, const void *weight, const void *bias,
+                            double eps, void *y, void *mean, void *rstd, void *workspace, size_t workspace_bytes,
+                            fvgb_stream_t stream);
+/* dx [n, channels], dweight and dbias [channels] (each may be null) of that forward. */
+int fvgb_group_norm_backward(int32_t dtype, const void *x, const void *dy, int64_t n, int32_t channels,
+                             int32_t groups, const int64_t *joffsets, int32_t num_grids, const void *weight,
+                             const void *mean, const void *rstd, void *dx, void *dweight, void *dbias,
+                             void *workspace, size_t workspace_bytes, fvgb_stream_t stream);
+
 #ifdef __cplusplus
 }
 #endif
