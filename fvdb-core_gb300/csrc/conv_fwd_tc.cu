@@ -89,6 +89,9 @@ struct FwdArgs {
     int32_t stages;
     int64_t n_tiles;
     int32_t direct_store;  // 1: output rows contiguous (ldy == cout, cout % 8 == 0): one bulk store per tile
+    // width of the epilogue's own stores where direct_store is off: 2 = 32 bytes (cout, ldy multiples
+    // of 16, y 32-byte aligned), 1 = 16 bytes (multiples of 8, y 16-byte aligned), 0 = one element
+    int32_t vec_store;
     const int32_t *out_rows;  // null: map row m computes output row m; else output row out_rows[m] (-1 = none)
 };
 
@@ -159,6 +162,13 @@ struct UnitWalker {
 
 __device__ __forceinline__ void st_shared_zero16(uint32_t addr) {
     asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(addr), "r"(0) : "memory");
+}
+
+// 32 bytes to global memory in one store (address 32-byte aligned)
+__device__ __forceinline__ void st_global_32(void *p, const uint32_t (&v)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+                 "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
 }
 
 template <int BN, int EBYTES, int PACK, int U>
@@ -430,12 +440,24 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
                     dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
                     if (c0 + 8 < a.cout) dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
                 } else {
-                    __nv_bfloat16 *yrow = reinterpret_cast<__nv_bfloat16 *>(a.y) + yrow_i * a.ldy;
+                    // each thread stores its own row: one whole 32-byte sector per instruction.  With
+                    // 2-byte stores a 256-channel tile took 32,768 partial-sector writes and the
+                    // epilogue, not the contraction, set the kernel's pace (4.3M rows, 128->256 FP8:
+                    // 12.7 ms with 2-byte stores, 4.0 ms with these)
+                    __nv_bfloat16 *yrow = reinterpret_cast<__nv_bfloat16 *>(a.y) + yrow_i * a.ldy + c0;
+                    if (a.vec_store == 2) {
+                        st_global_32(yrow, packed);
+                    } else if (a.vec_store == 1) {
+                        *reinterpret_cast<uint4 *>(yrow) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                        if (c0 + 8 < a.cout)
+                            *reinterpret_cast<uint4 *>(yrow + 8) = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+                    } else {
 #pragma unroll
-                    for (int t = 0; t < 8; ++t) {
-                        const __nv_bfloat162 h2 = *reinterpret_cast<const __nv_bfloat162 *>(&packed[t]);
-                        if (c0 + 2 * t < a.cout) yrow[c0 + 2 * t] = h2.x;
-                        if (c0 + 2 * t + 1 < a.cout) yrow[c0 + 2 * t + 1] = h2.y;
+                        for (int t = 0; t < 8; ++t) {
+                            const __nv_bfloat162 h2 = *reinterpret_cast<const __nv_bfloat162 *>(&packed[t]);
+                            if (c0 + 2 * t < a.cout) yrow[2 * t] = h2.x;
+                            if (c0 + 2 * t + 1 < a.cout) yrow[2 * t + 1] = h2.y;
+                        }
                     }
                 }
             }
@@ -722,6 +744,9 @@ extern "C" int fvgb_conv_fwd_tc_rows(int32_t dtype, const void *x, int64_t n_x, 
     a.stages = 0;
     a.n_tiles = ceil_div(n_out, kTileM);
     a.direct_store = (ldy == c_out && c_out % 8 == 0) ? 1 : 0;
+    a.vec_store = (c_out % 16 == 0 && ldy % 16 == 0 && ((uintptr_t)y & 31) == 0) ? 2
+                  : (c_out % 8 == 0 && ldy % 8 == 0)                             ? 1
+                                                                                 : 0;
     cudaStream_t s = as_stream(stream);
     return dispatch_fwd(eb, BN, a.pack, a, s);
 }

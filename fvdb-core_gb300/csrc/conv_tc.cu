@@ -45,6 +45,137 @@ __global__ void quantize_e4m3_kernel(const T *__restrict__ x, int64_t n, int32_t
         out[r * ldo + ch] = (uint8_t)__nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3);
     }
 }
+
+// Rows of 8-channel vectors: a thread keeps one vector column (its scales stay in registers) and
+// walks rows, eight of them in flight.  Bound by HBM.  4.3M x 128 BF16: 1.34 ms one element per
+// thread (a 64-bit division each), 0.27 ms here.
+constexpr int kVecThreads = 256;
+constexpr int kVecRows = 8;
+
+template <typename T>
+struct __align__(16) Vec8 {
+    T v[8];
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kVecThreads) quantize_e4m3_vec_kernel(const T *__restrict__ x, int64_t n, int32_t Q,
+                                                                        int64_t ldx,
+                                                                        const float *__restrict__ inv_scale,
+                                                                        uint8_t *__restrict__ out, int64_t ldo) {
+    const int q = threadIdx.x % Q, rr = threadIdx.x / Q, rpi = kVecThreads / Q;
+    if (rr >= rpi) return;
+    float s[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s[e] = inv_scale[8 * q + e];
+    const int64_t r0 = (int64_t)blockIdx.x * rpi * kVecRows + rr;
+    Vec8<T> p[kVecRows];
+#pragma unroll
+    for (int i = 0; i < kVecRows; ++i) {
+        const int64_t r = r0 + (int64_t)i * rpi;
+        if (r < n) p[i] = *reinterpret_cast<const Vec8<T> *>(x + r * ldx + 8 * q);
+    }
+#pragma unroll
+    for (int i = 0; i < kVecRows; ++i) {
+        const int64_t r = r0 + (int64_t)i * rpi;
+        if (r >= n) continue;
+        uint32_t w[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            uint32_t lo = __nv_cvt_float2_to_fp8x2(
+                make_float2(to_f32<T>(p[i].v[4 * h]) * s[4 * h], to_f32<T>(p[i].v[4 * h + 1]) * s[4 * h + 1]),
+                __NV_SATFINITE, __NV_E4M3);
+            uint32_t hi = __nv_cvt_float2_to_fp8x2(
+                make_float2(to_f32<T>(p[i].v[4 * h + 2]) * s[4 * h + 2], to_f32<T>(p[i].v[4 * h + 3]) * s[4 * h + 3]),
+                __NV_SATFINITE, __NV_E4M3);
+            w[h] = lo | (hi << 16);
+        }
+        *reinterpret_cast<uint2 *>(out + r * ldo + 8 * q) = make_uint2(w[0], w[1]);
+    }
+}
+
+// Largest |x| per channel, as the bits of a non-negative float: those order like the floats, with
+// every NaN above infinity, so an integer maximum returns NaN where a channel holds one.  One read
+// of x; 4.3M x 128 BF16: 1.14 ms as |x| and a column maximum, 0.20 ms here.
+__device__ __forceinline__ uint32_t abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+
+constexpr int kMaxIters = 16;  // row groups of kVecRows a CTA walks before it merges its maxima
+
+template <typename T>
+__global__ void __launch_bounds__(kVecThreads) channel_absmax_vec_kernel(const T *__restrict__ x, int64_t n, int32_t Q,
+                                                                         int64_t ldx, uint32_t *__restrict__ out) {
+    __shared__ uint32_t sm[8][kVecThreads];
+    const int q = threadIdx.x % Q, rr = threadIdx.x / Q, rpi = kVecThreads / Q;
+    uint32_t m[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) m[e] = 0;
+    const int64_t span = (int64_t)rpi * kVecRows * kMaxIters;
+    const int64_t base = (int64_t)blockIdx.x * span, end = min(n, base + span);
+    if (rr < rpi)
+        for (int64_t r0 = base + rr; r0 < end; r0 += (int64_t)rpi * kVecRows) {
+            Vec8<T> p[kVecRows];
+#pragma unroll
+            for (int i = 0; i < kVecRows; ++i) {
+                const int64_t r = r0 + (int64_t)i * rpi;
+                // rows past the end repeat the first one
+                p[i] = *reinterpret_cast<const Vec8<T> *>(x + (r < end ? r : r0) * ldx + 8 * q);
+            }
+#pragma unroll
+            for (int i = 0; i < kVecRows; ++i)
+#pragma unroll
+                for (int e = 0; e < 8; ++e) m[e] = max(m[e], abs_bits(to_f32<T>(p[i].v[e])));
+        }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) sm[e][threadIdx.x] = m[e];
+    __syncthreads();
+    for (int i = threadIdx.x; i < 8 * Q; i += kVecThreads) {
+        const int e = i & 7, c = i >> 3;
+        uint32_t v = 0;
+        for (int r = 0; r < rpi; ++r) v = max(v, sm[e][r * Q + c]);
+        atomicMax(out + i, v);
+    }
+}
+
+template <typename T>
+__global__ void channel_absmax_kernel(const T *__restrict__ x, int64_t n, int32_t c, int64_t ldx,
+                                      uint32_t *__restrict__ out) {
+    const int32_t ch = blockIdx.y * blockDim.x + threadIdx.x;
+    if (ch >= c) return;
+    uint32_t m = 0;
+    for (int64_t r = blockIdx.x; r < n; r += gridDim.x) m = max(m, abs_bits(to_f32<T>(x[r * ldx + ch])));
+    atomicMax(out + ch, m);
+}
+
+// the vector kernels: whole 8-channel vectors, 16-byte aligned rows, at most a CTA's columns
+bool vec8_rows(const void *x, int32_t c, int64_t ldx, int elem) {
+    return c % 8 == 0 && c / 8 <= kVecThreads && ((uintptr_t)x & 15) == 0 && (ldx * elem) % 16 == 0;
+}
+
+template <typename T>
+void launch_quantize(const void *x, int64_t n, int32_t c, int64_t ldx, const float *inv, void *out, int64_t ldo,
+                     cudaStream_t s) {
+    if (vec8_rows(x, c, ldx, sizeof(T)) && ((uintptr_t)out & 7) == 0 && ldo % 8 == 0) {
+        const int32_t Q = c / 8;
+        const int64_t rows = (int64_t)(kVecThreads / Q) * kVecRows;
+        quantize_e4m3_vec_kernel<T><<<(unsigned)ceil_div(n, rows), kVecThreads, 0, s>>>((const T *)x, n, Q, ldx, inv,
+                                                                                      (uint8_t *)out, ldo);
+    } else {
+        const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(n * c, 256), device_sm_count() * 64);
+        quantize_e4m3_kernel<T><<<blocks, 256, 0, s>>>((const T *)x, n, c, ldx, inv, (uint8_t *)out, ldo);
+    }
+}
+
+template <typename T>
+void launch_absmax(const void *x, int64_t n, int32_t c, int64_t ldx, float *out, cudaStream_t s) {
+    uint32_t *o = reinterpret_cast<uint32_t *>(out);
+    if (vec8_rows(x, c, ldx, sizeof(T))) {
+        const int32_t Q = c / 8;
+        const int64_t rows = (int64_t)(kVecThreads / Q) * kVecRows * kMaxIters;
+        channel_absmax_vec_kernel<T><<<(unsigned)ceil_div(n, rows), kVecThreads, 0, s>>>((const T *)x, n, Q, ldx, o);
+    } else {
+        const dim3 grid((unsigned)std::min<int64_t>(n, device_sm_count() * 8), (unsigned)ceil_div(c, 128));
+        channel_absmax_kernel<T><<<grid, 128, 0, s>>>((const T *)x, n, c, ldx, o);
+    }
+}
 }  // namespace
 }  // namespace fvgb
 
@@ -52,15 +183,23 @@ extern "C" int fvgb_quantize_e4m3(int32_t dtype, const void *x, int64_t n, int32
                                   const float *inv_scale, void *out, int64_t ldo, fvgb_stream_t stream) {
     if (n < 0 || c < 1 || ldx < c || ldo < c || !inv_scale || (n > 0 && (!x || !out))) return FVGB_EINVAL;
     if (n == 0) return FVGB_OK;
-    const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(n * c, 256), device_sm_count() * 64);
     cudaStream_t s = as_stream(stream);
-    if (dtype == FVGB_F32)
-        quantize_e4m3_kernel<float><<<blocks, 256, 0, s>>>((const float *)x, n, c, ldx, inv_scale, (uint8_t *)out, ldo);
-    else if (dtype == FVGB_BF16)
-        quantize_e4m3_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>((const __nv_bfloat16 *)x, n, c, ldx, inv_scale,
-                                                                   (uint8_t *)out, ldo);
-    else
-        return FVGB_ETYPE;
+    if (dtype == FVGB_F32) launch_quantize<float>(x, n, c, ldx, inv_scale, out, ldo, s);
+    else if (dtype == FVGB_BF16) launch_quantize<__nv_bfloat16>(x, n, c, ldx, inv_scale, out, ldo, s);
+    else return FVGB_ETYPE;
+    count_launches(1);
+    return launch_status();
+}
+
+extern "C" int fvgb_channel_absmax(int32_t dtype, const void *x, int64_t n, int32_t c, int64_t ldx, float *out,
+                                   fvgb_stream_t stream) {
+    if (n < 0 || c < 1 || c > 65535 * 128 || ldx < c || !out || (n > 0 && !x)) return FVGB_EINVAL;
+    if (dtype != FVGB_F32 && dtype != FVGB_BF16) return FVGB_ETYPE;
+    cudaStream_t s = as_stream(stream);
+    if (cudaMemsetAsync(out, 0, sizeof(float) * c, s) != cudaSuccess) return launch_status();
+    if (n == 0) return launch_status();
+    if (dtype == FVGB_F32) launch_absmax<float>(x, n, c, ldx, out, s);
+    else launch_absmax<__nv_bfloat16>(x, n, c, ldx, out, s);
     count_launches(1);
     return launch_status();
 }

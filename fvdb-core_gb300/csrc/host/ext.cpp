@@ -1143,9 +1143,9 @@ std::vector<Tensor> conv_backward(const Tensor &dy_in, const Tensor &x, const Te
 // FP8-E4M3 forward (inference): per-input-channel feature scales s_x (folded into the weights)
 // and per-output-channel weight scales s_w (applied in the epilogue), FP32 accumulation:
 //   y[m, co] = s_w[co] * sum_k sum_ci e4m3(x[., ci] / s_x[ci]) * e4m3(s_x[ci] W[k, ci, co] / s_w[co])
-// Returns (y bf16, s_x, s_w).
+// plus the bias (optional, [cout]) in the epilogue, rounded once to BF16.  Returns (y bf16, s_x, s_w).
 std::vector<Tensor> conv_forward_fp8(const Tensor &x, const Tensor &weights, PackPtr p, bool transposed,
-                                     bool relu = false) {
+                                     bool relu = false, const std::optional<Tensor> &bias = std::nullopt) {
     resolve_pack(p);
     TORCH_CHECK_VALUE(x.dim() == 2 && x.is_cuda() && x.is_floating_point(), "features must be a 2-D CUDA float tensor");
     TORCH_CHECK_VALUE(weights.dim() == 5, "Expected kernels to have 5 dimensions");
@@ -1163,16 +1163,29 @@ std::vector<Tensor> conv_forward_fp8(const Tensor &x, const Tensor &weights, Pac
                       .to(torch::kFloat32);
     const int64_t K = Wkio.size(0);
     Tensor xc = x.scalar_type() == torch::kBFloat16 ? x.contiguous() : x.to(torch::kFloat32).contiguous();
-    Tensor s_x = (xc.size(0) > 0 ? xc.abs().amax(0).to(torch::kFloat32) : torch::ones({cin}, Wkio.options()))
-                     .clamp_min(1e-12) / 448.0f;
+    Tensor b32;
+    if (bias) {
+        TORCH_CHECK_VALUE(bias->dim() == 1 && bias->size(0) == cout, "bias must have shape (", cout, ",)");
+        TORCH_CHECK_VALUE(bias->device() == x.device(), "bias must be on the features' device");
+        b32 = bias->to(torch::kFloat32).contiguous();
+    }
+    const float *bp = bias ? b32.data_ptr<float>() : nullptr;
+    const int32_t xdt = xc.scalar_type() == torch::kBFloat16 ? FVGB_BF16 : FVGB_F32;
+    Tensor s_x = torch::empty({cin}, Wkio.options());
+    if (xc.size(0) > 0)
+        check_status(fvgb_channel_absmax(xdt, xc.data_ptr(), xc.size(0), (int32_t)cin, xc.stride(0),
+                                         s_x.data_ptr<float>(), cur_stream()),
+                     "fp8 feature scales");
+    else s_x.fill_(1.0f);
+    s_x = s_x.clamp_min(1e-12) / 448.0f;
     Tensor wf = Wkio * s_x.view({1, cin, 1});
     Tensor s_w = wf.abs().amax({0, 1}).clamp_min(1e-12) / 448.0f;
     Tensor w8 = (wf / s_w.view({1, 1, cout})).to(at::ScalarType::Float8_e4m3fn).contiguous();
     Tensor x8 = torch::empty({xc.size(0), cin}, x.options().dtype(torch::kUInt8));
     Tensor inv = (1.0f / s_x).contiguous();
     auto s = cur_stream();
-    check_status(fvgb_quantize_e4m3(xc.scalar_type() == torch::kBFloat16 ? FVGB_BF16 : FVGB_F32, xc.data_ptr(),
-                                    xc.size(0), (int32_t)cin, xc.stride(0), inv.data_ptr<float>(), x8.data_ptr(), cin, s),
+    check_status(fvgb_quantize_e4m3(xdt, xc.data_ptr(), xc.size(0), (int32_t)cin, xc.stride(0), inv.data_ptr<float>(),
+                                    x8.data_ptr(), cin, s),
                  "fp8 quantisation");
     Tensor y = torch::empty({n_rows, cout}, x.options().dtype(torch::kBFloat16));
     if (n_rows == 0) return {y, s_x, s_w};
@@ -1191,7 +1204,7 @@ std::vector<Tensor> conv_forward_fp8(const Tensor &x, const Tensor &weights, Pac
     if (plan) {
         check_status(fvgb_conv_fwd_tc_planned(FVGB_E4M3, x8.data_ptr(), x8.size(0), (int32_t)cin, cin, plan->data_ptr(),
                                               n_rows, (int32_t)K, packed.data_ptr(), (int32_t)cout, y.data_ptr(),
-                                              y.stride(0), sw.data_ptr<float>(), nullptr, relu ? 1 : 0,
+                                              y.stride(0), sw.data_ptr<float>(), bp, relu ? 1 : 0,
                                               device_error_flag(x.device()).data_ptr<int32_t>(), s),
                      "sparse conv forward (fp8 tensor cores)");
         return {y, s_x, s_w};
@@ -1202,7 +1215,7 @@ std::vector<Tensor> conv_forward_fp8(const Tensor &x, const Tensor &weights, Pac
                                        order ? order->rows.data_ptr<int32_t>() : nullptr,
                                        tmo ? reinterpret_cast<const uint32_t *>(tmo->data_ptr<int32_t>()) : nullptr,
                                        packed.data_ptr(), (int32_t)cout, y.data_ptr(), y.stride(0),
-                                       sw.data_ptr<float>(), nullptr, relu ? 1 : 0,
+                                       sw.data_ptr<float>(), bp, relu ? 1 : 0,
                                        device_error_flag(x.device()).data_ptr<int32_t>(), s),
                  "sparse conv forward (fp8 tensor cores)");
     return {y, s_x, s_w};
@@ -1529,7 +1542,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           py::arg("transposed"), py::arg("bias") = py::none(), py::arg("relu") = false,
           py::arg("out_scale") = py::none(), py::call_guard<py::gil_scoped_release>());
     m.def("conv_forward_fp8", &conv_forward_fp8, py::arg("features"), py::arg("weights"), py::arg("pack"),
-          py::arg("transposed"), py::arg("relu") = false, py::call_guard<py::gil_scoped_release>());
+          py::arg("transposed"), py::arg("relu") = false, py::arg("bias") = py::none(),
+          py::call_guard<py::gil_scoped_release>());
     m.def("check_device_errors", [](const torch::Device &d) { check_device_errors(d); },
           py::call_guard<py::gil_scoped_release>());
     m.def("conv_backward", &conv_backward, py::call_guard<py::gil_scoped_release>());

@@ -447,6 +447,11 @@ int fvgb_conv_wgrad_tc(const void *x, int64_t n_x, int32_t c_in, int64_t ldx, co
  */
 int fvgb_quantize_e4m3(int32_t dtype, const void *x, int64_t n, int32_t c, int64_t ldx, const float *inv_scale,
                        void *out, int64_t ldo, fvgb_stream_t stream);
+/* out[c] = largest |x[r, c]| over the rows (0 without rows, NaN where a row holds one), FP32;
+ * dtype FVGB_F32 / FVGB_BF16.  The per-channel scales of the FP8 path; no counterpart in the
+ * reference. */
+int fvgb_channel_absmax(int32_t dtype, const void *x, int64_t n, int32_t c, int64_t ldx, float *out,
+                        fvgb_stream_t stream);
 
 /* ------------------------------------------------------------------- self test --- */
 

@@ -80,3 +80,42 @@ def test_fp8_through_module_is_forward_only(cuda_device):
     assert y.data.jdata.dtype == torch.bfloat16 and y.data.jdata.shape == (grid.total_voxels, 64)
     with pytest.raises(RuntimeError):
         conv(fvdb.nn.VDBTensor(grid, grid.jagged_like(x.requires_grad_(True))))
+
+
+@pytest.mark.parametrize("cin,dtype", [(32, torch.bfloat16), (160, torch.float32), (2080, torch.bfloat16)])
+@pytest.mark.parametrize("rows", [1, 700])
+def test_fp8_feature_scales_are_column_maxima(cuda_device, cin, dtype, rows):
+    """s_x equals |x|.amax(0) / 448 exactly (vector kernel up to 2,048 channels, scalar beyond),
+    a NaN in a channel reaching its scale."""
+    import fvdb
+
+    grid = fvdb.GridBatch.from_ijk(torch.from_numpy(random_sparse_ijk(rows, 24, cin)).to(cuda_device))
+    pack, _ = grid.sparse_conv_kernel_map(3, 1)
+    g = torch.Generator().manual_seed(cin + rows)
+    x = torch.randn(grid.total_voxels, cin, generator=g).to(cuda_device, dtype)
+    x[rows // 2, 5] = float("nan")
+    w = (torch.randn(16, cin, 3, 3, 3, generator=g) * 0.05).to(cuda_device, torch.bfloat16)
+    _, s_x, _ = fvdb._lib.load().conv_forward_fp8(x, w, pack._impl, False)
+    ref = x.abs().amax(0).float().clamp_min(1e-12) / 448.0
+    assert torch.equal(torch.nan_to_num(s_x, nan=-1.0), torch.nan_to_num(ref, nan=-1.0)) and s_x[5].isnan()
+
+
+@pytest.mark.parametrize("cout", [256, 200, 8])
+@pytest.mark.parametrize("relu", [False, True])
+def test_fp8_bias_in_the_epilogue(cuda_device, cout, relu):
+    """A BF16 bias is added before the one rounding to BF16: within the two roundings (2 x 2^-8 of
+    the summed magnitudes) of the sum of the rounded output and the bias; whole 32-byte, 16-byte
+    and staged stores."""
+    import fvdb
+
+    grid = fvdb.GridBatch.from_ijk(torch.from_numpy(random_sparse_ijk(3000, 24, 3)).to(cuda_device))
+    conv = fvdb.nn.SparseConv3d(64, cout, 3).to(cuda_device, torch.bfloat16)
+    conv.precision = "fp8"
+    x = fvdb.nn.VDBTensor(grid, torch.randn(grid.total_voxels, 64, device=cuda_device).bfloat16())
+    with torch.no_grad():
+        got = conv(x, relu=relu).data.jdata.double()
+        bias, conv.bias = conv.bias, None
+        y = conv(x).data.jdata.double()
+    want = y + bias.double()
+    lim = 2 * 2.0**-8 * (y.abs() + bias.double().abs())
+    assert ((got - (want.clamp(min=0) if relu else want)).abs() <= lim).all()
