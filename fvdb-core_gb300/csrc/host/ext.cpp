@@ -672,9 +672,21 @@ std::optional<RowOrder> pack_row_order(PackPtr p, bool transposed) {
 // (training re-uses every map for forward and data gradient).  The CUDA-core forms use the order
 // from the first call on large maps: it saves them far more than it costs (C2 layer 1 FP32:
 // 3.1 -> 2.0 ms).
-std::optional<RowOrder> pack_row_order_if_reused(PackPtr p, bool transposed) {
+// Two kinds of map take the order at the first tensor-core contraction too:
+//   * the transposed map of a convolution whose stride covers its kernel: a row has at most one
+//     entry, an index-order tile multiplies all K offsets for it (2^3 stride 2, 256->128 BF16,
+//     1.08M rows: 1.13 ms in index order, 0.31 ms ordered plus 0.06 ms for the order);
+//   * wide layers (row bytes times output channels of 128 x 256 and more), where a skipped offset
+//     saves more than its share of the sort: 128->256 FP8, 4.3M rows: 4.0 ms in index order, 2.7 ms
+//     ordered plus 0.6 ms for the order; 64->64 BF16 saves less than the order costs.
+// Below 2^14 rows the order's seven launches cost more than any of this.
+std::optional<RowOrder> pack_row_order_if_reused(PackPtr p, bool transposed, int64_t row_bytes, int64_t cout) {
     const int d = transposed ? 1 : 0;
-    if (!p->order_rows[d] && ++p->order_requests[d] < 2) return std::nullopt;
+    const bool one_entry = transposed && p->st.v[0] >= p->ks.v[0] && p->st.v[1] >= p->ks.v[1] && p->st.v[2] >= p->ks.v[2];
+    const bool wide = row_bytes * cout >= 128 * 256;
+    const int64_t n = transposed ? p->src->N : p->tgt->N;
+    if (!p->order_rows[d] && !((one_entry || wide) && n >= ((int64_t)1 << 14)) && ++p->order_requests[d] < 2)
+        return std::nullopt;
     return pack_row_order(p, transposed);
 }
 
@@ -944,7 +956,7 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
         // a map used again runs over its row order (measured faster than a tile plan: C2 layer 1,
         // 32->64: 0.30 ms ordered, 0.32 ms planned, 0.365 ms in index order); the tile plan serves
         // maps that have no row order (K < 4 or K > 32)
-        const auto order = pack ? pack_row_order_if_reused(pack, map_t) : std::nullopt;
+        const auto order = pack ? pack_row_order_if_reused(pack, map_t, cin * 2, cout) : std::nullopt;
         std::optional<Tensor> plan;
         if (pack && K < 4 && use_plan(FVGB_BF16, K, cin, cout, 2))
             plan = pack_plan_if_reused(pack, map_t, (int32_t)(cin * 2));
@@ -980,7 +992,7 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
         // build); small ones only once reused, where the build's launches would dominate
         const auto order = !pack ? std::nullopt
                                  : (n_out >= (int64_t)1 << 16 ? pack_row_order(pack, map_t)
-                                                              : pack_row_order_if_reused(pack, map_t));
+                                                              : pack_row_order_if_reused(pack, map_t, 0, 0));
         const Tensor &m_used = order ? order->map : map;
         check_status(fvgb_conv_fwd_simt_rows(dt, x.data_ptr(), x.size(0), (int32_t)cin, x.stride(0),
                                              m_used.data_ptr<int32_t>(), n_out, (int32_t)K, m_used.stride(0),
@@ -1198,7 +1210,7 @@ std::vector<Tensor> conv_forward_fp8(const Tensor &x, const Tensor &weights, Pac
     const Tensor &map = transposed ? pack_kmap_t(p) : pack_kmap(p);
     auto tm = pack_tile_mask(p, transposed);
     Tensor sw = s_w.contiguous();
-    const auto order = pack_row_order_if_reused(p, transposed);
+    const auto order = pack_row_order_if_reused(p, transposed, cin, cout);
     std::optional<Tensor> plan;
     if (K < 4 && use_plan(FVGB_E4M3, K, cin, cout, 1)) plan = pack_plan_if_reused(p, transposed, (int32_t)cin);
     if (plan) {
