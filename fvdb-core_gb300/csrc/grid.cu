@@ -9,6 +9,7 @@
 #include <cuda_fp16.h>
 
 #include <cub/cub.cuh>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -219,16 +220,10 @@ __global__ void leaf_finish_kernel(FvgbLeaf *__restrict__ leaves, int64_t L, int
 // FP32/FP16/BF16): scale and translation are the double quotients rounded once to T, the
 // transform is one fused multiply-add in T, and round() is floor(v + 1/2) in T
 // (src/fvdb/detail/VoxelCoordTransform.h:86-110,230-330, BuildGridFromPoints.cu:27-43).
-template <typename T>
-__device__ __forceinline__ int32_t voxelise(T p, double w, double o);
-template <>
-__device__ __forceinline__ int32_t voxelise<float>(float p, double w, double o) {
-    const float s = (float)(1.0 / w), t = (float)(-o / w);
+__device__ __forceinline__ int32_t voxelise(float p, float s, float t) {
     return (int32_t)floorf(__fadd_rn(__fmaf_rn(p, s, t), 0.5f));
 }
-template <>
-__device__ __forceinline__ int32_t voxelise<double>(double p, double w, double o) {
-    const double s = 1.0 / w, t = -o / w;
+__device__ __forceinline__ int32_t voxelise(double p, double s, double t) {
     return (int32_t)floor(__dadd_rn(__fma_rn(p, s, t), 0.5));
 }
 
@@ -240,19 +235,48 @@ template <>
 __device__ __forceinline__ float point_as_float<__half>(__half v) { return __half2float(v); }
 
 // P: storage type of the points; T: arithmetic type (double for FP64 points, else float).
+template <typename T, typename P>
+__device__ __forceinline__ T point_value(P v) {
+    if constexpr (sizeof(T) == 8) return (T)v;
+    else return point_as_float<P>(v);
+}
+
+// The scale and translation of the block's first grid are divided out once per block (FP64
+// divisions: per point and axis they took 1.18 ms for 7.9M points, 30 times what the bytes take).
+// A block that spans several grids divides for each row of the others.
+constexpr int kPointRows = 8;  // points per thread
+
 template <typename P, typename T>
-__global__ void points_kernel(const P *__restrict__ pts, const int64_t *__restrict__ joff, int32_t B, int64_t n,
-                              const double *__restrict__ vs, const double *__restrict__ org,
-                              int32_t *__restrict__ out) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int32_t b = batch_of(joff, B, i);
+__global__ void __launch_bounds__(256) points_kernel(const P *__restrict__ pts, const int64_t *__restrict__ joff,
+                                                     int32_t B, int64_t n, const double *__restrict__ vs,
+                                                     const double *__restrict__ org, int32_t *__restrict__ out) {
+    __shared__ T fac[6];
+    __shared__ int32_t sb[2];
+    const int64_t base = (int64_t)blockIdx.x * 256 * kPointRows;
+    const int64_t last = min(n, base + 256 * kPointRows) - 1;
+    if (threadIdx.x < 2) sb[threadIdx.x] = batch_of(joff, B, threadIdx.x == 0 ? base : last);
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        const double w = vs[3 * sb[0] + threadIdx.x], o = org[3 * sb[0] + threadIdx.x];
+        fac[threadIdx.x] = (T)(1.0 / w);
+        fac[3 + threadIdx.x] = (T)(-o / w);
+    }
+    __syncthreads();
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        T v;
-        if constexpr (sizeof(T) == 8) v = (T)pts[3 * i + a];
-        else v = point_as_float<P>(pts[3 * i + a]);
-        out[3 * i + a] = voxelise<T>(v, vs[3 * b + a], org[3 * b + a]);
+    for (int q = 0; q < kPointRows; ++q) {
+        const int64_t i = base + q * 256 + threadIdx.x;
+        if (i > last) return;
+        const int32_t b = sb[0] == sb[1] ? sb[0] : batch_of(joff, B, i);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            T s = fac[a], t = fac[3 + a];
+            if (b != sb[0]) {
+                const double w = vs[3 * b + a], o = org[3 * b + a];
+                s = (T)(1.0 / w);
+                t = (T)(-o / w);
+            }
+            out[3 * i + a] = voxelise(point_value<T>(pts[3 * i + a]), s, t);
+        }
     }
 }
 
@@ -469,22 +493,23 @@ extern "C" int fvgb_points_to_ijk(int32_t dtype, const void *points, const int64
         return FVGB_EINVAL;
     if (n == 0) return FVGB_OK;
     cudaStream_t s = as_stream(stream);
+    const unsigned blocks = (unsigned)ceil_div(n, (int64_t)kThreads * kPointRows);
     switch (dtype) {
         case FVGB_F64:
-            points_kernel<double, double><<<blocks_for(n), kThreads, 0, s>>>(
-                (const double *)points, joffsets, num_grids, n, voxel_sizes, origins, out_ijk);
+            points_kernel<double, double><<<blocks, kThreads, 0, s>>>((const double *)points, joffsets, num_grids, n,
+                                                                      voxel_sizes, origins, out_ijk);
             break;
         case FVGB_F16:
-            points_kernel<__half, float><<<blocks_for(n), kThreads, 0, s>>>(
-                (const __half *)points, joffsets, num_grids, n, voxel_sizes, origins, out_ijk);
+            points_kernel<__half, float><<<blocks, kThreads, 0, s>>>((const __half *)points, joffsets, num_grids, n,
+                                                                     voxel_sizes, origins, out_ijk);
             break;
         case FVGB_BF16:
-            points_kernel<__nv_bfloat16, float><<<blocks_for(n), kThreads, 0, s>>>(
+            points_kernel<__nv_bfloat16, float><<<blocks, kThreads, 0, s>>>(
                 (const __nv_bfloat16 *)points, joffsets, num_grids, n, voxel_sizes, origins, out_ijk);
             break;
         default:
-            points_kernel<float, float><<<blocks_for(n), kThreads, 0, s>>>(
-                (const float *)points, joffsets, num_grids, n, voxel_sizes, origins, out_ijk);
+            points_kernel<float, float><<<blocks, kThreads, 0, s>>>((const float *)points, joffsets, num_grids, n,
+                                                                    voxel_sizes, origins, out_ijk);
     }
     count_launches(1);
     return launch_status();
@@ -794,5 +819,402 @@ extern "C" int fvgb_coarse_grid_build(const FvgbGrid *fine, const int32_t factor
     coarse_offsets_kernel<<<(unsigned)ceil_div(fine->num_grids + 1, kThreads), kThreads, 0, s>>>(
         w.corig, w.cid, w.base, nl, fine->num_grids, meta);
     count_launches(launched);  // CUB's own launches are not counted
+    return launch_status();
+}
+
+// ---------------------------------------------------------------------------------------------
+// Grid build through a leaf hash, for inputs with many rows per leaf: the rows of ijk (or points)
+// are never sorted.  One pass inserts every row's leaf into an open-addressing table, a second ORs
+// the row's voxel into its leaf's 512-bit mask; then only the leaves are sorted and the voxels are
+// written leaf by leaf in bit order, with the leaf table and the leaf hash in the same kernel.
+// Leaves sorted by (grid, order key) and voxels by bit is the order of the voxel sort, so the grid
+// is identical to fvgb_ijk_sort_unique's.  7.9M points, 1.08M voxels, 27k leaves in four grids:
+// voxelise, sort, unique and index took 1.9 ms, 0.33 ms here (bound by the random reads of
+// the table, which stays in L2).  The table has room for rows / 8 leaves; an input with more
+// (fewer than eight rows per leaf) raises `overflow` and is left to the sort.
+namespace fvgb {
+namespace {
+
+constexpr uint64_t kEmptyLeaf = ~0ull;
+constexpr int kHashRows = 8;      // rows per thread
+constexpr int kHashProbes = 128;  // a full neighbourhood of the table counts as overflow
+constexpr int kHashMaxGrids = 1023;  // the grid index takes the key's top 10 bits (all ones: the empty slot)
+
+struct LeafHash {
+    uint64_t *table;    // [cap] leaf keys, kEmptyLeaf where free
+    int32_t *slot_id;   // [cap] leaf of a taken slot
+    uint64_t *keys;     // [max_leaves] key of each leaf, in insertion order
+    uint64_t *mask;     // [max_leaves][8]
+    uint32_t *row_slot; // [n]
+    uint16_t *row_bit;  // [n]
+    int64_t cap, max_leaves;
+};
+
+size_t leaf_hash_layout(int64_t n, LeafHash *w, char *base) {
+    int64_t cap = 1024;
+    while (cap < n / 4) cap <<= 1;
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        char *p = base ? base + off : nullptr;
+        off = align_up(off + bytes, 256);
+        return p;
+    };
+    LeafHash h;
+    h.cap = cap;
+    h.max_leaves = cap / 2;
+    h.table = (uint64_t *)take((size_t)cap * 8);
+    h.slot_id = (int32_t *)take((size_t)cap * 4);
+    h.keys = (uint64_t *)take((size_t)h.max_leaves * 8);
+    h.mask = (uint64_t *)take((size_t)h.max_leaves * 64);
+    h.row_slot = (uint32_t *)take((size_t)n * 4);
+    h.row_bit = (uint16_t *)take((size_t)n * 2);
+    if (w) *w = h;
+    return off;
+}
+
+// stat: [0] leaves, [1] error word, [2] overflow, [3..5] largest -x, -y, -z, [6..8] largest x, y, z
+__device__ __forceinline__ uint32_t insert_leaf(const LeafHash &h, uint64_t key, int32_t *__restrict__ stat) {
+    uint64_t m = key * 0x9E3779B97F4A7C15ull;
+    m ^= m >> 32;
+    m *= 0xD6E8FEB86659FD93ull;
+    m ^= m >> 29;
+    const uint64_t cap_mask = (uint64_t)h.cap - 1;
+    uint64_t s = m & cap_mask;
+    for (int probe = 0; probe < kHashProbes; ++probe) {
+        uint64_t k = *reinterpret_cast<volatile uint64_t *>(h.table + s);
+        if (k == kEmptyLeaf) {
+            k = atomicCAS(reinterpret_cast<unsigned long long *>(h.table + s), kEmptyLeaf, key);
+            if (k == kEmptyLeaf) {  // this thread's leaf: number it and clear its mask for the next pass
+                const int32_t id = atomicAdd(stat, 1);
+                h.slot_id[s] = id;
+                if (id < h.max_leaves) {
+                    h.keys[id] = key;
+#pragma unroll
+                    for (int w = 0; w < 8; ++w) h.mask[(int64_t)id * 8 + w] = 0;
+                } else {
+                    stat[2] = 1;
+                }
+                return (uint32_t)s;
+            }
+        }
+        if (k == key) return (uint32_t)s;
+        s = (s + 1) & cap_mask;
+    }
+    stat[2] = 1;
+    return 0;
+}
+
+// Pass 1 over ijk rows (P = int32_t) or points (P = the points' type, voxelised in T).
+template <typename P, typename T>
+__global__ void __launch_bounds__(256) leaf_insert_kernel(const P *__restrict__ in, const int64_t *__restrict__ joff,
+                                                          int32_t B, int64_t n, const double *__restrict__ vs,
+                                                          const double *__restrict__ org, LeafHash h,
+                                                          int32_t *__restrict__ stat) {
+    constexpr bool kPoints = !std::is_same<P, int32_t>::value;
+    __shared__ T fac[6];
+    __shared__ int32_t sb[2], full;
+    const int64_t base = (int64_t)blockIdx.x * 256 * kHashRows;
+    const int64_t last = min(n, base + 256 * kHashRows) - 1;
+    if (threadIdx.x < 2) sb[threadIdx.x] = batch_of(joff, B, threadIdx.x == 0 ? base : last);
+    if (threadIdx.x == 2) full = *reinterpret_cast<volatile int32_t *>(stat + 2);
+    __syncthreads();
+    if (full) return;  // the input is left to the sort
+    if (kPoints) {
+        if (threadIdx.x < 3) {
+            const double w = vs[3 * sb[0] + threadIdx.x], o = org[3 * sb[0] + threadIdx.x];
+            fac[threadIdx.x] = (T)(1.0 / w);
+            fac[3 + threadIdx.x] = (T)(-o / w);
+        }
+        __syncthreads();
+    }
+    int32_t c[kHashRows][3];
+    bool range = true;
+    int32_t lim[6];
+#pragma unroll
+    for (int e = 0; e < 6; ++e) lim[e] = INT32_MIN;
+#pragma unroll
+    for (int q = 0; q < kHashRows; ++q) {
+        const int64_t i = min(base + q * 256 + threadIdx.x, last);  // past the end: the last row again
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            if constexpr (kPoints) {
+                T s = fac[a], t = fac[3 + a];
+                if (sb[0] != sb[1]) {
+                    const int32_t b = batch_of(joff, B, i);
+                    if (b != sb[0]) {
+                        const double w = vs[3 * b + a], o = org[3 * b + a];
+                        s = (T)(1.0 / w);
+                        t = (T)(-o / w);
+                    }
+                }
+                c[q][a] = voxelise(point_value<T>(in[3 * i + a]), s, t);
+            } else {
+                c[q][a] = in[3 * i + a];
+            }
+            range = range && coord_in_range(c[q][a]);
+            lim[a] = max(lim[a], -c[q][a]);
+            lim[3 + a] = max(lim[3 + a], c[q][a]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < kHashRows; ++q) {
+        const int64_t i = base + q * 256 + threadIdx.x;
+        if (i > last) break;
+        const int32_t b = sb[0] == sb[1] ? sb[0] : batch_of(joff, B, i);
+        const uint64_t k = order_key(c[q][0], c[q][1], c[q][2]);
+        h.row_slot[i] = insert_leaf(h, ((uint64_t)b << 54) | (k >> 9), stat);
+        h.row_bit[i] = (uint16_t)(k & 511);
+    }
+    if (!range) stat[1] = FVGB_ERANGE;
+#pragma unroll
+    for (int e = 0; e < 6; ++e) {
+        const int32_t v = __reduce_max_sync(0xffffffffu, lim[e]);
+        if ((threadIdx.x & 31) == 0 && v > *reinterpret_cast<volatile int32_t *>(stat + 3 + e)) atomicMax(stat + 3 + e, v);
+    }
+}
+
+// Pass 2: the voxel bits (a bit already set, most rows of a dense cloud, costs no atomic)
+__global__ void __launch_bounds__(256) leaf_bits_kernel(int64_t n, LeafHash h) {
+    const int64_t base = (int64_t)blockIdx.x * 256 * kHashRows + threadIdx.x;
+    int32_t id[kHashRows];
+    uint32_t bit[kHashRows];
+#pragma unroll
+    for (int q = 0; q < kHashRows; ++q) {
+        const int64_t i = base + q * 256;
+        id[q] = i < n ? h.slot_id[h.row_slot[i]] : -1;
+        bit[q] = i < n ? h.row_bit[i] : 0;
+    }
+#pragma unroll
+    for (int q = 0; q < kHashRows; ++q) {
+        if (id[q] < 0) continue;
+        uint64_t *w = h.mask + (int64_t)id[q] * 8 + (bit[q] >> 6);
+        const uint64_t m = 1ull << (bit[q] & 63);
+        if (!(*reinterpret_cast<volatile uint64_t *>(w) & m)) atomicOr(reinterpret_cast<unsigned long long *>(w), m);
+    }
+}
+
+// sort key of leaf i: (grid << vb) | the order-key bits that vary inside the bounding box
+template <typename Key>
+__global__ void leaf_sort_keys_kernel(LeafHash h, int64_t L, uint64_t low, int vb, Key *__restrict__ keys,
+                                      int32_t *__restrict__ vals) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= L) return;
+    const uint64_t k = h.keys[i];
+    keys[i] = (Key)(((k >> 54) << vb) | (k & low));
+    vals[i] = (int32_t)i;
+}
+
+__global__ void leaf_counts_kernel(LeafHash h, int64_t L, const int32_t *__restrict__ vals, int32_t *__restrict__ count) {
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p > L) return;
+    int32_t c = 0;
+    if (p < L) {
+        const uint64_t *m = h.mask + (int64_t)vals[p] * 8;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) c += __popcll(m[w]);
+    }
+    count[p] = c;  // zero past the last leaf, for the exclusive scan over L + 1
+}
+
+// warp per leaf in index order: its voxels in bit order, its table entry and its hash slot
+__global__ void __launch_bounds__(256) leaf_emit_kernel(LeafHash h, int64_t L, const int32_t *__restrict__ vals,
+                                                        const int32_t *__restrict__ first,
+                                                        int32_t *__restrict__ out_ijk, FvgbLeaf *__restrict__ leaves,
+                                                        int32_t *__restrict__ slots, int64_t cap) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t p = (int64_t)blockIdx.x * 8 + warp;
+    if (p >= L) return;
+    const int32_t id = vals[p];
+    const uint64_t key = h.keys[id];
+    int32_t ox, oy, oz;
+    key_to_coord((key & ((1ull << 54) - 1ull)) << 9, ox, oy, oz);
+    const int32_t b = (int32_t)(key >> 54);
+    const int w = lane >> 2, sub = (lane & 3) * 16;
+    const uint64_t word = h.mask[(int64_t)id * 8 + w];
+    // exclusive prefix of the words' populations, the same for the four lanes of a word
+    int pre = 0;
+#pragma unroll
+    for (int v = 0; v < 7; ++v) {
+        const int c = __popcll(__shfl_sync(0xffffffffu, word, v * 4));
+        if (v < w) pre += c;
+    }
+    const int32_t base = first[p];
+    FvgbLeaf &lf = leaves[p];
+    if ((lane & 3) == 0) {
+        lf.mask[w] = word;
+        lf.prefix[w] = (uint16_t)pre;
+    }
+    if (lane < 3) {
+        lf.origin[lane] = lane == 0 ? ox : (lane == 1 ? oy : oz);
+        lf.pad[lane] = 0;
+    }
+    if (lane == 0) {
+        lf.batch = b;
+        lf.base = base;
+        const uint64_t cap_mask = (uint64_t)cap - 1;
+        uint64_t s = leaf_hash(b, ox >> 3, oy >> 3, oz >> 3) & cap_mask;
+        for (int64_t probe = 0; probe < cap; ++probe) {
+            if (atomicCAS(slots + s, -1, (int32_t)p) == -1) break;
+            s = (s + 1) & cap_mask;
+        }
+    }
+    int64_t r = (int64_t)base + pre + __popcll(sub ? (word & ((1ull << sub) - 1ull)) : 0ull);
+    uint32_t bits = (uint32_t)(word >> sub) & 0xffffu;
+    while (bits) {
+        const int i = w * 64 + sub + __ffs(bits) - 1;
+        bits &= bits - 1;
+        out_ijk[3 * r] = ox + (i >> 6);
+        out_ijk[3 * r + 1] = oy + ((i >> 3) & 7);
+        out_ijk[3 * r + 2] = oz + (i & 7);
+        ++r;
+    }
+}
+
+// meta[b] = first voxel of grid b (b <= B)
+__global__ void leaf_offsets_kernel(const FvgbLeaf *__restrict__ leaves, const int32_t *__restrict__ first, int64_t L,
+                                    int32_t B, int64_t *__restrict__ meta) {
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b > B) return;
+    int64_t lo = 0, hi = L;
+    while (lo < hi) {
+        const int64_t mid = (lo + hi) >> 1;
+        if (leaves[mid].batch < b) lo = mid + 1; else hi = mid;
+    }
+    meta[b] = first[lo];
+}
+
+struct LeafSortWs {
+    uint64_t *keys_a, *keys_b;
+    int32_t *vals_a, *vals_b, *count, *first;
+    void *cub_tmp;
+    size_t cub_bytes;
+};
+
+size_t leaf_sort_layout(int64_t L, LeafSortWs *w, char *base) {
+    size_t cub_bytes = 0, c = 0;
+    cub::DeviceRadixSort::SortPairs(nullptr, cub_bytes, (uint64_t *)nullptr, (uint64_t *)nullptr, (int32_t *)nullptr,
+                                    (int32_t *)nullptr, (int)L, 0, 64);
+    cub::DeviceRadixSort::SortPairs(nullptr, c, (uint32_t *)nullptr, (uint32_t *)nullptr, (int32_t *)nullptr,
+                                    (int32_t *)nullptr, (int)L, 0, 32);
+    cub_bytes = c > cub_bytes ? c : cub_bytes;
+    cub::DeviceScan::ExclusiveSum(nullptr, c, (int32_t *)nullptr, (int32_t *)nullptr, (int)L + 1);
+    cub_bytes = c > cub_bytes ? c : cub_bytes;
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        char *p = base ? base + off : nullptr;
+        off = align_up(off + bytes, 256);
+        return p;
+    };
+    LeafSortWs s;
+    s.keys_a = (uint64_t *)take((size_t)L * 8);
+    s.keys_b = (uint64_t *)take((size_t)L * 8);
+    s.vals_a = (int32_t *)take((size_t)L * 4);
+    s.vals_b = (int32_t *)take((size_t)L * 4);
+    s.count = (int32_t *)take((size_t)(L + 1) * 4);
+    s.first = (int32_t *)take((size_t)(L + 1) * 4);
+    s.cub_bytes = cub_bytes;
+    s.cub_tmp = take(cub_bytes);
+    if (w) *w = s;
+    return off;
+}
+
+char *align_ws(void *p) { return reinterpret_cast<char *>(((uintptr_t)p + 255) & ~(uintptr_t)255); }
+
+template <typename P, typename T>
+void launch_insert(const void *in, const int64_t *joff, int32_t B, int64_t n, const double *vs, const double *org,
+                   const LeafHash &h, int32_t *stat, cudaStream_t s) {
+    const unsigned blocks = (unsigned)ceil_div(n, (int64_t)256 * kHashRows);
+    leaf_insert_kernel<P, T><<<blocks, 256, 0, s>>>((const P *)in, joff, B, n, vs, org, h, stat);
+}
+
+}  // namespace
+}  // namespace fvgb
+
+extern "C" int fvgb_leaf_hash_workspace(int64_t n, size_t *bytes) {
+    if (!bytes || n < 1 || n >= (int64_t)INT32_MAX) return FVGB_EINVAL;
+    *bytes = leaf_hash_layout(n, nullptr, nullptr) + 256;
+    return FVGB_OK;
+}
+
+extern "C" int fvgb_leaf_hash_insert(int32_t dtype, const void *rows, const int64_t *joffsets, int32_t num_grids,
+                                     int64_t n, const double *voxel_sizes, const double *origins, int32_t *stat,
+                                     void *workspace, size_t workspace_bytes, fvgb_stream_t stream) {
+    size_t need = 0;
+    const int st = fvgb_leaf_hash_workspace(n, &need);
+    if (st) return st;
+    if (num_grids < 1 || num_grids > kHashMaxGrids || !rows || !joffsets || !stat) return FVGB_EINVAL;
+    if (dtype >= 0 && (!voxel_sizes || !origins)) return FVGB_EINVAL;
+    if (dtype >= 0 && dtype != FVGB_F32 && dtype != FVGB_F64 && dtype != FVGB_F16 && dtype != FVGB_BF16)
+        return FVGB_ETYPE;
+    if (!workspace || workspace_bytes < need) return FVGB_ENOSPACE;
+    cudaStream_t s = as_stream(stream);
+    LeafHash h;
+    leaf_hash_layout(n, &h, align_ws(workspace));
+    if (cudaMemsetAsync(h.table, 0xff, (size_t)h.cap * 8, s) != cudaSuccess ||
+        cudaMemsetAsync(stat, 0, 3 * 4, s) != cudaSuccess || cudaMemsetAsync(stat + 3, 0x80, 6 * 4, s) != cudaSuccess)
+        return launch_status();
+    if (dtype < 0) launch_insert<int32_t, float>(rows, joffsets, num_grids, n, nullptr, nullptr, h, stat, s);
+    else if (dtype == FVGB_F64) launch_insert<double, double>(rows, joffsets, num_grids, n, voxel_sizes, origins, h, stat, s);
+    else if (dtype == FVGB_F16) launch_insert<__half, float>(rows, joffsets, num_grids, n, voxel_sizes, origins, h, stat, s);
+    else if (dtype == FVGB_BF16)
+        launch_insert<__nv_bfloat16, float>(rows, joffsets, num_grids, n, voxel_sizes, origins, h, stat, s);
+    else launch_insert<float, float>(rows, joffsets, num_grids, n, voxel_sizes, origins, h, stat, s);
+    count_launches(1);
+    return launch_status();
+}
+
+extern "C" int fvgb_leaf_hash_finish_workspace(int64_t num_leaves, size_t *bytes) {
+    if (!bytes || num_leaves < 1 || num_leaves >= INT32_MAX) return FVGB_EINVAL;
+    *bytes = leaf_sort_layout(num_leaves, nullptr, nullptr) + 256;
+    return FVGB_OK;
+}
+
+extern "C" int fvgb_leaf_hash_finish(int64_t n, int32_t num_grids, int64_t num_leaves, const int32_t box_lo[3],
+                                     const int32_t box_hi[3], void *insert_workspace, size_t insert_bytes,
+                                     int32_t *out_ijk, int64_t *out_joffsets, FvgbLeaf *leaves, int32_t *hash_slots,
+                                     int64_t hash_capacity, void *workspace, size_t workspace_bytes,
+                                     fvgb_stream_t stream) {
+    size_t need = 0, need_insert = 0;
+    int st = fvgb_leaf_hash_finish_workspace(num_leaves, &need);
+    if (!st) st = fvgb_leaf_hash_workspace(n, &need_insert);
+    if (st) return st;
+    if (num_grids < 1 || num_grids > kHashMaxGrids || !out_ijk || !out_joffsets || !leaves || !hash_slots || !box_lo ||
+        !box_hi || hash_capacity < 2 * num_leaves || (hash_capacity & (hash_capacity - 1)))
+        return FVGB_EINVAL;
+    for (int a = 0; a < 3; ++a)
+        if (box_lo[a] > box_hi[a]) return FVGB_EINVAL;
+    if (!insert_workspace || insert_bytes < need_insert || !workspace || workspace_bytes < need) return FVGB_ENOSPACE;
+    cudaStream_t s = as_stream(stream);
+    LeafHash h;
+    leaf_hash_layout(n, &h, align_ws(insert_workspace));
+    if (num_leaves > h.max_leaves) return FVGB_EINVAL;
+    LeafSortWs w;
+    leaf_sort_layout(num_leaves, &w, align_ws(workspace));
+    const int64_t L = num_leaves;
+    if (cudaMemsetAsync(hash_slots, 0xff, sizeof(int32_t) * hash_capacity, s) != cudaSuccess) return launch_status();
+    leaf_bits_kernel<<<(unsigned)ceil_div(n, (int64_t)256 * kHashRows), 256, 0, s>>>(n, h);
+    const int end_bit = order_key_end_bit(box_lo, box_hi);
+    const int vb = end_bit > 9 ? end_bit - 9 : 0;
+    const uint64_t low = (1ull << vb) - 1ull;
+    int grid_bits = 0;
+    while ((1 << grid_bits) < num_grids) ++grid_bits;
+    const int bits = std::max(1, vb + grid_bits);
+    size_t tb = w.cub_bytes;
+    if (bits <= 32) {
+        uint32_t *ka = reinterpret_cast<uint32_t *>(w.keys_a), *kb = reinterpret_cast<uint32_t *>(w.keys_b);
+        leaf_sort_keys_kernel<uint32_t><<<blocks_for(L), kThreads, 0, s>>>(h, L, low, vb, ka, w.vals_a);
+        cub::DeviceRadixSort::SortPairs(w.cub_tmp, tb, ka, kb, w.vals_a, w.vals_b, (int)L, 0, bits, s);
+    } else {
+        leaf_sort_keys_kernel<uint64_t><<<blocks_for(L), kThreads, 0, s>>>(h, L, low, vb, w.keys_a, w.vals_a);
+        cub::DeviceRadixSort::SortPairs(w.cub_tmp, tb, w.keys_a, w.keys_b, w.vals_a, w.vals_b, (int)L, 0, bits, s);
+    }
+    leaf_counts_kernel<<<blocks_for(L + 1), kThreads, 0, s>>>(h, L, w.vals_b, w.count);
+    tb = w.cub_bytes;
+    cub::DeviceScan::ExclusiveSum(w.cub_tmp, tb, w.count, w.first, (int)L + 1, s);
+    leaf_emit_kernel<<<(unsigned)ceil_div(L, 8), 256, 0, s>>>(h, L, w.vals_b, w.first, out_ijk, leaves, hash_slots,
+                                                              hash_capacity);
+    leaf_offsets_kernel<<<(unsigned)ceil_div(num_grids + 1, kThreads), kThreads, 0, s>>>(leaves, w.first, L, num_grids,
+                                                                                         out_joffsets);
+    count_launches(5);
     return launch_status();
 }

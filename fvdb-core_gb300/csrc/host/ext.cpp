@@ -166,11 +166,77 @@ Tensor per_grid_vec(const Tensor &t, int64_t B, const char *name) {
     return v.contiguous().clone();
 }
 
+// The grid of n rows (ijk for dtype -1, else points with device voxel_sizes / origins) through the
+// leaf hash, or null where the input has too few rows per leaf for it (the caller sorts).  From
+// kLeafHashRows rows on: below it the build is a dozen launches of a few microseconds either way and
+// the sort's single count read is the cheaper one.
+constexpr int64_t kLeafHashRows = (int64_t)1 << 18;
+constexpr int64_t kLeafHashGrids = 1023;
+
+void fill_transforms(GridImpl &g, const Tensor &vs, const Tensor &org) {
+    g.voxel_sizes = per_grid_vec(vs, g.B, "voxel_sizes");
+    g.origins = per_grid_vec(org, g.B, "origins");
+}
+
+GridPtr build_by_leaf_hash(int32_t dtype, const void *rows, const Tensor &joff, int64_t n, const double *vsd,
+                           const double *ord) {
+    auto dev = joff.device();
+    const int64_t B = joff.size(0) - 1;
+    auto s = cur_stream();
+    cudaStream_t cs = reinterpret_cast<cudaStream_t>(s);
+    auto i32 = torch::dtype(torch::kInt32).device(dev);
+    size_t wsb = 0;
+    check_status(fvgb_leaf_hash_workspace(n, &wsb), "grid build (workspace)");
+    Tensor ws = workspace(wsb, dev);
+    Tensor stat = torch::empty({10}, i32);
+    check_status(fvgb_leaf_hash_insert(dtype, rows, joff.data_ptr<int64_t>(), (int32_t)B, n, vsd, ord,
+                                       stat.data_ptr<int32_t>(), ws.data_ptr(), ws.numel(), s),
+                 "grid build (leaves)");
+    int64_t *h = pinned_meta(dev.index(), std::max<size_t>(8, (size_t)B + 1));
+    TORCH_CHECK(cudaMemcpyAsync(h, stat.data_ptr<int32_t>(), 9 * sizeof(int32_t), cudaMemcpyDeviceToHost, cs) ==
+                        cudaSuccess &&
+                    cudaStreamSynchronize(cs) == cudaSuccess,
+                "grid build: reading the leaf count failed");
+    const int32_t *st = reinterpret_cast<const int32_t *>(h);
+    if (st[2]) return nullptr;
+    TORCH_CHECK_VALUE(st[1] == 0, "voxel coordinates must lie in [-2^20, 2^20) and inside their bounds");
+    auto g = std::make_shared<GridImpl>();
+    g->B = B;
+    g->L = st[0];
+    for (int a = 0; a < 3; ++a) {
+        g->box_lo[a] = -st[3 + a];
+        g->box_hi[a] = st[6 + a];
+    }
+    g->cap = next_pow2(2 * g->L);
+    Tensor out_ijk = torch::empty({std::min<int64_t>(n, 512 * g->L), 3}, i32);
+    g->joffsets = torch::empty({B + 1}, torch::dtype(torch::kInt64).device(dev));
+    g->leaves = torch::empty({g->L * (int64_t)sizeof(FvgbLeaf)}, torch::dtype(torch::kUInt8).device(dev));
+    g->hash = torch::empty({g->cap}, i32);
+    size_t fb = 0;
+    check_status(fvgb_leaf_hash_finish_workspace(g->L, &fb), "grid build (workspace)");
+    Tensor fws = workspace(fb, dev);
+    check_status(fvgb_leaf_hash_finish(n, (int32_t)B, g->L, g->box_lo, g->box_hi, ws.data_ptr(), ws.numel(),
+                                       out_ijk.data_ptr<int32_t>(), g->joffsets.data_ptr<int64_t>(),
+                                       reinterpret_cast<FvgbLeaf *>(g->leaves.data_ptr<uint8_t>()),
+                                       g->hash.data_ptr<int32_t>(), g->cap, fws.data_ptr(), fws.numel(), s),
+                 "grid build (index)");
+    TORCH_CHECK(cudaMemcpyAsync(h, g->joffsets.data_ptr<int64_t>(), (B + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost,
+                                cs) == cudaSuccess &&
+                    cudaStreamSynchronize(cs) == cudaSuccess,
+                "grid build: reading the counts failed");
+    g->joffsets_host = torch::from_blob(h, {B + 1}, torch::kInt64).clone();
+    g->N = h[B];
+    g->ijk = out_ijk.narrow(0, 0, g->N);
+    g->ready = std::make_shared<at::cuda::CUDAEvent>();
+    g->ready->record(at::cuda::getCurrentCUDAStream(dev.index()));
+    return g;
+}
+
 // Sorted-unique voxels in index order + leaf table + hash (one host sync for the counts and the
 // bounding box).  box_lo/box_hi (optional): bounds the caller knows for ijk, which shorten the
 // sort to the order-key bits that can differ.
 GridPtr build_grid(const Tensor &ijk_in, const Tensor &joff_in, const Tensor &vs, const Tensor &org,
-                   const int32_t *box_lo = nullptr, const int32_t *box_hi = nullptr) {
+                   const int32_t *box_lo = nullptr, const int32_t *box_hi = nullptr, bool leaf_hash = true) {
     TORCH_CHECK(ijk_in.is_cuda(), "fvdb_gb300 grids live on CUDA devices");
     c10::cuda::CUDAGuard guard(ijk_in.device());
     auto dev = ijk_in.device();
@@ -181,10 +247,14 @@ GridPtr build_grid(const Tensor &ijk_in, const Tensor &joff_in, const Tensor &vs
     const int64_t B = joff.size(0) - 1;
     TORCH_CHECK_VALUE(B >= 1, "a grid batch needs at least one grid");
     const int64_t n = ijk.size(0);
+    if (!(box_lo && box_hi) && leaf_hash && n >= kLeafHashRows && B <= kLeafHashGrids)
+        if (GridPtr h = build_by_leaf_hash(-1, ijk.data_ptr<int32_t>(), joff, n, nullptr, nullptr)) {
+            fill_transforms(*h, vs, org);
+            return h;
+        }
     auto g = std::make_shared<GridImpl>();
     g->B = B;
-    g->voxel_sizes = per_grid_vec(vs, B, "voxel_sizes");
-    g->origins = per_grid_vec(org, B, "origins");
+    fill_transforms(*g, vs, org);
     auto i32 = torch::dtype(torch::kInt32).device(dev);
     // Large inputs without known bounds: read their bounding box first (one small reduction and
     // one read) so the radix sort covers only the order-key bits that vary (3 of 8 passes for
@@ -288,12 +358,19 @@ GridPtr grid_from_points(const Tensor &points, const Tensor &joffsets, const Ten
     Tensor joff = joffsets.to(points.device(), torch::kInt64).contiguous();
     Tensor vsb = per_grid_vec(vs, B, "voxel_sizes"), orb = per_grid_vec(org, B, "origins");
     Tensor vsd = vsb.to(points.device()), ord = orb.to(points.device());
+    const bool hashed = p.size(0) >= kLeafHashRows && B <= kLeafHashGrids;
+    if (hashed)
+        if (GridPtr g = build_by_leaf_hash(fvgb_dtype(p), p.data_ptr(), joff, p.size(0), vsd.data_ptr<double>(),
+                                           ord.data_ptr<double>())) {
+            fill_transforms(*g, vsb, orb);
+            return g;
+        }
     Tensor ijk = torch::empty({p.size(0), 3}, torch::dtype(torch::kInt32).device(points.device()));
     check_status(fvgb_points_to_ijk(fvgb_dtype(p), p.data_ptr(), joff.data_ptr<int64_t>(), (int32_t)B, p.size(0),
                                     vsd.data_ptr<double>(), ord.data_ptr<double>(), ijk.data_ptr<int32_t>(),
                                     cur_stream()),
                  "points to ijk");
-    return build_grid(ijk, joff, vsb, orb);
+    return build_grid(ijk, joff, vsb, orb, nullptr, nullptr, !hashed);
 }
 
 // Coarse grid floor(ijk / f) of a grid, built leaf by leaf (fvgb_coarse_grid_build: one sort

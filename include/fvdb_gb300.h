@@ -117,6 +117,28 @@ int fvgb_ijk_sort_unique_in_box(const int32_t *ijk, const int64_t *joffsets, int
                                 int64_t *out_joffsets, int32_t *err_dev, void *workspace,
                                 size_t workspace_bytes, fvgb_stream_t stream);
 
+/* Grid build through a leaf hash, for inputs with at least eight rows per leaf (large point clouds
+ * and voxel lists): the same grid as fvgb_ijk_sort_unique + fvgb_grid_leaf_scan +
+ * fvgb_grid_index_build without sorting the rows.  num_grids <= 1023.
+ *   insert: rows are ijk (dtype -1, int32) or points (FVGB_F32 / F64 / F16 / BF16, voxelised with
+ *   voxel_sizes / origins as fvgb_points_to_ijk does).  stat (device int32 [9]): leaves, error word
+ *   (FVGB_ERANGE), overflow (more than one leaf per eight rows: the caller sorts instead), then the
+ *   largest -x, -y, -z, x, y, z.  The caller reads it and allocates.
+ *   finish: with the insert's workspace, the leaf count and the bounding box it reported: out_ijk
+ *   (min(n, 512 num_leaves) rows), out_joffsets [num_grids + 1], the leaf table and the leaf hash
+ *   (hash_capacity a power of two >= 2 num_leaves).
+ * Replaces dispatchCreateNanoGridFromPoints / FromIJK (BuildGridFromPoints.cu:27-130,
+ * BuildGridFromIjk.cu:26-83). */
+int fvgb_leaf_hash_workspace(int64_t n, size_t *bytes);
+int fvgb_leaf_hash_insert(int32_t dtype, const void *rows, const int64_t *joffsets, int32_t num_grids, int64_t n,
+                          const double *voxel_sizes, const double *origins, int32_t *stat, void *workspace,
+                          size_t workspace_bytes, fvgb_stream_t stream);
+int fvgb_leaf_hash_finish_workspace(int64_t num_leaves, size_t *bytes);
+int fvgb_leaf_hash_finish(int64_t n, int32_t num_grids, int64_t num_leaves, const int32_t box_lo[3],
+                          const int32_t box_hi[3], void *insert_workspace, size_t insert_bytes, int32_t *out_ijk,
+                          int64_t *out_joffsets, FvgbLeaf *leaves, int32_t *hash_slots, int64_t hash_capacity,
+                          void *workspace, size_t workspace_bytes, fvgb_stream_t stream);
+
 /*
  * Leaf ids of sorted unique ijk: leaf_ids[i] = 1 + id of the leaf of voxel i (inclusive scan
  * of leaf starts).  n is a capacity (>= joffsets[num_grids], the voxel count, read on the
