@@ -1,13 +1,14 @@
 // Tensor-core (tcgen05 / TMEM) implicit-GEMM sparse convolution, forward and data gradient.
 //
-//   y[m, :] = scale (.) sum_k x[map[m,k], :] . W[k]       (BF16 or FP8-E4M3 in, FP32 accumulate)
+//   y[m, :] = scale (.) sum_k x[map[m,k], :] . W[k]   (BF16, FP16 or FP8-E4M3 in, FP32 accumulate)
 //
 // Persistent kernel, one CTA per SM, looping over 128-row output tiles (tile t = blockIdx.x +
 // i * gridDim.x).  Each tile owns all (<= 256) output channels, so every output row is written
 // exactly once, without atomics.  The reduction dimension is cut into units of 128 bytes: one
-// 128-byte channel chunk of one kernel offset, or, when a feature row is 64 or 32 bytes, a fixed
-// group of 2 or 4 consecutive offsets whose rows share one 128-byte A row (one weight image per
-// group, so no half-empty weight tiles).  Units absent from all 128 rows of a tile (per-tile
+// 128-byte channel chunk of one kernel offset, or, when a feature row is at most 64 or 32 bytes, a
+// fixed group of 2 or 4 consecutive offsets whose rows share one 128-byte A row (one weight image per
+// group, so no half-empty weight tiles).  Rows are whole 16-byte pieces; what a row lacks of its
+// 64- or 32-byte slot, or of the 32 bytes of one MMA, is stored as zero.  Units absent from all 128 rows of a tile (per-tile
 // occupancy mask) are skipped.  A pipeline stage carries U units (2 for N <= 64), so every
 // barrier round trip feeds 8 MMAs: the per-stage handshakes, not bytes, set the pace of this
 // kernel, and tcgen05.mma with N <= 128 costs the same ~60-80 cycles whatever N is.
@@ -40,6 +41,7 @@
 // (src/fvdb/detail/ops/convolution/backend/SparseConvolutionImplicitGEMM.cu:120-3826,
 // SparseConvolutionImplicitGEMMSorted.cu:115-4639), sm_80 mma.sync code.
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include <mutex>
 
@@ -78,7 +80,8 @@ struct FwdArgs {
     int32_t nchunks;            // 128-byte chunks per row (pack == 1)
     int32_t pack;               // kernel offsets per 128-byte A row (1, 2 or 4); pack > 1 => nchunks == 1
     int32_t groups;             // offset groups (pack > 1): ceil(K / pack)
-    int32_t row_bytes;          // c_in * elem
+    int32_t row_bytes;          // c_in * elem, a multiple of 16
+    int32_t f16;                // 1: FP16 operands and output instead of BF16 (EBYTES == 2)
     int32_t cout;
     uint8_t *y;                 // bf16 [n_out, ldy]
     int64_t ldy;
@@ -225,6 +228,10 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
         const int row0 = warp * kRowsPerWarp;
         const int slot = j / kCpr;         // offset slot of chunk j within a group
         const int jj = j - slot * kCpr;    // chunk within that offset's row
+        // offsets this lane copies: none where its piece lies past a short row (PACK > 1); for whole
+        // chunks, the channel bytes left of its piece's end of the row and of the last MMA's end
+        const int k_lane = PACK > 1 && jj * 16 >= a.row_bytes ? 0 : a.K;
+        const int row_end = a.row_bytes - j * 16, mma_end = ((a.row_bytes + 31) & ~31) - j * 16;
         uint32_t it = 0, sig = 0, stage = 0, phase = 0, pstage = 0;
         int64_t tile = blockIdx.x;
         for (int i = 0; tile < a.n_tiles && !*abort; tile += stride, ++i) {
@@ -244,16 +251,17 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
                     int image = -1, k0 = 0, c = 0;
                     if (u0 + u < un.n) w.next(a, image, k0, c);
                     const int k = k0 + (PACK > 1 ? slot : 0);
-                    const int bytes = PACK > 1 ? kSlotBytes : min(kRowBytes, a.row_bytes - c * kRowBytes);
-                    // chunks past a short last chunk are never read by the MMA; group members past
-                    // K are zero-stored (their weights are zero, but stale A bytes could be NaN)
-                    on[u] = image >= 0 && (PACK > 1 || j * 16 < bytes);
+                    // pieces past the last MMA of a short last chunk are never read; group members past
+                    // K and the pieces a row lacks up to its slot or MMA are zero-stored (their
+                    // weights are zero, but stale A bytes could be NaN)
+                    on[u] = image >= 0 && (PACK > 1 || c * kRowBytes < mma_end);
+                    const int kmax = PACK > 1 || c * kRowBytes < row_end ? k_lane : 0;
                     colb[u] = PACK > 1 ? (int64_t)jj * 16 : (int64_t)c * kRowBytes + j * 16;
 #pragma unroll
                     for (int q = 0; q < kCopies; ++q) {
                         const int r = row0 + rsub + 4 * q;
                         int32_t v = -1;
-                        if (on[u] && k < a.K) {
+                        if (on[u] && k < kmax) {
                             if (stage_map) {
                                 v = mtile[r * a.K + k];
                             } else {
@@ -320,11 +328,11 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
         // advanced by constant offsets (16-byte units) from one base: shared addresses stay
         // below 2^18, so the 14-bit start-address field never carries.
         {
-            constexpr uint32_t idesc = EBYTES == 2 ? idesc_m128(BN, 1, 1) : idesc_m128(BN, 0, 0);
+            const uint32_t idesc = EBYTES == 2 && !a.f16 ? idesc_m128(BN, 1, 1) : idesc_m128(BN, 0, 0);
             constexpr uint32_t kStageD = kStage >> 4, kAD = kABytes >> 4, kBOffD = (U * kABytes) >> 4,
                                kBTileD = kBTile >> 4;
             const uint64_t adesc0 = desc_sw128(smem_u32(smem));
-            const int last_k32 = (a.row_bytes - (a.nchunks - 1) * kRowBytes) >> 5;  // pack == 1: last chunk
+            const int last_k32 = (a.row_bytes - (a.nchunks - 1) * kRowBytes + 31) >> 5;  // pack == 1: last chunk
             uint32_t stage = 0, phase = 0;
             bool ok = true;
             int64_t tile = blockIdx.x;
@@ -431,8 +439,13 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
                         lo = lo < 0.f ? 0.f : lo;
                         hi = hi < 0.f ? 0.f : hi;
                     }
-                    __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-                    packed[t] = *reinterpret_cast<uint32_t *>(&h);
+                    if (EBYTES == 2 && a.f16) {
+                        const __half2 h = __floats2half2_rn(lo, hi);
+                        packed[t] = *reinterpret_cast<const uint32_t *>(&h);
+                    } else {
+                        const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+                        packed[t] = *reinterpret_cast<const uint32_t *>(&h);
+                    }
                 }
                 if (a.direct_store) {
                     // cout % 8 == 0: whole 16-byte groups; the last group of a 16-wide block may be cut
@@ -444,7 +457,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
                     // 2-byte stores a 256-channel tile took 32,768 partial-sector writes and the
                     // epilogue, not the contraction, set the kernel's pace (4.3M rows, 128->256 FP8:
                     // 12.7 ms with 2-byte stores, 4.0 ms with these)
-                    __nv_bfloat16 *yrow = reinterpret_cast<__nv_bfloat16 *>(a.y) + yrow_i * a.ldy + c0;
+                    uint16_t *yrow = reinterpret_cast<uint16_t *>(a.y) + yrow_i * a.ldy + c0;
                     if (a.vec_store == 2) {
                         st_global_32(yrow, packed);
                     } else if (a.vec_store == 1) {
@@ -454,9 +467,8 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
                     } else {
 #pragma unroll
                         for (int t = 0; t < 8; ++t) {
-                            const __nv_bfloat162 h2 = *reinterpret_cast<const __nv_bfloat162 *>(&packed[t]);
-                            if (c0 + 2 * t < a.cout) yrow[2 * t] = h2.x;
-                            if (c0 + 2 * t + 1 < a.cout) yrow[2 * t + 1] = h2.y;
+                            if (c0 + 2 * t < a.cout) yrow[2 * t] = (uint16_t)packed[t];
+                            if (c0 + 2 * t + 1 < a.cout) yrow[2 * t + 1] = (uint16_t)(packed[t] >> 16);
                         }
                     }
                 }
@@ -538,7 +550,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
 // Packed weight image: per unit one [BN rows (output channel n) x 128 bytes] block laid out
 // exactly as the 128B-swizzled K-major shared-memory operand.  pack == 1: unit (k, chunk c)
 // holds W[k][c*CE + e][n] for e in [0, CE) (CE = 128/ebytes); pack > 1: unit g holds
-// W[g*pack + p][e][n] at element p*cin + e of the row.  Zero where the channel, the offset or
+// W[g*pack + p][e][n] at element p*CE/pack + e of the row.  Zero where the channel, the offset or
 // n is out of range.
 __global__ void pack_weights_kernel(const uint8_t *__restrict__ w, int64_t K, int32_t cin, int32_t cout,
                                     int64_t wsk, int64_t wsci, int64_t wsco, int32_t ebytes, int32_t BN,
@@ -552,9 +564,9 @@ __global__ void pack_weights_kernel(const uint8_t *__restrict__ w, int64_t K, in
         int64_t k;
         int ci;
         if (pack > 1) {
-            const int p = kk / cin;
+            const int slot = ce / pack, p = kk / slot;
             k = tilei * pack + p;
-            ci = kk - p * cin;
+            ci = kk - p * slot;
         } else {
             k = tilei / nchunks;
             ci = (int)(tilei % nchunks) * ce + kk;
@@ -582,7 +594,7 @@ int tile_n(int32_t cout) {
 
 // Units of the packed weight image for (K, c_in*elem bytes).
 int64_t weight_units(int64_t K, int64_t row_bytes, int *pack, int *nchunks) {
-    *pack = row_bytes < 128 ? (int)(128 / row_bytes) : 1;
+    *pack = row_bytes <= 32 ? 4 : (row_bytes <= 64 ? 2 : 1);
     *nchunks = (int)ceil_div(row_bytes, 128);
     return *pack > 1 ? ceil_div(K, (int64_t)*pack) : K * *nchunks;
 }
@@ -696,18 +708,18 @@ extern "C" int fvgb_conv_fwd_tc_epilogue(int32_t dtype, const void *x, int64_t n
                                  out_scale, bias, relu, err_dev, stream);
 }
 
-extern "C" int fvgb_conv_fwd_tc_rows(int32_t dtype, const void *x, int64_t n_x, int32_t c_in, int64_t ldx,
-                                     const int32_t *map, int64_t n_out, int32_t K, const int32_t *rows,
-                                     const uint32_t *tile_mask, const void *packed_w, int32_t c_out, void *y,
-                                     int64_t ldy, const float *out_scale, const float *bias, int32_t relu,
-                                     int32_t *err_dev, fvgb_stream_t stream) {
-    const int eb = dtype == FVGB_E4M3 ? 1 : (dtype == FVGB_BF16 ? 2 : 0);
-    if (!eb) return FVGB_ETYPE;
+namespace fvgb {
+namespace {
+// eb: bytes per element; f16: FP16 instead of BF16 (eb == 2)
+int conv_fwd(int eb, bool f16, const void *x, int64_t n_x, int32_t c_in, int64_t ldx, const int32_t *map,
+             int64_t n_out, int32_t K, const int32_t *rows, const uint32_t *tile_mask, const void *packed_w,
+             int32_t c_out, void *y, int64_t ldy, const float *out_scale, const float *bias, int32_t relu,
+             int32_t *err_dev, fvgb_stream_t stream) {
     if (c_in < 1 || c_out < 1 || K < 1 || n_out < 0 || n_x < 0 || ldx < c_in || ldy < c_out || !err_dev)
         return FVGB_EINVAL;
     const int64_t row_bytes = (int64_t)c_in * eb;
-    // each MMA consumes 32 bytes of K; rows shorter than 128 bytes must tile a 128-byte row
-    if (row_bytes % 32 != 0 || (row_bytes < 128 && 128 % row_bytes != 0) || (ldx * eb) % 16 != 0) return FVGB_EINVAL;
+    // rows are copied in 16-byte pieces
+    if (row_bytes % 16 != 0 || (ldx * eb) % 16 != 0) return FVGB_EINVAL;
     const int BN = tile_n(c_out);
     if (BN < 0) return FVGB_EINVAL;
     if (n_out == 0) return FVGB_OK;
@@ -728,12 +740,12 @@ extern "C" int fvgb_conv_fwd_tc_rows(int32_t dtype, const void *x, int64_t n_x, 
     a.wpack = (const uint8_t *)packed_w;
     int pack = 1, nchunks = 1;
     weight_units(K, row_bytes, &pack, &nchunks);
-    if (pack > 4) return FVGB_EINVAL;
     a.nchunks = nchunks;
     a.pack = pack;
     a.groups = (int32_t)ceil_div((int64_t)K, (int64_t)pack);
     // the group bit set of a K <= 32 mask has at most 16 bits; K > 32 walks units linearly
     a.row_bytes = (int32_t)row_bytes;
+    a.f16 = f16 ? 1 : 0;
     a.cout = c_out;
     a.y = (uint8_t *)y;
     a.ldy = ldy;
@@ -749,4 +761,30 @@ extern "C" int fvgb_conv_fwd_tc_rows(int32_t dtype, const void *x, int64_t n_x, 
                                                                                  : 0;
     cudaStream_t s = as_stream(stream);
     return dispatch_fwd(eb, BN, a.pack, a, s);
+}
+}  // namespace
+}  // namespace fvgb
+
+extern "C" int fvgb_conv_fwd_tc_rows(int32_t dtype, const void *x, int64_t n_x, int32_t c_in, int64_t ldx,
+                                     const int32_t *map, int64_t n_out, int32_t K, const int32_t *rows,
+                                     const uint32_t *tile_mask, const void *packed_w, int32_t c_out, void *y,
+                                     int64_t ldy, const float *out_scale, const float *bias, int32_t relu,
+                                     int32_t *err_dev, fvgb_stream_t stream) {
+    const int eb = dtype == FVGB_E4M3 ? 1 : (dtype == FVGB_BF16 ? 2 : 0);
+    if (!eb) return FVGB_ETYPE;
+    // each MMA consumes 32 bytes of K; rows shorter than 128 bytes must tile a 128-byte row
+    const int64_t row_bytes = (int64_t)c_in * eb;
+    if (c_in > 0 && (row_bytes % 32 != 0 || (row_bytes < 128 && 128 % row_bytes != 0))) return FVGB_EINVAL;
+    return conv_fwd(eb, false, x, n_x, c_in, ldx, map, n_out, K, rows, tile_mask, packed_w, c_out, y, ldy, out_scale,
+                    bias, relu, err_dev, stream);
+}
+
+extern "C" int fvgb_conv_fwd_tc_16bit(int32_t dtype, const void *x, int64_t n_x, int32_t c_in, int64_t ldx,
+                                      const int32_t *map, int64_t n_out, int32_t K, const int32_t *rows,
+                                      const uint32_t *tile_mask, const void *packed_w, int32_t c_out, void *y,
+                                      int64_t ldy, const float *out_scale, const float *bias, int32_t relu,
+                                      int32_t *err_dev, fvgb_stream_t stream) {
+    if (dtype != FVGB_BF16 && dtype != FVGB_F16) return FVGB_ETYPE;
+    return conv_fwd(2, dtype == FVGB_F16, x, n_x, c_in, ldx, map, n_out, K, rows, tile_mask, packed_w, c_out, y, ldy,
+                    out_scale, bias, relu, err_dev, stream);
 }

@@ -920,12 +920,14 @@ void check_device_errors(const torch::Device &dev) {
     }
 }
 
-// Shapes the tcgen05 contraction takes: 32-byte multiples of K per MMA, and rows shorter than
-// one 128-byte swizzle row must tile it (c_in 16 or 32 for bf16; any multiple of 16 from 64).
+// Features the tcgen05 contraction takes: BF16 or FP16 rows of whole, 16-byte aligned 16-byte pieces
+// (channels a multiple of 8) and at most 256 output channels.  Rows that do not fill their MMAs are
+// padded with zeros in shared memory, which costs far less than the CUDA cores: 24->40->40 FP16, 3^3
+// and 2^3 on 50k voxels: 297 us and 50 us of conversions to FP32 and back on the CUDA cores, 47 us
+// here; every other 16-bit shape keeps the CUDA-core form.
 bool use_tensor_cores(const Tensor &x, int64_t cin, int64_t cout) {
-    const int64_t row = cin * 2;
-    return x.scalar_type() == torch::kBFloat16 && row % 32 == 0 && (row >= 128 || 128 % row == 0) && cout <= 256 &&
-           x.stride(0) % 8 == 0;
+    return (x.scalar_type() == torch::kBFloat16 || x.scalar_type() == torch::kFloat16) && cin % 8 == 0 && cout <= 256 &&
+           x.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0;
 }
 
 // Derived weight tensors, cached per source tensor: the [K, Cin, Cout] view / copy of a 5-D
@@ -1012,7 +1014,8 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
     auto s = cur_stream();
     if (use_tensor_cores(x, cin, cout)) {
         const int tag = transpose_w ? 3 : 2;
-        std::optional<Tensor> cached = derived_get(Wkio, tag);
+        const bool same_type = Wkio.scalar_type() == x.scalar_type();  // the cached images are of the weights' own type
+        std::optional<Tensor> cached = same_type ? derived_get(Wkio, tag) : std::nullopt;
         Tensor packed;
         if (cached && cached->device() == x.device()) {
             packed = *cached;
@@ -1023,7 +1026,7 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
             check_status(fvgb_tc_pack_weights(FVGB_BF16, w.data_ptr(), K, (int32_t)cin, (int32_t)cout, wsk, wsci,
                                               wsco, packed.data_ptr(), wb, s),
                          "weight pack");
-            if (Wkio.scalar_type() == torch::kBFloat16) derived_put(Wkio, tag, packed);
+            if (same_type) derived_put(Wkio, tag, packed);
         }
         const uint32_t *tm = tile_mask ? reinterpret_cast<const uint32_t *>(tile_mask->data_ptr<int32_t>()) : nullptr;
         Tensor b32, s32;
@@ -1035,19 +1038,8 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
         // maps that have no row order (K < 4 or K > 32)
         const auto order = pack ? pack_row_order_if_reused(pack, map_t, cin * 2, cout) : std::nullopt;
         std::optional<Tensor> plan;
-        if (pack && K < 4 && use_plan(FVGB_BF16, K, cin, cout, 2))
+        if (pack && K < 4 && dt == FVGB_BF16 && use_plan(FVGB_BF16, K, cin, cout, 2))
             plan = pack_plan_if_reused(pack, map_t, (int32_t)(cin * 2));
-        if (order) {
-            check_status(fvgb_conv_fwd_tc_rows(FVGB_BF16, x.data_ptr(), x.size(0), (int32_t)cin, x.stride(0),
-                                               order->map.data_ptr<int32_t>(), n_out, (int32_t)K,
-                                               order->rows.data_ptr<int32_t>(),
-                                               reinterpret_cast<const uint32_t *>(order->mask.data_ptr<int32_t>()),
-                                               packed.data_ptr(), (int32_t)cout, y.data_ptr(), y.stride(0), sp,
-                                               bias ? b32.data_ptr<float>() : nullptr, relu ? 1 : 0,
-                                               device_error_flag(x.device()).data_ptr<int32_t>(), s),
-                         "sparse conv forward (tensor cores)");
-            return y;
-        }
         if (plan) {
             check_status(fvgb_conv_fwd_tc_planned(FVGB_BF16, x.data_ptr(), x.size(0), (int32_t)cin, x.stride(0),
                                                   plan->data_ptr(), n_out, (int32_t)K, packed.data_ptr(),
@@ -1057,11 +1049,14 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
                          "sparse conv forward (tensor cores)");
             return y;
         }
-        check_status(fvgb_conv_fwd_tc_epilogue(FVGB_BF16, x.data_ptr(), x.size(0), (int32_t)cin, x.stride(0),
-                                               map.data_ptr<int32_t>(), n_out, (int32_t)K, tm, packed.data_ptr(),
-                                               (int32_t)cout, y.data_ptr(), y.stride(0), sp,
-                                               bias ? b32.data_ptr<float>() : nullptr, relu ? 1 : 0,
-                                               device_error_flag(x.device()).data_ptr<int32_t>(), s),
+        const Tensor &m_used = order ? order->map : map;
+        const uint32_t *tm_used = order ? reinterpret_cast<const uint32_t *>(order->mask.data_ptr<int32_t>()) : tm;
+        check_status(fvgb_conv_fwd_tc_16bit(dt, x.data_ptr(), x.size(0), (int32_t)cin, x.stride(0),
+                                            m_used.data_ptr<int32_t>(), n_out, (int32_t)K,
+                                            order ? order->rows.data_ptr<int32_t>() : nullptr, tm_used,
+                                            packed.data_ptr(), (int32_t)cout, y.data_ptr(), y.stride(0), sp,
+                                            bias ? b32.data_ptr<float>() : nullptr, relu ? 1 : 0,
+                                            device_error_flag(x.device()).data_ptr<int32_t>(), s),
                      "sparse conv forward (tensor cores)");
         return y;
     } else if (dt == FVGB_F32 || dt == FVGB_F64) {

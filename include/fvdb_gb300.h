@@ -341,7 +341,7 @@ int fvgb_conv_wgrad_simt_noalloc(int32_t dtype, const void *x, int64_t n_x, int3
 
 /*
  * Bytes of the packed weight image that fvgb_conv_fwd_tc reads for a [K, c_in, c_out]
- * weight in `dtype` (FVGB_BF16 or FVGB_E4M3); c_out <= 256.  (host)
+ * weight in `dtype` (FVGB_BF16, which serves FP16 too, or FVGB_E4M3); c_out <= 256.  (host)
  */
 int fvgb_tc_weight_bytes(int32_t dtype, int64_t K, int32_t c_in, int32_t c_out, size_t *bytes);
 
@@ -410,6 +410,14 @@ int fvgb_conv_fwd_tc_rows(int32_t dtype, const void *x, int64_t n_x, int32_t c_i
                           int64_t n_out, int32_t K, const int32_t *rows, const uint32_t *tile_mask,
                           const void *packed_w, int32_t c_out, void *y, int64_t ldy, const float *out_scale,
                           const float *bias, int32_t relu, int32_t *err_dev, fvgb_stream_t stream);
+/* fvgb_conv_fwd_tc_rows for FVGB_BF16 or FVGB_F16 features of any channel count that is a multiple
+ * of 8 (rows of whole 16-byte pieces, padded with zeros in shared memory where they do not fill
+ * their MMAs); rows may be null (index order).  y has the features' type.  packed_w as for
+ * FVGB_BF16 (the image is a permutation of 2-byte elements). */
+int fvgb_conv_fwd_tc_16bit(int32_t dtype, const void *x, int64_t n_x, int32_t c_in, int64_t ldx, const int32_t *map,
+                           int64_t n_out, int32_t K, const int32_t *rows, const uint32_t *tile_mask,
+                           const void *packed_w, int32_t c_out, void *y, int64_t ldy, const float *out_scale,
+                           const float *bias, int32_t relu, int32_t *err_dev, fvgb_stream_t stream);
 
 /*
  * Tile plan of a kernel map for the planned tensor-core convolution: for every 128-row tile of
