@@ -135,6 +135,15 @@ __device__ inline int32_t batch_of(const int64_t *offsets, int32_t num_grids, in
     return lo;
 }
 
+// batch_of by a converged warp for one row: the offsets of up to 32 grids are compared at once (one
+// load instead of a chain of dependent ones).
+__device__ inline int32_t batch_of_warp(const int64_t *offsets, int32_t num_grids, int64_t row) {
+    if (num_grids > 32) return batch_of(offsets, num_grids, row);
+    const int lane = threadIdx.x & 31;
+    const bool past = lane < num_grids - 1 && __ldg(offsets + lane + 1) <= row;
+    return __popc(__ballot_sync(0xffffffffu, past));
+}
+
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 }  // namespace fvgb

@@ -8,8 +8,8 @@
 //
 // Bound by HBM: forward reads x twice and writes y, backward reads x and dy twice and writes dx.
 // 1.08M voxels x 64 channels in four grids, BF16, forward and backward together (GB300): 184 ms as
-// torch segment sums (their backward adds every row into one of four gradient rows), 0.59 ms here:
-// statistics 70 us, normalisation 77, gradient sums 190, dx 165, the merges 45.
+// torch segment sums (their backward adds every row into one of four gradient rows), 0.52 ms here:
+// statistics 59 us, normalisation 71, gradient sums 159, dx 114, the merges 70.
 //
 // A CTA owns a chunk of consecutive rows; every thread keeps one vector column (V channels of one
 // group) and kRowsPerThread rows of it in registers, so the chunk's variance is taken about the
@@ -28,7 +28,8 @@ namespace fvgb {
 namespace {
 
 constexpr int kNT = 256;
-constexpr int kRowsPerThread = 8;
+constexpr int kRowsPerThread = 8;  // forward: one operand
+constexpr int kRowsBackward = 4;   // backward: two operands in as many registers
 
 template <typename T>
 struct NNum;
@@ -79,11 +80,21 @@ __device__ __forceinline__ void grid_rows(const NormArgs &a, int32_t b, int64_t 
     hi = min(max(a.joff[b + 1], lo), a.n);
 }
 
-// Sum over the thread rows rr of the CTA for each column qq: the total is left in sm[qq] and
-// returned by every thread of the column.  sm: kNT entries.
+// Sum over the thread rows rr of the CTA for each column qq, returned by every thread of the column.
+// sm: kNT entries.  Columns that divide a warp fold its thread rows by shuffles first.
 template <typename A>
 __device__ __forceinline__ A column_sum(A v, A *sm, int rr, int qq, int QB, int rpi, int half) {
     __syncthreads();
+    if (QB <= 32 && (QB & (QB - 1)) == 0) {
+        for (int o = QB; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        const int lane = threadIdx.x & 31;
+        if (lane < QB) sm[(threadIdx.x >> 5) * QB + lane] = v;
+        __syncthreads();
+        A t = 0;
+#pragma unroll
+        for (int w = 0; w < kNT / 32; ++w) t += sm[w * QB + qq];
+        return t;
+    }
     if (rr < rpi) sm[rr * QB + qq] = v;
     for (int s = half; s > 0; s >>= 1) {
         __syncthreads();
@@ -105,13 +116,13 @@ __global__ void __launch_bounds__(kNT) gn_stats_kernel(NormArgs a, const T *__re
     int half = 1;
     while (half * 2 < a.rpi) half *= 2;
     const int64_t r0 = (int64_t)blockIdx.x * a.chunk_rows, r1 = min(a.n, r0 + a.chunk_rows);
+    const int32_t b0 = batch_of_warp(a.joff, a.B, r0), b1 = batch_of_warp(a.joff, a.B, r1 - 1);
     Pack<T, V> p[kRowsPerThread];
 #pragma unroll
     for (int i = 0; i < kRowsPerThread; ++i) {
         const int64_t r = r0 + rr + (int64_t)i * a.rpi;
         if (col && r < r1) p[i] = *reinterpret_cast<const Pack<T, V> *>(x + r * a.C + (int64_t)q * V);
     }
-    const int32_t b0 = batch_of(a.joff, a.B, r0), b1 = batch_of(a.joff, a.B, r1 - 1);
     for (int32_t b = b0; b <= b1; ++b) {
         int64_t lo, hi;
         grid_rows(a, b, lo, hi);
@@ -211,15 +222,15 @@ __global__ void __launch_bounds__(kNT) gn_apply_kernel(NormArgs a, const T *__re
     using A = typename NNum<T>::A;
     const int tid = threadIdx.x, qq = tid % a.QB, rr = tid / a.QB;
     const int q = blockIdx.y * a.QB + qq;
-    if (rr >= a.rpi || q >= a.Q) return;
     const int64_t r0 = (int64_t)blockIdx.x * a.chunk_rows, r1 = min(a.n, r0 + a.chunk_rows);
+    const int32_t b0 = batch_of_warp(a.joff, a.B, r0), b1 = batch_of_warp(a.joff, a.B, r1 - 1);
+    if (rr >= a.rpi || q >= a.Q) return;
     Pack<T, V> p[kRowsPerThread];
 #pragma unroll
     for (int i = 0; i < kRowsPerThread; ++i) {
         const int64_t r = r0 + rr + (int64_t)i * a.rpi;
         if (r < r1) p[i] = *reinterpret_cast<const Pack<T, V> *>(x + r * a.C + (int64_t)q * V);
     }
-    const int32_t b0 = batch_of(a.joff, a.B, r0), b1 = batch_of(a.joff, a.B, r1 - 1);
     const int32_t g = q * V / a.cpg;
     A wv[V], bv[V];
 #pragma unroll
@@ -242,7 +253,7 @@ __global__ void __launch_bounds__(kNT) gn_apply_kernel(NormArgs a, const T *__re
 
 // part[slot][0][c] = sum of dy, part[slot][1][c] = sum of dy * xhat over the slot's rows
 template <typename T, int V>
-__global__ void __launch_bounds__(kNT) gn_grad_sums_kernel(NormArgs a, const T *__restrict__ x,
+__global__ void __launch_bounds__(kNT, 4) gn_grad_sums_kernel(NormArgs a, const T *__restrict__ x,
                                                            const T *__restrict__ dy,
                                                            const typename NNum<T>::A *__restrict__ mean,
                                                            const typename NNum<T>::A *__restrict__ rstd,
@@ -255,16 +266,16 @@ __global__ void __launch_bounds__(kNT) gn_grad_sums_kernel(NormArgs a, const T *
     int half = 1;
     while (half * 2 < a.rpi) half *= 2;
     const int64_t r0 = (int64_t)blockIdx.x * a.chunk_rows, r1 = min(a.n, r0 + a.chunk_rows);
-    Pack<T, V> p[kRowsPerThread], d[kRowsPerThread];
+    const int32_t b0 = batch_of_warp(a.joff, a.B, r0), b1 = batch_of_warp(a.joff, a.B, r1 - 1);
+    Pack<T, V> p[kRowsBackward], d[kRowsBackward];
 #pragma unroll
-    for (int i = 0; i < kRowsPerThread; ++i) {
+    for (int i = 0; i < kRowsBackward; ++i) {
         const int64_t r = r0 + rr + (int64_t)i * a.rpi;
         if (col && r < r1) {
             p[i] = *reinterpret_cast<const Pack<T, V> *>(x + r * a.C + (int64_t)q * V);
             d[i] = *reinterpret_cast<const Pack<T, V> *>(dy + r * a.C + (int64_t)q * V);
         }
     }
-    const int32_t b0 = batch_of(a.joff, a.B, r0), b1 = batch_of(a.joff, a.B, r1 - 1);
     for (int32_t b = b0; b <= b1; ++b) {
         int64_t lo, hi;
         grid_rows(a, b, lo, hi);
@@ -278,7 +289,7 @@ __global__ void __launch_bounds__(kNT) gn_grad_sums_kernel(NormArgs a, const T *
             const int64_t k = (int64_t)b * a.G + q * V / a.cpg;
             const A m = mean[k], rs = rstd[k];
 #pragma unroll
-            for (int i = 0; i < kRowsPerThread; ++i) {
+            for (int i = 0; i < kRowsBackward; ++i) {
                 const int64_t r = r0 + rr + (int64_t)i * a.rpi;
                 if (r < lo || r >= hi) continue;
 #pragma unroll
@@ -288,6 +299,35 @@ __global__ void __launch_bounds__(kNT) gn_grad_sums_kernel(NormArgs a, const T *
                     s2[e] += g * ((NNum<T>::to(p[i].v[e]) - m) * rs);
                 }
             }
+        }
+        if (a.QB <= 32 && (a.QB & (a.QB - 1)) == 0) {
+            // columns that divide a warp: fold its thread rows by shuffles, then the warps' sums
+#pragma unroll
+            for (int e = 0; e < V; ++e)
+                for (int o = a.QB; o < 32; o <<= 1) {
+                    s1[e] += __shfl_xor_sync(0xffffffffu, s1[e], o);
+                    s2[e] += __shfl_xor_sync(0xffffffffu, s2[e], o);
+                }
+            __syncthreads();
+            const int lane = tid & 31;
+            if (lane < a.QB)
+#pragma unroll
+                for (int e = 0; e < V; ++e) {
+                    sm[e * kNT + (tid >> 5) * a.QB + lane] = s1[e];
+                    sm[(V + e) * kNT + (tid >> 5) * a.QB + lane] = s2[e];
+                }
+            __syncthreads();
+            // one thread per (sum, column): 2 V x QB of them, strided over the CTA
+            for (int i = tid; i < 2 * V * a.QB; i += kNT) {
+                const int j = i / a.QB, c = i % a.QB;
+                const int64_t qc = (int64_t)blockIdx.y * a.QB + c;
+                if (qc >= a.Q) continue;
+                A t = 0;
+#pragma unroll
+                for (int w = 0; w < kNT / 32; ++w) t += sm[j * kNT + w * a.QB + c];
+                part[((int64_t)blockIdx.x + b) * 2 * a.C + (j / V) * a.C + qc * V + j % V] = t;
+            }
+            continue;
         }
         // fold the thread rows together: entry j of thread t at sm[j * kNT + t]
         __syncthreads();
@@ -370,7 +410,7 @@ __global__ void gn_coef_kernel(NormArgs a, const double *__restrict__ sums, cons
 }
 
 template <typename T, int V>
-__global__ void __launch_bounds__(kNT) gn_dx_kernel(NormArgs a, const T *__restrict__ x, const T *__restrict__ dy,
+__global__ void __launch_bounds__(kNT, 4) gn_dx_kernel(NormArgs a, const T *__restrict__ x, const T *__restrict__ dy,
                                                     const typename NNum<T>::A *__restrict__ mean,
                                                     const typename NNum<T>::A *__restrict__ rstd,
                                                     const typename NNum<T>::A *__restrict__ w,
@@ -379,24 +419,24 @@ __global__ void __launch_bounds__(kNT) gn_dx_kernel(NormArgs a, const T *__restr
     using A = typename NNum<T>::A;
     const int tid = threadIdx.x, qq = tid % a.QB, rr = tid / a.QB;
     const int q = blockIdx.y * a.QB + qq;
-    if (rr >= a.rpi || q >= a.Q) return;
     const int64_t r0 = (int64_t)blockIdx.x * a.chunk_rows, r1 = min(a.n, r0 + a.chunk_rows);
-    Pack<T, V> p[kRowsPerThread], d[kRowsPerThread];
+    const int32_t b0 = batch_of_warp(a.joff, a.B, r0), b1 = batch_of_warp(a.joff, a.B, r1 - 1);
+    if (rr >= a.rpi || q >= a.Q) return;
+    Pack<T, V> p[kRowsBackward], d[kRowsBackward];
 #pragma unroll
-    for (int i = 0; i < kRowsPerThread; ++i) {
+    for (int i = 0; i < kRowsBackward; ++i) {
         const int64_t r = r0 + rr + (int64_t)i * a.rpi;
         if (r < r1) {
             p[i] = *reinterpret_cast<const Pack<T, V> *>(x + r * a.C + (int64_t)q * V);
             d[i] = *reinterpret_cast<const Pack<T, V> *>(dy + r * a.C + (int64_t)q * V);
         }
     }
-    const int32_t b0 = batch_of(a.joff, a.B, r0), b1 = batch_of(a.joff, a.B, r1 - 1);
     const int32_t g = q * V / a.cpg;
     A wv[V];
 #pragma unroll
     for (int e = 0; e < V; ++e) wv[e] = w ? w[q * V + e] : (A)1;
 #pragma unroll
-    for (int i = 0; i < kRowsPerThread; ++i) {
+    for (int i = 0; i < kRowsBackward; ++i) {
         const int64_t r = r0 + rr + (int64_t)i * a.rpi;
         if (r >= r1) continue;
         const int64_t k = (int64_t)(b0 == b1 ? b0 : batch_of(a.joff, a.B, r)) * a.G + g;
@@ -423,7 +463,7 @@ int pick_vec(int32_t cpg, int elem, const void *const *ptrs, int n_ptrs) {
     return v;
 }
 
-NormArgs norm_args(const int64_t *joff, int32_t B, int64_t n, int32_t C, int32_t G, int V) {
+NormArgs norm_args(const int64_t *joff, int32_t B, int64_t n, int32_t C, int32_t G, int V, bool backward) {
     NormArgs a;
     a.joff = joff;
     a.B = B;
@@ -434,7 +474,7 @@ NormArgs norm_args(const int64_t *joff, int32_t B, int64_t n, int32_t C, int32_t
     a.Q = C / V;
     a.QB = a.Q < kNT ? a.Q : kNT;
     a.rpi = kNT / a.QB;
-    a.chunk_rows = (int64_t)a.rpi * kRowsPerThread;
+    a.chunk_rows = (int64_t)a.rpi * (backward ? kRowsBackward : kRowsPerThread);
     return a;
 }
 
@@ -444,7 +484,7 @@ size_t norm_ws(int64_t n, int32_t B, int32_t C, int32_t G, size_t acc, bool back
     size_t need = 0;
     for (int V = 1; V <= 8; V *= 2) {
         if ((C / G) % V) break;
-        const NormArgs a = norm_args(nullptr, B, n, C, G, V);
+        const NormArgs a = norm_args(nullptr, B, n, C, G, V, backward);
         const size_t slots = (size_t)ceil_div(n > 0 ? n : 1, a.chunk_rows) + (size_t)B;
         const size_t s = backward ? slots * 2 * (size_t)C * acc : slots * (size_t)a.Q * 2 * acc;
         if (s > need) need = s;
@@ -517,7 +557,7 @@ int elem_size(int32_t dtype) { return dtype == FVGB_F64 ? 8 : (dtype == FVGB_F32
 int norm_check(int32_t dtype, int64_t n, int32_t C, int32_t G, int32_t B) {
     if (dtype != FVGB_F32 && dtype != FVGB_F64 && dtype != FVGB_BF16 && dtype != FVGB_F16) return FVGB_ETYPE;
     if (n < 0 || C < 1 || G < 1 || B < 1 || C % G != 0 || G > 65535 || C > 65535) return FVGB_EINVAL;
-    if (n / kRowsPerThread > INT32_MAX - 1) return FVGB_EINVAL;
+    if (n / kRowsBackward > INT32_MAX - 1) return FVGB_EINVAL;
     return FVGB_OK;
 }
 
@@ -546,7 +586,7 @@ extern "C" int fvgb_group_norm_forward(int32_t dtype, const void *x, int64_t n, 
     if (!workspace || workspace_bytes < need) return FVGB_ENOSPACE;
     const void *ptrs[2] = {x, y};
     const int V = pick_vec(channels / groups, elem_size(dtype), ptrs, 2);
-    const NormArgs a = norm_args(joffsets, num_grids, n, channels, groups, V);
+    const NormArgs a = norm_args(joffsets, num_grids, n, channels, groups, V, false);
     void *ws = reinterpret_cast<void *>(((uintptr_t)workspace + 255) & ~(uintptr_t)255);
     st = by_dtype(dtype, [&](auto *t) {
         using T = std::remove_pointer_t<decltype(t)>;
@@ -571,7 +611,7 @@ extern "C" int fvgb_group_norm_backward(int32_t dtype, const void *x, const void
     if (!workspace || workspace_bytes < need) return FVGB_ENOSPACE;
     const void *ptrs[3] = {x, dy, dx};
     const int V = pick_vec(channels / groups, elem_size(dtype), ptrs, 3);
-    const NormArgs a = norm_args(joffsets, num_grids, n, channels, groups, V);
+    const NormArgs a = norm_args(joffsets, num_grids, n, channels, groups, V, true);
     void *ws = reinterpret_cast<void *>(((uintptr_t)workspace + 255) & ~(uintptr_t)255);
     st = by_dtype(dtype, [&](auto *t) {
         using T = std::remove_pointer_t<decltype(t)>;
