@@ -1513,6 +1513,30 @@ Tensor upsample_backward(const GridPtr &coarse, const GridPtr &fine, const std::
     return dx.narrow(1, 0, C).reshape(x.sizes());
 }
 
+// Gradient of a convolution's fused bias and ReLU: (dy masked where the output y is not positive, or
+// dy itself without y; the bias gradient in FP32 or wider, where needed).
+std::vector<Tensor> bias_relu_backward(const Tensor &dy_in, const std::optional<Tensor> &y, bool need_db) {
+    c10::cuda::CUDAGuard guard(dy_in.device());
+    Tensor dy = dy_in.contiguous();
+    const int64_t n = dy.size(0), c = dy.size(1);
+    const auto acc = dy.scalar_type() == torch::kFloat64 ? torch::kFloat64 : torch::kFloat32;
+    Tensor out = y ? torch::empty_like(dy) : dy, db, ws, yc;
+    if (y) yc = y->contiguous();
+    if (need_db) {
+        db = torch::empty({c}, dy.options().dtype(acc));
+        size_t wsb = 0;
+        check_status(fvgb_bias_relu_backward_workspace(fvgb_dtype(dy), n, (int32_t)c, &wsb), "bias gradient (workspace)");
+        ws = workspace(wsb, dy.device());
+    }
+    if (y || need_db)
+        check_status(fvgb_bias_relu_backward(fvgb_dtype(dy), dy.data_ptr(), y ? yc.data_ptr() : nullptr, n, (int32_t)c,
+                                             out.data_ptr(), need_db ? db.data_ptr() : nullptr,
+                                             need_db ? ws.data_ptr() : nullptr, need_db ? (size_t)ws.numel() : 0,
+                                             cur_stream()),
+                     "bias and ReLU gradient");
+    return {out, db};
+}
+
 // Group normalisation of jagged rows: (y, mean, rstd); weight / bias in the accumulation type.
 std::vector<Tensor> group_norm_forward(const Tensor &x_in, const Tensor &joff, int64_t groups,
                                        const std::optional<Tensor> &weight, const std::optional<Tensor> &bias,
@@ -1633,6 +1657,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("conv_backward", &conv_backward, py::call_guard<py::gil_scoped_release>());
     m.def("halo_conv", &halo_conv, py::call_guard<py::gil_scoped_release>());
     m.def("halo_wgrad", &halo_wgrad, py::call_guard<py::gil_scoped_release>());
+    m.def("bias_relu_backward", &bias_relu_backward, py::call_guard<py::gil_scoped_release>());
     m.def("group_norm_forward", &group_norm_forward, py::call_guard<py::gil_scoped_release>());
     m.def("group_norm_backward", &group_norm_backward, py::call_guard<py::gil_scoped_release>());
     m.def("pool_forward", &pool_forward);

@@ -41,17 +41,21 @@ class SparseConvFunction(torch.autograd.Function):
             return None, None, None, None, None, None, None
         if ctx.scaled:
             raise RuntimeError("a convolution with a folded batch norm (out_scale) is inference-only")
-        if ctx.relu:
-            # fused ReLU: the gradient passes where the output is positive (torch.relu's rule)
-            grad_out = grad_out * (ctx.saved_tensors[2] > 0)
-        dx = dw = None
+        # fused ReLU: the gradient passes where the output is positive (torch.relu's rule); bias
+        # gradient = column sum of dy, accumulated in at least FP32 (FP64 stays FP64)
+        y = ctx.saved_tensors[2] if ctx.relu else None
+        dx = dw = db = None
+        if torch.is_grad_enabled():  # create_graph: operations that record their own gradient
+            if ctx.relu:
+                grad_out = grad_out * (y > 0)
+            if need_db:
+                db = grad_out.sum(0, dtype=torch.promote_types(grad_out.dtype, torch.float32))
+        else:
+            grad_out, db = C.bias_relu_backward(grad_out, y, need_db)
         if need_dx or need_dw:
             dx, dw = C.conv_backward(grad_out, features, wkio, ctx.pack_impl, ctx.transposed, need_dx, need_dw)
-        # bias gradient = column sum of dy, accumulated in at least FP32 (FP64 stays FP64)
-        db = None
         if need_db:
-            acc = torch.promote_types(grad_out.dtype, torch.float32)
-            db = grad_out.sum(0, dtype=acc).to(ctx.bias_dtype)
+            db = db.to(ctx.bias_dtype)
         return (dx if need_dx else None), (dw if need_dw else None), None, None, db, None, None
 
 

@@ -572,6 +572,16 @@ int fvgb_halo_wgrad(int32_t dtype, const FvgbGrid *grid, const void *x, int64_t 
                     fvgb_stream_t stream);
 
 /* ------------------------------------------------------------------------------------------
+ * Gradient of a fused bias and ReLU: out[r, c] = dy[r, c] * (y[r, c] > 0) (y null: no ReLU, out
+ * unused) and dbias[c] = sum of out (of dy without ReLU) over the rows, FP32 (FP64 for FP64) merged
+ * in FP64 in a fixed order (null: not needed).  Contiguous [n, c]; dtype FVGB_F32 / FVGB_F64 /
+ * FVGB_BF16 / FVGB_F16.
+ * ------------------------------------------------------------------------------------------ */
+int fvgb_bias_relu_backward_workspace(int32_t dtype, int64_t n, int32_t c, size_t *bytes);
+int fvgb_bias_relu_backward(int32_t dtype, const void *dy, const void *y, int64_t n, int32_t c, void *out,
+                            void *dbias, void *workspace, size_t workspace_bytes, fvgb_stream_t stream);
+
+/* ------------------------------------------------------------------------------------------
  * Group normalisation of jagged features: x [n, channels] contiguous rows, grid b's voxels are
  * rows joffsets[b] .. joffsets[b+1]-1 (device int64 [num_grids + 1], covering [0, n)); each
  * (grid, group of channels / groups consecutive channels) is normalised over its rows and
