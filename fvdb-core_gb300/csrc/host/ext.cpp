@@ -757,12 +757,14 @@ std::optional<RowOrder> pack_row_order(PackPtr p, bool transposed) {
 //     saves more than its share of the sort: 128->256 FP8, 4.3M rows: 4.0 ms in index order, 2.7 ms
 //     ordered plus 0.6 ms for the order; 64->64 BF16 saves less than the order costs.
 // Below 2^14 rows the order's seven launches cost more than any of this.
-std::optional<RowOrder> pack_row_order_if_reused(PackPtr p, bool transposed, int64_t row_bytes, int64_t cout) {
+// A contraction that announces another over the same map (reuse) counts as reused.
+std::optional<RowOrder> pack_row_order_if_reused(PackPtr p, bool transposed, int64_t row_bytes, int64_t cout,
+                                                 bool reuse) {
     const int d = transposed ? 1 : 0;
     const bool one_entry = transposed && p->st.v[0] >= p->ks.v[0] && p->st.v[1] >= p->ks.v[1] && p->st.v[2] >= p->ks.v[2];
     const bool wide = row_bytes * cout >= 128 * 256;
     const int64_t n = transposed ? p->src->N : p->tgt->N;
-    if (!p->order_rows[d] && !((one_entry || wide) && n >= ((int64_t)1 << 14)) && ++p->order_requests[d] < 2)
+    if (!p->order_rows[d] && !((one_entry || wide || reuse) && n >= ((int64_t)1 << 14)) && ++p->order_requests[d] < 2)
         return std::nullopt;
     return pack_row_order(p, transposed);
 }
@@ -942,7 +944,7 @@ struct DerivedKey {
     std::vector<int64_t> sizes, strides;
     c10::ScalarType dtype;
     int64_t version;
-    int tag;  // what is derived: 0/1 = [K, Cin, Cout] (not transposed / transposed), 2/3 = packed (W / W^T)
+    int tag;  // what is derived: 0/1 = [K, Cin, Cout] (not transposed / transposed), 2/3 = packed (W / W^T), 4/5 = mirrored
     bool operator==(const DerivedKey &o) const {
         return storage == o.storage && offset == o.offset && sizes == o.sizes && strides == o.strides &&
                dtype == o.dtype && version == o.version && tag == o.tag;
@@ -993,14 +995,28 @@ void derived_put(const Tensor &src, int tag, const Tensor &value) {
     while (g_derived.size() > kDerivedMax) g_derived.pop_back();
 }
 
+// A stride-1 map of a grid onto itself with odd kernel extents: offset k has its mirror image at
+// K-1-k, so map[m, k] == i exactly where map[i, K-1-k] == m, and a contraction over the transposed
+// map is one over the map itself with the weights in reverse offset order.  No transposed map is
+// built (its fill, scatter and masks), and both directions share one row order: on the 1.27M-voxel
+// training step (two 64->64 layers) the transposed map, its masks and its order were 0.5 ms.
+bool self_mirrored(const PackPtr &p) {
+    bool r = p->src == p->tgt;
+    for (int a = 0; a < 3; ++a) r = r && p->st.v[a] == 1 && p->ks.v[a] % 2 == 1;
+    return r;
+}
+
 // y[m] = sum_k x[map[m,k]] W[k]   for the first n_out rows of map
+// mirror: W in reverse offset order (see self_mirrored).  reuse: the caller will contract over this
+// map again (training: the data gradient), so a large map gets its row order at once.
 // bias (optional, [cout]): added in the tensor-core epilogue, else after the contraction.
 // pack / map_t (optional): the pack info that owns `map` and whether `map` is its transposed map;
 // with them, shapes the planned kernel takes run over the pack's cached tile plan.
 Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tensor &Wkio, bool transpose_w,
                    const std::optional<Tensor> &tile_mask = std::nullopt,
                    const std::optional<Tensor> &bias = std::nullopt, PackPtr pack = nullptr, bool map_t = false,
-                   bool relu = false, const std::optional<Tensor> &out_scale = std::nullopt) {
+                   bool relu = false, const std::optional<Tensor> &out_scale = std::nullopt, bool mirror = false,
+                   bool reuse = false) {
     c10::cuda::CUDAGuard guard(x.device());
     const int64_t K = map.size(1);
     const int64_t cin = transpose_w ? Wkio.size(2) : Wkio.size(1);
@@ -1009,11 +1025,15 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
     Tensor y = torch::empty({n_out, cout}, x.options());
     if (n_out == 0) return y;
     Tensor w = Wkio.to(x.scalar_type());
-    const int64_t wsk = w.stride(0), wsci = transpose_w ? w.stride(2) : w.stride(1), wsco = transpose_w ? w.stride(1) : w.stride(2);
+    const int64_t wsci = transpose_w ? w.stride(2) : w.stride(1), wsco = transpose_w ? w.stride(1) : w.stride(2);
+    const int64_t wsk = mirror ? -w.stride(0) : w.stride(0);
+    auto first_offset = [&](const Tensor &t) -> const void * {
+        return static_cast<const char *>(t.data_ptr()) + (mirror ? (K - 1) * t.stride(0) * t.element_size() : 0);
+    };
     const int32_t dt = fvgb_dtype(x);
     auto s = cur_stream();
     if (use_tensor_cores(x, cin, cout)) {
-        const int tag = transpose_w ? 3 : 2;
+        const int tag = (transpose_w ? 3 : 2) + (mirror ? 2 : 0);
         const bool same_type = Wkio.scalar_type() == x.scalar_type();  // the cached images are of the weights' own type
         std::optional<Tensor> cached = same_type ? derived_get(Wkio, tag) : std::nullopt;
         Tensor packed;
@@ -1023,7 +1043,7 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
             size_t wb = 0;
             check_status(fvgb_tc_weight_bytes(FVGB_BF16, K, (int32_t)cin, (int32_t)cout, &wb), "weight pack size");
             packed = torch::empty({(int64_t)wb}, torch::dtype(torch::kUInt8).device(x.device()));
-            check_status(fvgb_tc_pack_weights(FVGB_BF16, w.data_ptr(), K, (int32_t)cin, (int32_t)cout, wsk, wsci,
+            check_status(fvgb_tc_pack_weights(FVGB_BF16, first_offset(w), K, (int32_t)cin, (int32_t)cout, wsk, wsci,
                                               wsco, packed.data_ptr(), wb, s),
                          "weight pack");
             if (same_type) derived_put(Wkio, tag, packed);
@@ -1036,7 +1056,7 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
         // a map used again runs over its row order (measured faster than a tile plan: C2 layer 1,
         // 32->64: 0.30 ms ordered, 0.32 ms planned, 0.365 ms in index order); the tile plan serves
         // maps that have no row order (K < 4 or K > 32)
-        const auto order = pack ? pack_row_order_if_reused(pack, map_t, cin * 2, cout) : std::nullopt;
+        const auto order = pack ? pack_row_order_if_reused(pack, map_t, cin * 2, cout, reuse) : std::nullopt;
         std::optional<Tensor> plan;
         if (pack && K < 4 && dt == FVGB_BF16 && use_plan(FVGB_BF16, K, cin, cout, 2))
             plan = pack_plan_if_reused(pack, map_t, (int32_t)(cin * 2));
@@ -1064,11 +1084,11 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
         // build); small ones only once reused, where the build's launches would dominate
         const auto order = !pack ? std::nullopt
                                  : (n_out >= (int64_t)1 << 16 ? pack_row_order(pack, map_t)
-                                                              : pack_row_order_if_reused(pack, map_t, 0, 0));
+                                                              : pack_row_order_if_reused(pack, map_t, 0, 0, reuse));
         const Tensor &m_used = order ? order->map : map;
         check_status(fvgb_conv_fwd_simt_rows(dt, x.data_ptr(), x.size(0), (int32_t)cin, x.stride(0),
                                              m_used.data_ptr<int32_t>(), n_out, (int32_t)K, m_used.stride(0),
-                                             order ? order->rows.data_ptr<int32_t>() : nullptr, w.data_ptr(), wsk,
+                                             order ? order->rows.data_ptr<int32_t>() : nullptr, first_offset(w), wsk,
                                              wsci, wsco, y.data_ptr(), (int32_t)cout, y.stride(0), 0, s),
                      "sparse conv forward");
     } else {
@@ -1077,8 +1097,8 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
         Tensor xf = x.to(torch::kFloat32), wf = w.to(torch::kFloat32);
         Tensor yf = torch::empty({n_out, cout}, xf.options());
         check_status(fvgb_conv_fwd_simt(FVGB_F32, xf.data_ptr(), xf.size(0), (int32_t)cin, xf.stride(0),
-                                        map.data_ptr<int32_t>(), n_out, (int32_t)K, map.stride(0), wf.data_ptr(),
-                                        wf.stride(0), transpose_w ? wf.stride(2) : wf.stride(1),
+                                        map.data_ptr<int32_t>(), n_out, (int32_t)K, map.stride(0), first_offset(wf),
+                                        mirror ? -wf.stride(0) : wf.stride(0), transpose_w ? wf.stride(2) : wf.stride(1),
                                         transpose_w ? wf.stride(1) : wf.stride(2), yf.data_ptr(), (int32_t)cout,
                                         yf.stride(0), 0, s),
                      "sparse conv forward");
@@ -1134,7 +1154,7 @@ Tensor gather_wgrad(const Tensor &x, const Tensor &map, int64_t n_out, const Ten
 // into the layer), also in the epilogue.
 std::vector<Tensor> conv_forward(const Tensor &x, const Tensor &weights, PackPtr p, bool transposed,
                                  const std::optional<Tensor> &bias = std::nullopt, bool relu = false,
-                                 const std::optional<Tensor> &out_scale = std::nullopt) {
+                                 const std::optional<Tensor> &out_scale = std::nullopt, bool has_backward = false) {
     resolve_pack(p);
     TORCH_CHECK_VALUE(x.is_contiguous(), "features must be contiguous");
     TORCH_CHECK_TYPE(x.is_floating_point(), "features must have a floating point type");
@@ -1188,15 +1208,12 @@ std::vector<Tensor> conv_forward(const Tensor &x, const Tensor &weights, PackPtr
                           ",)");
         TORCH_CHECK_VALUE(out_scale->device() == x.device(), "out_scale must be on the features' device");
     }
-    Tensor y;
-    if (!transposed)
-        y = n_tgt > 0 ? gather_gemm(x, pack_kmap(p), n_tgt, Wkio, false, pack_tile_mask(p, false), bias, p, false, relu,
-                                    out_scale)
-                      : torch::empty({0, cout}, x.options());
-    else
-        y = n_src > 0 ? gather_gemm(x, pack_kmap_t(p), n_src, Wkio, false, pack_tile_mask(p, true), bias, p, true, relu,
-                                    out_scale)
-                      : torch::empty({0, cout}, x.options());
+    const bool mirror = transposed && self_mirrored(p);  // the map itself stands in for its transposed one
+    const bool map_t = transposed && !mirror;
+    const int64_t n_out = transposed ? n_src : n_tgt;
+    if (n_out == 0) return {torch::empty({0, cout}, x.options()), Wkio};
+    Tensor y = gather_gemm(x, map_t ? pack_kmap_t(p) : pack_kmap(p), n_out, Wkio, false, pack_tile_mask(p, map_t), bias,
+                           p, map_t, relu, out_scale, mirror, has_backward && self_mirrored(p));
     return {y, Wkio};
 }
 
@@ -1207,15 +1224,21 @@ std::vector<Tensor> conv_backward(const Tensor &dy_in, const Tensor &x, const Te
     Tensor dy = dy_in.contiguous();
     const int64_t K = Wkio.size(0), cin = Wkio.size(1), cout = Wkio.size(2);
     Tensor dx, dW;
+    const bool mirror = self_mirrored(p);
     if (!transposed) {
         // dgrad: dx[i] = sum_k dy[mapT[i,k]] W[k]^T ;  wgrad: dW[k] = sum_m x[map[m,k]]^T dy[m]
-        if (need_dx)
+        if (need_dx && mirror)
+            dx = gather_gemm(dy, pack_kmap(p), p->src->N, Wkio, true, pack_tile_mask(p, false), std::nullopt, p, false,
+                             false, std::nullopt, true);
+        else if (need_dx)
             dx = gather_gemm(dy, pack_kmap_t(p), p->src->N, Wkio, true, pack_tile_mask(p, true), std::nullopt, p, true);
         if (need_dw) dW = gather_wgrad(x, pack_kmap(p), p->tgt->N, dy, K, pack_tile_mask(p, false));
     } else {
         if (need_dx)
             dx = gather_gemm(dy, pack_kmap(p), p->tgt->N, Wkio, true, pack_tile_mask(p, false), std::nullopt, p, false);
-        if (need_dw) dW = gather_wgrad(x, pack_kmap_t(p), p->src->N, dy, K, pack_tile_mask(p, true));
+        if (need_dw && mirror)
+            dW = gather_wgrad(x, pack_kmap(p), p->src->N, dy, K, pack_tile_mask(p, false)).flip(0);
+        else if (need_dw) dW = gather_wgrad(x, pack_kmap_t(p), p->src->N, dy, K, pack_tile_mask(p, true));
     }
     if (need_dw) {
         dW = dW.reshape({p->ks.v[2], p->ks.v[1], p->ks.v[0], cin, cout});
@@ -1282,7 +1305,7 @@ std::vector<Tensor> conv_forward_fp8(const Tensor &x, const Tensor &weights, Pac
     const Tensor &map = transposed ? pack_kmap_t(p) : pack_kmap(p);
     auto tm = pack_tile_mask(p, transposed);
     Tensor sw = s_w.contiguous();
-    const auto order = pack_row_order_if_reused(p, transposed, cin, cout);
+    const auto order = pack_row_order_if_reused(p, transposed, cin, cout, false);
     std::optional<Tensor> plan;
     if (K < 4 && use_plan(FVGB_E4M3, K, cin, cout, 1)) plan = pack_plan_if_reused(p, transposed, (int32_t)cin);
     if (plan) {
@@ -1648,7 +1671,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     // so host threads of concurrent serving slots do not serialise on it
     m.def("conv_forward", &conv_forward, py::arg("features"), py::arg("weights"), py::arg("pack"),
           py::arg("transposed"), py::arg("bias") = py::none(), py::arg("relu") = false,
-          py::arg("out_scale") = py::none(), py::call_guard<py::gil_scoped_release>());
+          py::arg("out_scale") = py::none(), py::arg("has_backward") = false,
+          py::call_guard<py::gil_scoped_release>());
     m.def("conv_forward_fp8", &conv_forward_fp8, py::arg("features"), py::arg("weights"), py::arg("pack"),
           py::arg("transposed"), py::arg("relu") = false, py::arg("bias") = py::none(),
           py::call_guard<py::gil_scoped_release>());

@@ -20,7 +20,8 @@ class SparseConvFunction(torch.autograd.Function):
     def forward(ctx, features: torch.Tensor, weights: torch.Tensor, pack_impl, transposed: bool, bias=None,
                 relu: bool = False, scale=None):
         C = _lib.load()
-        y, wkio = C.conv_forward(features, weights, pack_impl, transposed, bias, relu, scale)
+        # a data gradient to come reuses the kernel map (and may share its row order)
+        y, wkio = C.conv_forward(features, weights, pack_impl, transposed, bias, relu, scale, ctx.needs_input_grad[0])
         ctx.scaled = scale is not None
         if relu:
             ctx.save_for_backward(features, wkio, y)
