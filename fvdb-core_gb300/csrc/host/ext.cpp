@@ -1438,6 +1438,13 @@ Tensor pool_backward(int32_t mode, const GridPtr &fine, const GridPtr &coarse, c
     FvgbGrid fv = fine->view(), cv = coarse->view();
     auto s = cur_stream();
     if (C == 0 || fine->N == 0) return torch::zeros_like(x);
+    if (mode == FVGB_POOL_MAX && st.v[0] >= p.v[0] && st.v[1] >= p.v[1] && st.v[2] >= p.v[2]) {
+        Tensor dx = torch::zeros({fine->N, C}, x.options());
+        check_status(fvgb_maxpool_backward_disjoint(fvgb_dtype(x), &fv, &cv, p.v, st.v, xf.data_ptr(), C, (int32_t)C,
+                                                    coarse->N ? df.data_ptr() : nullptr, C, dx.data_ptr(), s),
+                     "max_pool backward");
+        return dx.reshape(x.sizes());
+    }
     if (mode == FVGB_POOL_MAX) {
         const auto acc = x.scalar_type() == torch::kFloat64 ? torch::kFloat64 : torch::kFloat32;
         Tensor dacc = torch::zeros({fine->N, C}, x.options().dtype(acc));

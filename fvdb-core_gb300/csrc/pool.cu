@@ -18,11 +18,18 @@
 // (the reference reads the row before its grid's first), and gradients of overlapping windows
 // (stride < pool factor) add up (the reference's concurrent assignments keep one of them).
 //
-// Lookups go through the grids' leaf hash; one warp per output voxel gathers the window's
-// indices (lanes over window positions) into shared memory and then reduces channels (lanes over
-// channels, coalesced rows).  All of these kernels are bound by HBM and hash-probe latency.
+// Lookups go through the grids' leaf hash.  A group of G lanes owns one output voxel: the lanes share
+// the window's lookups, then each lane moves one 16-byte vector of the row (G = the power of two >=
+// vectors per row, so a 64-channel BF16 row takes 8 lanes and a warp works on four voxels).  Bound
+// by HBM for large rows and by the lookups' latency, which the groups of an SM hide, for short ones.
+// 1.08M fine and 0.29M coarse voxels, 64 BF16 channels, factor 2 (GB300), one warp per voxel and one
+// element per lane before: max 190 us, its gradient 235 + 115 for the FP32 buffer, upsampling 464,
+// its gradient 192; here 139, 231, 46 and 144 us.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+
+#include <initializer_list>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -73,12 +80,39 @@ __device__ __forceinline__ T mul_in(T a, double b) {
     return Num<T>::from(Num<T>::to(a) * Num<T>::to(Num<T>::from((A)b)));
 }
 
-// Window indices of one output voxel into the warp's shared array (window order i-outer,
-// k-inner); returns nothing, lanes fill positions lane, lane+32, ...
-__device__ __forceinline__ void window_indices(const FvgbGrid &g, int32_t b, int3 base, int3 ext, int32_t *idx,
-                                               int lane) {
+// V consecutive channels, one aligned load or store
+template <typename T, int V>
+struct __align__(sizeof(T) * V) Vec {
+    T v[V];
+};
+
+// Lane groups of a CTA: G = 1 << gs lanes per output voxel, and the shared window indices of each.
+struct Groups {
+    int gs;     // log2 lanes per group
+    int W;      // window entries stored per group
+    size_t smem;
+};
+
+constexpr int kGroupThreads = 256;
+constexpr int kGroupSmem = 32 * 1024;
+
+Groups groups_for(int32_t vecs, int W) {
+    Groups g;
+    g.gs = 0;
+    while ((1 << g.gs) < vecs && g.gs < 5) ++g.gs;
+    while (g.gs < 5 && (size_t)(kGroupThreads >> g.gs) * W * 4 > kGroupSmem) ++g.gs;
+    g.W = W;
+    g.smem = (size_t)(kGroupThreads >> g.gs) * W * 4;
+    return g;
+}
+
+// Window indices of one output voxel into the group's shared array (window order i-outer, k-inner):
+// lane l of the group fills positions l, l + G, ...  Every lane of the warp calls it (groups whose
+// voxel is past the end with an empty window).
+__device__ __forceinline__ void window_indices(const FvgbGrid &g, int32_t b, int3 base, int3 ext, int32_t *idx, int lane,
+                                               int G) {
     const int W = ext.x * ext.y * ext.z;
-    for (int w = lane; w < W; w += 32) {
+    for (int w = lane; w < W; w += G) {
         const int i = w / (ext.y * ext.z), j = (w / ext.z) % ext.y, k = w % ext.z;
         const int64_t v = voxel_at(g, b, base.x + i, base.y + j, base.z + k);
         idx[w] = (int32_t)v;
@@ -86,35 +120,128 @@ __device__ __forceinline__ void window_indices(const FvgbGrid &g, int32_t b, int
     __syncwarp();
 }
 
-template <typename T, bool MAX>
-__global__ void __launch_bounds__(kPoolWarps * 32) pool_fwd_kernel(FvgbGrid fine, FvgbGrid coarse, int3 pf, int3 st,
-                                                                   const T *__restrict__ x, int64_t ldx, int32_t C,
-                                                                   T *__restrict__ y, int64_t ldy, double avg) {
+constexpr int kAhead = 4;  // window rows a lane has in flight
+
+// Reduction over the window rows of every coarse voxel: maximum (MAX), or the sum, rounded and times
+// `avg` where SCALE.  Serves pooling and the upsampling gradient.
+template <typename T, int V, bool MAX, bool SCALE>
+__global__ void __launch_bounds__(kGroupThreads) window_reduce_kernel(FvgbGrid fine, FvgbGrid coarse, int3 pf, int3 st,
+                                                                      Groups gr, const T *__restrict__ x, int64_t ldx,
+                                                                      int32_t C, T *__restrict__ y, int64_t ldy,
+                                                                      double avg) {
     using A = typename Num<T>::Acc;
-    __shared__ int32_t widx[kPoolWarps][kMaxWindow];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int W = pf.x * pf.y * pf.z;
-    for (int64_t c = (int64_t)blockIdx.x * kPoolWarps + warp; c < coarse.num_voxels;
-         c += (int64_t)gridDim.x * kPoolWarps) {
-        const int32_t b = batch_of(coarse.voxel_offsets, coarse.num_grids, c);
-        const int3 base = make_int3(coarse.ijk[3 * c] * st.x, coarse.ijk[3 * c + 1] * st.y, coarse.ijk[3 * c + 2] * st.z);
-        window_indices(fine, b, base, pf, widx[warp], lane);
-        for (int ch = lane; ch < C; ch += 32) {
-            A acc = MAX ? (A)(-INFINITY) : (A)0;
-            for (int w = 0; w < W; ++w) {
-                const int32_t f = widx[warp][w];
-                if (f < 0) continue;
-                const A v = Num<T>::to(x[(int64_t)f * ldx + ch]);
-                acc = MAX ? (A)fmax((double)v, (double)acc) : acc + v;
+    extern __shared__ int32_t widx[];
+    const int G = 1 << gr.gs, group = threadIdx.x >> gr.gs, lane = threadIdx.x & (G - 1);
+    const int W = gr.W;
+    int32_t *idx = widx + group * W;
+    const int64_t c = (int64_t)blockIdx.x * (kGroupThreads >> gr.gs) + group;
+    const bool on = c < coarse.num_voxels;
+    int32_t b = 0;
+    int3 base = make_int3(0, 0, 0), ext = make_int3(0, 0, 0);
+    if (on) {
+        b = batch_of(coarse.voxel_offsets, coarse.num_grids, c);
+        base = make_int3(coarse.ijk[3 * c] * st.x, coarse.ijk[3 * c + 1] * st.y, coarse.ijk[3 * c + 2] * st.z);
+        ext = pf;
+    }
+    window_indices(fine, b, base, ext, idx, lane, G);
+    if (!on) return;
+    for (int32_t ch = lane * V; ch < C; ch += G * V) {
+        A acc[V];
+#pragma unroll
+        for (int e = 0; e < V; ++e) acc[e] = MAX ? (A)(-INFINITY) : (A)0;
+        for (int w0 = 0; w0 < W; w0 += kAhead) {
+            Vec<T, V> p[kAhead];
+            int32_t f[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                f[u] = w0 + u < W ? idx[w0 + u] : -1;
+                if (f[u] >= 0) p[u] = *reinterpret_cast<const Vec<T, V> *>(x + (int64_t)f[u] * ldx + ch);
             }
-            y[c * ldy + ch] = MAX ? Num<T>::from(acc) : mul_in<T>(Num<T>::from(acc), avg);
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                if (f[u] < 0) continue;
+#pragma unroll
+                for (int e = 0; e < V; ++e) {
+                    const A v = Num<T>::to(p[u].v[e]);
+                    if constexpr (MAX) {
+                        if constexpr (sizeof(A) == 8) acc[e] = fmax(v, acc[e]);
+                        else acc[e] = fmaxf(v, acc[e]);
+                    } else {
+                        acc[e] = acc[e] + v;
+                    }
+                }
+            }
         }
-        __syncwarp();
+        Vec<T, V> o;
+#pragma unroll
+        for (int e = 0; e < V; ++e) o.v[e] = SCALE ? mul_in<T>(Num<T>::from(acc[e]), avg) : Num<T>::from(acc[e]);
+        *reinterpret_cast<Vec<T, V> *>(y + c * ldy + ch) = o;
     }
 }
 
-// Max-pool gradient: per window and channel, grad to the first strict maximum, added into the
-// accumulation buffer dx (zero-initialised by the caller).
+// Max-pool gradient where no two windows overlap (stride >= window on every axis): each fine voxel
+// belongs to one window at most, so its row is written once -- the gradient where it holds the
+// window's first strict maximum, zero elsewhere -- without a buffer to add into.  Rows of voxels in
+// no window stay as the caller zeroed them.
+template <typename T, int V>
+__global__ void __launch_bounds__(kGroupThreads) maxpool_bwd_disjoint_kernel(FvgbGrid fine, FvgbGrid coarse, int3 pf,
+                                                                             int3 st, Groups gr,
+                                                                             const T *__restrict__ x, int64_t ldx,
+                                                                             int32_t C, const T *__restrict__ dy,
+                                                                             int64_t lddy, T *__restrict__ dx) {
+    using A = typename Num<T>::Acc;
+    extern __shared__ int32_t widx[];
+    const int G = 1 << gr.gs, group = threadIdx.x >> gr.gs, lane = threadIdx.x & (G - 1);
+    const int W = gr.W;
+    int32_t *idx = widx + group * W;
+    const int64_t c = (int64_t)blockIdx.x * (kGroupThreads >> gr.gs) + group;
+    const bool on = c < coarse.num_voxels;
+    int32_t b = 0;
+    int3 base = make_int3(0, 0, 0), ext = make_int3(0, 0, 0);
+    if (on) {
+        b = batch_of(coarse.voxel_offsets, coarse.num_grids, c);
+        base = make_int3(coarse.ijk[3 * c] * st.x, coarse.ijk[3 * c + 1] * st.y, coarse.ijk[3 * c + 2] * st.z);
+        ext = pf;
+    }
+    window_indices(fine, b, base, ext, idx, lane, G);
+    if (!on) return;
+    for (int32_t ch = lane * V; ch < C; ch += G * V) {
+        const Vec<T, V> g = *reinterpret_cast<const Vec<T, V> *>(dy + c * lddy + ch);
+        A best[V];
+        int32_t arg[V];
+#pragma unroll
+        for (int e = 0; e < V; ++e) best[e] = (A)(-INFINITY), arg[e] = -1;
+        for (int w0 = 0; w0 < W; w0 += kAhead) {
+            Vec<T, V> p[kAhead];
+            int32_t f[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                f[u] = w0 + u < W ? idx[w0 + u] : -1;
+                if (f[u] >= 0) p[u] = *reinterpret_cast<const Vec<T, V> *>(x + (int64_t)f[u] * ldx + ch);
+            }
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                if (f[u] < 0) continue;
+#pragma unroll
+                for (int e = 0; e < V; ++e) {
+                    const A v = Num<T>::to(p[u].v[e]);
+                    if (v > best[e]) best[e] = v, arg[e] = f[u];
+                }
+            }
+        }
+        for (int w = 0; w < W; ++w) {
+            const int32_t f = idx[w];
+            if (f < 0) continue;
+            Vec<T, V> o;
+#pragma unroll
+            for (int e = 0; e < V; ++e) o.v[e] = arg[e] == f ? g.v[e] : Num<T>::from((A)0);
+            *reinterpret_cast<Vec<T, V> *>(dx + (int64_t)f * C + ch) = o;
+        }
+    }
+}
+
+// Max-pool gradient of overlapping windows: per window and channel, grad to the first strict
+// maximum, added into the accumulation buffer dx (zero-initialised by the caller).
 template <typename T>
 __global__ void __launch_bounds__(kPoolWarps * 32) maxpool_bwd_kernel(FvgbGrid fine, FvgbGrid coarse, int3 pf, int3 st,
                                                                       const T *__restrict__ x, int64_t ldx, int32_t C,
@@ -128,7 +255,7 @@ __global__ void __launch_bounds__(kPoolWarps * 32) maxpool_bwd_kernel(FvgbGrid f
          c += (int64_t)gridDim.x * kPoolWarps) {
         const int32_t b = batch_of(coarse.voxel_offsets, coarse.num_grids, c);
         const int3 base = make_int3(coarse.ijk[3 * c] * st.x, coarse.ijk[3 * c + 1] * st.y, coarse.ijk[3 * c + 2] * st.z);
-        window_indices(fine, b, base, pf, widx[warp], lane);
+        window_indices(fine, b, base, pf, widx[warp], lane, 32);
         for (int ch = lane; ch < C; ch += 32) {
             A best = (A)(-INFINITY);
             int32_t arg = -1;
@@ -149,83 +276,94 @@ __global__ void __launch_bounds__(kPoolWarps * 32) maxpool_bwd_kernel(FvgbGrid f
 
 // Average-pool gradient, gathered per fine voxel: the coarse voxels whose window holds fine
 // voxel f are c with c*s <= f < c*s + p per axis.
-template <typename T>
-__global__ void __launch_bounds__(kPoolWarps * 32) avgpool_bwd_kernel(FvgbGrid fine, FvgbGrid coarse, int3 pf, int3 st,
-                                                                      int32_t C, const T *__restrict__ dy,
-                                                                      int64_t lddy, T *__restrict__ dx, int64_t lddx,
-                                                                      double avg) {
+template <typename T, int V>
+__global__ void __launch_bounds__(kGroupThreads) avgpool_bwd_kernel(FvgbGrid fine, FvgbGrid coarse, int3 pf, int3 st,
+                                                                    Groups gr, int32_t C, const T *__restrict__ dy,
+                                                                    int64_t lddy, T *__restrict__ dx, int64_t lddx,
+                                                                    double avg) {
     using A = typename Num<T>::Acc;
-    __shared__ int32_t widx[kPoolWarps][kMaxWindow];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    extern __shared__ int32_t widx[];
+    const int G = 1 << gr.gs, group = threadIdx.x >> gr.gs, lane = threadIdx.x & (G - 1);
+    int32_t *idx = widx + group * gr.W;
     auto fdiv = [](int32_t a, int32_t b) { return a >= 0 ? a / b : -((-a + b - 1) / b); };
-    for (int64_t f = (int64_t)blockIdx.x * kPoolWarps + warp; f < fine.num_voxels; f += (int64_t)gridDim.x * kPoolWarps) {
-        const int32_t b = batch_of(fine.voxel_offsets, fine.num_grids, f);
+    const int64_t f = (int64_t)blockIdx.x * (kGroupThreads >> gr.gs) + group;
+    const bool on = f < fine.num_voxels;
+    int32_t b = 0;
+    int3 lo = make_int3(0, 0, 0), ext = make_int3(0, 0, 0);
+    if (on) {
+        b = batch_of(fine.voxel_offsets, fine.num_grids, f);
         const int32_t fx = fine.ijk[3 * f], fy = fine.ijk[3 * f + 1], fz = fine.ijk[3 * f + 2];
         // candidate coarse range per axis: [ceil((f - p + 1) / s), floor(f / s)]
-        const int3 lo = make_int3(-fdiv(-(fx - pf.x + 1), st.x), -fdiv(-(fy - pf.y + 1), st.y), -fdiv(-(fz - pf.z + 1), st.z));
+        lo = make_int3(-fdiv(-(fx - pf.x + 1), st.x), -fdiv(-(fy - pf.y + 1), st.y), -fdiv(-(fz - pf.z + 1), st.z));
         const int3 hi = make_int3(fdiv(fx, st.x), fdiv(fy, st.y), fdiv(fz, st.z));
-        const int3 ext = make_int3(max(hi.x - lo.x + 1, 0), max(hi.y - lo.y + 1, 0), max(hi.z - lo.z + 1, 0));
-        const int W = ext.x * ext.y * ext.z;  // <= p0 p1 p2
-        window_indices(coarse, b, lo, ext, widx[warp], lane);
-        for (int ch = lane; ch < C; ch += 32) {
-            bool any = false;
-            A acc = (A)0;
-            for (int w = 0; w < W; ++w) {
-                const int32_t c = widx[warp][w];
-                if (c < 0) continue;
-                const T g = mul_in<T>(dy[(int64_t)c * lddy + ch], avg);
-                acc = any ? acc + Num<T>::to(g) : Num<T>::to(g);
-                any = true;
+        ext = make_int3(max(hi.x - lo.x + 1, 0), max(hi.y - lo.y + 1, 0), max(hi.z - lo.z + 1, 0));
+    }
+    const int W = ext.x * ext.y * ext.z;  // <= gr.W
+    window_indices(coarse, b, lo, ext, idx, lane, G);
+    if (!on) return;
+    for (int32_t ch = lane * V; ch < C; ch += G * V) {
+        bool any = false;
+        A acc[V];
+#pragma unroll
+        for (int e = 0; e < V; ++e) acc[e] = (A)0;
+        for (int w = 0; w < W; ++w) {
+            const int32_t c = idx[w];
+            if (c < 0) continue;
+            const Vec<T, V> p = *reinterpret_cast<const Vec<T, V> *>(dy + (int64_t)c * lddy + ch);
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+                const A g = Num<T>::to(mul_in<T>(p.v[e], avg));
+                acc[e] = any ? acc[e] + g : g;
             }
-            dx[f * lddx + ch] = Num<T>::from(acc);
+            any = true;
         }
-        __syncwarp();
+        Vec<T, V> o;
+#pragma unroll
+        for (int e = 0; e < V; ++e) o.v[e] = Num<T>::from(acc[e]);
+        *reinterpret_cast<Vec<T, V> *>(dx + f * lddx + ch) = o;
     }
 }
 
-// Nearest upsampling: fine voxel f copies coarse voxel floor(f / factor) (zero without one).
-template <typename T>
-__global__ void __launch_bounds__(kPoolWarps * 32) upsample_fwd_kernel(FvgbGrid coarse, FvgbGrid fine, int3 fac,
-                                                                       const T *__restrict__ x, int64_t ldx, int32_t C,
-                                                                       T *__restrict__ y, int64_t ldy) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// Nearest upsampling: fine voxel f copies coarse voxel floor(f / factor) (zero without one).  A warp
+// takes 32 consecutive fine voxels: each lane looks up one parent, then the warp's lane groups copy
+// the rows.
+template <typename T, int V>
+__global__ void __launch_bounds__(kGroupThreads) upsample_fwd_kernel(FvgbGrid coarse, FvgbGrid fine, int3 fac, int gs,
+                                                                     const T *__restrict__ x, int64_t ldx, int32_t C,
+                                                                     T *__restrict__ y, int64_t ldy) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int G = 1 << gs, sub = lane >> gs, gl = lane & (G - 1), per = 32 >> gs;
     auto fdiv = [](int32_t a, int32_t b) { return a >= 0 ? a / b : -((-a + b - 1) / b); };
-    for (int64_t f = (int64_t)blockIdx.x * kPoolWarps + warp; f < fine.num_voxels; f += (int64_t)gridDim.x * kPoolWarps) {
-        int64_t c = -1;
-        if (lane == 0) {
-            const int32_t b = batch_of(fine.voxel_offsets, fine.num_grids, f);
-            c = voxel_at(coarse, b, fdiv(fine.ijk[3 * f], fac.x), fdiv(fine.ijk[3 * f + 1], fac.y),
-                         fdiv(fine.ijk[3 * f + 2], fac.z));
-        }
-        c = __shfl_sync(0xffffffffu, c, 0);
-        for (int ch = lane; ch < C; ch += 32)
-            y[f * ldy + ch] = c >= 0 ? x[c * ldx + ch] : Num<T>::from(0.0f);
+    const int64_t f0 = ((int64_t)blockIdx.x * (kGroupThreads / 32) + warp) * 32;
+    if (f0 >= fine.num_voxels) return;  // warp-uniform
+    int32_t c = -1;
+    const int64_t fl = f0 + lane;
+    if (fl < fine.num_voxels) {
+        const int32_t b = batch_of(fine.voxel_offsets, fine.num_grids, fl);
+        c = (int32_t)voxel_at(coarse, b, fdiv(fine.ijk[3 * fl], fac.x), fdiv(fine.ijk[3 * fl + 1], fac.y),
+                              fdiv(fine.ijk[3 * fl + 2], fac.z));
     }
-}
-
-// Upsampling gradient: coarse voxel c sums its children c*factor + (i, j, k) (window order).
-template <typename T>
-__global__ void __launch_bounds__(kPoolWarps * 32) upsample_bwd_kernel(FvgbGrid coarse, FvgbGrid fine, int3 fac,
-                                                                       const T *__restrict__ dy, int64_t lddy, int32_t C,
-                                                                       T *__restrict__ dx, int64_t lddx) {
-    using A = typename Num<T>::Acc;
-    __shared__ int32_t widx[kPoolWarps][kMaxWindow];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int W = fac.x * fac.y * fac.z;
-    for (int64_t c = (int64_t)blockIdx.x * kPoolWarps + warp; c < coarse.num_voxels;
-         c += (int64_t)gridDim.x * kPoolWarps) {
-        const int32_t b = batch_of(coarse.voxel_offsets, coarse.num_grids, c);
-        const int3 base = make_int3(coarse.ijk[3 * c] * fac.x, coarse.ijk[3 * c + 1] * fac.y, coarse.ijk[3 * c + 2] * fac.z);
-        window_indices(fine, b, base, fac, widx[warp], lane);
-        for (int ch = lane; ch < C; ch += 32) {
-            A acc = (A)0;
-            for (int w = 0; w < W; ++w) {
-                const int32_t f = widx[warp][w];
-                if (f >= 0) acc += Num<T>::to(dy[(int64_t)f * lddy + ch]);
+    for (int i0 = 0; i0 < G; i0 += kAhead) {  // G = 32 / per rounds of `per` voxels, kAhead at a time
+        int32_t p[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) p[u] = __shfl_sync(0xffffffffu, c, ((i0 + u) * per + sub) & 31);
+        for (int32_t ch = gl * V; ch < C; ch += G * V) {
+            Vec<T, V> o[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                if (p[u] >= 0 && i0 + u < G) {
+                    o[u] = *reinterpret_cast<const Vec<T, V> *>(x + (int64_t)p[u] * ldx + ch);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < V; ++e) o[u].v[e] = Num<T>::from(0.0f);
+                }
             }
-            dx[c * lddx + ch] = Num<T>::from(acc);
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                const int64_t f = f0 + (i0 + u) * per + sub;
+                if (i0 + u < G && f < fine.num_voxels) *reinterpret_cast<Vec<T, V> *>(y + f * ldy + ch) = o[u];
+            }
         }
-        __syncwarp();
     }
 }
 
@@ -269,17 +407,41 @@ int dispatch_dtype(int32_t dtype, Args &&...args) {
     return launch_status();
 }
 
+// The vector width of rows of C channels at the given addresses and strides: 16 bytes where every
+// row is whole 16-byte pieces, else one element.
+template <typename T>
+bool whole_vectors(int32_t C, std::initializer_list<const void *> ptrs, std::initializer_list<int64_t> lds) {
+    constexpr int V = 16 / sizeof(T);
+    bool ok = C % V == 0;
+    for (const void *p : ptrs) ok = ok && ((uintptr_t)p & 15) == 0;
+    for (int64_t ld : lds) ok = ok && ld % V == 0;
+    return ok;
+}
+template <int V>
+using Width = std::integral_constant<int, V>;
+template <typename T, typename F>
+void by_width(bool vec, F &&f) {
+    if (vec) f(Width<16 / sizeof(T)>());
+    else f(Width<1>());
+}
+unsigned group_blocks(int64_t items, const Groups &g) { return (unsigned)ceil_div(items, (int64_t)(kGroupThreads >> g.gs)); }
+
 template <typename T>
 struct PoolFwd {
     static void run(int mode, const FvgbGrid &f, const FvgbGrid &c, int3 pf, int3 st, const void *x, int64_t ldx,
                     int32_t C, void *y, int64_t ldy, cudaStream_t s) {
         const double avg = 1.0 / ((double)pf.x * pf.y * pf.z);
-        if (mode == FVGB_POOL_MAX)
-            pool_fwd_kernel<T, true><<<pool_blocks(c.num_voxels), kPoolWarps * 32, 0, s>>>(
-                f, c, pf, st, (const T *)x, ldx, C, (T *)y, ldy, avg);
-        else
-            pool_fwd_kernel<T, false><<<pool_blocks(c.num_voxels), kPoolWarps * 32, 0, s>>>(
-                f, c, pf, st, (const T *)x, ldx, C, (T *)y, ldy, avg);
+        by_width<T>(whole_vectors<T>(C, {x, y}, {ldx, ldy}), [&](auto w) {
+            constexpr int V = decltype(w)::value;
+            const Groups g = groups_for(C / V, pf.x * pf.y * pf.z);
+            const unsigned blocks = group_blocks(c.num_voxels, g);
+            if (mode == FVGB_POOL_MAX)
+                window_reduce_kernel<T, V, true, false><<<blocks, kGroupThreads, g.smem, s>>>(
+                    f, c, pf, st, g, (const T *)x, ldx, C, (T *)y, ldy, avg);
+            else
+                window_reduce_kernel<T, V, false, true><<<blocks, kGroupThreads, g.smem, s>>>(
+                    f, c, pf, st, g, (const T *)x, ldx, C, (T *)y, ldy, avg);
+        });
     }
 };
 template <typename T>
@@ -291,28 +453,54 @@ struct MaxPoolBwd {
     }
 };
 template <typename T>
+struct MaxPoolBwdDisjoint {
+    static void run(const FvgbGrid &f, const FvgbGrid &c, int3 pf, int3 st, const void *x, int64_t ldx, int32_t C,
+                    const void *dy, int64_t lddy, void *dx, cudaStream_t s) {
+        by_width<T>(whole_vectors<T>(C, {x, dy, dx}, {ldx, lddy}), [&](auto w) {
+            constexpr int V = decltype(w)::value;
+            const Groups g = groups_for(C / V, pf.x * pf.y * pf.z);
+            maxpool_bwd_disjoint_kernel<T, V><<<group_blocks(c.num_voxels, g), kGroupThreads, g.smem, s>>>(
+                f, c, pf, st, g, (const T *)x, ldx, C, (const T *)dy, lddy, (T *)dx);
+        });
+    }
+};
+template <typename T>
 struct AvgPoolBwd {
     static void run(const FvgbGrid &f, const FvgbGrid &c, int3 pf, int3 st, int32_t C, const void *dy, int64_t lddy,
                     void *dx, int64_t lddx, cudaStream_t s) {
         const double avg = 1.0 / ((double)pf.x * pf.y * pf.z);
-        avgpool_bwd_kernel<T><<<pool_blocks(f.num_voxels), kPoolWarps * 32, 0, s>>>(f, c, pf, st, C, (const T *)dy,
-                                                                                      lddy, (T *)dx, lddx, avg);
+        // coarse voxels per axis whose window can hold one fine voxel
+        const int W = (int)(ceil_div(pf.x, st.x) * ceil_div(pf.y, st.y) * ceil_div(pf.z, st.z));
+        by_width<T>(whole_vectors<T>(C, {dy, dx}, {lddy, lddx}), [&](auto w) {
+            constexpr int V = decltype(w)::value;
+            const Groups g = groups_for(C / V, W);
+            avgpool_bwd_kernel<T, V><<<group_blocks(f.num_voxels, g), kGroupThreads, g.smem, s>>>(
+                f, c, pf, st, g, C, (const T *)dy, lddy, (T *)dx, lddx, avg);
+        });
     }
 };
 template <typename T>
 struct UpFwd {
     static void run(const FvgbGrid &c, const FvgbGrid &f, int3 fac, const void *x, int64_t ldx, int32_t C, void *y,
                     int64_t ldy, cudaStream_t s) {
-        upsample_fwd_kernel<T><<<pool_blocks(f.num_voxels), kPoolWarps * 32, 0, s>>>(c, f, fac, (const T *)x, ldx, C,
-                                                                                      (T *)y, ldy);
+        by_width<T>(whole_vectors<T>(C, {x, y}, {ldx, ldy}), [&](auto w) {
+            constexpr int V = decltype(w)::value;
+            const Groups g = groups_for(C / V, 1);
+            upsample_fwd_kernel<T, V><<<(unsigned)ceil_div(f.num_voxels, kGroupThreads), kGroupThreads, 0, s>>>(
+                c, f, fac, g.gs, (const T *)x, ldx, C, (T *)y, ldy);
+        });
     }
 };
 template <typename T>
 struct UpBwd {
     static void run(const FvgbGrid &c, const FvgbGrid &f, int3 fac, const void *dy, int64_t lddy, int32_t C, void *dx,
                     int64_t lddx, cudaStream_t s) {
-        upsample_bwd_kernel<T><<<pool_blocks(c.num_voxels), kPoolWarps * 32, 0, s>>>(c, f, fac, (const T *)dy, lddy, C,
-                                                                                      (T *)dx, lddx);
+        by_width<T>(whole_vectors<T>(C, {dy, dx}, {lddy, lddx}), [&](auto w) {
+            constexpr int V = decltype(w)::value;
+            const Groups g = groups_for(C / V, fac.x * fac.y * fac.z);
+            window_reduce_kernel<T, V, false, false><<<group_blocks(c.num_voxels, g), kGroupThreads, g.smem, s>>>(
+                f, c, fac, fac, g, (const T *)dy, lddy, C, (T *)dx, lddx, 1.0);
+        });
     }
 };
 
@@ -348,6 +536,21 @@ extern "C" int fvgb_maxpool_backward(int32_t dtype, const FvgbGrid *fine, const 
     return dispatch_dtype<MaxPoolBwd>(dtype, *fine, *coarse, make_int3(pool[0], pool[1], pool[2]),
                                       make_int3(stride[0], stride[1], stride[2]), x, ldx, C, dy, lddy, dx_acc,
                                       as_stream(stream));
+}
+
+extern "C" int fvgb_maxpool_backward_disjoint(int32_t dtype, const FvgbGrid *fine, const FvgbGrid *coarse,
+                                              const int32_t pool[3], const int32_t stride[3], const void *x, int64_t ldx,
+                                              int32_t C, const void *dy, int64_t lddy, void *dx, fvgb_stream_t stream) {
+    if (!grids_ok(fine, coarse) || !vec_ok(pool, kMaxWindow) || !vec_ok(stride, 1 << 30) || C < 1 || ldx < C ||
+        lddy < C)
+        return FVGB_EINVAL;
+    for (int a = 0; a < 3; ++a)
+        if (stride[a] < pool[a]) return FVGB_EINVAL;
+    if (coarse->num_voxels == 0 || fine->num_voxels == 0) return FVGB_OK;
+    if (!x || !dy || !dx) return FVGB_EINVAL;
+    return dispatch_dtype<MaxPoolBwdDisjoint>(dtype, *fine, *coarse, make_int3(pool[0], pool[1], pool[2]),
+                                              make_int3(stride[0], stride[1], stride[2]), x, ldx, C, dy, lddy, dx,
+                                              as_stream(stream));
 }
 
 extern "C" int fvgb_avgpool_backward(int32_t dtype, const FvgbGrid *fine, const FvgbGrid *coarse, const int32_t pool[3],

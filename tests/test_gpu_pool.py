@@ -125,3 +125,46 @@ def test_upsample_module_onto_user_grid(fvdb, cuda_device):
     assert out.grid.is_same(fine)
     # (1,1,1) has parent (0,0,0); (4,4,4) has none and reads zero
     assert out.data.jdata.cpu().tolist() == [[2.5, -1.0], [0.0, 0.0]]
+
+
+@pytest.mark.parametrize("c,dtype", [(1, torch.float32), (8, torch.float32), (24, torch.float64), (264, torch.float32),
+                                     (8, torch.bfloat16), (40, torch.float16), (20, torch.bfloat16), (272, torch.bfloat16)])
+@pytest.mark.parametrize("mode", ["max", "avg"])
+@pytest.mark.parametrize("pool,stride", [(2, 0), (3, 4), (8, 0)])
+def test_pool_and_upsampling_row_widths(fvdb, cuda_device, c, dtype, mode, pool, stride):
+    """Rows of one vector, of a lane group's vectors, of more than a warp's and of single elements;
+    windows of 8, 27 and 512; whole numbers, which every type adds exactly: equal to the oracle
+    (upsampling where the grids' factor is the pooling factor)."""
+    g, ijk, off = _grid(fvdb, cuda_device, n=700)
+    gen = torch.Generator().manual_seed(c)
+    x = torch.randint(-8, 9, (g.total_voxels, c), generator=gen).to(dtype)
+    if mode == "avg" and pool == 3:
+        x.zero_()  # 1/27 is not exact in 16 bits; zeros check the windows
+    xd = x.to(cuda_device).requires_grad_(True)
+    fn = g.max_pool if mode == "max" else g.avg_pool
+    y, cg = fn(pool, g.jagged_like(xd), stride=stride)
+    st = stride if stride else pool
+    cijk, coff = cg.ijk.jdata.cpu().numpy(), cg.joffsets.cpu().numpy()
+    ref = orc.pool_forward(ijk, off, cijk, coff, x.double().numpy(), pool, stride, mode)
+    assert np.array_equal(y.jdata.detach().double().cpu().numpy(), ref)
+    dy = torch.randint(-8, 9, y.jdata.shape, generator=gen).to(dtype)
+    y.jdata.backward(dy.to(cuda_device))
+    if not (mode == "avg" and pool == 3):
+        ref_dx = orc.pool_backward(ijk, off, cijk, coff, x.double().numpy(), dy.double().numpy(), pool, stride, mode)
+        assert np.array_equal(xd.grad.double().cpu().numpy(), ref_dx)
+    if stride:
+        return
+    z = dy.to(cuda_device).requires_grad_(True)
+    up, _ = cg.subdivide(pool, cg.jagged_like(z), fine_grid=g)
+    parent = torch.from_numpy(np.concatenate(
+        [np.full(off[b + 1] - off[b], b) for b in range(len(off) - 1)])).to(cuda_device)
+    key = torch.cat([parent[:, None], torch.div(g.ijk.jdata, pool, rounding_mode="floor")], 1)
+    ckey = torch.cat([cg.jidx.long()[:, None], cg.ijk.jdata], 1)
+    _, inv = torch.unique(torch.cat([ckey, key]), dim=0, return_inverse=True)
+    row = torch.empty(int(inv.max()) + 1, dtype=torch.long, device=cuda_device)
+    row[inv[:ckey.shape[0]]] = torch.arange(ckey.shape[0], device=cuda_device)
+    rows = row[inv[ckey.shape[0]:]]
+    assert torch.equal(up.jdata, z.detach()[rows])
+    ones = torch.ones_like(up.jdata)
+    up.jdata.backward(ones)
+    assert torch.equal(z.grad.double(), torch.bincount(rows, minlength=z.shape[0]).double()[:, None].expand_as(z))
