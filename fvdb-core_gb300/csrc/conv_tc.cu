@@ -205,23 +205,30 @@ extern "C" int fvgb_channel_absmax(int32_t dtype, const void *x, int64_t n, int3
 }
 
 // ---------------------------------------------------------------------------------------------
-// Tensor-core weight gradient (BF16 in, FP32 per-CTA partials, FP64 cross-CTA reduction):
+// Tensor-core weight gradient (BF16 / FP16 in, FP32 per-CTA partials, FP64 cross-CTA reduction):
 //
 //   dW[k, ci, co] = sum_m x[map[m,k], ci] * dy[m, co]
 //
 // A CTA owns a block of kernel offsets and a chunk of output rows.  The block's offsets form
-// sub-groups of G = 128 / c_in offsets (G x c_in = one M = 128 MMA, MN-major A) and every
-// sub-group accumulates in a TMEM accumulator of its own (512 / c_out of them, N = c_out
-// columns each).  So a 128-row tile of dy -- one TMA tile load per 64 channels, 128-byte
-// swizzle, straight into the MN-major B layout -- is loaded once and feeds every sub-group of
-// the block, and the tile's map rows (one bulk copy, K <= 32) feed every sub-group's gather.
+// sub-groups of G = 128 / slot offsets (slot = the power of two >= c_in; G x slot = one M = 128 MMA,
+// MN-major A, channels past c_in zero) and every sub-group accumulates in a TMEM accumulator of its
+// own (512 / BN of them, N = BN = c_out rounded up to 64, 128 or 256 columns each).  So a 128-row
+// tile of dy -- one TMA tile load per 64 channels, 128-byte swizzle, straight into the MN-major B
+// layout, zeros past c_out -- is loaded once and feeds every sub-group of the block, and the tile's
+// map rows (one bulk copy, K <= 32) feed every sub-group's gather.
+// Chunk c takes the tiles c, c + chunks, ...: over a row order neighbouring tiles have alike
+// sub-groups, and contiguous chunks would be unequal work.
+// Over a row order (ROWS) the tile's dy rows are scattered: the gather warps copy them too (their row
+// numbers come in with the map rows).  Rows of one occupancy share a tile then, and a tile has fewer sub-groups (0.8M
+// voxels of box faces, 64->64, 3^3: 545 us in index order with contiguous chunks, 318 us over the row order).
 // Per (tile, sub-group) the gather warps copy the sub-group's source rows into an A stage;
 // sub-groups with none of their offsets in the tile (per-tile occupancy mask) are skipped.
 // The epilogue writes the block's partial dW slice in FP32; a second kernel sums the partials
 // over chunks in FP64 in a fixed order (deterministic).
 //
 //   warps 0-7  gather the A operand with cp.async (lane -> 16-byte piece of four 128-byte MN
-//              atom rows per instruction), publish each stage one stage late; then the epilogue
+//              atom rows per instruction, zero fill for absent entries), published by asynchronous
+//              arrivals when the copies land; then the epilogue
 //   warp 8     MMA: owns the 512 TMEM columns; one elected lane issues, warp-uniform loop
 //   warp 9     loader: per active tile, the dy TMA loads and the map-row bulk copy (double-
 //              buffered, released by the tile's last MMA commit and the gather warps)
@@ -236,10 +243,6 @@ constexpr int kMNAtom = 16384;  // 128 K-rows x 128 bytes: one 64-element-wide M
 constexpr int kWgLoadWarp = kWgMmaWarp + 1;
 constexpr int kWgThreads = (kWgLoadWarp + 1) * 32;
 constexpr int kWgMaxMapK = 32;  // map tiles staged in shared memory up to K = 32
-
-__device__ __forceinline__ void st_shared_zero16(uint32_t addr) {
-    asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(addr), "r"(0) : "memory");
-}
 
 // MN-major operand, 128B swizzle: MN atoms (64 elements) kMNAtom apart (LBO), 8-row K groups
 // 1024 bytes apart (SBO).
@@ -267,16 +270,20 @@ struct WgArgs {
     int32_t K;
     const uint32_t *tile_mask;
     int32_t cout;
-    int32_t G;               // offsets per sub-group (128 / cin)
+    int32_t slot;            // MN elements per offset (power of two >= cin)
+    int32_t G;               // offsets per sub-group (128 / slot)
     int32_t offs_per_cta;    // offsets per block (a multiple of G)
-    int64_t rows_per_chunk;  // multiple of 128
     float *partials;         // [chunks][K][cin][cout]
     int32_t *err;
     int32_t stages;
     int32_t stage_map;
+    int32_t f16;             // 1: FP16 operands instead of BF16
+    const int32_t *rows;     // ROWS: output row of each map row (-1 = none)
+    const uint8_t *dy;       // ROWS: dy rows, lddy_bytes apart
+    int64_t lddy_bytes;
 };
 
-template <int BN>
+template <int BN, bool ROWS>
 __global__ void __launch_bounds__(kWgThreads, 1) conv_tc_wgrad_kernel(const __grid_constant__ CUtensorMap dy_map,
                                                                       WgArgs a) {
     extern __shared__ uint8_t smem_raw[];
@@ -287,8 +294,9 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv_tc_wgrad_kernel(const __gr
     uint8_t *dybuf = smem + S * kA;
     const int map_words = a.stage_map ? kTileM * a.K : 0;  // per buffer
     int32_t *map_sm = reinterpret_cast<int32_t *>(dybuf + 2 * kDy);
-    uint64_t *afull = reinterpret_cast<uint64_t *>(map_sm + 2 * map_words);
-    uint64_t *aempty = afull + S, *tfull = aempty + S, *tempty = tfull + 2, *accum = tempty + 2;
+    int32_t *rows_sm = map_sm + 2 * map_words;  // ROWS: [2][128]
+    uint64_t *afull = reinterpret_cast<uint64_t *>(rows_sm + (ROWS ? 2 * kTileM : 0));
+    uint64_t *aempty = afull + S, *tfull = aempty + S, *tempty = tfull + 2, *mfull = tempty + 2, *accum = mfull + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(accum + 1);
     volatile int *abort = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
@@ -297,18 +305,21 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv_tc_wgrad_kernel(const __gr
     const int k0 = blockIdx.x * a.offs_per_cta;
     const int k_end = min(a.K, k0 + a.offs_per_cta);
     const int nsg = (k_end - k0 + G - 1) / G;  // sub-groups of this block, <= 512 / BN
-    const int64_t r_begin = (int64_t)blockIdx.y * a.rows_per_chunk;
-    const int64_t r_end = min(a.n_out, r_begin + a.rows_per_chunk);
-    const int64_t t_begin = r_begin / kTileM;
-    const int64_t n_tiles = (r_end - r_begin + kTileM - 1) / kTileM;
+    // tile t of this chunk is tile blockIdx.y + t * gridDim.y of the map
+    const int64_t all_tiles = (a.n_out + kTileM - 1) / kTileM;
+    const int64_t n_tiles = (all_tiles - blockIdx.y + gridDim.y - 1) / gridDim.y;
+    auto tile_of = [&](int64_t t) { return (int64_t)blockIdx.y + t * gridDim.y; };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) {
-            mbar_init(&afull[s], kWgGatherWarps);  // one arrival per gather warp
+            mbar_init(&afull[s], kWgGatherWarps * 32);  // each gather thread, when its copies have landed
             mbar_init(&aempty[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
-            mbar_init(&tfull[b], 1);
+            // the tile's dy: the loader's expect_tx, or (ROWS) each gather thread; its map rows come in
+            // with dy, or (ROWS) with the row numbers on mfull
+            mbar_init(&tfull[b], ROWS ? kWgGatherWarps * 32 : 1);
+            mbar_init(&mfull[b], 1);
             mbar_init(&tempty[b], 1 + kWgGatherWarps);  // the tile's last MMA commit + each gather warp
         }
         mbar_init(accum, 1);
@@ -324,7 +335,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv_tc_wgrad_kernel(const __gr
     auto groups_of = [&](int64_t t) -> uint32_t {
         const uint32_t all = (1u << nsg) - 1u;
         if (!a.tile_mask || a.K > 32) return all;
-        const uint32_t m = __ldg(a.tile_mask + t_begin + t);
+        const uint32_t m = __ldg(a.tile_mask + tile_of(t));
         uint32_t r = 0;
         for (int g = 0; g < nsg; ++g) {
             const int kk = k0 + g * G, cnt = min(G, a.K - kk);
@@ -343,10 +354,16 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv_tc_wgrad_kernel(const __gr
 #pragma unroll
         for (int at = 0; at < 2; ++at) {
             const int m0 = at * 64 + jj * 8;
-            joff[at] = m0 / a.cin;
-            ci0[at] = m0 - joff[at] * a.cin;
+            joff[at] = m0 / a.slot;
+            ci0[at] = m0 - joff[at] * a.slot;
         }
-        uint32_t it = 0, sig = 0, stage = 0, phase = 0, pstage = 0, seen = 0;
+        // place of the lane's first row in an atom (rows 4 apart take the two halves of the swizzle
+        // pattern in turn), its source columns, and 32-bit row arithmetic: -1 is past every row count
+        const uint32_t even = mn_offset(row0 + rsub, jj * 8), odd = even ^ 64u;
+        const uint8_t *xcol[2] = {a.x + ci0[0] * 2, a.x + ci0[1] * 2};
+        const uint32_t nx32 = (uint32_t)a.n_x, ldx32 = (uint32_t)a.ldx_bytes, nout32 = (uint32_t)a.n_out,
+                       lddy32 = (uint32_t)a.lddy_bytes;
+        uint32_t stage = 0, phase = 0, seen = 0;
         int i = 0;
         bool ok = true;
         for (int64_t t = 0; t < n_tiles && ok && !*abort; ++t) {
@@ -354,58 +371,60 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv_tc_wgrad_kernel(const __gr
             if (!gm) continue;
             seen |= gm;
             const int b = i & 1;
-            if (a.stage_map && !mbar_wait_warp(&tfull[b], (i >> 1) & 1, abort)) break;
+            if (ROWS) {
+                if (!mbar_wait_warp(&mfull[b], (i >> 1) & 1, abort)) break;
+                // this warp's 16 dy rows
+                const uint32_t base = smem_u32(dybuf + b * kDy);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const uint32_t src = (uint32_t)rows_sm[b * kTileM + row0 + rsub + 4 * q];
+                    const uint8_t *row = a.dy + (uint64_t)src * lddy32 + jj * 16;
+#pragma unroll
+                    for (int at = 0; at < BN / 64; ++at) {
+                        const bool present = src < nout32 && at * 64 + jj * 8 < a.cout;
+                        cp_async_16(base + at * kMNAtom + q * 512 + (q & 1 ? odd : even), present ? row + at * 128 : a.dy,
+                                    present ? 16u : 0u);
+                    }
+                }
+                cp_async_arrive_noinc(&tfull[b]);
+            } else if (a.stage_map && !mbar_wait_warp(&tfull[b], (i >> 1) & 1, abort)) {
+                break;
+            }
             const int32_t *mt = map_sm + b * map_words;
-            const int64_t mrow0 = r_begin + t * kTileM;
+            const int64_t mrow0 = tile_of(t) * kTileM;
             while (gm) {
                 const int g = __ffs(gm) - 1;
                 gm &= gm - 1;
-                int32_t src[2][4];
+                uint32_t src[2][4];
 #pragma unroll
-                for (int at = 0; at < 2; ++at)
+                for (int at = 0; at < 2; ++at) {
+                    const int k = k0 + g * G + joff[at];
+                    const bool on = k < k_end && ci0[at] < a.cin;
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         const int r = row0 + rsub + 4 * q;
-                        const int k = k0 + g * G + joff[at];
                         int32_t v = -1;
-                        if (k < k_end) {
-                            v = a.stage_map ? mt[r * a.K + k] : a.map[(mrow0 + r) * a.K + k];
-                            if (v >= a.n_x) v = -1;
-                        }
-                        src[at][q] = v;
+                        if (on) v = a.stage_map ? mt[r * a.K + k] : a.map[(mrow0 + r) * a.K + k];
+                        src[at][q] = (uint32_t)v;
                     }
+                }
                 if (!mbar_wait_warp(&aempty[stage], phase ^ 1, abort)) {
                     ok = false;
                     break;
                 }
                 const uint32_t base = smem_u32(smem + stage * kA);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int r = row0 + rsub + 4 * q;
+                for (int q = 0; q < 4; ++q)
 #pragma unroll
                     for (int at = 0; at < 2; ++at) {
-                        const uint32_t dst = base + mn_offset(r, at * 64 + jj * 8);
-                        if (src[at][q] >= 0)
-                            cp_async_16(dst, a.x + (int64_t)src[at][q] * a.ldx_bytes + ci0[at] * 2, 16u);
-                        else
-                            st_shared_zero16(dst);
+                        const bool present = src[at][q] < nx32;
+                        cp_async_16(base + at * kMNAtom + q * 512 + (q & 1 ? odd : even),
+                                    present ? xcol[at] + (uint64_t)src[at][q] * ldx32 : a.x, present ? 16u : 0u);
                     }
-                }
-                // cp.async and st.shared are generic-proxy writes: each warp fences its own
-                // copies to the tensor core (async proxy), one stage late
-                cp_async_commit();
-                ++it;
+                cp_async_arrive_noinc(&afull[stage]);
                 if (++stage == (uint32_t)S) {
                     stage = 0;
                     phase ^= 1;
-                }
-                if (it - sig > 1) {
-                    cp_async_wait_group<1>();
-                    fence_proxy_async();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&afull[pstage]);
-                    ++sig;
-                    if (++pstage == (uint32_t)S) pstage = 0;
                 }
             }
             // the tile's map rows were read into registers: release its buffers (with the MMA)
@@ -413,24 +432,17 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv_tc_wgrad_kernel(const __gr
             if (lane == 0) mbar_arrive(&tempty[b]);
             ++i;
         }
-        cp_async_wait_group<0>();
-        fence_proxy_async();
-        __syncwarp();
-        if (lane == 0)
-            for (; sig < it; ++sig) {
-                mbar_arrive(&afull[pstage]);
-                if (++pstage == (uint32_t)S) pstage = 0;
-            }
+        cp_async_wait_all();
 
         // ---------------------------------------------------------------- epilogue
         const bool have = __all_sync(0xffffffffu, mbar_wait(accum, 0, abort) && !*abort);
         tc_fence_after();
         const int lg = warp & 3;
         const int row = lg * 32 + lane;  // M index = j * cin + ci
-        const int j = row / a.cin, ci = row % a.cin;
+        const int j = row / a.slot, ci = row % a.slot;
         for (int g = warp >> 2; g < nsg; g += 2) {
             const int k = k0 + g * G + j;
-            const bool mine = have && k < k_end;
+            const bool mine = have && k < k_end && ci < a.cin;
             const bool live = have && ((seen >> g) & 1u);  // warp-uniform
             float *dst = a.partials + (((int64_t)blockIdx.y * a.K + k) * a.cin + ci) * a.cout;
 #pragma unroll 1
@@ -445,13 +457,14 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv_tc_wgrad_kernel(const __gr
                 if (mine) {
 #pragma unroll
                     for (int e = 0; e < 16; e += 4)
-                        *reinterpret_cast<float4 *>(dst + c0 + e) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+                        if (c0 + e < a.cout)  // c_out is a multiple of 8
+                            *reinterpret_cast<float4 *>(dst + c0 + e) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
                 }
             }
         }
     } else if (warp == kWgMmaWarp) {
         // the whole warp runs the issue loop (warp-uniform); one elected lane issues each tcgen05 op
-        constexpr uint32_t idesc = idesc_m128(BN, 1, 1) | (1u << 15) | (1u << 16);  // bf16, A and B MN-major
+        const uint32_t idesc = (a.f16 ? idesc_m128(BN, 0, 0) : idesc_m128(BN, 1, 1)) | (1u << 15) | (1u << 16);  // A and B MN-major
         uint32_t inited = 0;
         int it = 0, i = 0;
         bool ok = true;
@@ -469,6 +482,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv_tc_wgrad_kernel(const __gr
                     ok = false;
                     break;
                 }
+                fence_proxy_async();  // the gather threads' copies, seen through the barriers -> tensor core
                 tc_fence_after();
                 const uint32_t As = smem_u32(smem + stage * kA);
                 const uint32_t d = tmem + (uint32_t)(g * BN);
@@ -492,25 +506,29 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv_tc_wgrad_kernel(const __gr
             mbar_arrive_warp(accum);
     } else {
         // ---------------------------------------------------------------- loader
+        const uint32_t map_bytes = (uint32_t)map_words * 4;
         if (lane == 0) {
-            const uint32_t map_bytes = (uint32_t)map_words * 4;
             int i = 0;
             for (int64_t t = 0; t < n_tiles && !*abort; ++t) {
                 if (!groups_of(t)) continue;
                 const int b = i & 1;
                 if (!mbar_wait_backoff(&tempty[b], ((i >> 1) & 1) ^ 1, abort, 64)) break;
-                const int64_t m0 = r_begin + t * kTileM;
-                mbar_arrive_expect_tx(&tfull[b], (uint32_t)kDy + map_bytes);
+                const int64_t m0 = tile_of(t) * kTileM;
+                uint64_t *full = ROWS ? &mfull[b] : &tfull[b];
+                mbar_arrive_expect_tx(full, (ROWS ? kTileM * 4u : (uint32_t)kDy) + map_bytes);
+                if (ROWS)
+                    bulk_g2s(smem_u32(rows_sm + b * kTileM), a.rows + m0, kTileM * 4, full);
+                else
 #pragma unroll
-                for (int at = 0; at < BN / 64; ++at)
-                    tma_load_2d(smem_u32(dybuf + b * kDy + at * kMNAtom), &dy_map, at * 64, (int32_t)m0, &tfull[b]);
-                if (map_bytes) bulk_g2s(smem_u32(map_sm + b * map_words), a.map + m0 * a.K, map_bytes, &tfull[b]);
+                    for (int at = 0; at < BN / 64; ++at)
+                        tma_load_2d(smem_u32(dybuf + b * kDy + at * kMNAtom), &dy_map, at * 64, (int32_t)m0, full);
+                if (map_bytes) bulk_g2s(smem_u32(map_sm + b * map_words), a.map + m0 * a.K, map_bytes, full);
                 ++i;
             }
             // the copies issued last land before the CTA exits (bounded: ~30 ms)
             for (int j = i > 2 ? i - 2 : 0; j < i; ++j) {
                 int give_up = 0;
-                mbar_wait_budget(&tfull[j & 1], (j >> 1) & 1, &give_up, 1ll << 26);
+                mbar_wait_budget(ROWS ? &mfull[j & 1] : &tfull[j & 1], (j >> 1) & 1, &give_up, 1ll << 26);
             }
         }
         __syncwarp();
@@ -529,21 +547,25 @@ __global__ void wgrad_reduce_f64_kernel(const float *__restrict__ partials, int6
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= per_chunk) return;
     double s = 0.0;
+#pragma unroll 16  // loads in flight; the sum keeps its order
     for (int64_t c = 0; c < chunks; ++c) s += (double)partials[c * per_chunk + e];
     dw[e] = (float)s;
 }
 
 struct TcWgradPlan {
-    int64_t blocks, chunks, rows_per_chunk;
-    int32_t G, offs_per_cta;
+    int64_t blocks, chunks;
+    int32_t slot, G, offs_per_cta, BN;
 };
 
-// Offset blocks of balanced sub-group counts (<= 512 / c_out accumulators each), then row chunks
+// Offset blocks of balanced sub-group counts (<= 512 / BN accumulators each), then row chunks
 // so that blocks x chunks fills the SMs once.
 TcWgradPlan tc_wgrad_plan(int64_t n_out, int32_t K, int32_t cin, int32_t cout) {
     TcWgradPlan p;
-    p.G = 128 / cin;
-    const int64_t subgroups = ceil_div(K, p.G), per_block_max = 512 / cout;
+    p.slot = 8;
+    while (p.slot < cin) p.slot *= 2;
+    p.BN = cout <= 64 ? 64 : (cout <= 128 ? 128 : 256);
+    p.G = 128 / p.slot;
+    const int64_t subgroups = ceil_div(K, p.G), per_block_max = 512 / p.BN;
     const int64_t blocks0 = ceil_div(subgroups, per_block_max);
     p.offs_per_cta = (int32_t)(ceil_div(subgroups, blocks0) * p.G);
     p.blocks = ceil_div(K, p.offs_per_cta);
@@ -551,8 +573,7 @@ TcWgradPlan tc_wgrad_plan(int64_t n_out, int32_t K, int32_t cin, int32_t cout) {
     int64_t chunks = ceil_div(device_sm_count(), p.blocks);
     if (chunks > tiles) chunks = tiles;
     if (chunks < 1) chunks = 1;
-    p.rows_per_chunk = ceil_div(tiles, chunks) * kTileM;
-    p.chunks = ceil_div(n_out > 0 ? n_out : 1, p.rows_per_chunk);
+    p.chunks = chunks;
     return p;
 }
 
@@ -575,17 +596,17 @@ EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-template <int BN>
+template <int BN, bool ROWS>
 int launch_wgrad(const CUtensorMap &dy_map, WgArgs a, int64_t blocks, int64_t chunks, cudaStream_t s) {
     constexpr int kA = 2 * kMNAtom, kDy = (BN / 64) * kMNAtom;
     const int map_bytes = a.stage_map ? 2 * kTileM * a.K * 4 : 0;
-    const int extra = 1024 + map_bytes + (2 * 4 + 4 + 1) * 8 + 16;
+    const int extra = 1024 + map_bytes + (ROWS ? 2 * kTileM * 4 : 0) + (2 * 4 + 6 + 1) * 8 + 16;
     int stages = 4;
     while (stages > 2 && stages * kA + 2 * kDy + extra > 227 * 1024) --stages;
     if (stages * kA + 2 * kDy + extra > 227 * 1024) return FVGB_EINVAL;
     a.stages = stages;
     const int smem = stages * kA + 2 * kDy + extra;
-    auto kern = conv_tc_wgrad_kernel<BN>;
+    auto kern = conv_tc_wgrad_kernel<BN, ROWS>;
     if (set_dynamic_smem(kern, smem) != cudaSuccess)
         return launch_status();
     kern<<<dim3((unsigned)blocks, (unsigned)chunks), kWgThreads, smem, s>>>(dy_map, a);
@@ -595,50 +616,57 @@ int launch_wgrad(const CUtensorMap &dy_map, WgArgs a, int64_t blocks, int64_t ch
 }  // namespace
 }  // namespace fvgb
 
-extern "C" int fvgb_tc_wgrad_workspace(int64_t n_out, int32_t K, int32_t c_in, int32_t c_out, size_t *bytes) {
-    if (!bytes || K < 1 || n_out < 0 || (c_in != 32 && c_in != 64 && c_in != 128) ||
-        (c_out != 64 && c_out != 128 && c_out != 256))
-        return FVGB_EINVAL;
-    const TcWgradPlan p = tc_wgrad_plan(n_out, K, c_in, c_out);
-    *bytes = (size_t)p.chunks * K * c_in * c_out * 4 + 256;
-    return FVGB_OK;
+namespace fvgb {
+namespace {
+
+bool wgrad_shape_ok(int32_t c_in, int32_t c_out) {
+    return c_in >= 8 && c_in <= 128 && c_in % 8 == 0 && c_out >= 8 && c_out <= 256 && c_out % 8 == 0;
 }
 
-extern "C" int fvgb_conv_wgrad_tc(const void *x, int64_t n_x, int32_t c_in, int64_t ldx, const int32_t *map,
-                                  int64_t n_out, int32_t K, const uint32_t *tile_mask, const void *dy, int32_t c_out,
-                                  int64_t lddy, float *dw, void *workspace, size_t workspace_bytes, int32_t *err_dev,
-                                  fvgb_stream_t stream) {
-    size_t need = 0;
-    int st = fvgb_tc_wgrad_workspace(n_out, K, c_in, c_out, &need);
-    if (st) return st;
+size_t wgrad_bytes(int64_t n_out, int32_t K, int32_t c_in, int32_t c_out) {
+    return (size_t)tc_wgrad_plan(n_out, K, c_in, c_out).chunks * K * c_in * c_out * 4 + 256;
+}
+
+int conv_wgrad(bool f16, const void *x, int64_t n_x, int32_t c_in, int64_t ldx, const int32_t *map, int64_t n_out,
+               int32_t K, const int32_t *rows, const uint32_t *tile_mask, const void *dy, int32_t c_out, int64_t lddy,
+               float *dw, void *workspace, size_t workspace_bytes, int32_t *err_dev, fvgb_stream_t stream) {
     if (!dw || !err_dev || ldx < c_in || lddy < c_out || (ldx % 8) || (lddy % 8) || n_x < 0) return FVGB_EINVAL;
     if (n_out > 0 && (!map || !dy)) return FVGB_EINVAL;
     if (n_out > INT32_MAX - kTileM) return FVGB_EINVAL;
-    if (!workspace || workspace_bytes < need) return FVGB_ENOSPACE;
-    if (((uintptr_t)x & 15) || ((uintptr_t)dy & 15) || ((uintptr_t)map & 15)) return FVGB_EINVAL;
+    // map entries are int32, so no more input rows can be named; row strides are 32-bit in the kernel
+    n_x = std::min<int64_t>(n_x, INT32_MAX);
+    if (n_x <= 1) ldx = c_in;
+    if (n_out <= 1) lddy = c_out;
+    if (ldx * 2 > UINT32_MAX || lddy * 2 > UINT32_MAX) return FVGB_EINVAL;
+    if (!workspace || workspace_bytes < wgrad_bytes(n_out, K, c_in, c_out)) return FVGB_ENOSPACE;
+    if (((uintptr_t)x & 15) || ((uintptr_t)dy & 15) || ((uintptr_t)map & 15) || ((uintptr_t)rows & 15)) return FVGB_EINVAL;
     const TcWgradPlan p = tc_wgrad_plan(n_out, K, c_in, c_out);
     cudaStream_t s = as_stream(stream);
     float *part = reinterpret_cast<float *>(((uintptr_t)workspace + 255) & ~(uintptr_t)255);
     const int64_t per_chunk = (int64_t)K * c_in * c_out;
     int launched = 0;
     if (n_out > 0) {
-        // dy as a 2-D tensor [n_out rows, c_out channels], boxes of 128 rows x 64 channels,
-        // 128-byte swizzle: each box is one MN atom of the B operand; rows past n_out read zero
-        EncodeTiledFn enc = encode_tiled();
-        if (!enc) {
-            record_message("cuTensorMapEncodeTiled is not available from the CUDA driver");
-            return FVGB_ECUDA;
-        }
-        CUtensorMap dy_map;
-        const cuuint64_t gdim[2] = {(cuuint64_t)c_out, (cuuint64_t)n_out};
-        const cuuint64_t gstride[1] = {(cuuint64_t)lddy * 2};
-        const cuuint32_t box[2] = {64, (cuuint32_t)kTileM};
-        const cuuint32_t estride[2] = {1, 1};
-        if (enc(&dy_map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(dy), gdim, gstride, box, estride,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
-            record_message("cuTensorMapEncodeTiled rejected the dy tensor");
-            return FVGB_EINVAL;
+        CUtensorMap dy_map = {};
+        if (!rows) {
+            // dy as a 2-D tensor [n_out rows, c_out channels], boxes of 128 rows x 64 channels,
+            // 128-byte swizzle: each box is one MN atom of the B operand; rows past n_out and
+            // channels past c_out read zero
+            EncodeTiledFn enc = encode_tiled();
+            if (!enc) {
+                record_message("cuTensorMapEncodeTiled is not available from the CUDA driver");
+                return FVGB_ECUDA;
+            }
+            const cuuint64_t gdim[2] = {(cuuint64_t)c_out, (cuuint64_t)n_out};
+            const cuuint64_t gstride[1] = {(cuuint64_t)lddy * 2};
+            const cuuint32_t box[2] = {64, (cuuint32_t)kTileM};
+            const cuuint32_t estride[2] = {1, 1};
+            if (enc(&dy_map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+                    const_cast<void *>(dy), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+                record_message("cuTensorMapEncodeTiled rejected the dy tensor");
+                return FVGB_EINVAL;
+            }
         }
         WgArgs a;
         a.x = (const uint8_t *)(n_x > 0 ? x : dy);
@@ -650,18 +678,31 @@ extern "C" int fvgb_conv_wgrad_tc(const void *x, int64_t n_x, int32_t c_in, int6
         a.K = K;
         a.tile_mask = tile_mask;
         a.cout = c_out;
+        a.slot = p.slot;
         a.G = p.G;
         a.offs_per_cta = p.offs_per_cta;
-        a.rows_per_chunk = p.rows_per_chunk;
         a.partials = part;
         a.err = err_dev;
         a.stages = 0;
         a.stage_map = K <= kWgMaxMapK ? 1 : 0;
+        a.f16 = f16 ? 1 : 0;
+        a.rows = rows;
+        a.dy = (const uint8_t *)dy;
+        a.lddy_bytes = lddy * 2;
         if (p.chunks > 65535 || p.blocks > 65535) return FVGB_EINVAL;
-        switch (c_out) {
-            case 64: st = launch_wgrad<64>(dy_map, a, p.blocks, p.chunks, s); break;
-            case 128: st = launch_wgrad<128>(dy_map, a, p.blocks, p.chunks, s); break;
-            default: st = launch_wgrad<256>(dy_map, a, p.blocks, p.chunks, s); break;
+        int st;
+        switch (p.BN) {
+            case 64:
+                st = rows ? launch_wgrad<64, true>(dy_map, a, p.blocks, p.chunks, s)
+                          : launch_wgrad<64, false>(dy_map, a, p.blocks, p.chunks, s);
+                break;
+            case 128:
+                st = rows ? launch_wgrad<128, true>(dy_map, a, p.blocks, p.chunks, s)
+                          : launch_wgrad<128, false>(dy_map, a, p.blocks, p.chunks, s);
+                break;
+            default:
+                st = rows ? launch_wgrad<256, true>(dy_map, a, p.blocks, p.chunks, s)
+                          : launch_wgrad<256, false>(dy_map, a, p.blocks, p.chunks, s);
         }
         if (st) return st;
         launched = 1;
@@ -670,6 +711,47 @@ extern "C" int fvgb_conv_wgrad_tc(const void *x, int64_t n_x, int32_t c_in, int6
                                                                                per_chunk, dw);
     count_launches(launched + 1);
     return launch_status();
+}
+
+}  // namespace
+}  // namespace fvgb
+
+extern "C" int fvgb_tc_wgrad_workspace(int64_t n_out, int32_t K, int32_t c_in, int32_t c_out, size_t *bytes) {
+    if (!bytes || K < 1 || n_out < 0 || (c_in != 32 && c_in != 64 && c_in != 128) ||
+        (c_out != 64 && c_out != 128 && c_out != 256))
+        return FVGB_EINVAL;
+    *bytes = wgrad_bytes(n_out, K, c_in, c_out);
+    return FVGB_OK;
+}
+
+extern "C" int fvgb_conv_wgrad_tc(const void *x, int64_t n_x, int32_t c_in, int64_t ldx, const int32_t *map,
+                                  int64_t n_out, int32_t K, const uint32_t *tile_mask, const void *dy, int32_t c_out,
+                                  int64_t lddy, float *dw, void *workspace, size_t workspace_bytes, int32_t *err_dev,
+                                  fvgb_stream_t stream) {
+    size_t need = 0;
+    const int st = fvgb_tc_wgrad_workspace(n_out, K, c_in, c_out, &need);
+    if (st) return st;
+    return conv_wgrad(false, x, n_x, c_in, ldx, map, n_out, K, nullptr, tile_mask, dy, c_out, lddy, dw, workspace,
+                      workspace_bytes, err_dev, stream);
+}
+
+extern "C" int fvgb_tc_wgrad_16bit_workspace(int64_t n_out, int32_t K, int32_t c_in, int32_t c_out, size_t *bytes) {
+    if (!bytes || K < 1 || n_out < 0 || !wgrad_shape_ok(c_in, c_out)) return FVGB_EINVAL;
+    *bytes = wgrad_bytes(n_out, K, c_in, c_out);
+    return FVGB_OK;
+}
+
+extern "C" int fvgb_conv_wgrad_tc_16bit(int32_t dtype, const void *x, int64_t n_x, int32_t c_in, int64_t ldx,
+                                        const int32_t *map, int64_t n_out, int32_t K, const int32_t *rows,
+                                        const uint32_t *tile_mask, const void *dy, int32_t c_out, int64_t lddy,
+                                        float *dw, void *workspace, size_t workspace_bytes, int32_t *err_dev,
+                                        fvgb_stream_t stream) {
+    size_t need = 0;
+    const int st = fvgb_tc_wgrad_16bit_workspace(n_out, K, c_in, c_out, &need);
+    if (st) return st;
+    if (dtype != FVGB_BF16 && dtype != FVGB_F16) return FVGB_ETYPE;
+    return conv_wgrad(dtype == FVGB_F16, x, n_x, c_in, ldx, map, n_out, K, rows, tile_mask, dy, c_out, lddy, dw,
+                      workspace, workspace_bytes, err_dev, stream);
 }
 
 namespace fvgb {

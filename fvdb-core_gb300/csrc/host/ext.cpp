@@ -743,6 +743,13 @@ std::optional<RowOrder> pack_row_order(PackPtr p, bool transposed) {
     return RowOrder{*p->order_rows[d], *p->order_mask[d], *p->order_map[d]};
 }
 
+// The row order if some contraction has built it.
+std::optional<RowOrder> built_row_order(const PackPtr &p, bool transposed) {
+    const int d = transposed ? 1 : 0;
+    if (!p->order_rows[d]) return std::nullopt;
+    return RowOrder{*p->order_rows[d], *p->order_mask[d], *p->order_map[d]};
+}
+
 // The row order for a tensor-core contraction once it is worth building: building it costs about
 // 0.19 ms for 1.08M rows x 27 (a sort and a permuted copy of the map), so the first tensor-core
 // contraction over a map runs in index order and the order serves the second and later ones
@@ -1111,25 +1118,35 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
 }
 
 // dW[k] = sum_m x[map[m,k]]^T dy[m]   -> [K, Cin, Cout]
+// order (optional): the map's row order, which the tensor-core form runs over where it exists.
 Tensor gather_wgrad(const Tensor &x, const Tensor &map, int64_t n_out, const Tensor &dy, int64_t K,
-                    const std::optional<Tensor> &tile_mask = std::nullopt) {
+                    const std::optional<Tensor> &tile_mask = std::nullopt,
+                    const std::optional<RowOrder> &order = std::nullopt) {
     c10::cuda::CUDAGuard guard(x.device());
     const int64_t cin = x.size(1), cout = dy.size(1);
-    if (x.scalar_type() == torch::kBFloat16 && (cin == 32 || cin == 64 || cin == 128) &&
-        (cout == 64 || cout == 128 || cout == 256)) {
-        // tensor cores: FP32 partials per CTA, FP64 reduction across CTAs
-        Tensor xx = x.contiguous(), dd = dy.to(torch::kBFloat16).contiguous();
+    const auto dtype = x.scalar_type();
+    // tensor cores: 16-bit operands of whole 16-byte pieces; FP32 partials per CTA, FP64 reduction
+    // across CTAs (the CUDA cores converted both operands to FP32 first)
+    if ((dtype == torch::kBFloat16 || dtype == torch::kFloat16) && cin % 8 == 0 && cin <= 128 && cout % 8 == 0 &&
+        cout <= 256) {
+        Tensor xx = x.contiguous(), dd = dy.to(dtype).contiguous();
+        auto aligned = [](const Tensor &t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0 ? t : t.clone(); };
+        xx = aligned(xx);
+        dd = aligned(dd);
         Tensor dw = torch::empty({K, cin, cout}, x.options().dtype(torch::kFloat32));
         size_t wsb = 0;
-        check_status(fvgb_tc_wgrad_workspace(n_out, (int32_t)K, (int32_t)cin, (int32_t)cout, &wsb), "wgrad workspace");
+        check_status(fvgb_tc_wgrad_16bit_workspace(n_out, (int32_t)K, (int32_t)cin, (int32_t)cout, &wsb), "wgrad workspace");
         Tensor ws = workspace(wsb, x.device());
-        const uint32_t *tm = tile_mask ? reinterpret_cast<const uint32_t *>(tile_mask->data_ptr<int32_t>()) : nullptr;
-        check_status(fvgb_conv_wgrad_tc(xx.data_ptr(), xx.size(0), (int32_t)cin, xx.stride(0), map.data_ptr<int32_t>(),
-                                        n_out, (int32_t)K, tm, dd.data_ptr(), (int32_t)cout, dd.stride(0),
-                                        dw.data_ptr<float>(), ws.data_ptr(), ws.numel(),
-                                        device_error_flag(x.device()).data_ptr<int32_t>(), cur_stream()),
+        const std::optional<Tensor> mask = order ? std::optional<Tensor>(order->mask) : tile_mask;
+        const uint32_t *tm = mask ? reinterpret_cast<const uint32_t *>(mask->data_ptr<int32_t>()) : nullptr;
+        check_status(fvgb_conv_wgrad_tc_16bit(fvgb_dtype(xx), xx.data_ptr(), xx.size(0), (int32_t)cin, xx.stride(0),
+                                              (order ? order->map : map).data_ptr<int32_t>(), n_out, (int32_t)K,
+                                              order ? order->rows.data_ptr<int32_t>() : nullptr, tm, dd.data_ptr(),
+                                              (int32_t)cout, dd.stride(0), dw.data_ptr<float>(), ws.data_ptr(),
+                                              ws.numel(), device_error_flag(x.device()).data_ptr<int32_t>(),
+                                              cur_stream()),
                      "sparse conv weight gradient (tensor cores)");
-        return dw.to(x.scalar_type());
+        return dw.to(dtype);
     }
     const bool wide = x.scalar_type() == torch::kFloat64;
     Tensor xx = wide ? x : x.to(torch::kFloat32).contiguous();
@@ -1232,13 +1249,15 @@ std::vector<Tensor> conv_backward(const Tensor &dy_in, const Tensor &x, const Te
                              false, std::nullopt, true);
         else if (need_dx)
             dx = gather_gemm(dy, pack_kmap_t(p), p->src->N, Wkio, true, pack_tile_mask(p, true), std::nullopt, p, true);
-        if (need_dw) dW = gather_wgrad(x, pack_kmap(p), p->tgt->N, dy, K, pack_tile_mask(p, false));
+        if (need_dw)
+            dW = gather_wgrad(x, pack_kmap(p), p->tgt->N, dy, K, pack_tile_mask(p, false), built_row_order(p, false));
     } else {
         if (need_dx)
             dx = gather_gemm(dy, pack_kmap(p), p->tgt->N, Wkio, true, pack_tile_mask(p, false), std::nullopt, p, false);
         if (need_dw && mirror)
-            dW = gather_wgrad(x, pack_kmap(p), p->src->N, dy, K, pack_tile_mask(p, false)).flip(0);
-        else if (need_dw) dW = gather_wgrad(x, pack_kmap_t(p), p->src->N, dy, K, pack_tile_mask(p, true));
+            dW = gather_wgrad(x, pack_kmap(p), p->src->N, dy, K, pack_tile_mask(p, false), built_row_order(p, false)).flip(0);
+        else if (need_dw)
+            dW = gather_wgrad(x, pack_kmap_t(p), p->src->N, dy, K, pack_tile_mask(p, true), built_row_order(p, true));
     }
     if (need_dw) {
         dW = dW.reshape({p->ks.v[2], p->ks.v[1], p->ks.v[0], cin, cout});

@@ -468,6 +468,14 @@ int fvgb_tc_wgrad_workspace(int64_t n_out, int32_t K, int32_t c_in, int32_t c_ou
 int fvgb_conv_wgrad_tc(const void *x, int64_t n_x, int32_t c_in, int64_t ldx, const int32_t *map, int64_t n_out,
                        int32_t K, const uint32_t *tile_mask, const void *dy, int32_t c_out, int64_t lddy, float *dw,
                        void *workspace, size_t workspace_bytes, int32_t *err_dev, fvgb_stream_t stream);
+/* fvgb_conv_wgrad_tc for FVGB_BF16 or FVGB_F16 operands of any channel counts that are multiples of
+ * 8 (c_in <= 128, c_out <= 256), in index order (rows null) or over a row order: map, tile_mask and
+ * rows (padded to whole 128-row tiles with -1) then come from fvgb_kmap_row_order. */
+int fvgb_tc_wgrad_16bit_workspace(int64_t n_out, int32_t K, int32_t c_in, int32_t c_out, size_t *bytes);
+int fvgb_conv_wgrad_tc_16bit(int32_t dtype, const void *x, int64_t n_x, int32_t c_in, int64_t ldx,
+                             const int32_t *map, int64_t n_out, int32_t K, const int32_t *rows,
+                             const uint32_t *tile_mask, const void *dy, int32_t c_out, int64_t lddy, float *dw,
+                             void *workspace, size_t workspace_bytes, int32_t *err_dev, fvgb_stream_t stream);
 
 /*
  * FP8-E4M3 quantisation of features: out[r, c] = e4m3_satfinite(x[r, c] * inv_scale[c]),
