@@ -36,11 +36,9 @@ class HaloConvFunction(torch.autograd.Function):
         data, w = ctx.saved_tensors
         C = _lib.load()
         dy = grad_out.to(data.dtype).contiguous()
-        dx = dw = None
-        if ctx.needs_input_grad[1]:
-            dx = C.halo_conv(ctx.grid_impl, dy, w, True)
-        if ctx.needs_input_grad[2]:
+        need_dx, need_dw = ctx.needs_input_grad[1:3]
+        dx, dw = C.halo_backward(ctx.grid_impl, data, w, dy, need_dx, need_dw)
+        if need_dw:  # [27, I, O]
             shape, wdtype = ctx.weight_meta
-            dw = C.halo_wgrad(ctx.grid_impl, data, dy)  # [27, I, O]
             dw = dw.reshape(3, 3, 3, shape[1], shape[0]).permute(4, 3, 2, 1, 0).to(wdtype).contiguous()
         return None, dx, dw
