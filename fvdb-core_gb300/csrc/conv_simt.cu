@@ -14,7 +14,7 @@
 namespace fvgb {
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16, NT = 256;  // wgrad tile
+constexpr int NT = 256;
 constexpr int FM = 128, FN = 64;                    // forward tile: 128 rows x 64 channels, 8 x 4 per thread
 
 template <typename T>
@@ -34,12 +34,26 @@ struct Vec4<double> {
     }
 };
 
+// One 16-byte vector from p (zeros for null)
+__device__ __forceinline__ void ldvec(const float *p, float *v) {
+    const float4 q = p ? __ldg(reinterpret_cast<const float4 *>(p)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+}
+__device__ __forceinline__ void ldvec(const double *p, double *v) {
+    const double2 q = p ? __ldg(reinterpret_cast<const double2 *>(p)) : make_double2(0.0, 0.0);
+    v[0] = q.x, v[1] = q.y;
+}
+
 // One CTA per 128-row x 64-channel output tile, 256 threads of 8 rows x 4 channels.  Per
 // offset with any present row and per 16-channel slice (8 for FP64), the gathered rows (transposed, so a
 // thread's 8 rows are two vector loads) and the weight slice go through shared memory; the
 // slice after is loaded into registers while this one is multiplied, so one barrier per slice
-// separates the two shared-memory buffers.
-template <typename T>
+// separates the two shared-memory buffers.  VEC (whole 16-byte pieces in x rows and W columns,
+// W's output channels contiguous): operands are fetched 16 bytes at a time; with one element per
+// load the fetches and their bounds checks took a third of the issue slots (0.11M voxels, row
+// order, the 32->64->32 FP32 training step's four contractions: 1.69 ms element by element, 1.34 ms
+// in vectors).
+template <typename T, bool VEC>
 __global__ void __launch_bounds__(NT) conv_fwd_simt_kernel(const T *__restrict__ x, int64_t n_x, int32_t cin,
                                                            int64_t ldx, const int32_t *__restrict__ map,
                                                            int64_t n_out, int32_t K, int64_t ldm,
@@ -76,32 +90,65 @@ __global__ void __launch_bounds__(NT) conv_fwd_simt_kernel(const T *__restrict__
     };
     // per thread: A elements e = tid + 256 q (q < QA) -> (row e / FK, channel e % FK); B elements
     // e = tid + 256 q (q < QB) -> (channel e / 64, column e % 64)
+    // VEC: the same slices in 16-byte vectors of VW elements
+    constexpr int VW = 16 / sizeof(T), VA = QA / VW, VB = QB / VW;
     T ra[QA], rb4[QB];
     auto fetch = [&](int32_t k, int32_t c0, int rbuf) {
+        if constexpr (VEC) {
 #pragma unroll
-        for (int q = 0; q < QA; ++q) {
-            const int e = tid + q * NT, r = e / FK, c = e % FK;
-            const int32_t src = rows[rbuf][r];
-            ra[q] = (src >= 0 && c0 + c < cin) ? x[(int64_t)src * ldx + c0 + c] : T(0);
-        }
+            for (int q = 0; q < VA; ++q) {
+                const int e = tid + q * NT, r = e / (FK / VW), c = (e % (FK / VW)) * VW;
+                const int32_t src = rows[rbuf][r];
+                const bool on = src >= 0 && c0 + c < cin;
+                ldvec(on ? x + (int64_t)src * ldx + c0 + c : nullptr, &ra[q * VW]);
+            }
 #pragma unroll
-        for (int q = 0; q < QB; ++q) {
-            const int e = tid + q * NT, c = e >> 6, n = e & 63;
-            rb4[q] = (c0 + c < cin && n0 + n < cout)
-                         ? w[k * wsk + (int64_t)(c0 + c) * wsci + (int64_t)(n0 + n) * wsco]
-                         : T(0);
+            for (int q = 0; q < VB; ++q) {
+                const int e = tid + q * NT, c = e / (FN / VW), n = (e % (FN / VW)) * VW;
+                const bool on = c0 + c < cin && n0 + n < cout;
+                ldvec(on ? w + k * wsk + (int64_t)(c0 + c) * wsci + n0 + n : nullptr, &rb4[q * VW]);
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < QA; ++q) {
+                const int e = tid + q * NT, r = e / FK, c = e % FK;
+                const int32_t src = rows[rbuf][r];
+                ra[q] = (src >= 0 && c0 + c < cin) ? x[(int64_t)src * ldx + c0 + c] : T(0);
+            }
+#pragma unroll
+            for (int q = 0; q < QB; ++q) {
+                const int e = tid + q * NT, c = e >> 6, n = e & 63;
+                rb4[q] = (c0 + c < cin && n0 + n < cout)
+                             ? w[k * wsk + (int64_t)(c0 + c) * wsci + (int64_t)(n0 + n) * wsco]
+                             : T(0);
+            }
         }
     };
     auto store = [&](int buf) {
+        if constexpr (VEC) {
 #pragma unroll
-        for (int q = 0; q < QA; ++q) {
-            const int e = tid + q * NT;
-            As[buf][e % FK][e / FK] = ra[q];
-        }
+            for (int q = 0; q < VA; ++q) {
+                const int e = tid + q * NT, r = e / (FK / VW), c = (e % (FK / VW)) * VW;
 #pragma unroll
-        for (int q = 0; q < QB; ++q) {
-            const int e = tid + q * NT;
-            Bs[buf][e >> 6][e & 63] = rb4[q];
+                for (int v = 0; v < VW; ++v) As[buf][c + v][r] = ra[q * VW + v];
+            }
+#pragma unroll
+            for (int q = 0; q < VB; ++q) {
+                const int e = tid + q * NT, c = e / (FN / VW), n = (e % (FN / VW)) * VW;
+#pragma unroll
+                for (int v = 0; v < VW; ++v) Bs[buf][c][n + v] = rb4[q * VW + v];
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < QA; ++q) {
+                const int e = tid + q * NT;
+                As[buf][e % FK][e / FK] = ra[q];
+            }
+#pragma unroll
+            for (int q = 0; q < QB; ++q) {
+                const int e = tid + q * NT;
+                Bs[buf][e >> 6][e & 63] = rb4[q];
+            }
         }
     };
 
@@ -163,81 +210,194 @@ __global__ void __launch_bounds__(NT) conv_fwd_simt_kernel(const T *__restrict__
     }
 }
 
+template <typename T>
+void launch_fwd_simt(dim3 grid, const void *x, int64_t n_x, int32_t cin, int64_t ldx, const int32_t *map, int64_t n_out,
+                     int32_t K, int64_t ldm, const void *w, int64_t wsk, int64_t wsci, int64_t wsco, void *y,
+                     int32_t cout, int64_t ldy, int32_t accumulate, const int32_t *rows, cudaStream_t s) {
+    constexpr int VW = 16 / sizeof(T);
+    const bool vec = cin % VW == 0 && ldx % VW == 0 && wsco == 1 && cout % VW == 0 && wsk % VW == 0 && wsci % VW == 0 &&
+                     (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
+    if (vec)
+        conv_fwd_simt_kernel<T, true><<<grid, NT, 0, s>>>((const T *)x, n_x, cin, ldx, map, n_out, K, ldm, (const T *)w, wsk,
+                                                          wsci, wsco, (T *)y, cout, ldy, accumulate, rows);
+    else
+        conv_fwd_simt_kernel<T, false><<<grid, NT, 0, s>>>((const T *)x, n_x, cin, ldx, map, n_out, K, ldm, (const T *)w,
+                                                           wsk, wsci, wsco, (T *)y, cout, ldy, accumulate, rows);
+}
+
 // Rows per wgrad chunk so that the grid has enough CTAs; deterministic in the sizes only.
 struct WgradPlan {
     int64_t chunks, rows_per_chunk;
+    int32_t tm, tn;              // tile of dW: tm input x tn output channels (32 or 64 each)
     int32_t tiles_ci, tiles_co;
 };
 
+// 64 wide unless the last 64 would be at most half used
+int32_t wgrad_tile(int32_t c) { return c % 64 == 0 || c % 64 > 32 ? 64 : 32; }
+
 WgradPlan wgrad_plan(int64_t n_out, int32_t K, int32_t cin, int32_t cout) {
     WgradPlan p;
-    p.tiles_ci = (int32_t)ceil_div(cin, BM);
-    p.tiles_co = (int32_t)ceil_div(cout, BN);
+    p.tm = wgrad_tile(cin);
+    p.tn = wgrad_tile(cout);
+    p.tiles_ci = (int32_t)ceil_div(cin, p.tm);
+    p.tiles_co = (int32_t)ceil_div(cout, p.tn);
     const int64_t per_chunk_ctas = (int64_t)K * p.tiles_ci * p.tiles_co;
     int64_t chunks = ceil_div(2048, per_chunk_ctas);
     const int64_t max_chunks = ceil_div(n_out > 0 ? n_out : 1, 256);
     if (chunks > max_chunks) chunks = max_chunks;
     if (chunks < 1) chunks = 1;
-    p.rows_per_chunk = ceil_div(ceil_div(n_out > 0 ? n_out : 1, chunks), BK) * BK;
+    p.rows_per_chunk = ceil_div(ceil_div(n_out > 0 ? n_out : 1, chunks), 16) * 16;
     p.chunks = ceil_div(n_out > 0 ? n_out : 1, p.rows_per_chunk);
     return p;
 }
 
-template <typename T, typename AccT>
-__global__ void __launch_bounds__(NT) wgrad_simt_kernel(const T *__restrict__ x, int64_t n_x, int32_t cin,
-                                                        int64_t ldx, const int32_t *__restrict__ map,
-                                                        int64_t n_out, int32_t K, int64_t ldm,
-                                                        const T *__restrict__ dy, int32_t cout, int64_t lddy,
-                                                        int64_t rows_per_chunk, int32_t tiles_co,
-                                                        AccT *__restrict__ partials) {
-    __shared__ int32_t rows[BK];
-    __shared__ AccT Xs[BK][BM + 4];
-    __shared__ AccT Ds[BK][BN + 4];
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+// dW partials of one (row chunk, offset, TM x TN channel tile) per CTA.  The chunk's map column is
+// read 256 rows at a time and its present entries are queued in row order, so the products run over
+// whole batches of BKP present (input row, output row) pairs: an offset of a surface grid is present
+// in under half of the rows, which the products would otherwise spend on zeros.  The 256 threads
+// form SL slices of TM x TN / 16 threads (4 x 4 outputs each); slice s takes pairs s, s + SL, ... of
+// a batch and the slices are added in order at the end, so a narrow tile keeps every thread busy.
+// The next batch is loaded into registers while this one is multiplied.  0.11M voxels, 32->64 and
+// 64->32 FP32, 3^3: 732 us each with zero rows and 64 x 64 tiles, 203 us here.
+constexpr int kPairQueue = 512;  // a batch's leftover and the next 256 rows
+
+template <typename T, int TM, int TN, bool VEC>
+__global__ void __launch_bounds__(NT) wgrad_simt_kernel(const T *__restrict__ x, int64_t n_x, int32_t cin, int64_t ldx,
+                                                        const int32_t *__restrict__ map, int64_t n_out, int32_t K,
+                                                        int64_t ldm, const T *__restrict__ dy, int32_t cout,
+                                                        int64_t lddy, int64_t rows_per_chunk, int32_t tiles_co,
+                                                        T *__restrict__ partials) {
+    constexpr int BKP = sizeof(T) == 8 ? 16 : 32;
+    constexpr int TPS = TM * TN / 16, SL = NT / TPS;
+    constexpr int VW = VEC ? 16 / sizeof(T) : 1;
+    constexpr int XV = BKP * TM / VW, DV = BKP * TN / VW;            // vectors per batch
+    constexpr int XQ = (XV + NT - 1) / NT, DQ = (DV + NT - 1) / NT;  // per thread
+    __shared__ __align__(16) T pool[2 * BKP * (TM + 4 + TN + 4)];
+    T(*Xs)[BKP][TM + 4] = reinterpret_cast<T(*)[BKP][TM + 4]>(pool);
+    T(*Ds)[BKP][TN + 4] = reinterpret_cast<T(*)[BKP][TN + 4]>(pool + 2 * BKP * (TM + 4));
+    __shared__ int2 queue[kPairQueue];
+    __shared__ int32_t wcount[NT / 32];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int slice = tid / TPS, ty = (tid % TPS) / (TN / 4), tx = (tid % TPS) % (TN / 4);
     const int64_t chunk = blockIdx.x;
     const int32_t k = blockIdx.y;
-    const int32_t ci0 = (blockIdx.z / tiles_co) * BM, co0 = (blockIdx.z % tiles_co) * BN;
-    const int64_t r_begin = chunk * rows_per_chunk;
-    int64_t r_end = r_begin + rows_per_chunk;
-    if (r_end > n_out) r_end = n_out;
-    AccT acc[4][4];
+    const int32_t ci0 = (blockIdx.z / tiles_co) * TM, co0 = (blockIdx.z % tiles_co) * TN;
+    int64_t r0 = chunk * rows_per_chunk;
+    const int64_t r_end = min(n_out, r0 + rows_per_chunk);
+    T acc[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = AccT(0);
-    for (int64_t r0 = r_begin; r0 < r_end; r0 += BK) {
-        int valid = 0;
-        if (tid < BK) {
+        for (int j = 0; j < 4; ++j) acc[i][j] = T(0);
+    int32_t head = 0, tail = 0;  // the same in every thread
+    // queue present pairs until a batch is full or the chunk ends
+    auto fill = [&]() {
+        while (tail - head < BKP && r0 < r_end) {
             const int64_t r = r0 + tid;
             int32_t v = r < r_end ? map[r * ldm + k] : -1;
             if (v >= n_x) v = -1;
-            rows[tid] = v;
-            valid = v >= 0;
-        }
-        if (!__syncthreads_or(valid)) continue;
+            const uint32_t present = __ballot_sync(0xffffffffu, v >= 0);
+            if (lane == 0) wcount[warp] = __popc(present);
+            __syncthreads();
+            int before = 0, total = 0;
 #pragma unroll
-        for (int q = 0; q < (BK * BM) / NT; ++q) {
-            const int e = tid + q * NT, r = e / BM, c = e % BM;
-            const int32_t src = rows[r];
-            Xs[r][c] = (src >= 0 && ci0 + c < cin) ? (AccT)x[(int64_t)src * ldx + ci0 + c] : AccT(0);
-            Ds[r][c] = (src >= 0 && co0 + c < cout) ? (AccT)dy[(r0 + r) * lddy + co0 + c] : AccT(0);
+            for (int w = 0; w < NT / 32; ++w) {
+                if (w < warp) before += wcount[w];
+                total += wcount[w];
+            }
+            if (v >= 0)
+                queue[(tail + before + __popc(present & ((1u << lane) - 1u))) & (kPairQueue - 1)] = make_int2(v, (int32_t)(r - chunk * rows_per_chunk));
+            tail += total;
+            r0 += NT;
+            __syncthreads();
         }
+    };
+    T rx[XQ * VW], rd[DQ * VW];
+    auto fetch = [&]() {
+        const int cnt = min(BKP, tail - head);
+#pragma unroll
+        for (int q = 0; q < XQ; ++q) {
+            const int e = tid + q * NT, p = e / (TM / VW), c = (e % (TM / VW)) * VW;
+            const T *src = nullptr;
+            if (e < XV && p < cnt && ci0 + c < cin)
+                src = x + (int64_t)queue[(head + p) & (kPairQueue - 1)].x * ldx + ci0 + c;
+            if constexpr (VEC) ldvec(src, &rx[q * VW]);
+            else rx[q] = src ? *src : T(0);
+        }
+#pragma unroll
+        for (int q = 0; q < DQ; ++q) {
+            const int e = tid + q * NT, p = e / (TN / VW), c = (e % (TN / VW)) * VW;
+            const T *src = nullptr;
+            if (e < DV && p < cnt && co0 + c < cout)
+                src = dy + (chunk * rows_per_chunk + queue[(head + p) & (kPairQueue - 1)].y) * lddy + co0 + c;
+            if constexpr (VEC) ldvec(src, &rd[q * VW]);
+            else rd[q] = src ? *src : T(0);
+        }
+        head += cnt;
+    };
+    auto store = [&](int buf) {
+#pragma unroll
+        for (int q = 0; q < XQ; ++q) {
+            const int e = tid + q * NT, p = e / (TM / VW), c = (e % (TM / VW)) * VW;
+            if (e < XV)
+#pragma unroll
+                for (int v = 0; v < VW; ++v) Xs[buf][p][c + v] = rx[q * VW + v];
+        }
+#pragma unroll
+        for (int q = 0; q < DQ; ++q) {
+            const int e = tid + q * NT, p = e / (TN / VW), c = (e % (TN / VW)) * VW;
+            if (e < DV)
+#pragma unroll
+                for (int v = 0; v < VW; ++v) Ds[buf][p][c + v] = rd[q * VW + v];
+        }
+    };
+    fill();
+    if (tail > head) {
+        fetch();
+        store(0);
         __syncthreads();
+        int buf = 0;
+        while (true) {
+            fill();
+            const bool more = tail > head;
+            if (more) fetch();
+#pragma unroll 8
+            for (int r = slice; r < BKP; r += SL) {
+                T a[4], b[4];
+                Vec4<T>::load(&Xs[buf][r][ty * 4], a);
+                Vec4<T>::load(&Ds[buf][r][tx * 4], b);
 #pragma unroll
-        for (int r = 0; r < BK; ++r) {
-            AccT a[4], bb[4];
+                for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = Xs[r][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) bb[j] = Ds[r][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], bb[j], acc[i][j]);
+                    for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+            }
+            if (!more) break;
+            store(buf ^ 1);
+            __syncthreads();
+            buf ^= 1;
         }
-        __syncthreads();
     }
-    AccT *dst = partials + ((chunk * K + k) * (int64_t)cin) * cout;
+    if constexpr (SL > 1) {
+        static_assert(2 * BKP * (TM + 4 + TN + 4) >= TM * TN, "the slice sums pass through the operand buffers");
+        T *red = pool;
+#pragma unroll
+        for (int s = 1; s < SL; ++s) {
+            __syncthreads();
+            if (slice == s)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) red[(ty * 4 + i) * TN + tx * 4 + j] = acc[i][j];
+            __syncthreads();
+            if (slice == 0)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[i][j] += red[(ty * 4 + i) * TN + tx * 4 + j];
+        }
+        if (slice != 0) return;
+    }
+    T *dst = partials + ((chunk * K + k) * (int64_t)cin) * cout;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int32_t ci = ci0 + ty * 4 + i;
@@ -250,6 +410,38 @@ __global__ void __launch_bounds__(NT) wgrad_simt_kernel(const T *__restrict__ x,
     }
 }
 
+template <typename T, int TM, int TN>
+void launch_wgrad_tile(const WgradPlan &p, const void *x, int64_t n_x, int32_t cin, int64_t ldx, const int32_t *map,
+                       int64_t n_out, int32_t K, int64_t ldm, const void *dy, int32_t cout, int64_t lddy, void *part,
+                       cudaStream_t s) {
+    constexpr int VW = 16 / sizeof(T);
+    const dim3 grid((unsigned)p.chunks, (unsigned)K, (unsigned)(p.tiles_ci * p.tiles_co));
+    const bool vec = cin % VW == 0 && cout % VW == 0 && ldx % VW == 0 && lddy % VW == 0 &&
+                     (((uintptr_t)x | (uintptr_t)dy) & 15) == 0;
+    if (vec)
+        wgrad_simt_kernel<T, TM, TN, true><<<grid, NT, 0, s>>>((const T *)x, n_x, cin, ldx, map, n_out, K, ldm,
+                                                               (const T *)dy, cout, lddy, p.rows_per_chunk, p.tiles_co,
+                                                               (T *)part);
+    else
+        wgrad_simt_kernel<T, TM, TN, false><<<grid, NT, 0, s>>>((const T *)x, n_x, cin, ldx, map, n_out, K, ldm,
+                                                                (const T *)dy, cout, lddy, p.rows_per_chunk, p.tiles_co,
+                                                                (T *)part);
+}
+
+template <typename T>
+void launch_wgrad_simt(const WgradPlan &p, const void *x, int64_t n_x, int32_t cin, int64_t ldx, const int32_t *map,
+                       int64_t n_out, int32_t K, int64_t ldm, const void *dy, int32_t cout, int64_t lddy, void *part,
+                       cudaStream_t s) {
+    if (p.tm == 64 && p.tn == 64)
+        launch_wgrad_tile<T, 64, 64>(p, x, n_x, cin, ldx, map, n_out, K, ldm, dy, cout, lddy, part, s);
+    else if (p.tm == 64)
+        launch_wgrad_tile<T, 64, 32>(p, x, n_x, cin, ldx, map, n_out, K, ldm, dy, cout, lddy, part, s);
+    else if (p.tn == 64)
+        launch_wgrad_tile<T, 32, 64>(p, x, n_x, cin, ldx, map, n_out, K, ldm, dy, cout, lddy, part, s);
+    else
+        launch_wgrad_tile<T, 32, 32>(p, x, n_x, cin, ldx, map, n_out, K, ldm, dy, cout, lddy, part, s);
+}
+
 // dW[e] = sum over chunks (ascending) of partials[chunk][e], accumulated in FP64.
 template <typename AccT, typename OutT>
 __global__ void wgrad_reduce_kernel(const AccT *__restrict__ partials, int64_t chunks, int64_t per_chunk,
@@ -257,6 +449,7 @@ __global__ void wgrad_reduce_kernel(const AccT *__restrict__ partials, int64_t c
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= per_chunk) return;
     double s = 0.0;
+#pragma unroll 16  // loads in flight; the sum keeps its order
     for (int64_t c = 0; c < chunks; ++c) s += (double)partials[c * per_chunk + e];
     dw[e] = (OutT)s;
 }
@@ -286,13 +479,11 @@ extern "C" int fvgb_conv_fwd_simt_rows(int32_t dtype, const void *x, int64_t n_x
     if (grid.y > 65535) return FVGB_EINVAL;
     cudaStream_t s = as_stream(stream);
     if (dtype == FVGB_F32) {
-        conv_fwd_simt_kernel<float><<<grid, NT, 0, s>>>((const float *)x, n_x, c_in, ldx, map, n_out, K, ldm,
-                                                        (const float *)w, wsk, wsci, wsco, (float *)y, c_out, ldy,
-                                                        accumulate, rows);
+        launch_fwd_simt<float>(grid, x, n_x, c_in, ldx, map, n_out, K, ldm, w, wsk, wsci, wsco, y, c_out, ldy, accumulate,
+                               rows, s);
     } else if (dtype == FVGB_F64) {
-        conv_fwd_simt_kernel<double><<<grid, NT, 0, s>>>((const double *)x, n_x, c_in, ldx, map, n_out, K, ldm,
-                                                         (const double *)w, wsk, wsci, wsco, (double *)y, c_out,
-                                                         ldy, accumulate, rows);
+        launch_fwd_simt<double>(grid, x, n_x, c_in, ldx, map, n_out, K, ldm, w, wsk, wsci, wsco, y, c_out, ldy, accumulate,
+                                rows, s);
     } else {
         return FVGB_ETYPE;
     }
@@ -327,17 +518,13 @@ extern "C" int fvgb_conv_wgrad_simt(int32_t dtype, const void *x, int64_t n_x, i
     if (dtype == FVGB_F32) {
         float *part = reinterpret_cast<float *>(base);
         if (n_out > 0)
-            wgrad_simt_kernel<float, float><<<grid, NT, 0, s>>>((const float *)x, n_x, c_in, ldx, map, n_out, K,
-                                                               ldm, (const float *)dy, c_out, lddy,
-                                                               p.rows_per_chunk, p.tiles_co, part);
+            launch_wgrad_simt<float>(p, x, n_x, c_in, ldx, map, n_out, K, ldm, dy, c_out, lddy, part, s);
         wgrad_reduce_kernel<float, float><<<(unsigned)ceil_div(per_chunk, 256), 256, 0, s>>>(
             part, n_out > 0 ? p.chunks : 0, per_chunk, (float *)dw);
     } else if (dtype == FVGB_F64) {
         double *part = reinterpret_cast<double *>(base);
         if (n_out > 0)
-            wgrad_simt_kernel<double, double><<<grid, NT, 0, s>>>((const double *)x, n_x, c_in, ldx, map, n_out,
-                                                                 K, ldm, (const double *)dy, c_out, lddy,
-                                                                 p.rows_per_chunk, p.tiles_co, part);
+            launch_wgrad_simt<double>(p, x, n_x, c_in, ldx, map, n_out, K, ldm, dy, c_out, lddy, part, s);
         wgrad_reduce_kernel<double, double><<<(unsigned)ceil_div(per_chunk, 256), 256, 0, s>>>(
             part, n_out > 0 ? p.chunks : 0, per_chunk, (double *)dw);
     } else {
@@ -421,7 +608,7 @@ extern "C" int fvgb_conv_wgrad_simt_noalloc(int32_t dtype, const void *x, int64_
     if (st != FVGB_OK) return st;
     WgradPlan p = wgrad_plan(n_out, K, c_in, c_out);
     if (p.chunks > cap_chunks) {
-        p.rows_per_chunk = ceil_div(ceil_div(n_out > 0 ? n_out : 1, cap_chunks), BK) * BK;
+        p.rows_per_chunk = ceil_div(ceil_div(n_out > 0 ? n_out : 1, cap_chunks), 16) * 16;
         p.chunks = ceil_div(n_out > 0 ? n_out : 1, p.rows_per_chunk);
     }
     cudaStream_t s = as_stream(stream);
@@ -431,17 +618,13 @@ extern "C" int fvgb_conv_wgrad_simt_noalloc(int32_t dtype, const void *x, int64_
     if (dtype == FVGB_F32) {
         float *part = reinterpret_cast<float *>(scratch);
         if (n_out > 0)
-            wgrad_simt_kernel<float, float><<<grid, NT, 0, s>>>((const float *)x, n_x, c_in, ldx, map, n_out, K,
-                                                               ldm, (const float *)dy, c_out, lddy,
-                                                               p.rows_per_chunk, p.tiles_co, part);
+            launch_wgrad_simt<float>(p, x, n_x, c_in, ldx, map, n_out, K, ldm, dy, c_out, lddy, part, s);
         wgrad_reduce_kernel<float, float><<<(unsigned)ceil_div(per_chunk, 256), 256, 0, s>>>(
             part, n_out > 0 ? p.chunks : 0, per_chunk, (float *)dw);
     } else {
         double *part = reinterpret_cast<double *>(scratch);
         if (n_out > 0)
-            wgrad_simt_kernel<double, double><<<grid, NT, 0, s>>>((const double *)x, n_x, c_in, ldx, map, n_out,
-                                                                 K, ldm, (const double *)dy, c_out, lddy,
-                                                                 p.rows_per_chunk, p.tiles_co, part);
+            launch_wgrad_simt<double>(p, x, n_x, c_in, ldx, map, n_out, K, ldm, dy, c_out, lddy, part, s);
         wgrad_reduce_kernel<double, double><<<(unsigned)ceil_div(per_chunk, 256), 256, 0, s>>>(
             part, n_out > 0 ? p.chunks : 0, per_chunk, (double *)dw);
     }

@@ -1093,10 +1093,20 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
                                  : (n_out >= (int64_t)1 << 16 ? pack_row_order(pack, map_t)
                                                               : pack_row_order_if_reused(pack, map_t, 0, 0, reuse));
         const Tensor &m_used = order ? order->map : map;
+        // W^T laid out with its output channels contiguous (a few hundred KB): the kernel reads the
+        // weights in whole vectors
+        Tensor wt = w;
+        int64_t tsk = wsk, tsci = wsci, tsco = wsco;
+        if (transpose_w && cout % 4 == 0) {
+            wt = w.transpose(1, 2).contiguous();
+            tsk = mirror ? -wt.stride(0) : wt.stride(0);
+            tsci = wt.stride(1);
+            tsco = wt.stride(2);
+        }
         check_status(fvgb_conv_fwd_simt_rows(dt, x.data_ptr(), x.size(0), (int32_t)cin, x.stride(0),
                                              m_used.data_ptr<int32_t>(), n_out, (int32_t)K, m_used.stride(0),
-                                             order ? order->rows.data_ptr<int32_t>() : nullptr, first_offset(w), wsk,
-                                             wsci, wsco, y.data_ptr(), (int32_t)cout, y.stride(0), 0, s),
+                                             order ? order->rows.data_ptr<int32_t>() : nullptr, first_offset(wt), tsk,
+                                             tsci, tsco, y.data_ptr(), (int32_t)cout, y.stride(0), 0, s),
                      "sparse conv forward");
     } else {
         // 16-bit features of shapes the tensor-core kernel does not take: CUDA cores, FP32
