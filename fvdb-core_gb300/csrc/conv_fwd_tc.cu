@@ -16,21 +16,24 @@
 // Warp roles (448 threads):
 //   warps 0-7  gather: each warp fills 16 rows of every unit's A tile.  Lane l copies chunk l%8 of
 //              rows l/8, l/8+4, l/8+8, l/8+12, so one warp instruction moves four whole 128-byte
-//              A rows (per-SM cp.async throughput is set by the number of issuing warps and the
-//              distinct lines per instruction, not by bytes).  Copies are 16-byte cp.async (L2
-//              evict_last: the input features stay L2-resident while the map and output stream)
-//              into the 128B-swizzled K-major A layout; absent entries (map -1) are zero-stored
-//              with st.shared.  Both are generic-proxy writes, so each warp publishes a stage to
-//              the tensor core (async proxy) itself, kLag stages late: cp.async.wait_group,
-//              fence.proxy.async, __syncwarp, one mbarrier arrive.  The MMA warp never fences
-//              and its MMAs stream back to back.  Map entries are read before the stage wait so
-//              their latency overlaps it.
+//              A rows into the 128B-swizzled K-major A layout with 16-byte cp.async; absent entries
+//              (map -1) are the same instruction with no source bytes (zero fill), so the copies of
+//              a warp never diverge.  A stage is published without waiting for it: every thread
+//              arrives on the stage's barrier asynchronously, when its copies have landed
+//              (cp.async.mbarrier.arrive.noinc), and the MMA warp, which sees the copies through
+//              that barrier, fences them to the async proxy.  So a gather warp runs ahead as far as
+//              the ring allows; publishing a stage itself (wait for the copies, fence, arrive) kept
+//              it to one stage ahead.  1.31M surface rows, 32->64 BF16, index order: 455 us
+//              published by the gather warps, 369 with zero fill and the padded output staging,
+//              349 asynchronously; box faces 64->64 over the row order 343 -> 271; 128->256 over the
+//              row order 1307 -> 1154.  16 gather warps gain nothing further (355).  Map entries are
+//              read before the stage wait so their latency overlaps it.
 //   warp 8     TMEM allocation (2 x N columns) and the MMA issuer: the whole warp runs the
 //              issue loop and one elected lane issues each tcgen05.mma; tile i accumulates into
 //              TMEM buffer i % 2.
 //   warps 9-12 epilogue: tcgen05.ld of the finished buffer -> scale -> BF16 -> a shared-memory
-//              copy of the output tile -> one bulk async store of the tile's contiguous rows;
-//              overlaps the next tile's main loop.
+//              copy of the output row -> one bulk async store per row; overlaps the next tile's
+//              main loop.
 //   warp 13    loader: bulk async copies of each tile's map rows (double-buffered) and of each
 //              unit's pre-packed, pre-swizzled weight image.
 //
@@ -61,7 +64,11 @@ constexpr int kMmaWarp = kGatherWarps;
 constexpr int kEpiWarps = 4;
 constexpr int kThreads = (kGatherWarps + 1 + kEpiWarps + 1) * 32;  // + loader warp
 constexpr int kMaxMapStage = 32;  // map tiles staged in shared memory up to K = 32
-constexpr int kLag = 1;  // cp.async groups a gather thread keeps in flight before publishing a stage
+constexpr int kMinStages = 2;
+// Row pitch of the output staging tile: 16 bytes past the row, so that the 32 rows a warp writes
+// spread over the banks (at the rows' own pitch, a multiple of 128 bytes, every store was an 8-way
+// conflict).
+constexpr int y_pitch(int BN) { return BN * 2 + 16; }
 
 // A "unit" is 128 bytes of the reduction dimension for all 128 rows of a tile: one 128-byte
 // channel chunk of one kernel offset (rows of >= 128 bytes), or a fixed group of `pack`
@@ -163,10 +170,6 @@ struct UnitWalker {
     }
 };
 
-__device__ __forceinline__ void st_shared_zero16(uint32_t addr) {
-    asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(addr), "r"(0) : "memory");
-}
-
 // 32 bytes to global memory in one store (address 32-byte aligned)
 __device__ __forceinline__ void st_global_32(void *p, const uint32_t (&v)[8]) {
     asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]),
@@ -183,12 +186,13 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
     constexpr int kSlotBytes = kRowBytes / PACK;             // one offset's share of an A row
     constexpr int kCpr = PACK > 1 ? kSlotBytes / 16 : 8;     // 16-byte chunks per offset slot
     constexpr int kCopies = kRowsPerWarp / 4;                // rows per lane per unit
+    constexpr int kYPitch = y_pitch(BN);
     const int S = a.stages;
     const bool stage_map = a.K <= kMaxMapStage;
     const int map_words = stage_map ? kTileM * a.K : 0;  // per buffer; 512*K bytes, 16-byte aligned
     int32_t *map_sm = reinterpret_cast<int32_t *>(smem + S * kStage);
     uint8_t *ystage = reinterpret_cast<uint8_t *>(map_sm + 2 * map_words);  // [128 rows x cout] bf16
-    uint64_t *bars = reinterpret_cast<uint64_t *>(ystage + (a.direct_store ? kTileM * BN * 2 : 0));
+    uint64_t *bars = reinterpret_cast<uint64_t *>(ystage + (a.direct_store ? kTileM * kYPitch : 0));
     uint64_t *full = bars, *empty = bars + S, *tfull = bars + 2 * S, *tempty = tfull + 2, *mfull = tempty + 2,
              *mempty = mfull + 2, *fin = mempty + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(fin + 1);
@@ -200,7 +204,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) {
-            mbar_init(&full[s], kGatherWarps + 1);  // one lane per gather warp + the loader's expect_tx
+            mbar_init(&full[s], kGatherWarps * 32 + 1);  // each gather thread + the loader's expect_tx
             mbar_init(&empty[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
@@ -222,7 +226,6 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
         // ----------------------------------------------------------------- gather (A operand)
         // Lane -> (16-byte chunk j of the 128-byte A row, rows rsub, rsub+4, rsub+8, rsub+12 of
         // this warp's 16): one warp instruction moves four whole A rows.
-        const uint64_t keep = policy_evict_last();
         const int j = lane & 7;
         const int rsub = lane >> 3;
         const int row0 = warp * kRowsPerWarp;
@@ -232,20 +235,25 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
         // chunks, the channel bytes left of its piece's end of the row and of the last MMA's end
         const int k_lane = PACK > 1 && jj * 16 >= a.row_bytes ? 0 : a.K;
         const int row_end = a.row_bytes - j * 16, mma_end = ((a.row_bytes + 31) & ~31) - j * 16;
-        uint32_t it = 0, sig = 0, stage = 0, phase = 0, pstage = 0;
+        // the lane's source column, its rows' place in a stage and 32-bit row arithmetic: a map entry of
+        // -1 is past n_x as an unsigned number
+        const uint8_t *xlane = a.x + (PACK > 1 ? jj : j) * 16;
+        const uint32_t dst0 = sw128_offset(row0 + rsub, j);
+        const uint32_t nx32 = (uint32_t)a.n_x, ldx32 = (uint32_t)a.ldx_bytes;
+        uint32_t stage = 0, phase = 0;
         int64_t tile = blockIdx.x;
         for (int i = 0; tile < a.n_tiles && !*abort; tile += stride, ++i) {
             const int mb = i & 1;
             if (stage_map && !__all_sync(0xffffffffu, mbar_wait_backoff(&mfull[mb], (i >> 1) & 1, abort, 64))) break;
-            const int32_t *mtile = map_sm + mb * map_words;
+            const int32_t *mlane = map_sm + mb * map_words + (row0 + rsub) * a.K;
             const Units un = tile_units<PACK>(a, tile);
             UnitWalker<PACK> w{un.bits, 0, 0, -1};
             bool ok = true;
             for (int u0 = 0; u0 < un.n; u0 += U) {
                 // map entries first: their latency overlaps the wait for the stage
-                int32_t src[U][kCopies];
+                uint32_t src[U][kCopies];
                 bool on[U];
-                int64_t colb[U];
+                const uint8_t *col[U];
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     int image = -1, k0 = 0, c = 0;
@@ -256,20 +264,19 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
                     // weights are zero, but stale A bytes could be NaN)
                     on[u] = image >= 0 && (PACK > 1 || c * kRowBytes < mma_end);
                     const int kmax = PACK > 1 || c * kRowBytes < row_end ? k_lane : 0;
-                    colb[u] = PACK > 1 ? (int64_t)jj * 16 : (int64_t)c * kRowBytes + j * 16;
+                    col[u] = xlane + (PACK > 1 ? 0 : c * kRowBytes);
 #pragma unroll
                     for (int q = 0; q < kCopies; ++q) {
-                        const int r = row0 + rsub + 4 * q;
                         int32_t v = -1;
                         if (on[u] && k < kmax) {
                             if (stage_map) {
-                                v = mtile[r * a.K + k];
+                                v = mlane[4 * q * a.K + k];
                             } else {
-                                const int64_t row = tile * kTileM + r;
+                                const int64_t row = tile * kTileM + row0 + rsub + 4 * q;
                                 v = row < a.n_out ? a.map[row * a.K + k] : -1;
                             }
                         }
-                        src[u][q] = v;
+                        src[u][q] = (uint32_t)v;
                     }
                 }
                 bool go = true;
@@ -280,47 +287,29 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
                     ok = false;
                     break;
                 }
-                const uint32_t As = smem_u32(smem + stage * kStage);
+                // rows 4 apart take the two halves of the swizzle pattern in turn
+                const uint32_t As = smem_u32(smem) + stage * kStage, even = As + dst0, odd = As + (dst0 ^ 64u);
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     if (!on[u]) continue;
 #pragma unroll
                     for (int q = 0; q < kCopies; ++q) {
-                        const uint32_t dst = As + u * kABytes + sw128_offset(row0 + rsub + 4 * q, j);
-                        if (src[u][q] >= 0 && src[u][q] < a.n_x)
-                            cp_async_16_hint(dst, a.x + (int64_t)src[u][q] * a.ldx_bytes + colb[u], 16u, keep);
-                        else
-                            st_shared_zero16(dst);
+                        const bool present = src[u][q] < nx32;
+                        cp_async_16((q & 1 ? odd : even) + u * kABytes + q * 4 * kRowBytes,
+                                    present ? col[u] + (uint64_t)src[u][q] * ldx32 : a.x, present ? 16u : 0u);
                     }
                 }
-                cp_async_commit();
-                ++it;
+                cp_async_arrive_noinc(&full[stage]);  // once this thread's copies have landed
                 if (++stage == (uint32_t)S) {
                     stage = 0;
                     phase ^= 1;
-                }
-                if (it - sig > kLag) {
-                    // the copies of stage `sig` have landed: publish them to the async proxy (tcgen05.mma)
-                    cp_async_wait_group<kLag>();
-                    fence_proxy_async();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&full[pstage]);
-                    ++sig;
-                    if (++pstage == (uint32_t)S) pstage = 0;
                 }
             }
             __syncwarp();
             if (stage_map && lane == 0) mbar_arrive(&mempty[mb]);
             if (!ok) break;
         }
-        cp_async_wait_group<0>();
-        fence_proxy_async();
-        __syncwarp();
-        if (lane == 0)
-            for (; sig < it; ++sig) {
-                mbar_arrive(&full[pstage]);
-                if (++pstage == (uint32_t)S) pstage = 0;
-            }
+        cp_async_wait_all();
     } else if (warp == kMmaWarp) {
         // ----------------------------------------------------------------- MMA issuer
         // The whole warp runs this loop (warp-uniform control flow, operands in uniform
@@ -349,6 +338,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
                         ok = false;
                         break;
                     }
+                    fence_proxy_async();  // the gather threads' copies, seen through the barrier -> tensor core
                     tc_fence_after();
                     const uint64_t ad = adesc0 + stage * kStageD, bd = ad + kBOffD;
 #pragma unroll
@@ -390,7 +380,6 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
         __syncwarp();
     } else if (warp < kMmaWarp + 1 + kEpiWarps) {
         // ----------------------------------------------------------------- epilogue
-        const int et = threadIdx.x - (kMmaWarp + 1) * 32;  // 0..127
         const int q4 = warp & 3;                           // TMEM lane quarter this warp may access
         const int rt = q4 * 32 + lane;                     // row of the tile this thread drains
         int64_t tile = blockIdx.x;
@@ -407,11 +396,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
             const uint32_t tbase = tmem + b * BN + ((uint32_t)(q4 * 32) << 16);
             // the output row this thread drains (rows of a given order: one bulk store per row)
             const int64_t yrow_i = rt >= rows ? -1 : (a.out_rows ? (int64_t)__ldg(a.out_rows + m0 + rt) : m0 + rt);
-            if (a.direct_store) {
-                // the staging tile of the previous store has been read
-                if (a.out_rows || et == 0) bulk_wait_read<0>();
-                named_barrier(1, kTileM);
-            }
+            if (a.direct_store) bulk_wait_read<0>();  // this thread's row of the previous tile has been read
 #pragma unroll 1
             for (int c0 = 0; c0 < BN; c0 += 16) {
                 float v[16];
@@ -449,7 +434,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
                 }
                 if (a.direct_store) {
                     // cout % 8 == 0: whole 16-byte groups; the last group of a 16-wide block may be cut
-                    uint4 *dst = reinterpret_cast<uint4 *>(ystage + ((size_t)rt * a.cout + c0) * 2);
+                    uint4 *dst = reinterpret_cast<uint4 *>(ystage + (size_t)rt * kYPitch + c0 * 2);
                     dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
                     if (c0 + 8 < a.cout) dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
                 } else {
@@ -477,21 +462,14 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
             __syncwarp();
             if (lane == 0) mbar_arrive(&tempty[b]);
             if (a.direct_store) {
-                fence_proxy_async();  // staging writes -> visible to the bulk store (async proxy)
-                named_barrier(1, kTileM);
-                if (a.out_rows) {
-                    if (yrow_i >= 0) {
-                        bulk_s2g(a.y + yrow_i * a.ldy * 2, smem_u32(ystage + (size_t)rt * a.cout * 2),
-                                 (uint32_t)(a.cout * 2));
-                        bulk_commit();
-                    }
-                } else if (et == 0) {
-                    bulk_s2g(a.y + m0 * a.ldy * 2, smem_u32(ystage), (uint32_t)(rows * a.cout * 2));
+                fence_proxy_async();  // this row's staging writes -> its bulk store (async proxy)
+                if (yrow_i >= 0) {
+                    bulk_s2g(a.y + yrow_i * a.ldy * 2, smem_u32(ystage + (size_t)rt * kYPitch), (uint32_t)(a.cout * 2));
                     bulk_commit();
                 }
             }
         }
-        if (a.direct_store && (a.out_rows || et == 0)) bulk_wait<0>();
+        if (a.direct_store) bulk_wait<0>();
     } else {
         // ----------------------------------------------------------------- loader (bulk copies)
         if (lane == 0) {
@@ -608,11 +586,10 @@ int launch_fwd(FwdArgs a, cudaStream_t s) {
     constexpr int stage = U * (kABytes + BN * kRowBytes);
     const int map_bytes = a.K <= kMaxMapStage ? 2 * kTileM * a.K * 4 : 0;
     a.direct_store = (a.direct_store && BN <= 128) ? 1 : 0;  // staging tile only where it fits
-    const int fixed = 1024 + map_bytes + (a.direct_store ? kTileM * BN * 2 : 0) + (2 * 8 + 9) * 8 + 16;
+    const int fixed = 1024 + map_bytes + (a.direct_store ? kTileM * y_pitch(BN) : 0) + (2 * 8 + 9) * 8 + 16;
     int stages = 8;
-    while (stages > kLag + 1 && stages * stage + fixed > 227 * 1024) --stages;
-    // a gather thread publishes a stage kLag stages late, so the ring needs more than kLag stages
-    if (stages < kLag + 1 || stages * stage + fixed > 227 * 1024) return FVGB_EINVAL;
+    while (stages > kMinStages && stages * stage + fixed > 227 * 1024) --stages;
+    if (stages * stage + fixed > 227 * 1024) return FVGB_EINVAL;
     a.stages = stages;
     const int smem = stages * stage + fixed;
     auto kern = conv_tc_fwd_kernel<BN, EB, PACK, U>;
@@ -720,6 +697,10 @@ int conv_fwd(int eb, bool f16, const void *x, int64_t n_x, int32_t c_in, int64_t
     const int64_t row_bytes = (int64_t)c_in * eb;
     // rows are copied in 16-byte pieces
     if (row_bytes % 16 != 0 || (ldx * eb) % 16 != 0) return FVGB_EINVAL;
+    // map entries are int32, so no more input rows can be named; row strides are 32-bit in the kernel
+    n_x = std::min<int64_t>(n_x, INT32_MAX);
+    if (n_x <= 1) ldx = c_in;
+    if (ldx * eb > UINT32_MAX) return FVGB_EINVAL;
     const int BN = tile_n(c_out);
     if (BN < 0) return FVGB_EINVAL;
     if (n_out == 0) return FVGB_OK;

@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(32 * kWarpLeaves) kmap_warp_kernel(KmapParams 
 // position -- against a window-leaf lookup, a mask test and a popcount per entry in
 // kmap_warp_kernel.  Rows are assembled in shared memory with stride 27 (odd: no bank conflicts),
 // which is the map's own layout, and copied out linearly.  Bound by the latency of a leaf's lookups; 1.31M rows of
-// a surface: 112 us with kmap_warp_kernel<3>, 84 us here; a dense 96^3 block 80 us, 40 us here.
+// a surface: 112 us with kmap_warp_kernel<3>, 84 us here; a dense 96^3 block 40 us.
 constexpr int kHaloLeaves = 4;  // target leaves (warps) per CTA
 struct HaloWarp {
     int32_t idx[1000];
