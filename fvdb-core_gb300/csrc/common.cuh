@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include <map>
 #include <mutex>
@@ -142,6 +143,39 @@ __device__ inline int32_t batch_of_warp(const int64_t *offsets, int32_t num_grid
     const int lane = threadIdx.x & 31;
     const bool past = lane < num_grids - 1 && __ldg(offsets + lane + 1) <= row;
     return __popc(__ballot_sync(0xffffffffu, past));
+}
+
+// A vector of V elements as one load or store of its bytes, kept as those bytes until it is used
+// (elements of 16 bits unpacked at the load take a register each while they wait).
+template <int BYTES>
+struct RawBytes;
+template <>
+struct RawBytes<16> { using type = uint4; };
+template <>
+struct RawBytes<8> { using type = uint2; };
+template <>
+struct RawBytes<4> { using type = uint32_t; };
+template <>
+struct RawBytes<2> { using type = uint16_t; };
+template <typename T, int V>
+using Raw = typename RawBytes<(int)sizeof(T) * V>::type;
+template <typename T, int V>
+struct Elems {
+    T v[V];
+};
+template <typename T, int V>
+__device__ __forceinline__ Raw<T, V> ld_raw(const T *p) { return *reinterpret_cast<const Raw<T, V> *>(p); }
+template <typename T, int V>
+__device__ __forceinline__ Elems<T, V> unpack(const Raw<T, V> &r) {
+    Elems<T, V> e;
+    memcpy(&e, &r, sizeof(e));
+    return e;
+}
+template <typename T, int V>
+__device__ __forceinline__ void st_vec(T *p, const Elems<T, V> &e) {
+    Raw<T, V> r;
+    memcpy(&r, &e, sizeof(r));
+    *reinterpret_cast<Raw<T, V> *>(p) = r;
 }
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }

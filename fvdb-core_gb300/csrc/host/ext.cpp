@@ -1425,6 +1425,20 @@ GridPtr grid_subdivided(const GridPtr &g, const std::vector<int64_t> &f, const s
 
 Tensor flat2d(const Tensor &t) { return t.reshape({t.size(0), -1}).contiguous(); }
 
+// Window map of a pooling pair (fvgb_window_map) where the leaf-by-leaf map kernel serves it, which
+// takes windows of up to 32 voxels (2^3 stride 2, 0.29M coarse voxels: 17 us; larger windows are
+// cheaper looked up by the pooling kernels themselves).  Lives for one call: 4 bytes per window
+// position.
+std::optional<Tensor> window_map(const GridPtr &fine, const GridPtr &coarse, const Vec3 &w, const Vec3 &st) {
+    const int64_t W = (int64_t)w.v[0] * w.v[1] * w.v[2];
+    if (W > 32 || fine->N == 0 || coarse->N == 0 || fine->B != coarse->B) return std::nullopt;
+    Tensor map = torch::empty({coarse->N, W}, torch::dtype(torch::kInt32).device(fine->device()));
+    FvgbGrid fv = fine->view(), cv = coarse->view();
+    check_status(fvgb_window_map(&fv, &cv, w.v, st.v, map.data_ptr<int32_t>(), cur_stream()), "window map");
+    return map;
+}
+constexpr int32_t kWindowSum = 2;  // mode of fvgb_pool_forward_map that sums the window rows
+
 // y [coarse N, C] = max / average pooling of x [fine N, *] (mode FVGB_POOL_MAX / FVGB_POOL_AVG)
 Tensor pool_forward(int32_t mode, const GridPtr &fine, const GridPtr &coarse, const std::vector<int64_t> &pool,
                     const std::vector<int64_t> &stride, const Tensor &x) {
@@ -1447,9 +1461,14 @@ Tensor pool_forward(int32_t mode, const GridPtr &fine, const GridPtr &coarse, co
     Tensor y = torch::empty({coarse->N, std::max<int64_t>(C, 1)}, x.options());
     if (C > 0 && coarse->N > 0) {
         FvgbGrid fv = fine->view(), cv = coarse->view();
-        check_status(fvgb_pool_forward(mode, fvgb_dtype(x), &fv, &cv, p.v, st.v, fine->N ? xf.data_ptr() : nullptr,
-                                       C, (int32_t)C, y.data_ptr(), C, cur_stream()),
-                     mode == FVGB_POOL_MAX ? "max_pool" : "avg_pool");
+        if (auto map = window_map(fine, coarse, p, st))
+            check_status(fvgb_pool_forward_map(mode, fvgb_dtype(x), map->data_ptr<int32_t>(), coarse->N, (int32_t)map->size(1),
+                                               xf.data_ptr(), C, (int32_t)C, y.data_ptr(), C, cur_stream()),
+                         mode == FVGB_POOL_MAX ? "max_pool" : "avg_pool");
+        else
+            check_status(fvgb_pool_forward(mode, fvgb_dtype(x), &fv, &cv, p.v, st.v, fine->N ? xf.data_ptr() : nullptr,
+                                           C, (int32_t)C, y.data_ptr(), C, cur_stream()),
+                         mode == FVGB_POOL_MAX ? "max_pool" : "avg_pool");
     }
     return y.narrow(1, 0, C).reshape(shape);
 }
@@ -1468,11 +1487,15 @@ Tensor pool_backward(int32_t mode, const GridPtr &fine, const GridPtr &coarse, c
     auto s = cur_stream();
     if (C == 0 || fine->N == 0) return torch::zeros_like(x);
     if (mode == FVGB_POOL_MAX && st.v[0] >= p.v[0] && st.v[1] >= p.v[1] && st.v[2] >= p.v[2]) {
-        Tensor dx = torch::zeros({fine->N, C}, x.options());
-        check_status(fvgb_maxpool_backward_disjoint(fvgb_dtype(x), &fv, &cv, p.v, st.v, xf.data_ptr(), C, (int32_t)C,
-                                                    coarse->N ? df.data_ptr() : nullptr, C, dx.data_ptr(), s),
-                     "max_pool backward");
-        return dx.reshape(x.sizes());
+        // windows that do not overlap: every row is written once, without a buffer to add into
+        if (auto map = window_map(fine, coarse, p, st)) {
+            Tensor dx = torch::zeros({fine->N, C}, x.options());
+            check_status(fvgb_maxpool_backward_map(fvgb_dtype(x), map->data_ptr<int32_t>(), coarse->N,
+                                                   (int32_t)map->size(1), xf.data_ptr(), C, (int32_t)C, df.data_ptr(), C,
+                                                   dx.data_ptr(), s),
+                         "max_pool backward");
+            return dx.reshape(x.sizes());
+        }
     }
     if (mode == FVGB_POOL_MAX) {
         const auto acc = x.scalar_type() == torch::kFloat64 ? torch::kFloat64 : torch::kFloat32;
@@ -1613,9 +1636,15 @@ Tensor upsample_backward(const GridPtr &coarse, const GridPtr &fine, const std::
     Tensor dx = torch::empty({coarse->N, std::max<int64_t>(C, 1)}, x.options());
     if (C > 0 && coarse->N > 0) {
         FvgbGrid fv = fine->view(), cv = coarse->view();
-        check_status(fvgb_upsample_backward(fvgb_dtype(x), &cv, &fv, f.v, fine->N ? df.data_ptr() : nullptr, C,
-                                            (int32_t)C, dx.data_ptr(), C, cur_stream()),
-                     "subdivide backward");
+        if (auto map = window_map(fine, coarse, f, f))
+            check_status(fvgb_pool_forward_map(kWindowSum, fvgb_dtype(x), map->data_ptr<int32_t>(), coarse->N,
+                                               (int32_t)map->size(1), df.data_ptr(), C, (int32_t)C, dx.data_ptr(), C,
+                                               cur_stream()),
+                         "subdivide backward");
+        else
+            check_status(fvgb_upsample_backward(fvgb_dtype(x), &cv, &fv, f.v, fine->N ? df.data_ptr() : nullptr, C,
+                                                (int32_t)C, dx.data_ptr(), C, cur_stream()),
+                         "subdivide backward");
     }
     return dx.narrow(1, 0, C).reshape(x.sizes());
 }

@@ -598,12 +598,12 @@ extern "C" int fvgb_kmap_row_order(const int32_t *kmap, int64_t n_out, int32_t K
     return launch_status();
 }
 
-extern "C" int fvgb_kmap_build(const FvgbGrid *src, const FvgbGrid *tgt, const int32_t ksize[3],
-                               const int32_t stride[3], int32_t *kmap, int64_t ld, int32_t *nbsizes,
-                               uint32_t *tile_mask, fvgb_stream_t stream) {
-    if (!src || !tgt || !ksize || !stride) return FVGB_EINVAL;
-    for (int a = 0; a < 3; ++a)
-        if (ksize[a] < 1 || stride[a] < 1) return FVGB_EINVAL;
+namespace fvgb {
+namespace {
+// start: source offset of kernel position 0, per user component
+int build_map(const FvgbGrid *src, const FvgbGrid *tgt, const int32_t ksize[3], const int32_t stride[3],
+              const int32_t start[3], int32_t *kmap, int64_t ld, int32_t *nbsizes, uint32_t *tile_mask,
+              fvgb_stream_t stream) {
     if (src->num_grids != tgt->num_grids) return FVGB_EINVAL;
     const int64_t K = (int64_t)ksize[0] * ksize[1] * ksize[2];
     if (K > (1 << 20) || ld < K) return FVGB_EINVAL;
@@ -616,10 +616,7 @@ extern "C" int fvgb_kmap_build(const FvgbGrid *src, const FvgbGrid *tgt, const i
     p.tgt = *tgt;
     p.K0 = ksize[0]; p.K1 = ksize[1]; p.K2 = ksize[2];
     p.S0 = stride[0]; p.S1 = stride[1]; p.S2 = stride[2];
-    // kernelStart = floor(-K/2 + 1) (ConvolutionKernelMap.cu:114-116)
-    p.st0 = (int32_t)floor(-ksize[0] / 2.0 + 1.0);
-    p.st1 = (int32_t)floor(-ksize[1] / 2.0 + 1.0);
-    p.st2 = (int32_t)floor(-ksize[2] / 2.0 + 1.0);
+    p.st0 = start[0]; p.st1 = start[1]; p.st2 = start[2];
     p.K = (int32_t)K;
     p.ld = ld;
     p.kmap = kmap;
@@ -631,7 +628,7 @@ extern "C" int fvgb_kmap_build(const FvgbGrid *src, const FvgbGrid *tgt, const i
     const int64_t W = (int64_t)span(p.S2, p.st2, p.K2) * span(p.S1, p.st1, p.K1) * span(p.S0, p.st0, p.K0);
     p.window = W <= kMaxWindow ? (int32_t)W : 0;
     if (!nbsizes && ld == 27 && ksize[0] == 3 && ksize[1] == 3 && ksize[2] == 3 && stride[0] == 1 && stride[1] == 1 &&
-        stride[2] == 1) {
+        stride[2] == 1 && start[0] == -1 && start[1] == -1 && start[2] == -1) {
         constexpr int smem = kHaloLeaves * (int)sizeof(HaloWarp);
         static_assert(smem <= 48 * 1024 && sizeof(HaloWarp) % 16 == 0, "halo tables of a CTA");
         kmap_halo3_kernel<<<(unsigned)ceil_div(tgt->num_leaves, (int64_t)kHaloLeaves), 32 * kHaloLeaves, smem,
@@ -662,6 +659,37 @@ extern "C" int fvgb_kmap_build(const FvgbGrid *src, const FvgbGrid *tgt, const i
     kmap_leaf_kernel<<<(unsigned)tgt->num_leaves, kKmapThreads, smem, as_stream(stream)>>>(p);
     count_launches(1);
     return launch_status();
+}
+}  // namespace
+}  // namespace fvgb
+
+extern "C" int fvgb_kmap_build(const FvgbGrid *src, const FvgbGrid *tgt, const int32_t ksize[3],
+                               const int32_t stride[3], int32_t *kmap, int64_t ld, int32_t *nbsizes,
+                               uint32_t *tile_mask, fvgb_stream_t stream) {
+    if (!src || !tgt || !ksize || !stride) return FVGB_EINVAL;
+    int32_t start[3];
+    for (int a = 0; a < 3; ++a) {
+        if (ksize[a] < 1 || stride[a] < 1) return FVGB_EINVAL;
+        // kernelStart = floor(-K/2 + 1) (ConvolutionKernelMap.cu:114-116)
+        start[a] = (int32_t)floor(-ksize[a] / 2.0 + 1.0);
+    }
+    return build_map(src, tgt, ksize, stride, start, kmap, ld, nbsizes, tile_mask, stream);
+}
+
+extern "C" int fvgb_window_map(const FvgbGrid *fine, const FvgbGrid *coarse, const int32_t window[3],
+                               const int32_t stride[3], int32_t *map, fvgb_stream_t stream) {
+    if (!fine || !coarse || !window || !stride) return FVGB_EINVAL;
+    // window axis a is ijk axis a; the kernel map's component 0 acts on axis 2
+    int32_t ks[3], st[3];
+    const int32_t start[3] = {0, 0, 0};
+    for (int a = 0; a < 3; ++a) {
+        if (window[a] < 1 || stride[a] < 1) return FVGB_EINVAL;
+        ks[a] = window[2 - a];
+        st[a] = stride[2 - a];
+    }
+    const int64_t W = (int64_t)ks[0] * ks[1] * ks[2];
+    if (W > 512) return FVGB_EINVAL;
+    return build_map(fine, coarse, ks, st, start, map, W, nullptr, nullptr, stream);
 }
 
 extern "C" int fvgb_kmap_transpose(const int32_t *kmap, int64_t n_out, int32_t K, int64_t ld, int32_t *mapT,

@@ -18,13 +18,14 @@
 // (the reference reads the row before its grid's first), and gradients of overlapping windows
 // (stride < pool factor) add up (the reference's concurrent assignments keep one of them).
 //
-// Lookups go through the grids' leaf hash.  A group of G lanes owns one output voxel: the lanes share
-// the window's lookups, then each lane moves one 16-byte vector of the row (G = the power of two >=
-// vectors per row, so a 64-channel BF16 row takes 8 lanes and a warp works on four voxels).  Bound
-// by HBM for large rows and by the lookups' latency, which the groups of an SM hide, for short ones.
-// 1.08M fine and 0.29M coarse voxels, 64 BF16 channels, factor 2 (GB300), one warp per voxel and one
-// element per lane before: max 190 us, its gradient 235 + 115 for the FP32 buffer, upsampling 464,
-// its gradient 192; here 139, 231, 46 and 144 us.
+// A group of G lanes owns one output voxel and each lane moves one 16-byte vector of its row (G = the
+// power of two >= vectors per row, so a 64-channel BF16 row takes 8 lanes and a warp works on four
+// voxels).  The window's rows come from a window map (fvgb_window_map, built leaf by leaf with one
+// hash probe per source leaf) or, without one, from one leaf-hash lookup per window position, which
+// the group's lanes share.  Bound by HBM with a map, by the lookups' latency without.  1.31M fine and
+// 0.36M coarse voxels, 64 BF16 channels, factor 2 (GB300), one warp per voxel and one element per
+// lane before: max 190 us, its gradient 235 + 115 for the FP32 buffer, upsampling 464, its gradient
+// 192; here 59, 113 + 43 for zeroing, 46 and 59, and 18 for each window map.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -80,12 +81,6 @@ __device__ __forceinline__ T mul_in(T a, double b) {
     return Num<T>::from(Num<T>::to(a) * Num<T>::to(Num<T>::from((A)b)));
 }
 
-// V consecutive channels, one aligned load or store
-template <typename T, int V>
-struct __align__(sizeof(T) * V) Vec {
-    T v[V];
-};
-
 // Lane groups of a CTA: G = 1 << gs lanes per output voxel, and the shared window indices of each.
 struct Groups {
     int gs;     // log2 lanes per group
@@ -120,12 +115,22 @@ __device__ __forceinline__ void window_indices(const FvgbGrid &g, int32_t b, int
     __syncwarp();
 }
 
-constexpr int kAhead = 4;  // window rows a lane has in flight
+// The same from a window map.
+__device__ __forceinline__ void map_indices(const int32_t *map, int64_t c, bool on, int W, int32_t *idx, int lane, int G) {
+    if (on)
+        for (int w = lane; w < W; w += G) idx[w] = __ldg(map + c * W + w);
+    __syncwarp();
+}
+
+constexpr int kAhead = 8;    // window rows a lane has in flight, 16 bytes each
+constexpr int kUpAhead = 4;  // rows of the upsampling copy, which its stores pace (eight: 67 us for 46)
 
 // Reduction over the window rows of every coarse voxel: maximum (MAX), or the sum, rounded and times
-// `avg` where SCALE.  Serves pooling and the upsampling gradient.
+// `avg` where SCALE.  Serves pooling and the upsampling gradient.  Over `map` where given (the grids
+// are then not read), else by lookups.
 template <typename T, int V, bool MAX, bool SCALE>
-__global__ void __launch_bounds__(kGroupThreads) window_reduce_kernel(FvgbGrid fine, FvgbGrid coarse, int3 pf, int3 st,
+__global__ void __launch_bounds__(kGroupThreads, 4) window_reduce_kernel(FvgbGrid fine, FvgbGrid coarse, int3 pf, int3 st,
+                                                                      const int32_t *__restrict__ map, int64_t n_coarse,
                                                                       Groups gr, const T *__restrict__ x, int64_t ldx,
                                                                       int32_t C, T *__restrict__ y, int64_t ldy,
                                                                       double avg) {
@@ -135,34 +140,39 @@ __global__ void __launch_bounds__(kGroupThreads) window_reduce_kernel(FvgbGrid f
     const int W = gr.W;
     int32_t *idx = widx + group * W;
     const int64_t c = (int64_t)blockIdx.x * (kGroupThreads >> gr.gs) + group;
-    const bool on = c < coarse.num_voxels;
-    int32_t b = 0;
-    int3 base = make_int3(0, 0, 0), ext = make_int3(0, 0, 0);
-    if (on) {
-        b = batch_of(coarse.voxel_offsets, coarse.num_grids, c);
-        base = make_int3(coarse.ijk[3 * c] * st.x, coarse.ijk[3 * c + 1] * st.y, coarse.ijk[3 * c + 2] * st.z);
-        ext = pf;
+    const bool on = c < n_coarse;
+    if (map) {
+        map_indices(map, c, on, W, idx, lane, G);
+    } else {
+        int32_t b = 0;
+        int3 base = make_int3(0, 0, 0), ext = make_int3(0, 0, 0);
+        if (on) {
+            b = batch_of(coarse.voxel_offsets, coarse.num_grids, c);
+            base = make_int3(coarse.ijk[3 * c] * st.x, coarse.ijk[3 * c + 1] * st.y, coarse.ijk[3 * c + 2] * st.z);
+            ext = pf;
+        }
+        window_indices(fine, b, base, ext, idx, lane, G);
     }
-    window_indices(fine, b, base, ext, idx, lane, G);
     if (!on) return;
     for (int32_t ch = lane * V; ch < C; ch += G * V) {
         A acc[V];
 #pragma unroll
         for (int e = 0; e < V; ++e) acc[e] = MAX ? (A)(-INFINITY) : (A)0;
         for (int w0 = 0; w0 < W; w0 += kAhead) {
-            Vec<T, V> p[kAhead];
+            Raw<T, V> p[kAhead];
             int32_t f[kAhead];
 #pragma unroll
             for (int u = 0; u < kAhead; ++u) {
                 f[u] = w0 + u < W ? idx[w0 + u] : -1;
-                if (f[u] >= 0) p[u] = *reinterpret_cast<const Vec<T, V> *>(x + (int64_t)f[u] * ldx + ch);
+                if (f[u] >= 0) p[u] = ld_raw<T, V>(x + (int64_t)f[u] * ldx + ch);
             }
 #pragma unroll
             for (int u = 0; u < kAhead; ++u) {
                 if (f[u] < 0) continue;
+                const Elems<T, V> row = unpack<T, V>(p[u]);
 #pragma unroll
                 for (int e = 0; e < V; ++e) {
-                    const A v = Num<T>::to(p[u].v[e]);
+                    const A v = Num<T>::to(row.v[e]);
                     if constexpr (MAX) {
                         if constexpr (sizeof(A) == 8) acc[e] = fmax(v, acc[e]);
                         else acc[e] = fmaxf(v, acc[e]);
@@ -172,10 +182,10 @@ __global__ void __launch_bounds__(kGroupThreads) window_reduce_kernel(FvgbGrid f
                 }
             }
         }
-        Vec<T, V> o;
+        Elems<T, V> o;
 #pragma unroll
         for (int e = 0; e < V; ++e) o.v[e] = SCALE ? mul_in<T>(Num<T>::from(acc[e]), avg) : Num<T>::from(acc[e]);
-        *reinterpret_cast<Vec<T, V> *>(y + c * ldy + ch) = o;
+        st_vec<T, V>(y + c * ldy + ch, o);
     }
 }
 
@@ -184,8 +194,8 @@ __global__ void __launch_bounds__(kGroupThreads) window_reduce_kernel(FvgbGrid f
 // window's first strict maximum, zero elsewhere -- without a buffer to add into.  Rows of voxels in
 // no window stay as the caller zeroed them.
 template <typename T, int V>
-__global__ void __launch_bounds__(kGroupThreads) maxpool_bwd_disjoint_kernel(FvgbGrid fine, FvgbGrid coarse, int3 pf,
-                                                                             int3 st, Groups gr,
+__global__ void __launch_bounds__(kGroupThreads, 4) maxpool_bwd_disjoint_kernel(const int32_t *__restrict__ map,
+                                                                             int64_t n_coarse, Groups gr,
                                                                              const T *__restrict__ x, int64_t ldx,
                                                                              int32_t C, const T *__restrict__ dy,
                                                                              int64_t lddy, T *__restrict__ dx) {
@@ -195,36 +205,30 @@ __global__ void __launch_bounds__(kGroupThreads) maxpool_bwd_disjoint_kernel(Fvg
     const int W = gr.W;
     int32_t *idx = widx + group * W;
     const int64_t c = (int64_t)blockIdx.x * (kGroupThreads >> gr.gs) + group;
-    const bool on = c < coarse.num_voxels;
-    int32_t b = 0;
-    int3 base = make_int3(0, 0, 0), ext = make_int3(0, 0, 0);
-    if (on) {
-        b = batch_of(coarse.voxel_offsets, coarse.num_grids, c);
-        base = make_int3(coarse.ijk[3 * c] * st.x, coarse.ijk[3 * c + 1] * st.y, coarse.ijk[3 * c + 2] * st.z);
-        ext = pf;
-    }
-    window_indices(fine, b, base, ext, idx, lane, G);
+    const bool on = c < n_coarse;
+    map_indices(map, c, on, W, idx, lane, G);
     if (!on) return;
     for (int32_t ch = lane * V; ch < C; ch += G * V) {
-        const Vec<T, V> g = *reinterpret_cast<const Vec<T, V> *>(dy + c * lddy + ch);
+        const Elems<T, V> g = unpack<T, V>(ld_raw<T, V>(dy + c * lddy + ch));
         A best[V];
         int32_t arg[V];
 #pragma unroll
         for (int e = 0; e < V; ++e) best[e] = (A)(-INFINITY), arg[e] = -1;
         for (int w0 = 0; w0 < W; w0 += kAhead) {
-            Vec<T, V> p[kAhead];
+            Raw<T, V> p[kAhead];
             int32_t f[kAhead];
 #pragma unroll
             for (int u = 0; u < kAhead; ++u) {
                 f[u] = w0 + u < W ? idx[w0 + u] : -1;
-                if (f[u] >= 0) p[u] = *reinterpret_cast<const Vec<T, V> *>(x + (int64_t)f[u] * ldx + ch);
+                if (f[u] >= 0) p[u] = ld_raw<T, V>(x + (int64_t)f[u] * ldx + ch);
             }
 #pragma unroll
             for (int u = 0; u < kAhead; ++u) {
                 if (f[u] < 0) continue;
+                const Elems<T, V> row = unpack<T, V>(p[u]);
 #pragma unroll
                 for (int e = 0; e < V; ++e) {
-                    const A v = Num<T>::to(p[u].v[e]);
+                    const A v = Num<T>::to(row.v[e]);
                     if (v > best[e]) best[e] = v, arg[e] = f[u];
                 }
             }
@@ -232,10 +236,10 @@ __global__ void __launch_bounds__(kGroupThreads) maxpool_bwd_disjoint_kernel(Fvg
         for (int w = 0; w < W; ++w) {
             const int32_t f = idx[w];
             if (f < 0) continue;
-            Vec<T, V> o;
+            Elems<T, V> o;
 #pragma unroll
             for (int e = 0; e < V; ++e) o.v[e] = arg[e] == f ? g.v[e] : Num<T>::from((A)0);
-            *reinterpret_cast<Vec<T, V> *>(dx + (int64_t)f * C + ch) = o;
+            st_vec<T, V>(dx + (int64_t)f * C + ch, o);
         }
     }
 }
@@ -277,7 +281,7 @@ __global__ void __launch_bounds__(kPoolWarps * 32) maxpool_bwd_kernel(FvgbGrid f
 // Average-pool gradient, gathered per fine voxel: the coarse voxels whose window holds fine
 // voxel f are c with c*s <= f < c*s + p per axis.
 template <typename T, int V>
-__global__ void __launch_bounds__(kGroupThreads) avgpool_bwd_kernel(FvgbGrid fine, FvgbGrid coarse, int3 pf, int3 st,
+__global__ void __launch_bounds__(kGroupThreads, 4) avgpool_bwd_kernel(FvgbGrid fine, FvgbGrid coarse, int3 pf, int3 st,
                                                                     Groups gr, int32_t C, const T *__restrict__ dy,
                                                                     int64_t lddy, T *__restrict__ dx, int64_t lddx,
                                                                     double avg) {
@@ -309,7 +313,7 @@ __global__ void __launch_bounds__(kGroupThreads) avgpool_bwd_kernel(FvgbGrid fin
         for (int w = 0; w < W; ++w) {
             const int32_t c = idx[w];
             if (c < 0) continue;
-            const Vec<T, V> p = *reinterpret_cast<const Vec<T, V> *>(dy + (int64_t)c * lddy + ch);
+            const Elems<T, V> p = unpack<T, V>(ld_raw<T, V>(dy + (int64_t)c * lddy + ch));
 #pragma unroll
             for (int e = 0; e < V; ++e) {
                 const A g = Num<T>::to(mul_in<T>(p.v[e], avg));
@@ -317,10 +321,10 @@ __global__ void __launch_bounds__(kGroupThreads) avgpool_bwd_kernel(FvgbGrid fin
             }
             any = true;
         }
-        Vec<T, V> o;
+        Elems<T, V> o;
 #pragma unroll
         for (int e = 0; e < V; ++e) o.v[e] = Num<T>::from(acc[e]);
-        *reinterpret_cast<Vec<T, V> *>(dx + f * lddx + ch) = o;
+        st_vec<T, V>(dx + f * lddx + ch, o);
     }
 }
 
@@ -328,7 +332,7 @@ __global__ void __launch_bounds__(kGroupThreads) avgpool_bwd_kernel(FvgbGrid fin
 // takes 32 consecutive fine voxels: each lane looks up one parent, then the warp's lane groups copy
 // the rows.
 template <typename T, int V>
-__global__ void __launch_bounds__(kGroupThreads) upsample_fwd_kernel(FvgbGrid coarse, FvgbGrid fine, int3 fac, int gs,
+__global__ void __launch_bounds__(kGroupThreads, 4) upsample_fwd_kernel(FvgbGrid coarse, FvgbGrid fine, int3 fac, int gs,
                                                                      const T *__restrict__ x, int64_t ldx, int32_t C,
                                                                      T *__restrict__ y, int64_t ldy) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -343,25 +347,21 @@ __global__ void __launch_bounds__(kGroupThreads) upsample_fwd_kernel(FvgbGrid co
         c = (int32_t)voxel_at(coarse, b, fdiv(fine.ijk[3 * fl], fac.x), fdiv(fine.ijk[3 * fl + 1], fac.y),
                               fdiv(fine.ijk[3 * fl + 2], fac.z));
     }
-    for (int i0 = 0; i0 < G; i0 += kAhead) {  // G = 32 / per rounds of `per` voxels, kAhead at a time
-        int32_t p[kAhead];
+    for (int i0 = 0; i0 < G; i0 += kUpAhead) {  // G = 32 / per rounds of `per` voxels, kUpAhead at a time
+        int32_t p[kUpAhead];
 #pragma unroll
-        for (int u = 0; u < kAhead; ++u) p[u] = __shfl_sync(0xffffffffu, c, ((i0 + u) * per + sub) & 31);
+        for (int u = 0; u < kUpAhead; ++u) p[u] = __shfl_sync(0xffffffffu, c, ((i0 + u) * per + sub) & 31);
         for (int32_t ch = gl * V; ch < C; ch += G * V) {
-            Vec<T, V> o[kAhead];
+            Raw<T, V> o[kUpAhead];  // copied as bytes; zero is all zero bits in every type
 #pragma unroll
-            for (int u = 0; u < kAhead; ++u) {
-                if (p[u] >= 0 && i0 + u < G) {
-                    o[u] = *reinterpret_cast<const Vec<T, V> *>(x + (int64_t)p[u] * ldx + ch);
-                } else {
-#pragma unroll
-                    for (int e = 0; e < V; ++e) o[u].v[e] = Num<T>::from(0.0f);
-                }
+            for (int u = 0; u < kUpAhead; ++u) {
+                o[u] = Raw<T, V>{};
+                if (p[u] >= 0 && i0 + u < G) o[u] = ld_raw<T, V>(x + (int64_t)p[u] * ldx + ch);
             }
 #pragma unroll
-            for (int u = 0; u < kAhead; ++u) {
+            for (int u = 0; u < kUpAhead; ++u) {
                 const int64_t f = f0 + (i0 + u) * per + sub;
-                if (i0 + u < G && f < fine.num_voxels) *reinterpret_cast<Vec<T, V> *>(y + f * ldy + ch) = o[u];
+                if (i0 + u < G && f < fine.num_voxels) *reinterpret_cast<Raw<T, V> *>(y + f * ldy + ch) = o[u];
             }
         }
     }
@@ -426,21 +426,35 @@ void by_width(bool vec, F &&f) {
 }
 unsigned group_blocks(int64_t items, const Groups &g) { return (unsigned)ceil_div(items, (int64_t)(kGroupThreads >> g.gs)); }
 
+constexpr int kPoolSum = 2;  // mode of the window sum (upsampling gradient)
+
+// Windows over a map, or by lookups between two grids (map null).
+struct Windows {
+    FvgbGrid fine, coarse;
+    int3 pf, st;
+    const int32_t *map;
+    int64_t n_coarse;
+    int W;
+};
+
 template <typename T>
 struct PoolFwd {
-    static void run(int mode, const FvgbGrid &f, const FvgbGrid &c, int3 pf, int3 st, const void *x, int64_t ldx,
-                    int32_t C, void *y, int64_t ldy, cudaStream_t s) {
-        const double avg = 1.0 / ((double)pf.x * pf.y * pf.z);
-        by_width<T>(whole_vectors<T>(C, {x, y}, {ldx, ldy}), [&](auto w) {
-            constexpr int V = decltype(w)::value;
-            const Groups g = groups_for(C / V, pf.x * pf.y * pf.z);
-            const unsigned blocks = group_blocks(c.num_voxels, g);
+    static void run(int mode, const Windows &w, const void *x, int64_t ldx, int32_t C, void *y, int64_t ldy,
+                    cudaStream_t s) {
+        const double avg = 1.0 / (double)w.W;
+        by_width<T>(whole_vectors<T>(C, {x, y}, {ldx, ldy}), [&](auto v) {
+            constexpr int V = decltype(v)::value;
+            const Groups g = groups_for(C / V, w.W);
+            const unsigned blocks = group_blocks(w.n_coarse, g);
             if (mode == FVGB_POOL_MAX)
                 window_reduce_kernel<T, V, true, false><<<blocks, kGroupThreads, g.smem, s>>>(
-                    f, c, pf, st, g, (const T *)x, ldx, C, (T *)y, ldy, avg);
-            else
+                    w.fine, w.coarse, w.pf, w.st, w.map, w.n_coarse, g, (const T *)x, ldx, C, (T *)y, ldy, avg);
+            else if (mode == FVGB_POOL_AVG)
                 window_reduce_kernel<T, V, false, true><<<blocks, kGroupThreads, g.smem, s>>>(
-                    f, c, pf, st, g, (const T *)x, ldx, C, (T *)y, ldy, avg);
+                    w.fine, w.coarse, w.pf, w.st, w.map, w.n_coarse, g, (const T *)x, ldx, C, (T *)y, ldy, avg);
+            else
+                window_reduce_kernel<T, V, false, false><<<blocks, kGroupThreads, g.smem, s>>>(
+                    w.fine, w.coarse, w.pf, w.st, w.map, w.n_coarse, g, (const T *)x, ldx, C, (T *)y, ldy, avg);
         });
     }
 };
@@ -454,13 +468,13 @@ struct MaxPoolBwd {
 };
 template <typename T>
 struct MaxPoolBwdDisjoint {
-    static void run(const FvgbGrid &f, const FvgbGrid &c, int3 pf, int3 st, const void *x, int64_t ldx, int32_t C,
-                    const void *dy, int64_t lddy, void *dx, cudaStream_t s) {
-        by_width<T>(whole_vectors<T>(C, {x, dy, dx}, {ldx, lddy}), [&](auto w) {
-            constexpr int V = decltype(w)::value;
-            const Groups g = groups_for(C / V, pf.x * pf.y * pf.z);
-            maxpool_bwd_disjoint_kernel<T, V><<<group_blocks(c.num_voxels, g), kGroupThreads, g.smem, s>>>(
-                f, c, pf, st, g, (const T *)x, ldx, C, (const T *)dy, lddy, (T *)dx);
+    static void run(const int32_t *map, int64_t n_coarse, int W, const void *x, int64_t ldx, int32_t C, const void *dy,
+                    int64_t lddy, void *dx, cudaStream_t s) {
+        by_width<T>(whole_vectors<T>(C, {x, dy, dx}, {ldx, lddy}), [&](auto v) {
+            constexpr int V = decltype(v)::value;
+            const Groups g = groups_for(C / V, W);
+            maxpool_bwd_disjoint_kernel<T, V><<<group_blocks(n_coarse, g), kGroupThreads, g.smem, s>>>(
+                map, n_coarse, g, (const T *)x, ldx, C, (const T *)dy, lddy, (T *)dx);
         });
     }
 };
@@ -491,19 +505,6 @@ struct UpFwd {
         });
     }
 };
-template <typename T>
-struct UpBwd {
-    static void run(const FvgbGrid &c, const FvgbGrid &f, int3 fac, const void *dy, int64_t lddy, int32_t C, void *dx,
-                    int64_t lddx, cudaStream_t s) {
-        by_width<T>(whole_vectors<T>(C, {dy, dx}, {lddy, lddx}), [&](auto w) {
-            constexpr int V = decltype(w)::value;
-            const Groups g = groups_for(C / V, fac.x * fac.y * fac.z);
-            window_reduce_kernel<T, V, false, false><<<group_blocks(c.num_voxels, g), kGroupThreads, g.smem, s>>>(
-                f, c, fac, fac, g, (const T *)dy, lddy, C, (T *)dx, lddx, 1.0);
-        });
-    }
-};
-
 bool grids_ok(const FvgbGrid *a, const FvgbGrid *b) {
     return a && b && a->num_grids == b->num_grids && a->num_voxels >= 0 && b->num_voxels >= 0;
 }
@@ -521,8 +522,9 @@ extern "C" int fvgb_pool_forward(int32_t mode, int32_t dtype, const FvgbGrid *fi
         return FVGB_EINVAL;
     if (coarse->num_voxels == 0) return FVGB_OK;
     if (!y || (fine->num_voxels > 0 && !x)) return FVGB_EINVAL;
-    return dispatch_dtype<PoolFwd>(dtype, mode, *fine, *coarse, make_int3(pool[0], pool[1], pool[2]),
-                                   make_int3(stride[0], stride[1], stride[2]), x, ldx, C, y, ldy, as_stream(stream));
+    const Windows w{*fine,   *coarse, make_int3(pool[0], pool[1], pool[2]), make_int3(stride[0], stride[1], stride[2]),
+                    nullptr, coarse->num_voxels, pool[0] * pool[1] * pool[2]};
+    return dispatch_dtype<PoolFwd>(dtype, mode, w, x, ldx, C, y, ldy, as_stream(stream));
 }
 
 extern "C" int fvgb_maxpool_backward(int32_t dtype, const FvgbGrid *fine, const FvgbGrid *coarse, const int32_t pool[3],
@@ -538,19 +540,28 @@ extern "C" int fvgb_maxpool_backward(int32_t dtype, const FvgbGrid *fine, const 
                                       as_stream(stream));
 }
 
-extern "C" int fvgb_maxpool_backward_disjoint(int32_t dtype, const FvgbGrid *fine, const FvgbGrid *coarse,
-                                              const int32_t pool[3], const int32_t stride[3], const void *x, int64_t ldx,
-                                              int32_t C, const void *dy, int64_t lddy, void *dx, fvgb_stream_t stream) {
-    if (!grids_ok(fine, coarse) || !vec_ok(pool, kMaxWindow) || !vec_ok(stride, 1 << 30) || C < 1 || ldx < C ||
-        lddy < C)
+extern "C" int fvgb_pool_forward_map(int32_t mode, int32_t dtype, const int32_t *map, int64_t n_coarse, int32_t window,
+                                     const void *x, int64_t ldx, int32_t C, void *y, int64_t ldy,
+                                     fvgb_stream_t stream) {
+    if ((mode != FVGB_POOL_MAX && mode != FVGB_POOL_AVG && mode != kPoolSum) || n_coarse < 0 || window < 1 ||
+        window > kMaxWindow || C < 1 || ldx < C || ldy < C)
         return FVGB_EINVAL;
-    for (int a = 0; a < 3; ++a)
-        if (stride[a] < pool[a]) return FVGB_EINVAL;
-    if (coarse->num_voxels == 0 || fine->num_voxels == 0) return FVGB_OK;
-    if (!x || !dy || !dx) return FVGB_EINVAL;
-    return dispatch_dtype<MaxPoolBwdDisjoint>(dtype, *fine, *coarse, make_int3(pool[0], pool[1], pool[2]),
-                                              make_int3(stride[0], stride[1], stride[2]), x, ldx, C, dy, lddy, dx,
-                                              as_stream(stream));
+    if (n_coarse == 0) return FVGB_OK;
+    if (!map || !y) return FVGB_EINVAL;
+    Windows w{};
+    w.map = map;
+    w.n_coarse = n_coarse;
+    w.W = window;
+    return dispatch_dtype<PoolFwd>(dtype, mode, w, x, ldx, C, y, ldy, as_stream(stream));
+}
+
+extern "C" int fvgb_maxpool_backward_map(int32_t dtype, const int32_t *map, int64_t n_coarse, int32_t window,
+                                         const void *x, int64_t ldx, int32_t C, const void *dy, int64_t lddy, void *dx,
+                                         fvgb_stream_t stream) {
+    if (n_coarse < 0 || window < 1 || window > kMaxWindow || C < 1 || ldx < C || lddy < C) return FVGB_EINVAL;
+    if (n_coarse == 0) return FVGB_OK;
+    if (!map || !x || !dy || !dx) return FVGB_EINVAL;
+    return dispatch_dtype<MaxPoolBwdDisjoint>(dtype, map, n_coarse, window, x, ldx, C, dy, lddy, dx, as_stream(stream));
 }
 
 extern "C" int fvgb_avgpool_backward(int32_t dtype, const FvgbGrid *fine, const FvgbGrid *coarse, const int32_t pool[3],
@@ -582,8 +593,9 @@ extern "C" int fvgb_upsample_backward(int32_t dtype, const FvgbGrid *coarse, con
     if (!grids_ok(fine, coarse) || !vec_ok(factor, kMaxWindow) || C < 1 || lddy < C || lddx < C) return FVGB_EINVAL;
     if (coarse->num_voxels == 0) return FVGB_OK;
     if (!dx || (fine->num_voxels > 0 && !dy)) return FVGB_EINVAL;
-    return dispatch_dtype<UpBwd>(dtype, *coarse, *fine, make_int3(factor[0], factor[1], factor[2]), dy, lddy, C, dx,
-                                 lddx, as_stream(stream));
+    const int3 f = make_int3(factor[0], factor[1], factor[2]);
+    const Windows w{*fine, *coarse, f, f, nullptr, coarse->num_voxels, factor[0] * factor[1] * factor[2]};
+    return dispatch_dtype<PoolFwd>(dtype, kPoolSum, w, dy, lddy, C, dx, lddx, as_stream(stream));
 }
 
 extern "C" int fvgb_subdivide_candidates(const FvgbGrid *coarse, const int32_t factor[3], const uint8_t *mask,

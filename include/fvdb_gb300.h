@@ -523,12 +523,18 @@ int fvgb_pool_forward(int32_t mode, int32_t dtype, const FvgbGrid *fine, const F
 int fvgb_maxpool_backward(int32_t dtype, const FvgbGrid *fine, const FvgbGrid *coarse, const int32_t pool[3],
                           const int32_t stride[3], const void *x, int64_t ldx, int32_t C, const void *dy, int64_t lddy,
                           void *dx_acc, fvgb_stream_t stream);
-/* Max-pool gradient of windows that do not overlap (stride >= pool on every axis, else FVGB_EINVAL):
- * written into dx [fine n, C] of the data type, which the caller zeroes (rows of voxels in no window
- * are not touched). */
-int fvgb_maxpool_backward_disjoint(int32_t dtype, const FvgbGrid *fine, const FvgbGrid *coarse, const int32_t pool[3],
-                                   const int32_t stride[3], const void *x, int64_t ldx, int32_t C, const void *dy,
-                                   int64_t lddy, void *dx, fvgb_stream_t stream);
+/* Window map of a pooling or upsampling pair: map[c, w] = row of fine voxel c*stride + (i, j, k), -1
+ * where absent, w = (i * window[1] + j) * window[2] + k; int32 [coarse n, window volume <= 512]. */
+int fvgb_window_map(const FvgbGrid *fine, const FvgbGrid *coarse, const int32_t window[3], const int32_t stride[3],
+                    int32_t *map, fvgb_stream_t stream);
+/* fvgb_pool_forward over a window map; mode 2 sums the window rows (the upsampling gradient). */
+int fvgb_pool_forward_map(int32_t mode, int32_t dtype, const int32_t *map, int64_t n_coarse, int32_t window,
+                          const void *x, int64_t ldx, int32_t C, void *y, int64_t ldy, fvgb_stream_t stream);
+/* Max-pool gradient over the window map of windows that do not overlap (stride >= pool on every
+ * axis): written into dx [fine n, C] of the data type, which the caller zeroes (rows of voxels in no
+ * window are not touched). */
+int fvgb_maxpool_backward_map(int32_t dtype, const int32_t *map, int64_t n_coarse, int32_t window, const void *x,
+                              int64_t ldx, int32_t C, const void *dy, int64_t lddy, void *dx, fvgb_stream_t stream);
 /* Average-pool gradient dx [fine n, C] = sum over the windows holding a fine voxel of
  * dy * 1/(pool volume).  Replaces DownsampleGridAvgPoolBackward (DownsampleGridAvgPool.cu:68-112,203-283). */
 int fvgb_avgpool_backward(int32_t dtype, const FvgbGrid *fine, const FvgbGrid *coarse, const int32_t pool[3],
