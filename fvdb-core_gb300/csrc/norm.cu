@@ -8,8 +8,8 @@
 //
 // Bound by HBM: forward reads x twice and writes y, backward reads x and dy twice and writes dx.
 // 1.08M voxels x 64 channels in four grids, BF16, forward and backward together (GB300): 184 ms as
-// torch segment sums (their backward adds every row into one of four gradient rows), 0.52 ms here:
-// statistics 59 us, normalisation 71, gradient sums 159, dx 114, the merges 70.
+// torch segment sums (their backward adds every row into one of four gradient rows), 0.37 ms here:
+// statistics 61 us, normalisation 48, gradient sums 66, dx 69, the merges 31.
 //
 // A CTA owns a chunk of consecutive rows; every thread keeps one vector column (V channels of one
 // group) and kRowsPerThread rows of it in registers, so the chunk's variance is taken about the
@@ -30,6 +30,7 @@ namespace {
 constexpr int kNT = 256;
 constexpr int kRowsPerThread = 8;  // forward: one operand
 constexpr int kRowsBackward = 4;   // backward: two operands in as many registers
+constexpr int kSumIters = 4;       // row groups a CTA adds up before it folds its thread rows
 
 template <typename T>
 struct NNum;
@@ -56,12 +57,6 @@ struct NNum<__half> {
     using A = float;
     __device__ static float to(__half v) { return __half2float(v); }
     __device__ static __half from(float v) { return __float2half_rn(v); }
-};
-
-// V consecutive elements as one aligned load / store (V * sizeof(T) <= 16)
-template <typename T, int V>
-struct __align__(sizeof(T) * V) Pack {
-    T v[V];
 };
 
 struct NormArgs {
@@ -106,7 +101,7 @@ __device__ __forceinline__ A column_sum(A v, A *sm, int rr, int qq, int QB, int 
 
 // stat[slot][q] = {mean, M2} of the slot's rows in vector column q
 template <typename T, int V>
-__global__ void __launch_bounds__(kNT) gn_stats_kernel(NormArgs a, const T *__restrict__ x,
+__global__ void __launch_bounds__(kNT, 4) gn_stats_kernel(NormArgs a, const T *__restrict__ x,
                                                        typename NNum<T>::A *__restrict__ stat) {
     using A = typename NNum<T>::A;
     __shared__ A sm[kNT];
@@ -117,11 +112,11 @@ __global__ void __launch_bounds__(kNT) gn_stats_kernel(NormArgs a, const T *__re
     while (half * 2 < a.rpi) half *= 2;
     const int64_t r0 = (int64_t)blockIdx.x * a.chunk_rows, r1 = min(a.n, r0 + a.chunk_rows);
     const int32_t b0 = batch_of_warp(a.joff, a.B, r0), b1 = batch_of_warp(a.joff, a.B, r1 - 1);
-    Pack<T, V> p[kRowsPerThread];
+    Raw<T, V> p[kRowsPerThread];
 #pragma unroll
     for (int i = 0; i < kRowsPerThread; ++i) {
         const int64_t r = r0 + rr + (int64_t)i * a.rpi;
-        if (col && r < r1) p[i] = *reinterpret_cast<const Pack<T, V> *>(x + r * a.C + (int64_t)q * V);
+        if (col && r < r1) p[i] = ld_raw<T, V>(x + r * a.C + (int64_t)q * V);
     }
     for (int32_t b = b0; b <= b1; ++b) {
         int64_t lo, hi;
@@ -133,21 +128,25 @@ __global__ void __launch_bounds__(kNT) gn_stats_kernel(NormArgs a, const T *__re
 #pragma unroll
         for (int i = 0; i < kRowsPerThread; ++i) {
             const int64_t r = r0 + rr + (int64_t)i * a.rpi;
-            if (col && r >= lo && r < hi)
+            if (col && r >= lo && r < hi) {
+                const Elems<T, V> x_ = unpack<T, V>(p[i]);
 #pragma unroll
-                for (int e = 0; e < V; ++e) s += NNum<T>::to(p[i].v[e]);
+                for (int e = 0; e < V; ++e) s += NNum<T>::to(x_.v[e]);
+            }
         }
         const A mean = column_sum<A>(s, sm, rr, qq, a.QB, a.rpi, half) / (A)((hi - lo) * V);
         A m2 = 0;
 #pragma unroll
         for (int i = 0; i < kRowsPerThread; ++i) {
             const int64_t r = r0 + rr + (int64_t)i * a.rpi;
-            if (col && r >= lo && r < hi)
+            if (col && r >= lo && r < hi) {
+                const Elems<T, V> x_ = unpack<T, V>(p[i]);
 #pragma unroll
                 for (int e = 0; e < V; ++e) {
-                    const A d = NNum<T>::to(p[i].v[e]) - mean;
+                    const A d = NNum<T>::to(x_.v[e]) - mean;
                     m2 += d * d;
                 }
+            }
         }
         m2 = column_sum<A>(m2, sm, rr, qq, a.QB, a.rpi, half);
         if (col && rr == 0) {
@@ -213,7 +212,7 @@ __global__ void __launch_bounds__(kNT) gn_merge_kernel(NormArgs a, int32_t V, co
 }
 
 template <typename T, int V>
-__global__ void __launch_bounds__(kNT) gn_apply_kernel(NormArgs a, const T *__restrict__ x,
+__global__ void __launch_bounds__(kNT, 4) gn_apply_kernel(NormArgs a, const T *__restrict__ x,
                                                        const typename NNum<T>::A *__restrict__ mean,
                                                        const typename NNum<T>::A *__restrict__ rstd,
                                                        const typename NNum<T>::A *__restrict__ w,
@@ -225,11 +224,11 @@ __global__ void __launch_bounds__(kNT) gn_apply_kernel(NormArgs a, const T *__re
     const int64_t r0 = (int64_t)blockIdx.x * a.chunk_rows, r1 = min(a.n, r0 + a.chunk_rows);
     const int32_t b0 = batch_of_warp(a.joff, a.B, r0), b1 = batch_of_warp(a.joff, a.B, r1 - 1);
     if (rr >= a.rpi || q >= a.Q) return;
-    Pack<T, V> p[kRowsPerThread];
+    Raw<T, V> p[kRowsPerThread];
 #pragma unroll
     for (int i = 0; i < kRowsPerThread; ++i) {
         const int64_t r = r0 + rr + (int64_t)i * a.rpi;
-        if (r < r1) p[i] = *reinterpret_cast<const Pack<T, V> *>(x + r * a.C + (int64_t)q * V);
+        if (r < r1) p[i] = ld_raw<T, V>(x + r * a.C + (int64_t)q * V);
     }
     const int32_t g = q * V / a.cpg;
     A wv[V], bv[V];
@@ -244,10 +243,11 @@ __global__ void __launch_bounds__(kNT) gn_apply_kernel(NormArgs a, const T *__re
         if (r >= r1) continue;
         const int64_t k = (int64_t)(b0 == b1 ? b0 : batch_of(a.joff, a.B, r)) * a.G + g;
         const A m = mean[k], s = rstd[k];
-        Pack<T, V> o;
+        const Elems<T, V> x_ = unpack<T, V>(p[i]);
+        Elems<T, V> o;
 #pragma unroll
-        for (int e = 0; e < V; ++e) o.v[e] = NNum<T>::from((NNum<T>::to(p[i].v[e]) - m) * s * wv[e] + bv[e]);
-        *reinterpret_cast<Pack<T, V> *>(y + r * a.C + (int64_t)q * V) = o;
+        for (int e = 0; e < V; ++e) o.v[e] = NNum<T>::from((NNum<T>::to(x_.v[e]) - m) * s * wv[e] + bv[e]);
+        st_vec<T, V>(y + r * a.C + (int64_t)q * V, o);
     }
 }
 
@@ -267,15 +267,6 @@ __global__ void __launch_bounds__(kNT, 4) gn_grad_sums_kernel(NormArgs a, const 
     while (half * 2 < a.rpi) half *= 2;
     const int64_t r0 = (int64_t)blockIdx.x * a.chunk_rows, r1 = min(a.n, r0 + a.chunk_rows);
     const int32_t b0 = batch_of_warp(a.joff, a.B, r0), b1 = batch_of_warp(a.joff, a.B, r1 - 1);
-    Pack<T, V> p[kRowsBackward], d[kRowsBackward];
-#pragma unroll
-    for (int i = 0; i < kRowsBackward; ++i) {
-        const int64_t r = r0 + rr + (int64_t)i * a.rpi;
-        if (col && r < r1) {
-            p[i] = *reinterpret_cast<const Pack<T, V> *>(x + r * a.C + (int64_t)q * V);
-            d[i] = *reinterpret_cast<const Pack<T, V> *>(dy + r * a.C + (int64_t)q * V);
-        }
-    }
     for (int32_t b = b0; b <= b1; ++b) {
         int64_t lo, hi;
         grid_rows(a, b, lo, hi);
@@ -288,15 +279,27 @@ __global__ void __launch_bounds__(kNT, 4) gn_grad_sums_kernel(NormArgs a, const 
         if (col) {
             const int64_t k = (int64_t)b * a.G + q * V / a.cpg;
             const A m = mean[k], rs = rstd[k];
+            const int64_t group = (int64_t)a.rpi * kRowsBackward;
+            for (int64_t g0 = r0 + (lo - r0) / group * group; g0 < hi; g0 += group) {
+                Raw<T, V> p[kRowsBackward], d[kRowsBackward];
 #pragma unroll
-            for (int i = 0; i < kRowsBackward; ++i) {
-                const int64_t r = r0 + rr + (int64_t)i * a.rpi;
-                if (r < lo || r >= hi) continue;
+                for (int i = 0; i < kRowsBackward; ++i) {
+                    const int64_t r = g0 + rr + (int64_t)i * a.rpi;
+                    if (r < lo || r >= hi) continue;
+                    p[i] = ld_raw<T, V>(x + r * a.C + (int64_t)q * V);
+                    d[i] = ld_raw<T, V>(dy + r * a.C + (int64_t)q * V);
+                }
 #pragma unroll
-                for (int e = 0; e < V; ++e) {
-                    const A g = NNum<T>::to(d[i].v[e]);
-                    s1[e] += g;
-                    s2[e] += g * ((NNum<T>::to(p[i].v[e]) - m) * rs);
+                for (int i = 0; i < kRowsBackward; ++i) {
+                    const int64_t r = g0 + rr + (int64_t)i * a.rpi;
+                    if (r < lo || r >= hi) continue;
+                    const Elems<T, V> x_ = unpack<T, V>(p[i]), g_ = unpack<T, V>(d[i]);
+#pragma unroll
+                    for (int e = 0; e < V; ++e) {
+                        const A g = NNum<T>::to(g_.v[e]);
+                        s1[e] += g;
+                        s2[e] += g * ((NNum<T>::to(x_.v[e]) - m) * rs);
+                    }
                 }
             }
         }
@@ -354,8 +357,10 @@ __global__ void __launch_bounds__(kNT, 4) gn_grad_sums_kernel(NormArgs a, const 
     }
 }
 
-// CTA per (grid, 32 of the 2C sums): sums[b][j] over the grid's slots in FP64 (fixed order)
+// CTA per (grid, 32 of the 2C sums, one of kSlices interleaved shares of the grid's slots):
+// sums[z][b][j] in FP64 (fixed order)
 constexpr int kSumWarps = 32;
+constexpr int kSlices = 8;
 template <typename A>
 __global__ void __launch_bounds__(32 * kSumWarps) gn_grad_merge_kernel(NormArgs a, const A *__restrict__ part,
                                                                        double *__restrict__ sums) {
@@ -367,14 +372,16 @@ __global__ void __launch_bounds__(32 * kSumWarps) gn_grad_merge_kernel(NormArgs 
     grid_chunks(a, b, lo, hi, first, last);
     double s = 0;
     if (j < 2 * a.C)
-        for (int64_t c = first + warp; c <= last; c += kSumWarps) s += (double)part[(c + b) * 2 * a.C + j];
+#pragma unroll 4
+        for (int64_t c = first + blockIdx.z * kSumWarps + warp; c <= last; c += kSumWarps * kSlices)
+            s += (double)part[(c + b) * 2 * a.C + j];
     sm[warp][lane] = s;
     __syncthreads();
     if (warp == 0 && j < 2 * a.C) {
         double t = 0;
 #pragma unroll
         for (int w = 0; w < kSumWarps; ++w) t += sm[w][lane];
-        sums[(int64_t)b * 2 * a.C + j] = t;
+        sums[((int64_t)blockIdx.z * a.B + b) * 2 * a.C + j] = t;
     }
 }
 
@@ -384,6 +391,12 @@ __global__ void gn_coef_kernel(NormArgs a, const double *__restrict__ sums, cons
                                A *__restrict__ coef, A *__restrict__ dw, A *__restrict__ db) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t bg = (int64_t)a.B * a.G;
+    auto sum_of = [&](int32_t b, int32_t j) {
+        double t = 0;
+#pragma unroll
+        for (int z = 0; z < kSlices; ++z) t += sums[((int64_t)z * a.B + b) * 2 * a.C + j];
+        return t;
+    };
     if (i < bg) {
         const int32_t b = (int32_t)(i / a.G), g = (int32_t)(i % a.G);
         int64_t lo, hi;
@@ -392,8 +405,8 @@ __global__ void gn_coef_kernel(NormArgs a, const double *__restrict__ sums, cons
         double s1 = 0, s2 = 0;
         for (int32_t c = g * a.cpg; c < (g + 1) * a.cpg; ++c) {
             const double wc = w ? (double)w[c] : 1.0;
-            s1 += wc * sums[(int64_t)b * 2 * a.C + c];
-            s2 += wc * sums[(int64_t)b * 2 * a.C + a.C + c];
+            s1 += wc * sum_of(b, c);
+            s2 += wc * sum_of(b, a.C + c);
         }
         coef[2 * i] = (A)(count > 0 ? s1 / count : 0.0);
         coef[2 * i + 1] = (A)(count > 0 ? s2 / count : 0.0);
@@ -401,8 +414,8 @@ __global__ void gn_coef_kernel(NormArgs a, const double *__restrict__ sums, cons
         const int32_t c = (int32_t)(i - bg);
         double s1 = 0, s2 = 0;
         for (int32_t b = 0; b < a.B; ++b) {
-            s1 += sums[(int64_t)b * 2 * a.C + c];
-            s2 += sums[(int64_t)b * 2 * a.C + a.C + c];
+            s1 += sum_of(b, c);
+            s2 += sum_of(b, a.C + c);
         }
         if (db) db[c] = (A)s1;
         if (dw) dw[c] = (A)s2;
@@ -422,13 +435,13 @@ __global__ void __launch_bounds__(kNT, 4) gn_dx_kernel(NormArgs a, const T *__re
     const int64_t r0 = (int64_t)blockIdx.x * a.chunk_rows, r1 = min(a.n, r0 + a.chunk_rows);
     const int32_t b0 = batch_of_warp(a.joff, a.B, r0), b1 = batch_of_warp(a.joff, a.B, r1 - 1);
     if (rr >= a.rpi || q >= a.Q) return;
-    Pack<T, V> p[kRowsBackward], d[kRowsBackward];
+    Raw<T, V> p[kRowsBackward], d[kRowsBackward];
 #pragma unroll
     for (int i = 0; i < kRowsBackward; ++i) {
         const int64_t r = r0 + rr + (int64_t)i * a.rpi;
         if (r < r1) {
-            p[i] = *reinterpret_cast<const Pack<T, V> *>(x + r * a.C + (int64_t)q * V);
-            d[i] = *reinterpret_cast<const Pack<T, V> *>(dy + r * a.C + (int64_t)q * V);
+            p[i] = ld_raw<T, V>(x + r * a.C + (int64_t)q * V);
+            d[i] = ld_raw<T, V>(dy + r * a.C + (int64_t)q * V);
         }
     }
     const int32_t g = q * V / a.cpg;
@@ -441,13 +454,14 @@ __global__ void __launch_bounds__(kNT, 4) gn_dx_kernel(NormArgs a, const T *__re
         if (r >= r1) continue;
         const int64_t k = (int64_t)(b0 == b1 ? b0 : batch_of(a.joff, a.B, r)) * a.G + g;
         const A m = mean[k], s = rstd[k], c1 = coef[2 * k], c2 = coef[2 * k + 1];
-        Pack<T, V> o;
+        const Elems<T, V> x_ = unpack<T, V>(p[i]), g_ = unpack<T, V>(d[i]);
+        Elems<T, V> o;
 #pragma unroll
         for (int e = 0; e < V; ++e) {
-            const A xhat = (NNum<T>::to(p[i].v[e]) - m) * s;
-            o.v[e] = NNum<T>::from(s * (NNum<T>::to(d[i].v[e]) * wv[e] - c1 - xhat * c2));
+            const A xhat = (NNum<T>::to(x_.v[e]) - m) * s;
+            o.v[e] = NNum<T>::from(s * (NNum<T>::to(g_.v[e]) * wv[e] - c1 - xhat * c2));
         }
-        *reinterpret_cast<Pack<T, V> *>(dx + r * a.C + (int64_t)q * V) = o;
+        st_vec<T, V>(dx + r * a.C + (int64_t)q * V, o);
     }
 }
 
@@ -463,7 +477,7 @@ int pick_vec(int32_t cpg, int elem, const void *const *ptrs, int n_ptrs) {
     return v;
 }
 
-NormArgs norm_args(const int64_t *joff, int32_t B, int64_t n, int32_t C, int32_t G, int V, bool backward) {
+NormArgs norm_args(const int64_t *joff, int32_t B, int64_t n, int32_t C, int32_t G, int V, int rows) {
     NormArgs a;
     a.joff = joff;
     a.B = B;
@@ -474,7 +488,7 @@ NormArgs norm_args(const int64_t *joff, int32_t B, int64_t n, int32_t C, int32_t
     a.Q = C / V;
     a.QB = a.Q < kNT ? a.Q : kNT;
     a.rpi = kNT / a.QB;
-    a.chunk_rows = (int64_t)a.rpi * (backward ? kRowsBackward : kRowsPerThread);
+    a.chunk_rows = (int64_t)a.rpi * rows;
     return a;
 }
 
@@ -484,13 +498,13 @@ size_t norm_ws(int64_t n, int32_t B, int32_t C, int32_t G, size_t acc, bool back
     size_t need = 0;
     for (int V = 1; V <= 8; V *= 2) {
         if ((C / G) % V) break;
-        const NormArgs a = norm_args(nullptr, B, n, C, G, V, backward);
+        const NormArgs a = norm_args(nullptr, B, n, C, G, V, backward ? kRowsBackward * kSumIters : kRowsPerThread);
         const size_t slots = (size_t)ceil_div(n > 0 ? n : 1, a.chunk_rows) + (size_t)B;
         const size_t s = backward ? slots * 2 * (size_t)C * acc : slots * (size_t)a.Q * 2 * acc;
         if (s > need) need = s;
     }
     need = (need + 255) & ~(size_t)255;
-    if (backward) need += (((size_t)B * 2 * C * 8 + 255) & ~(size_t)255) + (((size_t)B * G * 2 * acc + 255) & ~(size_t)255);
+    if (backward) need += (((size_t)kSlices * B * 2 * C * 8 + 255) & ~(size_t)255) + (((size_t)B * G * 2 * acc + 255) & ~(size_t)255);
     return need + 256;
 }
 
@@ -514,15 +528,18 @@ void run_backward(const NormArgs &a, const void *x, const void *dy, const void *
     A *part = (A *)p;
     p += ((size_t)(chunks + a.B) * 2 * a.C * sizeof(A) + 255) & ~(size_t)255;
     double *sums = (double *)p;
-    p += ((size_t)a.B * 2 * a.C * 8 + 255) & ~(size_t)255;
+    p += ((size_t)kSlices * a.B * 2 * a.C * 8 + 255) & ~(size_t)255;
     A *coef = (A *)p;
     const dim3 grid((unsigned)chunks, (unsigned)ceil_div(a.Q, a.QB));
     gn_grad_sums_kernel<T, V><<<grid, kNT, 0, s>>>(a, (const T *)x, (const T *)dy, (const A *)mean, (const A *)rstd, part);
-    gn_grad_merge_kernel<A><<<dim3((unsigned)a.B, (unsigned)ceil_div(2 * a.C, 32)), 32 * kSumWarps, 0, s>>>(a, part, sums);
+    gn_grad_merge_kernel<A><<<dim3((unsigned)a.B, (unsigned)ceil_div(2 * a.C, 32), kSlices), 32 * kSumWarps, 0, s>>>(a, part, sums);
     gn_coef_kernel<A><<<(unsigned)ceil_div((int64_t)a.B * a.G + a.C, 128), 128, 0, s>>>(a, sums, (const A *)w, coef,
                                                                                        (A *)dw, (A *)db);
+    NormArgs ax = a;  // dx: one row group per CTA
+    ax.chunk_rows = (int64_t)a.rpi * kRowsBackward;
+    const dim3 grid_dx((unsigned)ceil_div(a.n, ax.chunk_rows), grid.y);
     if (dx)
-        gn_dx_kernel<T, V><<<grid, kNT, 0, s>>>(a, (const T *)x, (const T *)dy, (const A *)mean, (const A *)rstd,
+        gn_dx_kernel<T, V><<<grid_dx, kNT, 0, s>>>(ax, (const T *)x, (const T *)dy, (const A *)mean, (const A *)rstd,
                                                 (const A *)w, coef, (T *)dx);
 }
 
@@ -586,7 +603,7 @@ extern "C" int fvgb_group_norm_forward(int32_t dtype, const void *x, int64_t n, 
     if (!workspace || workspace_bytes < need) return FVGB_ENOSPACE;
     const void *ptrs[2] = {x, y};
     const int V = pick_vec(channels / groups, elem_size(dtype), ptrs, 2);
-    const NormArgs a = norm_args(joffsets, num_grids, n, channels, groups, V, false);
+    const NormArgs a = norm_args(joffsets, num_grids, n, channels, groups, V, kRowsPerThread);
     void *ws = reinterpret_cast<void *>(((uintptr_t)workspace + 255) & ~(uintptr_t)255);
     st = by_dtype(dtype, [&](auto *t) {
         using T = std::remove_pointer_t<decltype(t)>;
@@ -611,7 +628,7 @@ extern "C" int fvgb_group_norm_backward(int32_t dtype, const void *x, const void
     if (!workspace || workspace_bytes < need) return FVGB_ENOSPACE;
     const void *ptrs[3] = {x, dy, dx};
     const int V = pick_vec(channels / groups, elem_size(dtype), ptrs, 3);
-    const NormArgs a = norm_args(joffsets, num_grids, n, channels, groups, V, true);
+    const NormArgs a = norm_args(joffsets, num_grids, n, channels, groups, V, kRowsBackward * kSumIters);
     void *ws = reinterpret_cast<void *>(((uintptr_t)workspace + 255) & ~(uintptr_t)255);
     st = by_dtype(dtype, [&](auto *t) {
         using T = std::remove_pointer_t<decltype(t)>;
