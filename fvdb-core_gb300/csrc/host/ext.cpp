@@ -419,7 +419,10 @@ GridPtr build_coarse_by_leaves(const GridPtr &g, const Vec3 &f, const int32_t lo
         c10::cuda::CUDAStreamGuard sg(side);
         pb->out_ijk = torch::empty({std::max<int64_t>(g->N, 1), 3}, i32);
         pb->leaf_ids = torch::empty({std::max<int64_t>(g->N, 1)}, i32);
-        pb->meta = torch::zeros({B + 4}, torch::dtype(torch::kInt64).device(dev));
+        pb->meta = torch::empty({B + 4}, torch::dtype(torch::kInt64).device(dev));
+        TORCH_CHECK(cudaMemsetAsync(pb->meta.data_ptr<int64_t>(), 0, (B + 4) * sizeof(int64_t), side.stream()) ==
+                        cudaSuccess,
+                    "coarse grid: clearing the counts failed");
         size_t wsb = 0;
         check_status(fvgb_coarse_grid_workspace(g->L, &wsb), "coarse grid (workspace)");
         Tensor ws = workspace(wsb, dev);
@@ -639,12 +642,18 @@ Tensor build_kmap(const GridPtr &src, const GridPtr &tgt, const Vec3 &ks, const 
     TORCH_CHECK_VALUE(src->B == tgt->B, "source and target grids must have the same grid count");
     const int64_t npad = (tgt->N + 127) / 128 * 128;
     Tensor kmap = torch::empty({npad, K}, torch::dtype(torch::kInt32).device(tgt->device()));
-    if (npad > tgt->N) kmap.narrow(0, tgt->N, npad - tgt->N).fill_(-1);
+    cudaStream_t cs = reinterpret_cast<cudaStream_t>(cur_stream());
+    bool ok = true;
+    if (npad > tgt->N)  // padding rows are -1
+        ok = cudaMemsetAsync(kmap.data_ptr<int32_t>() + tgt->N * K, 0xff, (npad - tgt->N) * K * sizeof(int32_t), cs) ==
+             cudaSuccess;
     uint32_t *tm = nullptr;
     if (tile_mask && K <= 32) {
-        *tile_mask = torch::zeros({std::max<int64_t>(npad / 128, 1)}, kmap.options());
+        *tile_mask = torch::empty({std::max<int64_t>(npad / 128, 1)}, kmap.options());
         tm = reinterpret_cast<uint32_t *>(tile_mask->data_ptr<int32_t>());
+        ok = ok && cudaMemsetAsync(tm, 0, tile_mask->numel() * sizeof(int32_t), cs) == cudaSuccess;
     }
+    TORCH_CHECK(ok, "kernel map build: clearing the padding failed");
     FvgbGrid s = src->view(), t = tgt->view();
     check_status(fvgb_kmap_build(&s, &t, ks.v, st.v, kmap.data_ptr<int32_t>(), K, nullptr, tm, cur_stream()),
                  "kernel map build");
@@ -1673,6 +1682,29 @@ std::vector<Tensor> bias_relu_backward(const Tensor &dy_in, const std::optional<
     return {out, db};
 }
 
+// (scale, shift) FP32 of an inference-mode batch norm; every parameter [c], contiguous, of one type.
+std::vector<Tensor> fold_batch_norm(const Tensor &mean, const Tensor &var, const std::optional<Tensor> &weight,
+                                    const std::optional<Tensor> &bias, double eps) {
+    c10::cuda::CUDAGuard guard(mean.device());
+    const int64_t c = mean.size(0);
+    Tensor st = torch::empty({2, c}, mean.options().dtype(torch::kFloat32));
+    check_status(fvgb_fold_batch_norm(fvgb_dtype(mean), mean.data_ptr(), var.data_ptr(),
+                                      weight ? weight->data_ptr() : nullptr, bias ? bias->data_ptr() : nullptr, (int32_t)c,
+                                      (float)eps, st.data_ptr<float>(), st.data_ptr<float>() + c, cur_stream()),
+                 "batch norm folding");
+    return {st.select(0, 0), st.select(0, 1)};
+}
+
+// bias * s + t, FP32
+Tensor fold_bias(const Tensor &bias, const Tensor &s, const Tensor &t) {
+    c10::cuda::CUDAGuard guard(bias.device());
+    Tensor shift = torch::empty_like(t);
+    check_status(fvgb_fold_bias(fvgb_dtype(bias), bias.data_ptr(), s.data_ptr<float>(), t.data_ptr<float>(),
+                                (int32_t)bias.size(0), shift.data_ptr<float>(), cur_stream()),
+                 "bias folding");
+    return shift;
+}
+
 // Group normalisation of jagged rows: (y, mean, rstd); weight / bias in the accumulation type.
 std::vector<Tensor> group_norm_forward(const Tensor &x_in, const Tensor &joff, int64_t groups,
                                        const std::optional<Tensor> &weight, const std::optional<Tensor> &bias,
@@ -1795,6 +1827,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("halo_conv", &halo_conv, py::call_guard<py::gil_scoped_release>());
     m.def("halo_wgrad", &halo_wgrad, py::call_guard<py::gil_scoped_release>());
     m.def("halo_backward", &halo_backward, py::call_guard<py::gil_scoped_release>());
+    m.def("fold_batch_norm", &fold_batch_norm);
+    m.def("fold_bias", &fold_bias);
     m.def("bias_relu_backward", &bias_relu_backward, py::call_guard<py::gil_scoped_release>());
     m.def("group_norm_forward", &group_norm_forward, py::call_guard<py::gil_scoped_release>());
     m.def("group_norm_backward", &group_norm_backward, py::call_guard<py::gil_scoped_release>());

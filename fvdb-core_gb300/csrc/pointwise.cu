@@ -111,6 +111,44 @@ __global__ void __launch_bounds__(32 * kWarps) column_merge_kernel(const A *__re
     }
 }
 
+// s = rsqrt(var + eps) * weight, t = -mean * s + bias: an inference-mode batch norm as
+// x -> x s + t, in FP32 with one rounding per operation; every parameter of one type, weight and bias
+// optional.
+template <typename T>
+__global__ void fold_batch_norm_kernel(const T *__restrict__ mean, const T *__restrict__ var, const T *__restrict__ weight,
+                                       const T *__restrict__ bias, int32_t c, float eps, float *__restrict__ s,
+                                       float *__restrict__ t) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= c) return;
+    float a = rsqrtf(__fadd_rn((float)up(var[i]), eps));
+    if (weight) a = __fmul_rn(a, (float)up(weight[i]));
+    float b = __fmul_rn(-(float)up(mean[i]), a);
+    if (bias) b = __fadd_rn(b, (float)up(bias[i]));
+    s[i] = a;
+    t[i] = b;
+}
+
+// shift = bias * s + t (FP32)
+template <typename T>
+__global__ void fold_bias_kernel(const T *__restrict__ bias, const float *__restrict__ s, const float *__restrict__ t,
+                                 int32_t c, float *__restrict__ shift) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < c) shift[i] = __fadd_rn(__fmul_rn((float)up(bias[i]), s[i]), t[i]);
+}
+
+template <typename F>
+int by_type(int32_t dtype, F &&f) {
+    switch (dtype) {
+        case FVGB_F32: f((float *)nullptr); break;
+        case FVGB_F64: f((double *)nullptr); break;
+        case FVGB_BF16: f((__nv_bfloat16 *)nullptr); break;
+        case FVGB_F16: f((__half *)nullptr); break;
+        default: return FVGB_ETYPE;
+    }
+    count_launches(1);
+    return launch_status();
+}
+
 int64_t part_ctas(int64_t n) { return std::min<int64_t>(std::max<int64_t>(ceil_div(n, 64), 1), (int64_t)device_sm_count() * 4); }
 
 template <typename T, int V>
@@ -162,4 +200,24 @@ extern "C" int fvgb_bias_relu_backward(int32_t dtype, const void *dy, const void
     }
     count_launches(dbias ? 2 : 1);
     return launch_status();
+}
+
+extern "C" int fvgb_fold_batch_norm(int32_t dtype, const void *mean, const void *var, const void *weight,
+                                    const void *bias, int32_t c, float eps, float *scale, float *shift,
+                                    fvgb_stream_t stream) {
+    if (c < 1 || !mean || !var || !scale || !shift) return FVGB_EINVAL;
+    return by_type(dtype, [&](auto *p) {
+        using T = std::remove_pointer_t<decltype(p)>;
+        fold_batch_norm_kernel<T><<<(unsigned)ceil_div(c, 128), 128, 0, as_stream(stream)>>>(
+            (const T *)mean, (const T *)var, (const T *)weight, (const T *)bias, c, eps, scale, shift);
+    });
+}
+
+extern "C" int fvgb_fold_bias(int32_t dtype, const void *bias, const float *s, const float *t, int32_t c, float *shift,
+                              fvgb_stream_t stream) {
+    if (c < 1 || !bias || !s || !t || !shift) return FVGB_EINVAL;
+    return by_type(dtype, [&](auto *p) {
+        using T = std::remove_pointer_t<decltype(p)>;
+        fold_bias_kernel<T><<<(unsigned)ceil_div(c, 128), 128, 0, as_stream(stream)>>>((const T *)bias, s, t, c, shift);
+    });
 }

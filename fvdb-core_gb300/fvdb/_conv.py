@@ -13,6 +13,7 @@ from __future__ import annotations
 import torch
 
 from . import _lib
+from ._dispatch import plain_cuda, wants_grad
 
 
 class SparseConvFunction(torch.autograd.Function):
@@ -66,4 +67,6 @@ def sparse_conv(features: torch.Tensor, weights: torch.Tensor, pack_impl, transp
     the output clamped at zero, in the contraction's epilogue on the tensor-core path (one pass
     over the output instead of two or three).  `scale` ([C_out], optional, inference only)
     multiplies the contraction before the bias: an eval-mode batch norm folded into the layer."""
+    if not wants_grad(features, weights, bias, scale) and plain_cuda(features, weights, bias, scale):
+        return _lib.load().conv_forward(features, weights, pack_impl, transposed, bias, relu, scale)[0]
     return SparseConvFunction.apply(features, weights, pack_impl, transposed, bias, relu, scale)

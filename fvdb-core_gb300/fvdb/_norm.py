@@ -6,6 +6,7 @@ from __future__ import annotations
 import torch
 
 from . import _lib
+from ._dispatch import plain_cuda
 
 _DTYPES = (torch.float32, torch.float64, torch.bfloat16, torch.float16)
 
@@ -36,16 +37,9 @@ def group_norm_kernel_takes(x: torch.Tensor, weight, bias) -> bool:
     """Whether the kernels serve this call: plain CUDA tensors outside function transforms,
     forward-mode differentiation and tracing (where composed operations carry the derivative)."""
     params = [p for p in (weight, bias) if p is not None]
-    if not x.is_cuda or x.dtype not in _DTYPES or x.shape[1] > 65535:
+    if not plain_cuda(x, weight, bias) or x.dtype not in _DTYPES or x.shape[1] > 65535:
         return False
-    if (weight is None) != (bias is None) or any(not p.is_floating_point() or p.device != x.device for p in params):
-        return False
-    if any(type(t) not in (torch.Tensor, torch.nn.Parameter) for t in (x, *params)):
-        return False
-    if torch.jit.is_tracing() or torch.compiler.is_compiling() or torch._C._are_functorch_transforms_active():
-        return False
-    return not any(torch.autograd.forward_ad.unpack_dual(t).tangent is not None for t in (x, *params)) \
-        if torch.autograd.forward_ad._current_level >= 0 else True
+    return (weight is None) == (bias is None) and all(p.is_floating_point() and p.device == x.device for p in params)
 
 
 class GroupNormFunction(torch.autograd.Function):

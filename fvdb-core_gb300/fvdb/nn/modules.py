@@ -16,10 +16,24 @@ from typing import Optional, Sequence, Union
 import torch
 import torch.nn as nn
 
+from .. import _lib
+from .._dispatch import plain_cuda
 from .._norm import GroupNormFunction, group_norm_composed, group_norm_kernel_takes
 from ..grid_batch import GridBatch
 from ..sparse_conv_pack_info import ConvPackBackend, SparseConvPackInfo
 from .vdbtensor import VDBTensor
+
+
+def _vectors(*tensors) -> bool:
+    """Contiguous 1-D tensors of one size and one type: what the parameter-folding kernels read
+    (None entries are skipped)."""
+    ts = [t for t in tensors if t is not None]
+    return all(t.dim() == 1 and t.is_contiguous() and t.shape == ts[0].shape and t.device == ts[0].device and
+               t.dtype == ts[0].dtype and t.is_floating_point() and t.numel() > 0 for t in ts)
+
+
+def _detached(t):
+    return None if t is None else t.detach()
 
 
 class SparseConv3d(nn.Module):
@@ -104,7 +118,11 @@ class SparseConv3d(nn.Module):
         """(scale, shift) of conv * scale + shift with a following per-channel affine map
         (s, t) folded in: scale = s, shift = bias * s + t (FP32)."""
         s, t = (v.detach().float() for v in out_affine)
-        return s, (t if self.bias is None else self.bias.detach().float() * s + t)
+        if self.bias is None:
+            return s, t
+        if plain_cuda(s, t, self.bias) and _vectors(s, t) and _vectors(self.bias) and self.bias.shape == s.shape:
+            return s, _lib.load().fold_bias(self.bias.detach(), s, t)
+        return s, self.bias.detach().float() * s + t
 
     def forward(self, input: VDBTensor, out_grid: Optional[GridBatch] = None, *, relu: bool = False,
                 out_affine=None) -> VDBTensor:
@@ -203,6 +221,10 @@ class BatchNorm(nn.BatchNorm1d):
         running statistics, or None when it normalises with batch statistics."""
         if self.training or self.running_mean is None or self.running_var is None:
             return None
+        params = (self.running_mean, self.running_var, self.weight, self.bias)
+        if plain_cuda(*params) and _vectors(*params):
+            # one launch in place of seven
+            return tuple(_lib.load().fold_batch_norm(*map(_detached, params), self.eps))
         s = torch.rsqrt(self.running_var.detach().float() + self.eps)
         if self.weight is not None:
             s = s * self.weight.detach().float()

@@ -600,6 +600,13 @@ int fvgb_halo_wgrad(int32_t dtype, const FvgbGrid *grid, const void *x, int64_t 
 int fvgb_bias_relu_backward_workspace(int32_t dtype, int64_t n, int32_t c, size_t *bytes);
 int fvgb_bias_relu_backward(int32_t dtype, const void *dy, const void *y, int64_t n, int32_t c, void *out,
                             void *dbias, void *workspace, size_t workspace_bytes, fvgb_stream_t stream);
+/* An inference-mode batch norm as x -> x * scale + shift: scale = rsqrt(var + eps) * weight,
+ * shift = bias - mean * scale, FP32 [c]; parameters of one dtype (weight, bias may be null). */
+int fvgb_fold_batch_norm(int32_t dtype, const void *mean, const void *var, const void *weight, const void *bias,
+                         int32_t c, float eps, float *scale, float *shift, fvgb_stream_t stream);
+/* shift = bias * s + t: a convolution's bias ahead of such a map. */
+int fvgb_fold_bias(int32_t dtype, const void *bias, const float *s, const float *t, int32_t c, float *shift,
+                   fvgb_stream_t stream);
 
 /* ------------------------------------------------------------------------------------------
  * Group normalisation of jagged features: x [n, channels] contiguous rows, grid b's voxels are
