@@ -279,11 +279,8 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
                         src[u][q] = (uint32_t)v;
                     }
                 }
-                bool go = true;
-                if (lane == 0) go = mbar_wait(&empty[stage], phase ^ 1, abort);
-                go = __shfl_sync(0xffffffffu, go, 0);
-                __syncwarp();
-                if (!go) {
+                // every lane polls: one lane polling for the warp and passing the answer on cost 7 %
+                if (!mbar_wait_warp(&empty[stage], phase ^ 1, abort)) {
                     ok = false;
                     break;
                 }

@@ -1029,7 +1029,6 @@ bool self_mirrored(const PackPtr &p) {
 // pack / map_t (optional): the pack info that owns `map` and whether `map` is its transposed map;
 // with them, shapes the planned kernel takes run over the pack's cached tile plan.
 Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tensor &Wkio, bool transpose_w,
-                   const std::optional<Tensor> &tile_mask = std::nullopt,
                    const std::optional<Tensor> &bias = std::nullopt, PackPtr pack = nullptr, bool map_t = false,
                    bool relu = false, const std::optional<Tensor> &out_scale = std::nullopt, bool mirror = false,
                    bool reuse = false) {
@@ -1064,7 +1063,6 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
                          "weight pack");
             if (same_type) derived_put(Wkio, tag, packed);
         }
-        const uint32_t *tm = tile_mask ? reinterpret_cast<const uint32_t *>(tile_mask->data_ptr<int32_t>()) : nullptr;
         Tensor b32, s32;
         if (bias) b32 = bias->to(torch::kFloat32).contiguous();
         if (out_scale) s32 = out_scale->to(torch::kFloat32).contiguous();
@@ -1086,7 +1084,10 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
             return y;
         }
         const Tensor &m_used = order ? order->map : map;
-        const uint32_t *tm_used = order ? reinterpret_cast<const uint32_t *>(order->mask.data_ptr<int32_t>()) : tm;
+        // the index order's tile masks are made only where no row order stands in for them
+        const std::optional<Tensor> mask = order ? std::optional<Tensor>(order->mask) : pack ? pack_tile_mask(pack, map_t)
+                                                                                             : std::nullopt;
+        const uint32_t *tm_used = mask ? reinterpret_cast<const uint32_t *>(mask->data_ptr<int32_t>()) : nullptr;
         check_status(fvgb_conv_fwd_tc_16bit(dt, x.data_ptr(), x.size(0), (int32_t)cin, x.stride(0),
                                             m_used.data_ptr<int32_t>(), n_out, (int32_t)K,
                                             order ? order->rows.data_ptr<int32_t>() : nullptr, tm_used,
@@ -1137,10 +1138,10 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
 }
 
 // dW[k] = sum_m x[map[m,k]]^T dy[m]   -> [K, Cin, Cout]
-// order (optional): the map's row order, which the tensor-core form runs over where it exists.
+// pack, map_t: the owner of `map`; the tensor-core form runs over the map's row order where some
+// contraction has built one.
 Tensor gather_wgrad(const Tensor &x, const Tensor &map, int64_t n_out, const Tensor &dy, int64_t K,
-                    const std::optional<Tensor> &tile_mask = std::nullopt,
-                    const std::optional<RowOrder> &order = std::nullopt) {
+                    PackPtr pack = nullptr, bool map_t = false) {
     c10::cuda::CUDAGuard guard(x.device());
     const int64_t cin = x.size(1), cout = dy.size(1);
     const auto dtype = x.scalar_type();
@@ -1156,7 +1157,9 @@ Tensor gather_wgrad(const Tensor &x, const Tensor &map, int64_t n_out, const Ten
         size_t wsb = 0;
         check_status(fvgb_tc_wgrad_16bit_workspace(n_out, (int32_t)K, (int32_t)cin, (int32_t)cout, &wsb), "wgrad workspace");
         Tensor ws = workspace(wsb, x.device());
-        const std::optional<Tensor> mask = order ? std::optional<Tensor>(order->mask) : tile_mask;
+        const std::optional<RowOrder> order = pack ? built_row_order(pack, map_t) : std::nullopt;
+        const std::optional<Tensor> mask = order ? std::optional<Tensor>(order->mask) : pack ? pack_tile_mask(pack, map_t)
+                                                                                             : std::nullopt;
         const uint32_t *tm = mask ? reinterpret_cast<const uint32_t *>(mask->data_ptr<int32_t>()) : nullptr;
         check_status(fvgb_conv_wgrad_tc_16bit(fvgb_dtype(xx), xx.data_ptr(), xx.size(0), (int32_t)cin, xx.stride(0),
                                               (order ? order->map : map).data_ptr<int32_t>(), n_out, (int32_t)K,
@@ -1248,7 +1251,7 @@ std::vector<Tensor> conv_forward(const Tensor &x, const Tensor &weights, PackPtr
     const bool map_t = transposed && !mirror;
     const int64_t n_out = transposed ? n_src : n_tgt;
     if (n_out == 0) return {torch::empty({0, cout}, x.options()), Wkio};
-    Tensor y = gather_gemm(x, map_t ? pack_kmap_t(p) : pack_kmap(p), n_out, Wkio, false, pack_tile_mask(p, map_t), bias,
+    Tensor y = gather_gemm(x, map_t ? pack_kmap_t(p) : pack_kmap(p), n_out, Wkio, false, bias,
                            p, map_t, relu, out_scale, mirror, has_backward && self_mirrored(p));
     return {y, Wkio};
 }
@@ -1264,19 +1267,19 @@ std::vector<Tensor> conv_backward(const Tensor &dy_in, const Tensor &x, const Te
     if (!transposed) {
         // dgrad: dx[i] = sum_k dy[mapT[i,k]] W[k]^T ;  wgrad: dW[k] = sum_m x[map[m,k]]^T dy[m]
         if (need_dx && mirror)
-            dx = gather_gemm(dy, pack_kmap(p), p->src->N, Wkio, true, pack_tile_mask(p, false), std::nullopt, p, false,
+            dx = gather_gemm(dy, pack_kmap(p), p->src->N, Wkio, true, std::nullopt, p, false,
                              false, std::nullopt, true);
         else if (need_dx)
-            dx = gather_gemm(dy, pack_kmap_t(p), p->src->N, Wkio, true, pack_tile_mask(p, true), std::nullopt, p, true);
+            dx = gather_gemm(dy, pack_kmap_t(p), p->src->N, Wkio, true, std::nullopt, p, true);
         if (need_dw)
-            dW = gather_wgrad(x, pack_kmap(p), p->tgt->N, dy, K, pack_tile_mask(p, false), built_row_order(p, false));
+            dW = gather_wgrad(x, pack_kmap(p), p->tgt->N, dy, K, p, false);
     } else {
         if (need_dx)
-            dx = gather_gemm(dy, pack_kmap(p), p->tgt->N, Wkio, true, pack_tile_mask(p, false), std::nullopt, p, false);
+            dx = gather_gemm(dy, pack_kmap(p), p->tgt->N, Wkio, true, std::nullopt, p, false);
         if (need_dw && mirror)
-            dW = gather_wgrad(x, pack_kmap(p), p->src->N, dy, K, pack_tile_mask(p, false), built_row_order(p, false)).flip(0);
+            dW = gather_wgrad(x, pack_kmap(p), p->src->N, dy, K, p, false).flip(0);
         else if (need_dw)
-            dW = gather_wgrad(x, pack_kmap_t(p), p->src->N, dy, K, pack_tile_mask(p, true), built_row_order(p, true));
+            dW = gather_wgrad(x, pack_kmap_t(p), p->src->N, dy, K, p, true);
     }
     if (need_dw) {
         dW = dW.reshape({p->ks.v[2], p->ks.v[1], p->ks.v[0], cin, cout});
@@ -1341,7 +1344,6 @@ std::vector<Tensor> conv_forward_fp8(const Tensor &x, const Tensor &weights, Pac
                                       packed.data_ptr(), wb, s),
                  "fp8 weight pack");
     const Tensor &map = transposed ? pack_kmap_t(p) : pack_kmap(p);
-    auto tm = pack_tile_mask(p, transposed);
     Tensor sw = s_w.contiguous();
     const auto order = pack_row_order_if_reused(p, transposed, cin, cout, false);
     std::optional<Tensor> plan;
@@ -1354,7 +1356,7 @@ std::vector<Tensor> conv_forward_fp8(const Tensor &x, const Tensor &weights, Pac
                      "sparse conv forward (fp8 tensor cores)");
         return {y, s_x, s_w};
     }
-    const std::optional<Tensor> tmo = order ? std::optional<Tensor>(order->mask) : tm;
+    const std::optional<Tensor> tmo = order ? std::optional<Tensor>(order->mask) : pack_tile_mask(p, transposed);
     check_status(fvgb_conv_fwd_tc_rows(FVGB_E4M3, x8.data_ptr(), x8.size(0), (int32_t)cin, cin,
                                        (order ? order->map : map).data_ptr<int32_t>(), n_rows, (int32_t)K,
                                        order ? order->rows.data_ptr<int32_t>() : nullptr,
@@ -1551,7 +1553,7 @@ Tensor halo_conv_over(const GridPtr &g, const Tensor &x, const Tensor &w, bool m
     if (g->N > 0 && cin > 0 && cout > 0 && use_tensor_cores(xc, cin, cout)) {
         if (!map) map = halo_map(g);
         if (map)
-            return gather_gemm(xc, pack_kmap(map), g->N, wc, mirror, pack_tile_mask(map, false), std::nullopt, map, false,
+            return gather_gemm(xc, pack_kmap(map), g->N, wc, mirror, std::nullopt, map, false,
                                false, std::nullopt, mirror);
     }
     Tensor y = torch::empty({g->N, cout}, x.options());
@@ -1583,7 +1585,7 @@ Tensor halo_wgrad_over(const GridPtr &g, const Tensor &x, const Tensor &dy, Pack
     const bool by_map = x.scalar_type() == torch::kFloat32 || (use_tensor_cores(xc, cin, cout) && cin <= 128 && cout % 8 == 0);
     if (g->N > 0 && by_map) {
         if (!map) map = halo_map(g);
-        if (map) return gather_wgrad(xc, pack_kmap(map), g->N, dc, 27, pack_tile_mask(map, false));
+        if (map) return gather_wgrad(xc, pack_kmap(map), g->N, dc, 27, map, false);
     }
     FvgbGrid v = g->view();
     size_t wsb = 0;

@@ -406,11 +406,6 @@ __global__ void __launch_bounds__(32 * kHaloLeaves) kmap_halo3_kernel(KmapParams
     if (p.tile_mask && lane < 8 && sm.tmask[lane]) atomicOr(p.tile_mask + t0 + lane, sm.tmask[lane]);
 }
 
-__global__ void fill_kernel(int32_t *__restrict__ p, int64_t n, int32_t v) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        p[i] = v;
-}
-
 __global__ void transpose_kernel(const int32_t *__restrict__ kmap, int64_t n_out, int32_t K, int64_t ld,
                                  int32_t *__restrict__ mapT, int64_t n_in, int64_t ldT) {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -696,10 +691,12 @@ extern "C" int fvgb_kmap_transpose(const int32_t *kmap, int64_t n_out, int32_t K
                                    int64_t n_in, int64_t ldT, fvgb_stream_t stream) {
     if (K < 1 || ld < K || ldT < K || n_out < 0 || n_in < 0) return FVGB_EINVAL;
     cudaStream_t s = as_stream(stream);
-    if (n_in > 0) fill_kernel<<<(unsigned)std::min<int64_t>(ceil_div(n_in * ldT, 256), 65535 * 8), 256, 0, s>>>(mapT, n_in * ldT, -1);
+    // -1 everywhere (all bits set); a store kernel took four times the memset (1.27M x 8: 30 us)
+    if (n_in > 0 && cudaMemsetAsync(mapT, 0xff, sizeof(int32_t) * (size_t)n_in * ldT, s) != cudaSuccess)
+        return launch_status();
     if (n_out > 0)
         transpose_kernel<<<(unsigned)ceil_div(n_out * K, 256), 256, 0, s>>>(kmap, n_out, K, ld, mapT, n_in, ldT);
-    count_launches((n_in > 0) + (n_out > 0));
+    count_launches(n_out > 0);
     return launch_status();
 }
 
