@@ -15,7 +15,6 @@ namespace fvgb {
 namespace {
 
 constexpr int NT = 256;
-constexpr int FM = 128, FN = 64;                    // forward tile: 128 rows x 64 channels, 8 x 4 per thread
 
 template <typename T>
 struct Vec4;
@@ -44,7 +43,9 @@ __device__ __forceinline__ void ldvec(const double *p, double *v) {
     v[0] = q.x, v[1] = q.y;
 }
 
-// One CTA per 128-row x 64-channel output tile, 256 threads of 8 rows x 4 channels.  Per
+// One CTA per FM-row x FN-channel output tile, a thread per 8 rows x 4 channels: 128 x 64, or 128 x 32
+// where the last 64 channels would be at most half used (64->32 FP32, 0.11M voxels: 438 us with
+// 64-wide tiles, 334 us with 256 x 32, whose 427 CTAs left the second wave half empty, 280 us with 128 x 32).  Per
 // offset with any present row and per 16-channel slice (8 for FP64), the gathered rows (transposed, so a
 // thread's 8 rows are two vector loads) and the weight slice go through shared memory; the
 // slice after is loaded into registers while this one is multiplied, so one barrier per slice
@@ -53,8 +54,10 @@ __device__ __forceinline__ void ldvec(const double *p, double *v) {
 // load the fetches and their bounds checks took a third of the issue slots (0.11M voxels, row
 // order, the 32->64->32 FP32 training step's four contractions: 1.69 ms element by element, 1.34 ms
 // in vectors).
-template <typename T, bool VEC>
-__global__ void __launch_bounds__(NT) conv_fwd_simt_kernel(const T *__restrict__ x, int64_t n_x, int32_t cin,
+constexpr int kStageK = 32;  // offsets up to which a tile's map rows are staged in shared memory
+
+template <typename T, bool VEC, int FM, int FN>
+__global__ void __launch_bounds__((FM / 8) * (FN / 4)) conv_fwd_simt_kernel(const T *__restrict__ x, int64_t n_x, int32_t cin,
                                                            int64_t ldx, const int32_t *__restrict__ map,
                                                            int64_t n_out, int32_t K, int64_t ldm,
                                                            const T *__restrict__ w, int64_t wsk, int64_t wsci,
@@ -62,12 +65,17 @@ __global__ void __launch_bounds__(NT) conv_fwd_simt_kernel(const T *__restrict__
                                                            int64_t ldy, int32_t accumulate,
                                                            const int32_t *__restrict__ out_rows) {
     // map row m (m < n_out) computes output row out_rows[m] (m itself when out_rows is null)
+    constexpr int NT = (FM / 8) * (FN / 4);  // threads: 8 rows x 4 channels each
     constexpr int FK = sizeof(T) == 8 ? 8 : 16;  // channels per slice (static shared memory < 48 KB)
     constexpr int QA = FM * FK / NT, QB = FK * FN / NT;
+    // the tile's map rows, all offsets, where they were staged (K <= kStageK): one coalesced read, and
+    // the offsets no row has are known at once; else one offset's column at a time
+    extern __shared__ __align__(16) int32_t tile_map[];
     __shared__ int32_t rows[2][FM];
+    __shared__ uint32_t wmask[NT / 32];
     __shared__ __align__(16) T As[2][FK][FM + 4];
     __shared__ __align__(16) T Bs[2][FK][FN + 4];
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int tid = threadIdx.x, tx = tid % (FN / 4), ty = tid / (FN / 4);
     const int64_t m0 = (int64_t)blockIdx.x * FM;
     const int32_t n0 = blockIdx.y * FN;
     T acc[8][4];
@@ -76,48 +84,76 @@ __global__ void __launch_bounds__(NT) conv_fwd_simt_kernel(const T *__restrict__
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = T(0);
 
+    const bool staged = K <= kStageK;
+    uint32_t offsets = 0;  // staged: the offsets some row of the tile has
+    if (staged) {
+        const int64_t n_here = n_out - m0 < FM ? n_out - m0 : FM;
+        const int32_t words = (int32_t)n_here * K;
+        uint32_t mine = 0;
+        if (ldm == K) {
+            for (int e = tid; e < FM * K; e += NT) {
+                int32_t v = e < words ? map[m0 * K + e] : -1;
+                if (v >= n_x) v = -1;
+                tile_map[e] = v;
+                if (v >= 0) mine |= 1u << (e % K);
+            }
+        } else {
+            for (int e = tid; e < FM * K; e += NT) {
+                int32_t v = e < words ? map[(m0 + e / K) * ldm + e % K] : -1;
+                if (v >= n_x) v = -1;
+                tile_map[e] = v;
+                if (v >= 0) mine |= 1u << (e % K);
+            }
+        }
+        mine = __reduce_or_sync(0xffffffffu, mine);
+        if ((tid & 31) == 0) wmask[tid >> 5] = mine;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < NT / 32; ++i) offsets |= wmask[i];
+    }
     // rows of offset k into rows[rb]; true if any is present (a CTA-wide vote)
     auto load_rows = [&](int32_t k, int rb) -> bool {
+        if (staged) return (offsets >> k) & 1u;
         int valid = 0;
-        if (tid < FM) {
-            const int64_t r = m0 + tid;
+        for (int t = tid; t < FM; t += NT) {
+            const int64_t r = m0 + t;
             int32_t v = r < n_out ? map[r * ldm + k] : -1;
             if (v >= n_x) v = -1;
-            rows[rb][tid] = v;
-            valid = v >= 0;
+            rows[rb][t] = v;
+            valid |= v >= 0;
         }
         return __syncthreads_or(valid) != 0;
     };
     // per thread: A elements e = tid + 256 q (q < QA) -> (row e / FK, channel e % FK); B elements
     // e = tid + 256 q (q < QB) -> (channel e / 64, column e % 64)
     // VEC: the same slices in 16-byte vectors of VW elements
-    constexpr int VW = 16 / sizeof(T), VA = QA / VW, VB = QB / VW;
-    T ra[QA], rb4[QB];
+    constexpr int VW = 16 / sizeof(T), VA = QA / VW, VB = (QB + VW - 1) / VW;
+    T ra[QA], rb4[VB * VW];
     auto fetch = [&](int32_t k, int32_t c0, int rbuf) {
         if constexpr (VEC) {
 #pragma unroll
             for (int q = 0; q < VA; ++q) {
                 const int e = tid + q * NT, r = e / (FK / VW), c = (e % (FK / VW)) * VW;
-                const int32_t src = rows[rbuf][r];
+                const int32_t src = staged ? tile_map[r * K + k] : rows[rbuf][r];
                 const bool on = src >= 0 && c0 + c < cin;
                 ldvec(on ? x + (int64_t)src * ldx + c0 + c : nullptr, &ra[q * VW]);
             }
 #pragma unroll
             for (int q = 0; q < VB; ++q) {
                 const int e = tid + q * NT, c = e / (FN / VW), n = (e % (FN / VW)) * VW;
-                const bool on = c0 + c < cin && n0 + n < cout;
+                const bool on = c < FK && c0 + c < cin && n0 + n < cout;
                 ldvec(on ? w + k * wsk + (int64_t)(c0 + c) * wsci + n0 + n : nullptr, &rb4[q * VW]);
             }
         } else {
 #pragma unroll
             for (int q = 0; q < QA; ++q) {
                 const int e = tid + q * NT, r = e / FK, c = e % FK;
-                const int32_t src = rows[rbuf][r];
+                const int32_t src = staged ? tile_map[r * K + k] : rows[rbuf][r];
                 ra[q] = (src >= 0 && c0 + c < cin) ? x[(int64_t)src * ldx + c0 + c] : T(0);
             }
 #pragma unroll
             for (int q = 0; q < QB; ++q) {
-                const int e = tid + q * NT, c = e >> 6, n = e & 63;
+                const int e = tid + q * NT, c = e / FN, n = e % FN;
                 rb4[q] = (c0 + c < cin && n0 + n < cout)
                              ? w[k * wsk + (int64_t)(c0 + c) * wsci + (int64_t)(n0 + n) * wsco]
                              : T(0);
@@ -135,8 +171,9 @@ __global__ void __launch_bounds__(NT) conv_fwd_simt_kernel(const T *__restrict__
 #pragma unroll
             for (int q = 0; q < VB; ++q) {
                 const int e = tid + q * NT, c = e / (FN / VW), n = (e % (FN / VW)) * VW;
+                if (c < FK)
 #pragma unroll
-                for (int v = 0; v < VW; ++v) Bs[buf][c][n + v] = rb4[q * VW + v];
+                    for (int v = 0; v < VW; ++v) Bs[buf][c][n + v] = rb4[q * VW + v];
             }
         } else {
 #pragma unroll
@@ -147,7 +184,7 @@ __global__ void __launch_bounds__(NT) conv_fwd_simt_kernel(const T *__restrict__
 #pragma unroll
             for (int q = 0; q < QB; ++q) {
                 const int e = tid + q * NT;
-                Bs[buf][e >> 6][e & 63] = rb4[q];
+                Bs[buf][e / FN][e % FN] = rb4[q];
             }
         }
     };
@@ -210,19 +247,109 @@ __global__ void __launch_bounds__(NT) conv_fwd_simt_kernel(const T *__restrict__
     }
 }
 
+// Short rows: few output channels, or few rows (whose maps have no row order).  A lane group of
+// cout / 4 lanes owns one output row and walks that row's present entries only -- the tiles above
+// multiply an offset for all of their rows as soon as one row has it -- with the whole weight tensor
+// in shared memory.  Sums run over offsets, then channels, as in the tiles: the same results.
+// 20,000 scattered voxels (2.9 of 27 offsets present per row), 16->16: 55 us in 128 x 64 tiles,
+// 13 us here, bound by the latency of one row's dependent loads.
+constexpr int kShortSmem = 96 * 1024;
+
 template <typename T>
-void launch_fwd_simt(dim3 grid, const void *x, int64_t n_x, int32_t cin, int64_t ldx, const int32_t *map, int64_t n_out,
-                     int32_t K, int64_t ldm, const void *w, int64_t wsk, int64_t wsci, int64_t wsco, void *y,
-                     int32_t cout, int64_t ldy, int32_t accumulate, const int32_t *rows, cudaStream_t s) {
+__global__ void __launch_bounds__(NT) conv_fwd_short_kernel(const T *__restrict__ x, int64_t n_x, int32_t cin, int64_t ldx,
+                                                            const int32_t *__restrict__ map, int64_t n_out, int32_t K,
+                                                            int64_t ldm, const T *__restrict__ w, int64_t wsk,
+                                                            int64_t wsci, T *__restrict__ y, int32_t cout, int64_t ldy,
+                                                            int32_t accumulate, const int32_t *__restrict__ out_rows,
+                                                            int gs) {
+    constexpr int VW = 16 / sizeof(T);
+    extern __shared__ __align__(16) uint8_t short_smem[];
+    T *ws = reinterpret_cast<T *>(short_smem);  // [K][cin][cout]
+    const int lane = threadIdx.x & 31;
+    const int G = 1 << gs, gl = lane & (G - 1);
+    const int64_t m = ((int64_t)blockIdx.x * NT + threadIdx.x) >> gs;
+    // the row's occupancy, entries shared over the group's lanes
+    uint32_t present = 0;
+    if (m < n_out)
+        for (int k = gl; k < K; k += G) {
+            const int32_t v = __ldg(map + m * ldm + k);
+            if (v >= 0 && v < n_x) present |= 1u << k;
+        }
+    for (int o = 1; o < G; o <<= 1) present |= __shfl_xor_sync(0xffffffffu, present, o);
+    const int cv = cout / VW;
+    for (int e = threadIdx.x; e < K * cin * cv; e += NT) {
+        const int k = e / (cin * cv), ci = (e / cv) % cin, c = (e % cv) * VW;
+        T t[VW];
+        ldvec(w + k * wsk + (int64_t)ci * wsci + c, t);
+#pragma unroll
+        for (int i = 0; i < VW; ++i) ws[(k * cin + ci) * cout + c + i] = t[i];
+    }
+    __syncthreads();
+    if (m >= n_out || gl * 4 >= cout) return;
+    T acc[4] = {T(0), T(0), T(0), T(0)};
+    while (present) {
+        const int k = __ffs(present) - 1;
+        present &= present - 1;
+        const T *xr = x + (int64_t)__ldg(map + m * ldm + k) * ldx;
+        const T *wk = ws + k * cin * cout + gl * 4;
+        for (int c0 = 0; c0 < cin; c0 += 8) {
+            T xv[8];
+#pragma unroll
+            for (int c = 0; c < 8; c += VW) ldvec(c0 + c < cin ? xr + c0 + c : nullptr, &xv[c]);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                if (c0 + c >= cin) break;
+                T b[4];
+                Vec4<T>::load(wk + (c0 + c) * cout, b);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[j] = fma(xv[c], b[j], acc[j]);
+            }
+        }
+    }
+    const int64_t r = out_rows ? (int64_t)out_rows[m] : m;
+    T *dst = y + r * ldy + gl * 4;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) dst[j] = accumulate ? (T)(dst[j] + acc[j]) : acc[j];
+}
+
+template <typename T>
+int launch_fwd_simt(const void *x, int64_t n_x, int32_t cin, int64_t ldx, const int32_t *map, int64_t n_out, int32_t K,
+                    int64_t ldm, const void *w, int64_t wsk, int64_t wsci, int64_t wsco, void *y, int32_t cout,
+                    int64_t ldy, int32_t accumulate, const int32_t *rows, cudaStream_t s) {
     constexpr int VW = 16 / sizeof(T);
     const bool vec = cin % VW == 0 && ldx % VW == 0 && wsco == 1 && cout % VW == 0 && wsk % VW == 0 && wsci % VW == 0 &&
                      (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
-    if (vec)
-        conv_fwd_simt_kernel<T, true><<<grid, NT, 0, s>>>((const T *)x, n_x, cin, ldx, map, n_out, K, ldm, (const T *)w, wsk,
-                                                          wsci, wsco, (T *)y, cout, ldy, accumulate, rows);
-    else
-        conv_fwd_simt_kernel<T, false><<<grid, NT, 0, s>>>((const T *)x, n_x, cin, ldx, map, n_out, K, ldm, (const T *)w,
-                                                           wsk, wsci, wsco, (T *)y, cout, ldy, accumulate, rows);
+    // the short-row kernel: 16 channels and fewer always (a 64-wide tile would be three quarters
+    // empty); up to 32 only below 2^16 rows, where tiles have no row order
+    const int64_t wbytes = (int64_t)K * cin * cout * sizeof(T);
+    if (vec && cout % 4 == 0 && K <= 32 && wbytes <= kShortSmem &&
+        (cout <= 16 || (cout <= 32 && n_out < ((int64_t)1 << 16)))) {
+        int gs = 0;
+        while ((4 << gs) < cout) ++gs;
+        if (set_dynamic_smem(conv_fwd_short_kernel<T>, kShortSmem) != cudaSuccess) return launch_status();
+        conv_fwd_short_kernel<T><<<(unsigned)ceil_div(n_out << gs, (int64_t)NT), NT, (size_t)wbytes, s>>>(
+            (const T *)x, n_x, cin, ldx, map, n_out, K, ldm, (const T *)w, wsk, wsci, (T *)y, cout, ldy, accumulate, rows,
+            gs);
+        return FVGB_OK;
+    }
+    const bool narrow = cout % 64 != 0 && cout % 64 <= 32;
+    const int fm = 128, fn = narrow ? 32 : 64, threads = narrow ? 128 : 256;
+    const dim3 grid((unsigned)ceil_div(n_out, fm), (unsigned)ceil_div(cout, fn));
+    if (ceil_div(cout, fn) > 65535) return FVGB_EINVAL;
+    const int smem = K <= kStageK ? fm * K * 4 : 0;
+    auto go = [&](auto kern) {
+        if (set_dynamic_smem(kern, smem) != cudaSuccess) return;
+        kern<<<grid, threads, smem, s>>>((const T *)x, n_x, cin, ldx, map, n_out, K, ldm, (const T *)w, wsk, wsci, wsco, (T *)y, cout,
+                                 ldy, accumulate, rows);
+    };
+    if (narrow) {
+        if (vec) go(conv_fwd_simt_kernel<T, true, 128, 32>);
+        else go(conv_fwd_simt_kernel<T, false, 128, 32>);
+    } else {
+        if (vec) go(conv_fwd_simt_kernel<T, true, 128, 64>);
+        else go(conv_fwd_simt_kernel<T, false, 128, 64>);
+    }
+    return FVGB_OK;
 }
 
 // Rows per wgrad chunk so that the grid has enough CTAs; deterministic in the sizes only.
@@ -475,18 +602,18 @@ extern "C" int fvgb_conv_fwd_simt_rows(int32_t dtype, const void *x, int64_t n_x
         return FVGB_EINVAL;
     if (n_out == 0) return FVGB_OK;
     if (!map || !w || !y || (n_x > 0 && !x)) return FVGB_EINVAL;
-    const dim3 grid((unsigned)ceil_div(n_out, FM), (unsigned)ceil_div(c_out, FN));
-    if (grid.y > 65535) return FVGB_EINVAL;
+    if (ceil_div(c_out, 64) > 65535) return FVGB_EINVAL;
     cudaStream_t s = as_stream(stream);
-    if (dtype == FVGB_F32) {
-        launch_fwd_simt<float>(grid, x, n_x, c_in, ldx, map, n_out, K, ldm, w, wsk, wsci, wsco, y, c_out, ldy, accumulate,
-                               rows, s);
-    } else if (dtype == FVGB_F64) {
-        launch_fwd_simt<double>(grid, x, n_x, c_in, ldx, map, n_out, K, ldm, w, wsk, wsci, wsco, y, c_out, ldy, accumulate,
-                                rows, s);
-    } else {
+    int st;
+    if (dtype == FVGB_F32)
+        st = launch_fwd_simt<float>(x, n_x, c_in, ldx, map, n_out, K, ldm, w, wsk, wsci, wsco, y, c_out, ldy, accumulate,
+                                    rows, s);
+    else if (dtype == FVGB_F64)
+        st = launch_fwd_simt<double>(x, n_x, c_in, ldx, map, n_out, K, ldm, w, wsk, wsci, wsco, y, c_out, ldy, accumulate,
+                                     rows, s);
+    else
         return FVGB_ETYPE;
-    }
+    if (st) return st;
     count_launches(1);
     return launch_status();
 }
