@@ -335,6 +335,50 @@ __global__ void compact_offsets_kernel(const int64_t *__restrict__ src_joff, int
     out[b] = pos[src_joff[b] * per];
 }
 
+// Writes leaf p of the index order (its grid b, origin and first voxel; `word` = mask word lane / 4 of a
+// converged warp): its voxels in bit order, its table entry and its hash slot.
+__device__ __forceinline__ void emit_leaf(uint64_t word, int32_t ox, int32_t oy, int32_t oz, int32_t b, int32_t base,
+                                          int64_t p, int lane, int32_t *out_ijk, FvgbLeaf *leaves, int32_t *slots,
+                                          int64_t cap) {
+    const int w = lane >> 2, sub = (lane & 3) * 16;
+    // exclusive prefix of the words' populations, the same for the four lanes of a word
+    int pre = 0;
+#pragma unroll
+    for (int v = 0; v < 7; ++v) {
+        const int c = __popcll(__shfl_sync(0xffffffffu, word, v * 4));
+        if (v < w) pre += c;
+    }
+    FvgbLeaf &lf = leaves[p];
+    if ((lane & 3) == 0) {
+        lf.mask[w] = word;
+        lf.prefix[w] = (uint16_t)pre;
+    }
+    if (lane < 3) {
+        lf.origin[lane] = lane == 0 ? ox : (lane == 1 ? oy : oz);
+        lf.pad[lane] = 0;
+    }
+    if (lane == 0) {
+        lf.batch = b;
+        lf.base = base;
+        const uint64_t cap_mask = (uint64_t)cap - 1;
+        uint64_t s = leaf_hash(b, ox >> 3, oy >> 3, oz >> 3) & cap_mask;
+        for (int64_t probe = 0; probe < cap; ++probe) {
+            if (atomicCAS(slots + s, -1, (int32_t)p) == -1) break;
+            s = (s + 1) & cap_mask;
+        }
+    }
+    int64_t r = (int64_t)base + pre + __popcll(sub ? (word & ((1ull << sub) - 1ull)) : 0ull);
+    uint32_t bits = (uint32_t)(word >> sub) & 0xffffu;
+    while (bits) {
+        const int i = w * 64 + sub + __ffs(bits) - 1;
+        bits &= bits - 1;
+        out_ijk[3 * r] = ox + (i >> 6);
+        out_ijk[3 * r + 1] = oy + ((i >> 3) & 7);
+        out_ijk[3 * r + 2] = oz + (i & 7);
+        ++r;
+    }
+}
+
 constexpr int kThreads = 256;
 inline unsigned blocks_for(int64_t n) { return (unsigned)ceil_div(n > 0 ? n : 1, kThreads); }
 
@@ -744,6 +788,192 @@ __global__ void coarse_offsets_kernel(const int4 *__restrict__ corig, const int3
     }
 }
 
+// Up to kHashLeaves fine leaves the coarse leaves are found through a hash table and put in order by
+// counting, for each, the keys below its own: five launches with little shared memory instead of
+// seventeen.  The build runs beside convolutions whose CTAs leave about 30 KB of shared memory per SM;
+// the radix sort's passes waited for those CTAs to end, and the host, which waits for the counts,
+// waited with them (inference step, 1.31M voxels in 21.7k fine leaves: 763 us a step with the sort, 646 us
+// with this; pooling over the same grid, nothing beside it: 652 -> 575 us).  Counting is quadratic in the
+// coarse leaves (a quarter of the fine ones on surfaces), which at kHashLeaves coarse leaves is about the
+// sort's time.
+constexpr int64_t kHashLeaves = 49152;
+constexpr int kRankThreads = 256, kScanThreads = 1024;
+
+// Workspace of the hashed build.
+struct CoarseHash {
+    uint64_t *table;   // [cap] keys, all ones where free
+    int32_t *slot_id;  // [cap] coarse leaf of a taken slot, in insertion order
+    uint64_t *key;     // [nl]
+    int32_t *slot;     // [nl] slot of each fine leaf
+    int32_t *order;    // [nl] coarse leaf at each place of the index order
+    int32_t *count;    // [nl] voxels of the coarse leaf at each place
+    int32_t *base;     // [nl + 1] first voxel of each place
+    int32_t *found;    // [1] coarse leaves
+    uint64_t *cmask;   // [nl][8]
+    int4 *corig;       // [nl]
+    int64_t cap;
+};
+
+__global__ void coarse_insert_kernel(const FvgbLeaf *__restrict__ leaves, int64_t nl, int3 sh, uint64_t low_mask, int vb,
+                                     CoarseHash h) {
+    const int64_t l = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (l >= nl) return;
+    const FvgbLeaf &lf = leaves[l];
+    const int32_t cx = (lf.origin[0] >> (sh.x + 3)) << 3, cy = (lf.origin[1] >> (sh.y + 3)) << 3,
+                  cz = (lf.origin[2] >> (sh.z + 3)) << 3;
+    const uint64_t key = ((uint64_t)lf.batch << vb) | ((order_key(cx, cy, cz) & low_mask) >> 9);
+    const uint64_t cap_mask = (uint64_t)h.cap - 1;
+    uint64_t m = key * 0x9E3779B97F4A7C15ull;
+    m ^= m >> 32;
+    uint64_t s = m & cap_mask;
+    for (int64_t probe = 0; probe < h.cap; ++probe) {  // at most half full: a free slot is found
+        const uint64_t k = atomicCAS(reinterpret_cast<unsigned long long *>(h.table + s), ~0ull, key);
+        if (k == ~0ull) {
+            const int32_t id = atomicAdd(h.found, 1);
+            h.slot_id[s] = id;
+            h.key[id] = key;
+            h.corig[id] = make_int4(cx, cy, cz, lf.batch);
+#pragma unroll
+            for (int w = 0; w < 8; ++w) h.cmask[(int64_t)id * 8 + w] = 0;
+            break;
+        }
+        if (k == key) break;
+        s = (s + 1) & cap_mask;
+    }
+    h.slot[l] = (int32_t)s;
+}
+
+// warp per fine leaf: OR its voxels, mapped down, into its coarse leaf's mask
+__global__ void __launch_bounds__(256) coarse_or_kernel(const FvgbLeaf *__restrict__ leaves, int64_t nl, int3 sh,
+                                                        CoarseHash h) {
+    __shared__ unsigned long long wm[8][8];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t l = (int64_t)blockIdx.x * 8 + warp;
+    if (l >= nl) return;  // whole warps leave together
+    const FvgbLeaf &lf = leaves[l];
+    const int64_t c = h.slot_id[h.slot[l]];
+    if (lane < 8) wm[warp][lane] = 0ull;
+    __syncwarp();
+    const uint64_t word = lf.mask[lane >> 2];
+    const int sub = (lane & 3) * 16;
+    uint32_t bits = (uint32_t)(word >> sub) & 0xffffu;
+    while (bits) {
+        const int b = (lane >> 2) * 64 + sub + __ffs(bits) - 1;
+        bits &= bits - 1;
+        const uint32_t cb = leaf_bit((lf.origin[0] + (b >> 6)) >> sh.x, (lf.origin[1] + ((b >> 3) & 7)) >> sh.y,
+                                     (lf.origin[2] + (b & 7)) >> sh.z);
+        atomicOr(&wm[warp][cb >> 6], 1ull << (cb & 63));
+    }
+    __syncwarp();
+    if (lane < 8) {
+        const unsigned long long m = wm[warp][lane];
+        if (m) atomicOr(reinterpret_cast<unsigned long long *>(h.cmask) + c * 8 + lane, m);
+    }
+}
+
+// place of coarse leaf i in the index order = keys below its own (keys are distinct)
+template <typename Key>
+__global__ void __launch_bounds__(kRankThreads) coarse_rank_kernel(CoarseHash h) {
+    __shared__ Key keys[kRankThreads];
+    const int32_t n = *h.found;
+    if ((int64_t)blockIdx.x * kRankThreads >= n) return;
+    const int32_t i = blockIdx.x * kRankThreads + threadIdx.x;
+    const Key mine = i < n ? (Key)h.key[i] : (Key)0;
+    int32_t rank = 0;
+    for (int32_t j0 = 0; j0 < n; j0 += kRankThreads) {
+        const int32_t j = j0 + threadIdx.x;
+        __syncthreads();
+        keys[threadIdx.x] = j < n ? (Key)h.key[j] : (Key)~(Key)0;  // never below a key
+        __syncthreads();
+#pragma unroll 32
+        for (int t = 0; t < kRankThreads; ++t) rank += keys[t] < mine ? 1 : 0;
+    }
+    if (i >= n) return;
+    int32_t c = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) c += __popcll(h.cmask[(int64_t)i * 8 + w]);
+    h.order[rank] = i;
+    h.count[rank] = c;
+}
+
+// one CTA: first voxel of every place, and meta[b] = first voxel of grid b, meta[B+1] = coarse leaves,
+// meta[B+2] = voxels
+__global__ void __launch_bounds__(kScanThreads) coarse_scan_kernel(CoarseHash h, int32_t B, int64_t *meta) {
+    using Scan = cub::BlockScan<int32_t, kScanThreads>;
+    __shared__ typename Scan::TempStorage tmp;
+    const int32_t n = *h.found;
+    int32_t run = 0;
+    constexpr int kItems = 8;
+    for (int32_t p0 = 0; p0 < n; p0 += kScanThreads * kItems) {
+        int32_t v[kItems], total;
+#pragma unroll
+        for (int i = 0; i < kItems; ++i) {
+            const int32_t p = p0 + threadIdx.x * kItems + i;
+            v[i] = p < n ? h.count[p] : 0;
+        }
+        __syncthreads();
+        Scan(tmp).ExclusiveSum(v, v, total);
+#pragma unroll
+        for (int i = 0; i < kItems; ++i) {
+            const int32_t p = p0 + threadIdx.x * kItems + i;
+            if (p < n) h.base[p] = run + v[i];
+        }
+        run += total;
+    }
+    if (threadIdx.x == 0) h.base[n] = run;
+    __syncthreads();
+    for (int b = threadIdx.x; b <= B; b += kScanThreads) {
+        int32_t lo = 0, hi = n;  // first place with grid >= b
+        while (lo < hi) {
+            const int32_t mid = (lo + hi) >> 1;
+            if (h.corig[h.order[mid]].w < b) lo = mid + 1; else hi = mid;
+        }
+        meta[b] = h.base[lo];
+    }
+    if (threadIdx.x == 0) {
+        meta[B + 1] = n;
+        meta[B + 2] = run;
+    }
+}
+
+// warp per place: its voxels in bit order, its leaf table entry and its hash slot
+__global__ void __launch_bounds__(256) coarse_place_kernel(CoarseHash h, int32_t *__restrict__ out_ijk,
+                                                           FvgbLeaf *__restrict__ leaves, int32_t *__restrict__ slots,
+                                                           int64_t cap) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t p = (int64_t)blockIdx.x * 8 + warp;
+    if (p >= *h.found) return;
+    const int64_t c = h.order[p];
+    const int4 o = h.corig[c];
+    emit_leaf(h.cmask[c * 8 + (lane >> 2)], o.x, o.y, o.z, o.w, h.base[p], p, lane, out_ijk, leaves, slots, cap);
+}
+
+// 8 + 4 bytes per slot (2 to 4 slots per fine leaf) and 112 per fine leaf
+size_t coarse_hash_layout(int64_t nl, CoarseHash *w, char *base) {
+    CoarseHash h;
+    h.cap = 64;
+    while (h.cap < 2 * nl) h.cap <<= 1;
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        char *p = base ? base + off : nullptr;
+        off += (bytes + 255) & ~(size_t)255;
+        return p;
+    };
+    const size_t n = (size_t)nl;
+    h.table = (uint64_t *)take((size_t)h.cap * 8);
+    h.slot_id = (int32_t *)take((size_t)h.cap * 4);
+    h.key = (uint64_t *)take(n * 8);
+    h.slot = (int32_t *)take(n * 4);
+    h.order = (int32_t *)take(n * 4);
+    h.count = (int32_t *)take(n * 4);
+    h.base = (int32_t *)take((n + 1) * 4);
+    h.found = (int32_t *)take(4);
+    h.cmask = (uint64_t *)take(n * 64);
+    h.corig = (int4 *)take(n * 16);
+    if (w) *w = h;
+    return off;
+}
+
 }  // namespace
 }  // namespace fvgb
 
@@ -1016,7 +1246,7 @@ __global__ void leaf_counts_kernel(LeafHash h, int64_t L, const int32_t *__restr
     count[p] = c;  // zero past the last leaf, for the exclusive scan over L + 1
 }
 
-// warp per leaf in index order: its voxels in bit order, its table entry and its hash slot
+// warp per leaf in index order
 __global__ void __launch_bounds__(256) leaf_emit_kernel(LeafHash h, int64_t L, const int32_t *__restrict__ vals,
                                                         const int32_t *__restrict__ first,
                                                         int32_t *__restrict__ out_ijk, FvgbLeaf *__restrict__ leaves,
@@ -1028,46 +1258,8 @@ __global__ void __launch_bounds__(256) leaf_emit_kernel(LeafHash h, int64_t L, c
     const uint64_t key = h.keys[id];
     int32_t ox, oy, oz;
     key_to_coord((key & ((1ull << 54) - 1ull)) << 9, ox, oy, oz);
-    const int32_t b = (int32_t)(key >> 54);
-    const int w = lane >> 2, sub = (lane & 3) * 16;
-    const uint64_t word = h.mask[(int64_t)id * 8 + w];
-    // exclusive prefix of the words' populations, the same for the four lanes of a word
-    int pre = 0;
-#pragma unroll
-    for (int v = 0; v < 7; ++v) {
-        const int c = __popcll(__shfl_sync(0xffffffffu, word, v * 4));
-        if (v < w) pre += c;
-    }
-    const int32_t base = first[p];
-    FvgbLeaf &lf = leaves[p];
-    if ((lane & 3) == 0) {
-        lf.mask[w] = word;
-        lf.prefix[w] = (uint16_t)pre;
-    }
-    if (lane < 3) {
-        lf.origin[lane] = lane == 0 ? ox : (lane == 1 ? oy : oz);
-        lf.pad[lane] = 0;
-    }
-    if (lane == 0) {
-        lf.batch = b;
-        lf.base = base;
-        const uint64_t cap_mask = (uint64_t)cap - 1;
-        uint64_t s = leaf_hash(b, ox >> 3, oy >> 3, oz >> 3) & cap_mask;
-        for (int64_t probe = 0; probe < cap; ++probe) {
-            if (atomicCAS(slots + s, -1, (int32_t)p) == -1) break;
-            s = (s + 1) & cap_mask;
-        }
-    }
-    int64_t r = (int64_t)base + pre + __popcll(sub ? (word & ((1ull << sub) - 1ull)) : 0ull);
-    uint32_t bits = (uint32_t)(word >> sub) & 0xffffu;
-    while (bits) {
-        const int i = w * 64 + sub + __ffs(bits) - 1;
-        bits &= bits - 1;
-        out_ijk[3 * r] = ox + (i >> 6);
-        out_ijk[3 * r + 1] = oy + ((i >> 3) & 7);
-        out_ijk[3 * r + 2] = oz + (i & 7);
-        ++r;
-    }
+    emit_leaf(h.mask[(int64_t)id * 8 + (lane >> 2)], ox, oy, oz, (int32_t)(key >> 54), first[p], p, lane, out_ijk, leaves,
+              slots, cap);
 }
 
 // meta[b] = first voxel of grid b (b <= B)
@@ -1215,6 +1407,56 @@ extern "C" int fvgb_leaf_hash_finish(int64_t n, int32_t num_grids, int64_t num_l
                                                               hash_capacity);
     leaf_offsets_kernel<<<(unsigned)ceil_div(num_grids + 1, kThreads), kThreads, 0, s>>>(leaves, w.first, L, num_grids,
                                                                                          out_joffsets);
+    count_launches(5);
+    return launch_status();
+}
+
+extern "C" int fvgb_coarse_grid_index_workspace(int64_t num_fine_leaves, size_t *bytes) {
+    if (!bytes || num_fine_leaves < 1 || num_fine_leaves > fvgb::kHashLeaves) return FVGB_EINVAL;
+    *bytes = fvgb::coarse_hash_layout(num_fine_leaves, nullptr, nullptr) + 256;
+    return FVGB_OK;
+}
+
+extern "C" int fvgb_coarse_grid_index(const FvgbGrid *fine, const int32_t factor[3], const int32_t box_lo[3],
+                                      const int32_t box_hi[3], int32_t *out_ijk, int64_t *meta, FvgbLeaf *leaves,
+                                      int32_t *hash_slots, int64_t hash_capacity, void *workspace,
+                                      size_t workspace_bytes, fvgb_stream_t stream) {
+    if (!fine || !factor || !meta || !out_ijk || !leaves || !hash_slots || !box_lo || !box_hi) return FVGB_EINVAL;
+    if (fine->num_grids < 1 || fine->num_grids > kCoarseMaxGrids || !fine->leaves) return FVGB_EINVAL;
+    size_t need = 0;
+    const int64_t nl = fine->num_leaves;
+    const int st = fvgb_coarse_grid_index_workspace(nl, &need);
+    if (st) return st;
+    if (hash_capacity < 2 * nl || (hash_capacity & (hash_capacity - 1))) return FVGB_EINVAL;
+    if (!workspace || workspace_bytes < need) return FVGB_ENOSPACE;
+    int sh[3];
+    for (int a = 0; a < 3; ++a) {
+        const int f = factor[a];
+        if ((f != 1 && f != 2 && f != 4 && f != 8) || box_lo[a] > box_hi[a]) return FVGB_EINVAL;
+        sh[a] = f == 1 ? 0 : (f == 2 ? 1 : (f == 4 ? 2 : 3));
+    }
+    const int3 shv = make_int3(sh[0], sh[1], sh[2]);
+    const int end_bit = order_key_end_bit(box_lo, box_hi);
+    const int vb = end_bit > 9 ? end_bit - 9 : 0;
+    const uint64_t low_mask = end_bit >= 63 ? ~0ull : ((1ull << end_bit) - 1ull);
+    int grid_bits = 0;
+    while ((1 << grid_bits) < fine->num_grids) ++grid_bits;
+    const int bits = vb + grid_bits;
+    if (bits >= 64) return FVGB_EINVAL;  // a key of all ones is the table's free slot
+    cudaStream_t s = as_stream(stream);
+    CoarseHash h;
+    coarse_hash_layout(nl, &h, align_ws(workspace));
+    if (cudaMemsetAsync(h.table, 0xff, (size_t)h.cap * 8, s) != cudaSuccess ||
+        cudaMemsetAsync(h.found, 0, 4, s) != cudaSuccess ||
+        cudaMemsetAsync(hash_slots, 0xff, sizeof(int32_t) * hash_capacity, s) != cudaSuccess)
+        return launch_status();
+    coarse_insert_kernel<<<blocks_for(nl), kThreads, 0, s>>>(fine->leaves, nl, shv, low_mask, vb, h);
+    coarse_or_kernel<<<(unsigned)ceil_div(nl, 8), 256, 0, s>>>(fine->leaves, nl, shv, h);
+    const unsigned ranks = (unsigned)ceil_div(nl, (int64_t)kRankThreads);
+    if (bits <= 32) coarse_rank_kernel<uint32_t><<<ranks, kRankThreads, 0, s>>>(h);
+    else coarse_rank_kernel<uint64_t><<<ranks, kRankThreads, 0, s>>>(h);
+    coarse_scan_kernel<<<1, kScanThreads, 0, s>>>(h, fine->num_grids, meta);
+    coarse_place_kernel<<<(unsigned)ceil_div(nl, 8), 256, 0, s>>>(h, out_ijk, leaves, hash_slots, hash_capacity);
     count_launches(5);
     return launch_status();
 }

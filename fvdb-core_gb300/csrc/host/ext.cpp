@@ -119,6 +119,7 @@ struct GridImpl {
         at::cuda::CUDAEvent counted;  // on the build stream, after the counts' copy to the host
         Tensor meta_host;             // pinned int64 [B + 4]
         Tensor out_ijk, leaf_ids, meta;
+        Tensor leaves, hash;          // an indexed build (fvgb_coarse_grid_index): room for the fine leaves
         // the counts' copy into meta_host must land before the pinned block can be reused
         ~PendingBuild() {
             try {
@@ -404,7 +405,7 @@ GridPtr build_coarse_by_leaves(const GridPtr &g, const Vec3 &f, const int32_t lo
     // The build runs on the library's build stream once the fine grid is complete (its ready
     // event), so it does not wait for work queued on the caller's stream (e.g. the previous
     // step's convolutions); the host reads its counts only when the coarse grid is first used.
-    // Buffers are allocated for the build stream and handed to the caller's stream.
+    // Buffers are allocated for the build stream and handed to the using stream by resolve().
     auto main = at::cuda::getCurrentCUDAStream(dev.index());
     auto side = build_stream(dev.index());
     if (g->ready) g->ready->block(side);
@@ -418,29 +419,40 @@ GridPtr build_coarse_by_leaves(const GridPtr &g, const Vec3 &f, const int32_t lo
     {
         c10::cuda::CUDAStreamGuard sg(side);
         pb->out_ijk = torch::empty({std::max<int64_t>(g->N, 1), 3}, i32);
-        pb->leaf_ids = torch::empty({std::max<int64_t>(g->N, 1)}, i32);
         pb->meta = torch::empty({B + 4}, torch::dtype(torch::kInt64).device(dev));
         TORCH_CHECK(cudaMemsetAsync(pb->meta.data_ptr<int64_t>(), 0, (B + 4) * sizeof(int64_t), side.stream()) ==
                         cudaSuccess,
                     "coarse grid: clearing the counts failed");
         size_t wsb = 0;
-        check_status(fvgb_coarse_grid_workspace(g->L, &wsb), "coarse grid (workspace)");
-        Tensor ws = workspace(wsb, dev);
         FvgbGrid fv = g->view();
         cudaStream_t cs = side.stream();
-        check_status(fvgb_coarse_grid_build(&fv, f.v, lo, hi, pb->out_ijk.data_ptr<int32_t>(),
-                                            pb->meta.data_ptr<int64_t>(), pb->leaf_ids.data_ptr<int32_t>(),
-                                            ws.data_ptr(), ws.numel(), cs),
-                     "coarse grid");
+        if (fvgb_coarse_grid_index_workspace(g->L, &wsb) == FVGB_OK) {
+            // the leaf table and hash come out of the build, sized for the fine grid's leaves
+            const int64_t cap = next_pow2(2 * g->L);
+            pb->leaves = torch::empty({g->L * (int64_t)sizeof(FvgbLeaf)}, torch::dtype(torch::kUInt8).device(dev));
+            pb->hash = torch::empty({cap}, i32);
+            Tensor ws = workspace(wsb, dev);
+            const int st = fvgb_coarse_grid_index(&fv, f.v, lo, hi, pb->out_ijk.data_ptr<int32_t>(),
+                                                  pb->meta.data_ptr<int64_t>(),
+                                                  reinterpret_cast<FvgbLeaf *>(pb->leaves.data_ptr<uint8_t>()),
+                                                  pb->hash.data_ptr<int32_t>(), cap, ws.data_ptr(), ws.numel(), cs);
+            if (st == FVGB_EINVAL) pb->leaves = pb->hash = Tensor();  // keys too wide: the sort
+            else check_status(st, "coarse grid");
+        }
+        if (!pb->leaves.defined()) {
+            pb->leaf_ids = torch::empty({std::max<int64_t>(g->N, 1)}, i32);
+            check_status(fvgb_coarse_grid_workspace(g->L, &wsb), "coarse grid (workspace)");
+            Tensor ws = workspace(wsb, dev);
+            check_status(fvgb_coarse_grid_build(&fv, f.v, lo, hi, pb->out_ijk.data_ptr<int32_t>(),
+                                                pb->meta.data_ptr<int64_t>(), pb->leaf_ids.data_ptr<int32_t>(),
+                                                ws.data_ptr(), ws.numel(), cs),
+                         "coarse grid");
+        }
         TORCH_CHECK(cudaMemcpyAsync(pb->meta_host.data_ptr<int64_t>(), pb->meta.data_ptr<int64_t>(),
                                     (B + 4) * sizeof(int64_t), cudaMemcpyDeviceToHost, cs) == cudaSuccess,
                     "coarse grid: copying the counts failed");
         pb->counted.record(side);
     }
-    // the buffers live on in the caller's stream
-    pb->out_ijk.record_stream(main);
-    pb->leaf_ids.record_stream(main);
-    pb->meta.record_stream(main);
     c->joffsets = pb->meta.narrow(0, 0, B + 1);  // the device, for guards; values after resolve()
     c->N = -1;
     c->L = -1;
@@ -464,15 +476,24 @@ void GridImpl::resolve() const {
     self->N = h[B + 2];
     self->L = h[B + 1];
     self->ijk = P.out_ijk.narrow(0, 0, self->N);
-    self->cap = next_pow2(2 * self->L);
     auto main = at::cuda::getCurrentCUDAStream(dev.index());
-    P.counted.block(main);  // the index build follows the coarse build on the device
-    auto i32 = torch::dtype(torch::kInt32).device(dev);
-    self->leaves = torch::empty({std::max<int64_t>(self->L, 1) * (int64_t)sizeof(FvgbLeaf)},
-                                torch::dtype(torch::kUInt8).device(dev));
-    self->hash = torch::empty({self->cap}, i32);
-    FvgbGrid v = self->view_unchecked();
-    check_status(fvgb_grid_index_build(&v, P.leaf_ids.data_ptr<int32_t>(), main.stream()), "coarse grid (index)");
+    P.counted.block(main);  // what uses the grid follows its build on the device
+    // the buffers, allocated for the build stream, live on in the stream that uses the grid
+    for (const Tensor &t : {P.out_ijk, P.meta, P.leaves, P.hash, P.leaf_ids})
+        if (t.defined()) t.record_stream(main);
+    if (P.leaves.defined()) {
+        self->cap = P.hash.size(0);
+        self->leaves = P.leaves.narrow(0, 0, self->L * (int64_t)sizeof(FvgbLeaf));
+        self->hash = P.hash;
+    } else {
+        self->cap = next_pow2(2 * self->L);
+        auto i32 = torch::dtype(torch::kInt32).device(dev);
+        self->leaves = torch::empty({std::max<int64_t>(self->L, 1) * (int64_t)sizeof(FvgbLeaf)},
+                                    torch::dtype(torch::kUInt8).device(dev));
+        self->hash = torch::empty({self->cap}, i32);
+        FvgbGrid v = self->view_unchecked();
+        check_status(fvgb_grid_index_build(&v, P.leaf_ids.data_ptr<int32_t>(), main.stream()), "coarse grid (index)");
+    }
     self->ready = std::make_shared<at::cuda::CUDAEvent>();
     self->ready->record(main);
     self->pending.reset();

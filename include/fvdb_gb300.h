@@ -176,6 +176,16 @@ int fvgb_coarse_grid_workspace(int64_t num_fine_leaves, size_t *bytes);
 int fvgb_coarse_grid_build(const FvgbGrid *fine, const int32_t factor[3], const int32_t *box_lo, const int32_t *box_hi,
                            int32_t *out_ijk, int64_t *meta, int32_t *leaf_ids, void *workspace, size_t workspace_bytes,
                            fvgb_stream_t stream);
+/* The same coarse grid with its index, for up to 49,152 fine leaves: ijk, meta (offsets, coarse leaves,
+ * voxels; meta[num_grids + 3] is not written), leaf table [num_fine_leaves entries of room] and leaf
+ * hash (hash_capacity a power of two >= 2 num_fine_leaves).  Found through a hash table and ordered by
+ * counting instead of sorting; FVGB_EINVAL where the grid is larger (fvgb_coarse_grid_build serves
+ * it).  No counterpart in the reference. */
+int fvgb_coarse_grid_index_workspace(int64_t num_fine_leaves, size_t *bytes);
+int fvgb_coarse_grid_index(const FvgbGrid *fine, const int32_t factor[3], const int32_t box_lo[3],
+                           const int32_t box_hi[3], int32_t *out_ijk, int64_t *meta, FvgbLeaf *leaves,
+                           int32_t *hash_slots, int64_t hash_capacity, void *workspace, size_t workspace_bytes,
+                           fvgb_stream_t stream);
 
 /*
  * Index of each query coordinate (query q belongs to grid b with joffsets[b] <= q <

@@ -109,3 +109,30 @@ def test_coarse_grid_by_leaves_equals_voxel_sort(cuda_device, factor):
         assert np.array_equal(coarse.joffsets.cpu().numpy(), c_off)
         idx = coarse.ijk_to_index(coarse.ijk, cumulative=True).jdata.cpu().numpy()
         assert np.array_equal(idx, np.arange(c_ijk.shape[0]))
+
+
+@pytest.mark.parametrize("leaves", [1, 257, 9000, 49152, 49153])
+@pytest.mark.parametrize("factor", [2, 8])
+def test_coarse_grid_leaf_counts(cuda_device, leaves, factor):
+    """The hashed build (up to 49,152 fine leaves, remainders of its tiles) and the sorting build above
+    it, two grids, both signs: the voxel sort's grid."""
+    import fvdb
+
+    from oracle import oracle as orc
+
+    rng = np.random.default_rng(leaves)
+    origin = rng.permutation(40**3)[:leaves]
+    origin = np.stack([origin // 1600, origin // 40 % 40, origin % 40], 1) * 8 - 160
+    ijk = (origin[:, None] + rng.integers(0, 8, (leaves, 5, 3))).reshape(-1, 3).astype(np.int32)
+    cut = (leaves // 3) * 5
+    off = np.array([0, cut, ijk.shape[0]], dtype=np.int64)
+    if cut == 0:
+        off = np.array([0, ijk.shape[0]], dtype=np.int64)
+    grid = fvdb.GridBatch.from_ijk(fvdb.JaggedTensor.from_data_and_offsets(
+        torch.from_numpy(ijk).to(cuda_device), torch.from_numpy(off).to(cuda_device)))
+    o_ijk, o_off = orc.grid_from_ijk(ijk, off)
+    c_ijk, c_off = orc.conv_grid(o_ijk, o_off, factor, factor)
+    assert grid._impl.total_leaf_nodes == leaves
+    coarse = grid.conv_grid(factor, factor)
+    assert np.array_equal(coarse.ijk.jdata.cpu().numpy(), c_ijk)
+    assert np.array_equal(coarse.joffsets.cpu().numpy(), c_off)
