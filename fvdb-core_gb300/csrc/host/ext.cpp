@@ -607,6 +607,7 @@ struct PackInfo {
     std::optional<Tensor> out_in_map;      // [ceil(N_tgt/128)*128, K]
     std::optional<Tensor> out_in_map_bwd;  // [ceil(N_src/128)*128, K]
     std::optional<Tensor> nbmap, nbsizes;  // GS form
+    Tensor row_mask;  // occupancy of the forward map's rows where its build made it (3^3, stride 1)
     std::optional<Tensor> tile_mask, tile_mask_t;  // OR of row occupancy per 128-row tile (K <= 32)
     std::optional<Tensor> reorder_loc, sorted_mask, reorder_out_in_map, reduced_sorted_mask;
     std::optional<Tensor> reorder_loc_bwd, reorder_out_in_map_bwd, sorted_mask_bwd_w, sorted_mask_bwd_d;
@@ -658,7 +659,7 @@ PackPtr make_pack(const std::vector<int64_t> &ks_in, const std::vector<int64_t> 
 // Kernel map [ceil(N_tgt/128)*128, K] (padding rows -1); for K <= 32 the per-128-row-tile
 // occupancy masks come out of the same pass into *tile_mask.
 Tensor build_kmap(const GridPtr &src, const GridPtr &tgt, const Vec3 &ks, const Vec3 &st, int32_t K,
-                  Tensor *tile_mask = nullptr) {
+                  Tensor *tile_mask = nullptr, Tensor *row_mask = nullptr) {
     c10::cuda::CUDAGuard guard(tgt->device());
     TORCH_CHECK_VALUE(src->B == tgt->B, "source and target grids must have the same grid count");
     const int64_t npad = (tgt->N + 127) / 128 * 128;
@@ -676,6 +677,15 @@ Tensor build_kmap(const GridPtr &src, const GridPtr &tgt, const Vec3 &ks, const 
     }
     TORCH_CHECK(ok, "kernel map build: clearing the padding failed");
     FvgbGrid s = src->view(), t = tgt->view();
+    bool cube3 = tm && row_mask && tgt->N > 0;
+    for (int a = 0; a < 3; ++a) cube3 = cube3 && ks.v[a] == 3 && st.v[a] == 1;
+    if (cube3) {
+        *row_mask = torch::empty({tgt->N}, kmap.options());
+        check_status(fvgb_kmap_build_masks(&s, &t, ks.v, st.v, kmap.data_ptr<int32_t>(), tm,
+                                           reinterpret_cast<uint32_t *>(row_mask->data_ptr<int32_t>()), cur_stream()),
+                     "kernel map build");
+        return kmap;
+    }
     check_status(fvgb_kmap_build(&s, &t, ks.v, st.v, kmap.data_ptr<int32_t>(), K, nullptr, tm, cur_stream()),
                  "kernel map build");
     return kmap;
@@ -685,7 +695,7 @@ const Tensor &pack_kmap(PackPtr p) {
     resolve_pack(p);
     if (!p->out_in_map) {
         Tensor tm;
-        p->out_in_map = build_kmap(p->src, p->tgt, p->ks, p->st, p->K, &tm);
+        p->out_in_map = build_kmap(p->src, p->tgt, p->ks, p->st, p->K, &tm, &p->row_mask);
         if (tm.defined()) p->tile_mask = tm;
     }
     return *p->out_in_map;
@@ -762,10 +772,18 @@ std::optional<RowOrder> pack_row_order(PackPtr p, bool transposed) {
         size_t wsb = 0;
         check_status(fvgb_kmap_row_order_workspace(n, p->K, &wsb), "row order workspace");
         Tensor ws = workspace(wsb, m.device());
-        check_status(fvgb_kmap_row_order(m.data_ptr<int32_t>(), n, p->K, m.stride(0), rows.data_ptr<int32_t>(),
-                                         reinterpret_cast<uint32_t *>(tmask.data_ptr<int32_t>()),
-                                         smap.data_ptr<int32_t>(), ws.data_ptr(), ws.numel(), cur_stream()),
-                     "row order");
+        if (!transposed && p->row_mask.defined())
+            check_status(fvgb_kmap_row_order_masked(
+                             m.data_ptr<int32_t>(), reinterpret_cast<const uint32_t *>(p->row_mask.data_ptr<int32_t>()), n,
+                             p->K, m.stride(0), rows.data_ptr<int32_t>(),
+                             reinterpret_cast<uint32_t *>(tmask.data_ptr<int32_t>()), smap.data_ptr<int32_t>(),
+                             ws.data_ptr(), ws.numel(), cur_stream()),
+                         "row order");
+        else
+            check_status(fvgb_kmap_row_order(m.data_ptr<int32_t>(), n, p->K, m.stride(0), rows.data_ptr<int32_t>(),
+                                             reinterpret_cast<uint32_t *>(tmask.data_ptr<int32_t>()),
+                                             smap.data_ptr<int32_t>(), ws.data_ptr(), ws.numel(), cur_stream()),
+                         "row order");
         p->order_rows[d] = rows;
         p->order_mask[d] = tmask;
         p->order_map[d] = smap;

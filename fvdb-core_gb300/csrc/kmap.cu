@@ -31,6 +31,7 @@ struct KmapParams {
     int32_t *kmap;
     int32_t *nbsizes;
     uint32_t *tile_mask;    // OR of row occupancy per 128-row tile (K <= 32), may be null
+    uint32_t *row_mask;     // occupancy of every row (kmap_halo3_kernel only), may be null
     int32_t window;         // source leaves staged per CTA (0: not staged)
     int32_t disp_table;     // 1: per-offset displacements tabulated in shared memory
 };
@@ -322,7 +323,9 @@ __global__ void __launch_bounds__(32 * kWarpLeaves) kmap_warp_kernel(KmapParams 
 // position -- against a window-leaf lookup, a mask test and a popcount per entry in
 // kmap_warp_kernel.  Rows are assembled in shared memory with stride 27 (odd: no bank conflicts),
 // which is the map's own layout, and copied out linearly.  Bound by the latency of a leaf's lookups; 1.31M rows of
-// a surface: 112 us with kmap_warp_kernel<3>, 84 us here; a dense 96^3 block 40 us.
+// a surface: 112 us with kmap_warp_kernel<3>, 84 us here, 76 us where the grid maps onto itself and the
+// leaf's own voxels need no walk over its mask words; a dense 96^3 block 40 us.  The rows' occupancy,
+// at hand here, is written out for the row order (a pass over the map for it: 137 us at 5.1M rows).
 constexpr int kHaloLeaves = 4;  // target leaves (warps) per CTA
 struct HaloWarp {
     int32_t idx[1000];
@@ -359,11 +362,19 @@ __global__ void __launch_bounds__(32 * kHaloLeaves) kmap_halo3_kernel(KmapParams
     }
     const int32_t cnt = (int32_t)tl.prefix[7] + __popcll(tl.mask[7]);
     __syncwarp();
+    // a map of a grid onto itself: the leaf's own voxels, most of its halo, are its rows in order
+    const bool own = p.src.leaves == p.tgt.leaves && p.src.num_leaves == p.tgt.num_leaves;
+    if (own)
+        for (int32_t r = lane; r < cnt; r += 32) {
+            const uint32_t s = sm.slots[r];
+            sm.idx[((s >> 6) + 1) * 100 + (((s >> 3) & 7) + 1) * 10 + (s & 7) + 1] = (int32_t)tbase + r;
+        }
 #pragma unroll
     for (int i0 = 0; i0 < 96; i0 += 32) {
         const int i = i0 + lane;
         if (i >= 90) break;
         const int hx = i / 9, iy = (i % 9) / 3, iz = i % 3;
+        if (own && hx >= 1 && hx <= 8 && iy == 1 && iz == 1) continue;  // the leaf itself, above
         const int ix = hx == 0 ? 0 : (hx == 9 ? 2 : 1), q = (hx + 7) & 7;
         const int32_t id = sm.leaf[ix * 9 + iy * 3 + iz];
         if (id < 0) continue;
@@ -396,6 +407,7 @@ __global__ void __launch_bounds__(32 * kHaloLeaves) kmap_halo3_kernel(KmapParams
                 dst[k] = v;
             }
             if (p.tile_mask) atomicOr(&sm.tmask[((tbase + r) >> 7) - t0], bits);
+            if (p.row_mask) p.row_mask[tbase + r] = bits;
         }
         __syncwarp();
         const int32_t n = min(32, cnt - r0) * 27;
@@ -552,9 +564,11 @@ extern "C" int fvgb_kmap_row_order_workspace(int64_t n_out, int32_t K, size_t *b
     return FVGB_OK;
 }
 
-extern "C" int fvgb_kmap_row_order(const int32_t *kmap, int64_t n_out, int32_t K, int64_t ld, int32_t *rows,
-                                   uint32_t *tile_mask, int32_t *sorted_map, void *workspace, size_t workspace_bytes,
-                                   fvgb_stream_t stream) {
+namespace fvgb {
+namespace {
+// given_mask: the rows' occupancy where the map's build already made it (null: read from the map)
+int row_order(const int32_t *kmap, const uint32_t *given_mask, int64_t n_out, int32_t K, int64_t ld, int32_t *rows,
+              uint32_t *tile_mask, int32_t *sorted_map, void *workspace, size_t workspace_bytes, fvgb_stream_t stream) {
     size_t need = 0;
     int st = fvgb_kmap_row_order_workspace(n_out, K, &need);
     if (st) return st;
@@ -570,20 +584,21 @@ extern "C" int fvgb_kmap_row_order(const int32_t *kmap, int64_t n_out, int32_t K
     };
     uint8_t *p = reinterpret_cast<uint8_t *>(((uintptr_t)workspace + 255) & ~(uintptr_t)255);
     const size_t n = (size_t)n_out;
-    uint32_t *mask = (uint32_t *)carve(p, n * 4);
+    uint32_t *own_mask = (uint32_t *)carve(p, n * 4);
+    const uint32_t *mask = given_mask ? given_mask : own_mask;
     uint32_t *smask = (uint32_t *)carve(p, n * 4);
     int32_t *iota = (int32_t *)carve(p, n * 4);
     size_t cub_bytes = 0;
     cub::DeviceRadixSort::SortPairsDescending(nullptr, cub_bytes, mask, smask, iota, rows, (int)n_out, 0, K, s);
     if ((size_t)(p - (uint8_t *)workspace) + cub_bytes > workspace_bytes) return FVGB_ENOSPACE;
     const unsigned tiles = (unsigned)ceil_div(n_out, 128);
-    masks_kernel<<<tiles, 128, 0, s>>>(kmap, n_out, K, ld, mask, nullptr);
+    if (!given_mask) masks_kernel<<<tiles, 128, 0, s>>>(kmap, n_out, K, ld, own_mask, nullptr);
     iota_kernel<<<(unsigned)ceil_div(n_out, 256), 256, 0, s>>>(iota, n_out);
     if (cub::DeviceRadixSort::SortPairsDescending(p, cub_bytes, mask, smask, iota, rows, (int)n_out, 0, K, s) !=
         cudaSuccess)
         return launch_status();
     order_tiles_kernel<<<tiles, 128, 0, s>>>(smask, n_out, rows, tile_mask);
-    int launched = 3;
+    int launched = given_mask ? 2 : 3;
     if (sorted_map) {
         const int64_t n_pad = (int64_t)tiles * 128;
         launch_permute(kmap, ld, K, rows, n_pad, sorted_map, s);
@@ -592,13 +607,28 @@ extern "C" int fvgb_kmap_row_order(const int32_t *kmap, int64_t n_out, int32_t K
     count_launches(launched);
     return launch_status();
 }
+}  // namespace
+}  // namespace fvgb
+
+extern "C" int fvgb_kmap_row_order(const int32_t *kmap, int64_t n_out, int32_t K, int64_t ld, int32_t *rows,
+                                   uint32_t *tile_mask, int32_t *sorted_map, void *workspace, size_t workspace_bytes,
+                                   fvgb_stream_t stream) {
+    return row_order(kmap, nullptr, n_out, K, ld, rows, tile_mask, sorted_map, workspace, workspace_bytes, stream);
+}
+
+extern "C" int fvgb_kmap_row_order_masked(const int32_t *kmap, const uint32_t *row_mask, int64_t n_out, int32_t K,
+                                          int64_t ld, int32_t *rows, uint32_t *tile_mask, int32_t *sorted_map,
+                                          void *workspace, size_t workspace_bytes, fvgb_stream_t stream) {
+    if (!row_mask) return FVGB_EINVAL;
+    return row_order(kmap, row_mask, n_out, K, ld, rows, tile_mask, sorted_map, workspace, workspace_bytes, stream);
+}
 
 namespace fvgb {
 namespace {
 // start: source offset of kernel position 0, per user component
 int build_map(const FvgbGrid *src, const FvgbGrid *tgt, const int32_t ksize[3], const int32_t stride[3],
               const int32_t start[3], int32_t *kmap, int64_t ld, int32_t *nbsizes, uint32_t *tile_mask,
-              fvgb_stream_t stream) {
+              uint32_t *row_mask, fvgb_stream_t stream) {
     if (src->num_grids != tgt->num_grids) return FVGB_EINVAL;
     const int64_t K = (int64_t)ksize[0] * ksize[1] * ksize[2];
     if (K > (1 << 20) || ld < K) return FVGB_EINVAL;
@@ -617,6 +647,7 @@ int build_map(const FvgbGrid *src, const FvgbGrid *tgt, const int32_t ksize[3], 
     p.kmap = kmap;
     p.nbsizes = nbsizes;
     p.tile_mask = tile_mask;
+    p.row_mask = row_mask;
     // The source-leaf window of a target leaf has the same extent for every leaf (leaf origins
     // are multiples of 8, so origin*stride is too): size shared memory to it.
     auto span = [](int32_t s, int32_t st, int32_t k) { return ((7 * s + st + k - 1) >> 3) - (st >> 3) + 1; };
@@ -668,7 +699,17 @@ extern "C" int fvgb_kmap_build(const FvgbGrid *src, const FvgbGrid *tgt, const i
         // kernelStart = floor(-K/2 + 1) (ConvolutionKernelMap.cu:114-116)
         start[a] = (int32_t)floor(-ksize[a] / 2.0 + 1.0);
     }
-    return build_map(src, tgt, ksize, stride, start, kmap, ld, nbsizes, tile_mask, stream);
+    return build_map(src, tgt, ksize, stride, start, kmap, ld, nbsizes, tile_mask, nullptr, stream);
+}
+
+extern "C" int fvgb_kmap_build_masks(const FvgbGrid *src, const FvgbGrid *tgt, const int32_t ksize[3],
+                                     const int32_t stride[3], int32_t *kmap, uint32_t *tile_mask, uint32_t *row_mask,
+                                     fvgb_stream_t stream) {
+    if (!src || !tgt || !ksize || !stride || !tile_mask || !row_mask) return FVGB_EINVAL;
+    for (int a = 0; a < 3; ++a)
+        if (ksize[a] != 3 || stride[a] != 1) return FVGB_EINVAL;
+    const int32_t start[3] = {-1, -1, -1};
+    return build_map(src, tgt, ksize, stride, start, kmap, 27, nullptr, tile_mask, row_mask, stream);
 }
 
 extern "C" int fvgb_window_map(const FvgbGrid *fine, const FvgbGrid *coarse, const int32_t window[3],
@@ -684,7 +725,7 @@ extern "C" int fvgb_window_map(const FvgbGrid *fine, const FvgbGrid *coarse, con
     }
     const int64_t W = (int64_t)ks[0] * ks[1] * ks[2];
     if (W > 512) return FVGB_EINVAL;
-    return build_map(fine, coarse, ks, st, start, map, W, nullptr, nullptr, stream);
+    return build_map(fine, coarse, ks, st, start, map, W, nullptr, nullptr, nullptr, stream);
 }
 
 extern "C" int fvgb_kmap_transpose(const int32_t *kmap, int64_t n_out, int32_t K, int64_t ld, int32_t *mapT,

@@ -246,6 +246,10 @@ int fvgb_compact_ijk(const int32_t *ijk, const uint8_t *valid, const int64_t *sr
 int fvgb_kmap_build(const FvgbGrid *src, const FvgbGrid *tgt, const int32_t ksize[3],
                     const int32_t stride[3], int32_t *kmap, int64_t ld, int32_t *nbsizes,
                     uint32_t *tile_mask, fvgb_stream_t stream);
+/* fvgb_kmap_build of a 3^3 stride-1 map (ld = 27) with the occupancy of every row as well (row_mask
+ * [tgt voxels], bit k = offset k present): what fvgb_kmap_row_order_masked sorts by. */
+int fvgb_kmap_build_masks(const FvgbGrid *src, const FvgbGrid *tgt, const int32_t ksize[3], const int32_t stride[3],
+                          int32_t *kmap, uint32_t *tile_mask, uint32_t *row_mask, fvgb_stream_t stream);
 
 /*
  * mapT[i*ldT + k] = t where kmap[t*ld + k] == i, else -1 (fills all n_in rows).
@@ -288,6 +292,10 @@ int fvgb_kmap_row_order_workspace(int64_t n_out, int32_t K, size_t *bytes);
 int fvgb_kmap_row_order(const int32_t *kmap, int64_t n_out, int32_t K, int64_t ld, int32_t *rows,
                         uint32_t *tile_mask, int32_t *sorted_map, void *workspace, size_t workspace_bytes,
                         fvgb_stream_t stream);
+/* The same with the rows' occupancy masks given (a map build's row_mask). */
+int fvgb_kmap_row_order_masked(const int32_t *kmap, const uint32_t *row_mask, int64_t n_out, int32_t K, int64_t ld,
+                               int32_t *rows, uint32_t *tile_mask, int32_t *sorted_map, void *workspace,
+                               size_t workspace_bytes, fvgb_stream_t stream);
 
 /* ---------------------------------------------------------------- contractions --- */
 

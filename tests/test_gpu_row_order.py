@@ -150,3 +150,61 @@ def test_simt_rows_equals_index_order(cuda_device, dtype, code):
     w5 = w.double().cpu().numpy().reshape(3, 3, 3, cin, cout).transpose(4, 3, 2, 1, 0)
     ref = orc.conv_forward_f64(x.double().cpu().numpy(), w5, km)
     assert rel_l2(y1.double().cpu().numpy(), ref) <= (1e-6 if dtype == torch.float32 else 1e-13)
+
+
+@pytest.mark.parametrize("n_vox,extent,same", [(1, 4, True), (9000, 30, True), (9000, 30, False), (30000, 34, True)])
+def test_map_build_row_masks(cuda_device, n_vox, extent, same):
+    """fvgb_kmap_build_masks: the map, tile masks and row masks of a 3^3 map (of a grid onto itself and
+    onto another grid), and fvgb_kmap_row_order_masked equal to the order read from the map."""
+    import fvdb
+    from fvdb import _lib
+
+    lib = _lib.cdll()
+
+    class Grid(ctypes.Structure):
+        _fields_ = [
+            ("num_grids", ctypes.c_int32), ("reserved", ctypes.c_int32), ("num_voxels", ctypes.c_int64),
+            ("num_leaves", ctypes.c_int64), ("hash_capacity", ctypes.c_int64), ("voxel_offsets", ctypes.c_void_p),
+            ("ijk", ctypes.c_void_p), ("leaves", ctypes.c_void_p), ("hash_slots", ctypes.c_void_p),
+        ]
+
+    def grid(seed):
+        return fvdb.GridBatch.from_ijk(torch.from_numpy(random_sparse_ijk(n_vox, extent, seed)).to(cuda_device))
+
+    def view(g):
+        i = g._impl
+        return Grid(i.grid_count, 0, i.total_voxels, i.total_leaf_nodes, i.hash.numel(), i.joffsets.data_ptr(),
+                    i.ijk.data_ptr(), i.leaves.data_ptr(), i.hash.data_ptr())
+
+    tgt = grid(3)
+    src = tgt if same else grid(4)
+    n, K, tiles = tgt.total_voxels, 27, (tgt.total_voxels + 127) // 128
+    kmap = torch.full((tiles * 128, K), -7, dtype=torch.int32, device=cuda_device)
+    kmap[n:] = -1
+    tm = torch.zeros(tiles, dtype=torch.int32, device=cuda_device)
+    rm = torch.full((n,), -7, dtype=torch.int32, device=cuda_device)
+    ks, st = (ctypes.c_int32 * 3)(3, 3, 3), (ctypes.c_int32 * 3)(1, 1, 1)
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    s, t = view(src), view(tgt)
+    assert lib.fvgb_kmap_build_masks(ctypes.byref(s), ctypes.byref(t), ks, st, P(kmap), P(tm), P(rm), stream) == 0
+    torch.cuda.synchronize()
+    off = np.array([0, n])
+    a, b = src.ijk.jdata.cpu().numpy(), tgt.ijk.jdata.cpu().numpy()
+    o = orc.kernel_map(a, np.array([0, len(a)]), b, off, (3, 3, 3), (1, 1, 1))
+    assert np.array_equal(kmap[:n].cpu().numpy(), o)
+    bits = ((o >= 0).astype(np.int64) << np.arange(K)).sum(1)
+    assert np.array_equal(rm.cpu().numpy().astype(np.int64) & 0xFFFFFFFF, bits)
+    pad = np.zeros(tiles * 128, np.int64)
+    pad[:n] = bits
+    assert np.array_equal(tm.cpu().numpy().astype(np.int64) & 0xFFFFFFFF, np.bitwise_or.reduce(pad.reshape(tiles, 128), axis=1))
+    ref = _row_order(lib, kmap, n, K, cuda_device)
+    got = [torch.empty_like(ref[0]), torch.zeros_like(ref[1]), torch.empty_like(ref[2])]
+    wsb = ctypes.c_size_t(0)
+    assert lib.fvgb_kmap_row_order_workspace(ctypes.c_int64(n), K, ctypes.byref(wsb)) == 0
+    ws = torch.empty(wsb.value, dtype=torch.uint8, device=cuda_device)
+    assert lib.fvgb_kmap_row_order_masked(P(kmap), P(rm), ctypes.c_int64(n), K, ctypes.c_int64(K), P(got[0]), P(got[1]),
+                                          P(got[2]), P(ws), ctypes.c_size_t(ws.numel()), stream) == 0
+    torch.cuda.synchronize()
+    assert all(torch.equal(x, y) for x, y in zip(got, ref))
+    st2 = (ctypes.c_int32 * 3)(2, 2, 2)  # refused before any launch
+    assert lib.fvgb_kmap_build_masks(ctypes.byref(s), ctypes.byref(t), ks, st2, P(kmap), P(tm), P(rm), stream) == 1
