@@ -1152,11 +1152,16 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
             tsci = wt.stride(1);
             tsco = wt.stride(2);
         }
-        check_status(fvgb_conv_fwd_simt_rows(dt, x.data_ptr(), x.size(0), (int32_t)cin, x.stride(0),
-                                             m_used.data_ptr<int32_t>(), n_out, (int32_t)K, m_used.stride(0),
-                                             order ? order->rows.data_ptr<int32_t>() : nullptr, first_offset(wt), tsk,
-                                             tsci, tsco, y.data_ptr(), (int32_t)cout, y.stride(0), 0, s),
+        // without a scale ahead of them, bias and ReLU go with the contraction's stores
+        Tensor bc;
+        if (bias && !out_scale) bc = bias->to(y.scalar_type()).contiguous();
+        check_status(fvgb_conv_fwd_simt_finish(dt, x.data_ptr(), x.size(0), (int32_t)cin, x.stride(0),
+                                               m_used.data_ptr<int32_t>(), n_out, (int32_t)K, m_used.stride(0),
+                                               order ? order->rows.data_ptr<int32_t>() : nullptr, first_offset(wt), tsk,
+                                               tsci, tsco, y.data_ptr(), (int32_t)cout, y.stride(0),
+                                               bc.defined() ? bc.data_ptr() : nullptr, relu && !out_scale ? 1 : 0, s),
                      "sparse conv forward");
+        if (!out_scale) return y;
     } else {
         // 16-bit features of shapes the tensor-core kernel does not take: CUDA cores, FP32
         // accumulate, rounded once at the end.

@@ -322,6 +322,12 @@ int fvgb_conv_fwd_simt_rows(int32_t dtype, const void *x, int64_t n_x, int32_t c
                             int64_t n_out, int32_t K, int64_t ldm, const int32_t *rows, const void *w, int64_t wsk,
                             int64_t wsci, int64_t wsco, void *y, int32_t c_out, int64_t ldy, int32_t accumulate,
                             fvgb_stream_t stream);
+/* The same (rows may be null: index order) with a bias [c_out] of the features' dtype (null: none) added
+ * to the finished sum and, where relu != 0, negative results replaced by zero. */
+int fvgb_conv_fwd_simt_finish(int32_t dtype, const void *x, int64_t n_x, int32_t c_in, int64_t ldx, const int32_t *map,
+                              int64_t n_out, int32_t K, int64_t ldm, const int32_t *rows, const void *w, int64_t wsk,
+                              int64_t wsci, int64_t wsco, void *y, int32_t c_out, int64_t ldy, const void *bias,
+                              int32_t relu, fvgb_stream_t stream);
 
 /*
  * Weight gradient on CUDA cores:  dW[k, ci, co] = sum_m x[map[m,k], ci] * dy[m, co].

@@ -42,3 +42,30 @@ def test_forward_and_gradients(cuda_device, dtype, tol, cin, cout, n):
         assert rel(f64(y), y_ref) <= tol
         assert rel(f64(dx), dx_ref) <= tol
         assert rel(f64(dw), dw_ref) <= tol
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("cin,cout,n", [(8, 16, 900), (64, 32, 70000), (32, 64, 500), (3, 5, 300), (100, 36, 300)])
+def test_bias_and_relu(cuda_device, dtype, cin, cout, n):
+    """Bias and ReLU with the contraction's stores (short rows, narrow, wide and element-wise tiles, row
+    order) equal the separate additions and clamps, bit for bit, NaN included."""
+    import fvdb
+    from fvdb import _lib
+
+    grid = fvdb.GridBatch.from_ijk(torch.from_numpy(random_sparse_ijk(n, 64, n)).to(cuda_device))
+    pack, _ = grid.sparse_conv_kernel_map(3, 1)
+    g = torch.Generator().manual_seed(cin + cout)
+    x = torch.randn(grid.total_voxels, cin, generator=g, dtype=dtype).to(cuda_device)
+    x[5] = float("nan")
+    w = (torch.randn(cout, cin, 3, 3, 3, generator=g, dtype=dtype) / (27 * cin) ** 0.5).to(cuda_device)
+    bias = torch.randn(cout, generator=g, dtype=dtype).to(cuda_device)
+    conv = _lib.load().conv_forward
+    y = conv(x, w, pack._impl, False)[0]
+    bits = torch.int32 if dtype == torch.float32 else torch.int64
+    for b, relu in ((bias, False), (bias, True), (None, True)):
+        got = conv(x, w, pack._impl, False, b, relu)[0]
+        ref = y if b is None else y + b
+        ref = torch.relu(ref) if relu else ref
+        nan = torch.isnan(ref)
+        assert torch.equal(torch.isnan(got), nan)
+        assert torch.equal(got[~nan].view(bits), ref[~nan].view(bits))
