@@ -809,7 +809,7 @@ struct CoarseHash {
     int32_t *count;    // [nl] voxels of the coarse leaf at each place
     int32_t *grid;     // [nl] grid of the coarse leaf at each place
     int32_t *base;     // [nl + 1] first voxel of each place
-    int32_t *found;    // [1] coarse leaves
+    int32_t *found;    // [1] coarse leaves - 1 (cleared to all ones together with the table before it)
     uint64_t *cmask;   // [nl][8]
     int4 *corig;       // [nl]
     int64_t cap;
@@ -830,7 +830,7 @@ __global__ void coarse_insert_kernel(const FvgbLeaf *__restrict__ leaves, int64_
     for (int64_t probe = 0; probe < h.cap; ++probe) {  // at most half full: a free slot is found
         const uint64_t k = atomicCAS(reinterpret_cast<unsigned long long *>(h.table + s), ~0ull, key);
         if (k == ~0ull) {
-            const int32_t id = atomicAdd(h.found, 1);
+            const int32_t id = atomicAdd(h.found, 1) + 1;
             h.slot_id[s] = id;
             h.key[id] = key;
             h.corig[id] = make_int4(cx, cy, cz, lf.batch);
@@ -848,10 +848,12 @@ __global__ void coarse_insert_kernel(const FvgbLeaf *__restrict__ leaves, int64_
 // rows of eight z positions as bytes, so it costs two shared-memory updates however full the leaf is
 // (21.7k leaves: 15.6 us voxel by voxel, 4.6 us).
 __global__ void __launch_bounds__(256) coarse_or_kernel(const FvgbLeaf *__restrict__ leaves, int64_t nl, int3 sh,
-                                                        CoarseHash h) {
+                                                        CoarseHash h, int32_t *__restrict__ slots, int64_t cap) {
     __shared__ uint32_t wm[8][16];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t l = (int64_t)blockIdx.x * 8 + warp;
+    // the leaf hash that coarse_place_kernel fills starts out free
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < cap; i += (int64_t)gridDim.x * 256) slots[i] = -1;
     if (l >= nl) return;  // whole warps leave together
     const FvgbLeaf &lf = leaves[l];
     const int64_t c = h.slot_id[h.slot[l]];
@@ -889,7 +891,7 @@ template <typename Key>
 __global__ void __launch_bounds__(kRankThreads) coarse_rank_kernel(CoarseHash h) {
     __shared__ Key keys[kRankThreads];
     constexpr int kOwn = kRankThreads / kRankSplit;  // leaves per CTA
-    const int32_t n = *h.found;
+    const int32_t n = *h.found + 1;
     if ((int64_t)blockIdx.x * kOwn >= n) return;
     const int part = threadIdx.x % kRankSplit;
     const int32_t i = blockIdx.x * kOwn + threadIdx.x / kRankSplit;
@@ -918,41 +920,66 @@ __global__ void __launch_bounds__(kRankThreads) coarse_rank_kernel(CoarseHash h)
     h.grid[rank] = h.corig[i].w;
 }
 
-// one CTA: first voxel of every place, and meta[b] = first voxel of grid b, meta[B+1] = coarse leaves,
-// meta[B+2] = voxels
-__global__ void __launch_bounds__(kScanThreads) coarse_scan_kernel(CoarseHash h, int32_t B, int64_t *meta) {
+// One CTA: first voxel of every place (count and grid of each of n > 0 places given, base [n + 1]) and
+// first voxel of every grid, offsets [B + 1]; returns the voxels.
+__device__ __forceinline__ int32_t scan_places(int32_t n, const int32_t *__restrict__ count,
+                                               const int32_t *__restrict__ grid, int32_t B, int32_t *__restrict__ base,
+                                               int64_t *__restrict__ offsets) {
     using Scan = cub::BlockScan<int32_t, kScanThreads>;
     __shared__ typename Scan::TempStorage tmp;
-    const int32_t n = *h.found;
     int32_t run = 0;
     constexpr int kItems = 8;
     for (int32_t p0 = 0; p0 < n; p0 += kScanThreads * kItems) {
         int32_t v[kItems], g[kItems + 1], total;
-        g[0] = -1;
+        const int32_t q = p0 + threadIdx.x * kItems;
+        const bool whole = q + kItems <= n;  // 16-byte accesses: the arrays start on 256 bytes
+        g[0] = q > 0 && q < n ? grid[q - 1] : -1;
+        if (whole) {
 #pragma unroll
-        for (int i = 0; i < kItems; ++i) {
-            const int32_t p = p0 + threadIdx.x * kItems + i;
-            v[i] = p < n ? h.count[p] : 0;
-            g[i + 1] = p < n ? h.grid[p] : -1;
-            if (i == 0 && p > 0 && p < n) g[0] = h.grid[p - 1];
+            for (int i = 0; i < kItems; i += 4) {
+                const int4 a = *reinterpret_cast<const int4 *>(count + q + i);
+                const int4 b = *reinterpret_cast<const int4 *>(grid + q + i);
+                v[i] = a.x, v[i + 1] = a.y, v[i + 2] = a.z, v[i + 3] = a.w;
+                g[i + 1] = b.x, g[i + 2] = b.y, g[i + 3] = b.z, g[i + 4] = b.w;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < kItems; ++i) {
+                v[i] = q + i < n ? count[q + i] : 0;
+                g[i + 1] = q + i < n ? grid[q + i] : -1;
+            }
         }
         __syncthreads();
         Scan(tmp).ExclusiveSum(v, v, total);
+        if (whole) {
+#pragma unroll
+            for (int i = 0; i < kItems; i += 4)
+                *reinterpret_cast<int4 *>(base + q + i) =
+                    make_int4(run + v[i], run + v[i + 1], run + v[i + 2], run + v[i + 3]);
+        }
 #pragma unroll
         for (int i = 0; i < kItems; ++i) {
-            const int32_t p = p0 + threadIdx.x * kItems + i;
+            const int32_t p = q + i;
             if (p >= n) break;
-            h.base[p] = run + v[i];
-            for (int32_t b = g[i] + 1; b <= g[i + 1]; ++b) meta[b] = run + v[i];  // grids that begin here
+            if (!whole) base[p] = run + v[i];
+            for (int32_t b = g[i] + 1; b <= g[i + 1]; ++b) offsets[b] = run + v[i];  // grids that begin here
             if (p == n - 1)
-                for (int32_t b = g[i + 1] + 1; b <= B; ++b) meta[b] = run + total;  // and those after the last
+                for (int32_t b = g[i + 1] + 1; b <= B; ++b) offsets[b] = run + total;  // and those after the last
         }
         run += total;
     }
+    if (threadIdx.x == 0) base[n] = run;
+    return run;
+}
+
+// meta[b] = first voxel of grid b, meta[B+1] = coarse leaves, meta[B+2] = voxels
+__global__ void __launch_bounds__(kScanThreads) coarse_scan_kernel(CoarseHash h, int32_t B, int64_t *meta) {
+    const int32_t n = *h.found + 1;
+    const int32_t voxels = scan_places(n, h.count, h.grid, B, h.base, meta);
     if (threadIdx.x == 0) {
-        h.base[n] = run;
         meta[B + 1] = n;
-        meta[B + 2] = run;
+        meta[B + 2] = voxels;
+        meta[B + 3] = 0;
     }
 }
 
@@ -962,7 +989,7 @@ __global__ void __launch_bounds__(256) coarse_place_kernel(CoarseHash h, int32_t
                                                            int64_t cap) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t p = (int64_t)blockIdx.x * 8 + warp;
-    if (p >= *h.found) return;
+    if (p > *h.found) return;
     const int64_t c = h.order[p];
     const int4 o = h.corig[c];
     emit_leaf(h.cmask[c * 8 + (lane >> 2)], o.x, o.y, o.z, o.w, h.base[p], p, lane, out_ijk, leaves, slots, cap);
@@ -981,6 +1008,7 @@ size_t coarse_hash_layout(int64_t nl, CoarseHash *w, char *base) {
     };
     const size_t n = (size_t)nl;
     h.table = (uint64_t *)take((size_t)h.cap * 8);
+    h.found = (int32_t *)take(4);
     h.slot_id = (int32_t *)take((size_t)h.cap * 4);
     h.key = (uint64_t *)take(n * 8);
     h.slot = (int32_t *)take(n * 4);
@@ -988,7 +1016,6 @@ size_t coarse_hash_layout(int64_t nl, CoarseHash *w, char *base) {
     h.count = (int32_t *)take(n * 4);
     h.grid = (int32_t *)take(n * 4);
     h.base = (int32_t *)take((n + 1) * 4);
-    h.found = (int32_t *)take(4);
     h.cmask = (uint64_t *)take(n * 64);
     h.corig = (int4 *)take(n * 16);
     if (w) *w = h;
@@ -1075,35 +1102,33 @@ extern "C" int fvgb_coarse_grid_build(const FvgbGrid *fine, const int32_t factor
 
 // ---------------------------------------------------------------------------------------------
 // Grid build through a leaf hash, for inputs with many rows per leaf: the rows of ijk (or points)
-// are never sorted.  One pass inserts every row's leaf into an open-addressing table, a second ORs
-// the row's voxel into its leaf's 512-bit mask; then only the leaves are sorted and the voxels are
-// written leaf by leaf in bit order, with the leaf table and the leaf hash in the same kernel.
-// Leaves sorted by (grid, order key) and voxels by bit is the order of the voxel sort, so the grid
-// is identical to fvgb_ijk_sort_unique's.  7.9M points, 1.08M voxels, 27k leaves in four grids:
-// voxelise, sort, unique and index took 1.9 ms, 0.33 ms here (bound by the random reads of
-// the table, which stays in L2).  The table has room for rows / 8 leaves; an input with more
-// (fewer than eight rows per leaf) raises `overflow` and is left to the sort.
+// are never sorted.  One pass inserts every row's leaf into an open-addressing table, ORs the row's
+// voxel into the slot's 512-bit mask and counts the voxels that were new, so one read tells the host
+// every size; then only the leaves are sorted and the voxels are written leaf by leaf in bit order,
+// with the leaf table and the leaf hash in the same kernel.  Leaves sorted by (grid, order key) and
+// voxels by bit is the order of the voxel sort, so the grid is identical to fvgb_ijk_sort_unique's.
+// 7.9M points, 1.31M voxels, 22k leaves in four grids: voxelise, sort, unique and index took 1.9 ms,
+// 0.20 ms here, bound by the random reads of the table and the masks.  The table has room for
+// rows / 8 leaves at three quarters full; an input with more (fewer than eight rows per leaf) raises
+// `overflow` and is left to the sort.
 namespace fvgb {
 namespace {
 
 constexpr uint64_t kEmptyLeaf = ~0ull;
-constexpr int kHashRows = 8;      // rows per thread
-constexpr int kHashProbes = 128;  // a full neighbourhood of the table counts as overflow
+constexpr int kHashRows = 4;      // rows per thread (more cost occupancy: 169 us with 8, 151 with 2, 132 with 4)
+constexpr int kHashProbes = 512;  // a full neighbourhood of the table counts as overflow
 constexpr int kHashMaxGrids = 1023;  // the grid index takes the key's top 10 bits (all ones: the empty slot)
 
 struct LeafHash {
     uint64_t *table;    // [cap] leaf keys, kEmptyLeaf where free
-    int32_t *slot_id;   // [cap] leaf of a taken slot
+    uint64_t *mask;     // [cap][8] voxels of the slot's leaf, cleared with the pass
     uint64_t *keys;     // [max_leaves] key of each leaf, in insertion order
-    uint64_t *mask;     // [max_leaves][8]
-    uint32_t *row_slot; // [n]
-    uint16_t *row_bit;  // [n]
-    int64_t cap, max_leaves;
+    uint32_t *leaf_slot;  // [max_leaves] its slot
+    uint32_t cap;
+    int32_t max_leaves;
 };
 
 size_t leaf_hash_layout(int64_t n, LeafHash *w, char *base) {
-    int64_t cap = 1024;
-    while (cap < n / 4) cap <<= 1;
     size_t off = 0;
     auto take = [&](size_t bytes) {
         char *p = base ? base + off : nullptr;
@@ -1111,51 +1136,56 @@ size_t leaf_hash_layout(int64_t n, LeafHash *w, char *base) {
         return p;
     };
     LeafHash h;
-    h.cap = cap;
-    h.max_leaves = cap / 2;
-    h.table = (uint64_t *)take((size_t)cap * 8);
-    h.slot_id = (int32_t *)take((size_t)cap * 4);
+    h.max_leaves = (int32_t)std::max<int64_t>(512, ceil_div(n, (int64_t)8));
+    h.cap = (uint32_t)((int64_t)h.max_leaves / 3 * 4 + 4);
+    h.table = (uint64_t *)take((size_t)h.cap * 8);
+    h.mask = (uint64_t *)take((size_t)h.cap * 64);
     h.keys = (uint64_t *)take((size_t)h.max_leaves * 8);
-    h.mask = (uint64_t *)take((size_t)h.max_leaves * 64);
-    h.row_slot = (uint32_t *)take((size_t)n * 4);
-    h.row_bit = (uint16_t *)take((size_t)n * 2);
+    h.leaf_slot = (uint32_t *)take((size_t)h.max_leaves * 4);
     if (w) *w = h;
     return off;
 }
 
-// stat: [0] leaves, [1] error word, [2] overflow, [3..5] largest -x, -y, -z, [6..8] largest x, y, z
-__device__ __forceinline__ uint32_t insert_leaf(const LeafHash &h, uint64_t key, int32_t *__restrict__ stat) {
+// first slot tried for a leaf: the key's hash scaled to the table (its size is no power of two)
+__device__ __forceinline__ uint32_t leaf_home(const LeafHash &h, uint64_t key) {
     uint64_t m = key * 0x9E3779B97F4A7C15ull;
     m ^= m >> 32;
     m *= 0xD6E8FEB86659FD93ull;
-    m ^= m >> 29;
-    const uint64_t cap_mask = (uint64_t)h.cap - 1;
-    uint64_t s = m & cap_mask;
+    return __umulhi((uint32_t)(m >> 32), h.cap);
+}
+
+// The slot of a leaf, from slot s on.  stat: [0] leaves, [1] error word, [2] overflow, [3..5] largest
+// -x, -y, -z, [6..8] largest x, y, z, [9..] voxels of each grid
+__device__ __forceinline__ uint32_t insert_leaf(uint64_t *table, uint64_t *keys, uint32_t *leaf_slot, uint32_t cap,
+                                              int32_t max_leaves, uint64_t key, uint32_t s, int32_t *stat) {
     for (int probe = 0; probe < kHashProbes; ++probe) {
-        uint64_t k = *reinterpret_cast<volatile uint64_t *>(h.table + s);
+        uint64_t k = *reinterpret_cast<volatile uint64_t *>(table + s);
         if (k == kEmptyLeaf) {
-            k = atomicCAS(reinterpret_cast<unsigned long long *>(h.table + s), kEmptyLeaf, key);
-            if (k == kEmptyLeaf) {  // this thread's leaf: number it and clear its mask for the next pass
+            k = atomicCAS(reinterpret_cast<unsigned long long *>(table + s), kEmptyLeaf, key);
+            if (k == kEmptyLeaf) {  // this thread's leaf
                 const int32_t id = atomicAdd(stat, 1);
-                h.slot_id[s] = id;
-                if (id < h.max_leaves) {
-                    h.keys[id] = key;
-#pragma unroll
-                    for (int w = 0; w < 8; ++w) h.mask[(int64_t)id * 8 + w] = 0;
+                if (id < max_leaves) {
+                    keys[id] = key;
+                    leaf_slot[id] = s;
                 } else {
                     stat[2] = 1;
                 }
-                return (uint32_t)s;
+                return s;
             }
         }
-        if (k == key) return (uint32_t)s;
-        s = (s + 1) & cap_mask;
+        if (k == key) return s;
+        s = s + 1 < cap ? s + 1 : 0;
     }
     stat[2] = 1;
-    return 0;
+    return s;
 }
 
-// Pass 1 over ijk rows (P = int32_t) or points (P = the points' type, voxelised in T).
+__global__ void stat_init_kernel(int32_t *stat, int32_t n) {
+    const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) stat[i] = i >= 3 && i < 9 ? INT32_MIN : 0;
+}
+
+// The pass over ijk rows (P = int32_t) or points (P = the points' type, voxelised in T).
 template <typename P, typename T>
 __global__ void __launch_bounds__(256) leaf_insert_kernel(const P *__restrict__ in, const int64_t *__restrict__ joff,
                                                           int32_t B, int64_t n, const double *__restrict__ vs,
@@ -1163,7 +1193,7 @@ __global__ void __launch_bounds__(256) leaf_insert_kernel(const P *__restrict__ 
                                                           int32_t *__restrict__ stat) {
     constexpr bool kPoints = !std::is_same<P, int32_t>::value;
     __shared__ T fac[6];
-    __shared__ int32_t sb[2], full, box[6][8];
+    __shared__ int32_t sb[2], full, box[7][8];
     const int64_t base = (int64_t)blockIdx.x * 256 * kHashRows;
     const int64_t last = min(n, base + 256 * kHashRows) - 1;
     if (threadIdx.x < 2) sb[threadIdx.x] = batch_of(joff, B, threadIdx.x == 0 ? base : last);
@@ -1207,49 +1237,61 @@ __global__ void __launch_bounds__(256) leaf_insert_kernel(const P *__restrict__ 
             lim[3 + a] = max(lim[3 + a], c[q][a]);
         }
     }
+    // Every step's accesses for all rows go out together: the first probe, which finds most leaves, the
+    // mask words, and the updates, whose results are looked at last (one after another each update's
+    // wait added up: 200 us for 7.9M points, 132 us).
+    uint64_t key[kHashRows], word[kHashRows];
+    uint32_t slot[kHashRows], bit[kHashRows];
 #pragma unroll
     for (int q = 0; q < kHashRows; ++q) {
-        const int64_t i = base + q * 256 + threadIdx.x;
-        if (i > last) break;
+        const int64_t i = min(base + q * 256 + threadIdx.x, last);
         const int32_t b = sb[0] == sb[1] ? sb[0] : batch_of(joff, B, i);
         const uint64_t k = order_key(c[q][0], c[q][1], c[q][2]);
-        h.row_slot[i] = insert_leaf(h, ((uint64_t)b << 54) | (k >> 9), stat);
-        h.row_bit[i] = (uint16_t)(k & 511);
+        bit[q] = (uint32_t)(k & 511);
+        key[q] = ((uint64_t)b << 54) | (k >> 9);
+        slot[q] = leaf_home(h, key[q]);
+        word[q] = __ldcg(h.table + slot[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < kHashRows; ++q)
+        if (word[q] != key[q]) slot[q] = insert_leaf(h.table, h.keys, h.leaf_slot, h.cap, h.max_leaves, key[q], slot[q], stat);
+#pragma unroll
+    for (int q = 0; q < kHashRows; ++q)
+        word[q] = __ldcg(h.mask + (size_t)slot[q] * 8 + (bit[q] >> 6));
+#pragma unroll
+    for (int q = 0; q < kHashRows; ++q) {
+        const uint64_t m = 1ull << (bit[q] & 63);
+        if (!(word[q] & m))  // most rows of a dense cloud have nothing to set
+            word[q] = atomicOr(reinterpret_cast<unsigned long long *>(h.mask + (size_t)slot[q] * 8 + (bit[q] >> 6)), m);
+    }
+    int32_t fresh = 0;  // voxels this thread set
+#pragma unroll
+    for (int q = 0; q < kHashRows; ++q) {
+        if (word[q] >> (bit[q] & 63) & 1) continue;
+        if (sb[0] == sb[1]) ++fresh;
+        else atomicAdd(stat + 9 + (int32_t)(key[q] >> 54), 1);
     }
     if (!range) stat[1] = FVGB_ERANGE;
     // the bounding box, once per CTA: every update reads one address (a read per warp, 31k warps on
-    // 7.9M points, set the kernel's pace: 170 us, 102 us now)
+    // 7.9M points, set the kernel's pace: 170 us against 102), and the new voxels of the CTA's grid
 #pragma unroll
     for (int e = 0; e < 6; ++e) {
         const int32_t v = __reduce_max_sync(0xffffffffu, lim[e]);
         if ((threadIdx.x & 31) == 0) box[e][threadIdx.x >> 5] = v;
     }
+    fresh = __reduce_add_sync(0xffffffffu, fresh);
+    if ((threadIdx.x & 31) == 0) box[6][threadIdx.x >> 5] = fresh;
     __syncthreads();
     if (threadIdx.x < 6) {
         int32_t v = box[threadIdx.x][0];
 #pragma unroll
         for (int w = 1; w < 8; ++w) v = max(v, box[threadIdx.x][w]);
         if (v > *reinterpret_cast<volatile int32_t *>(stat + 3 + threadIdx.x)) atomicMax(stat + 3 + threadIdx.x, v);
-    }
-}
-
-// Pass 2: the voxel bits (a bit already set, most rows of a dense cloud, costs no atomic)
-__global__ void __launch_bounds__(256) leaf_bits_kernel(int64_t n, LeafHash h) {
-    const int64_t base = (int64_t)blockIdx.x * 256 * kHashRows + threadIdx.x;
-    int32_t id[kHashRows];
-    uint32_t bit[kHashRows];
+    } else if (threadIdx.x == 32) {
+        int32_t v = 0;
 #pragma unroll
-    for (int q = 0; q < kHashRows; ++q) {
-        const int64_t i = base + q * 256;
-        id[q] = i < n ? h.slot_id[h.row_slot[i]] : -1;
-        bit[q] = i < n ? h.row_bit[i] : 0;
-    }
-#pragma unroll
-    for (int q = 0; q < kHashRows; ++q) {
-        if (id[q] < 0) continue;
-        uint64_t *w = h.mask + (int64_t)id[q] * 8 + (bit[q] >> 6);
-        const uint64_t m = 1ull << (bit[q] & 63);
-        if (!(__ldcg(w) & m)) atomicOr(reinterpret_cast<unsigned long long *>(w), m);
+        for (int w = 0; w < 8; ++w) v += box[6][w];
+        if (v) atomicAdd(stat + 9 + sb[0], v);
     }
 }
 
@@ -1269,11 +1311,86 @@ __global__ void leaf_counts_kernel(LeafHash h, int64_t L, const int32_t *__restr
     if (p > L) return;
     int32_t c = 0;
     if (p < L) {
-        const uint64_t *m = h.mask + (int64_t)vals[p] * 8;
+        const uint64_t *m = h.mask + (size_t)h.leaf_slot[vals[p]] * 8;
 #pragma unroll
         for (int w = 0; w < 8; ++w) c += __popcll(m[w]);
     }
     count[p] = c;  // zero past the last leaf, for the exclusive scan over L + 1
+}
+
+// Up to kTileLeaves leaves are sorted by two kernels: tiles of kSortTile leaves each in shared memory
+// (place = keys of the tile below its own), then every leaf finds by binary search the keys below its
+// own in the other tiles: a CTA takes 32 leaves next to each other in a tile, whose searches read the
+// same entries, and its eight warps share the tiles.  The second kernel also counts the leaf's voxels,
+// and one CTA scans them (leaf_scan_kernel).  Four launches against the radix sort's and scan's
+// nineteen (22k leaves: 71 us of small kernels, 27 us here).  A leaf searches every tile, so the
+// cost grows with the square: at kTileLeaves it is about the radix sort's.
+constexpr int kSortTile = 512;
+constexpr int64_t kTileLeaves = 65536;
+
+template <typename Key>
+__global__ void __launch_bounds__(kSortTile) leaf_tile_kernel(LeafHash h, int64_t L, uint64_t low, int vb,
+                                                              Key *__restrict__ keys, int32_t *__restrict__ vals,
+                                                              int32_t *__restrict__ slots, int64_t cap) {
+    __shared__ __align__(16) Key tile[kSortTile];
+    const int64_t base = (int64_t)blockIdx.x * kSortTile, i = base + threadIdx.x;
+    // the leaf hash that leaf_emit_kernel fills starts out free
+    for (int64_t j = i; j < cap; j += (int64_t)gridDim.x * kSortTile) slots[j] = -1;
+    Key mine = ~(Key)0;  // past the last leaf: never below a key
+    if (i < L) {
+        const uint64_t k = h.keys[i];
+        mine = (Key)(((k >> 54) << vb) | (k & low));
+    }
+    tile[threadIdx.x] = mine;
+    __syncthreads();
+    if (i >= L) return;
+    int32_t place = 0;
+#pragma unroll 16
+    for (int t = 0; t < kSortTile; ++t) place += tile[t] < mine ? 1 : 0;
+    keys[base + place] = mine;
+    vals[base + place] = (int32_t)i;
+}
+
+template <typename Key>
+__global__ void __launch_bounds__(256) leaf_rank_kernel(LeafHash h, int32_t L, const Key *__restrict__ keys,
+                                                        const int32_t *__restrict__ vals, int32_t *__restrict__ order,
+                                                        int32_t *__restrict__ count, int32_t *__restrict__ grid) {
+    __shared__ int32_t part[8][32], voxels[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int32_t p = min(blockIdx.x * 32 + lane, L - 1), own = p / kSortTile;
+    const Key mine = keys[p];
+    const int32_t id = vals[p];
+    voxels[warp][lane] = __popcll(h.mask[(size_t)h.leaf_slot[id] * 8 + warp]);  // a mask word per warp
+    int32_t below = 0;
+    for (int32_t t = warp; t * kSortTile < L; t += 8) {
+        const int32_t first = t * kSortTile;
+        if (t == own) {
+            below += p - first;
+            continue;
+        }
+        int32_t lo = first, hi = min(L, first + kSortTile);
+        while (lo < hi) {
+            const int32_t mid = (lo + hi) >> 1;
+            if (__ldg(keys + mid) < mine) lo = mid + 1; else hi = mid;
+        }
+        below += lo - first;
+    }
+    part[warp][lane] = below;
+    __syncthreads();
+    if (warp != 0 || blockIdx.x * 32 + lane >= L) return;
+    int32_t rank = 0, c = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) rank += part[w][lane], c += voxels[w][lane];
+    order[rank] = id;
+    count[rank] = c;
+    grid[rank] = (int32_t)(h.keys[id] >> 54);
+}
+
+__global__ void __launch_bounds__(kScanThreads) leaf_scan_kernel(int32_t L, const int32_t *__restrict__ count,
+                                                                 const int32_t *__restrict__ grid, int32_t B,
+                                                                 int32_t *__restrict__ first,
+                                                                 int64_t *__restrict__ offsets) {
+    scan_places(L, count, grid, B, first, offsets);
 }
 
 // warp per leaf in index order
@@ -1288,7 +1405,7 @@ __global__ void __launch_bounds__(256) leaf_emit_kernel(LeafHash h, int64_t L, c
     const uint64_t key = h.keys[id];
     int32_t ox, oy, oz;
     key_to_coord((key & ((1ull << 54) - 1ull)) << 9, ox, oy, oz);
-    emit_leaf(h.mask[(int64_t)id * 8 + (lane >> 2)], ox, oy, oz, (int32_t)(key >> 54), first[p], p, lane, out_ijk, leaves,
+    emit_leaf(h.mask[(size_t)h.leaf_slot[id] * 8 + (lane >> 2)], ox, oy, oz, (int32_t)(key >> 54), first[p], p, lane, out_ijk, leaves,
               slots, cap);
 }
 
@@ -1307,20 +1424,22 @@ __global__ void leaf_offsets_kernel(const FvgbLeaf *__restrict__ leaves, const i
 
 struct LeafSortWs {
     uint64_t *keys_a, *keys_b;
-    int32_t *vals_a, *vals_b, *count, *first;
+    int32_t *vals_a, *vals_b, *count, *first, *grid;
     void *cub_tmp;
     size_t cub_bytes;
 };
 
 size_t leaf_sort_layout(int64_t L, LeafSortWs *w, char *base) {
     size_t cub_bytes = 0, c = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, cub_bytes, (uint64_t *)nullptr, (uint64_t *)nullptr, (int32_t *)nullptr,
-                                    (int32_t *)nullptr, (int)L, 0, 64);
-    cub::DeviceRadixSort::SortPairs(nullptr, c, (uint32_t *)nullptr, (uint32_t *)nullptr, (int32_t *)nullptr,
-                                    (int32_t *)nullptr, (int)L, 0, 32);
-    cub_bytes = c > cub_bytes ? c : cub_bytes;
-    cub::DeviceScan::ExclusiveSum(nullptr, c, (int32_t *)nullptr, (int32_t *)nullptr, (int)L + 1);
-    cub_bytes = c > cub_bytes ? c : cub_bytes;
+    if (L > kTileLeaves) {
+        cub::DeviceRadixSort::SortPairs(nullptr, cub_bytes, (uint64_t *)nullptr, (uint64_t *)nullptr, (int32_t *)nullptr,
+                                        (int32_t *)nullptr, (int)L, 0, 64);
+        cub::DeviceRadixSort::SortPairs(nullptr, c, (uint32_t *)nullptr, (uint32_t *)nullptr, (int32_t *)nullptr,
+                                        (int32_t *)nullptr, (int)L, 0, 32);
+        cub_bytes = c > cub_bytes ? c : cub_bytes;
+        cub::DeviceScan::ExclusiveSum(nullptr, c, (int32_t *)nullptr, (int32_t *)nullptr, (int)L + 1);
+        cub_bytes = c > cub_bytes ? c : cub_bytes;
+    }
     size_t off = 0;
     auto take = [&](size_t bytes) {
         char *p = base ? base + off : nullptr;
@@ -1334,6 +1453,7 @@ size_t leaf_sort_layout(int64_t L, LeafSortWs *w, char *base) {
     s.vals_b = (int32_t *)take((size_t)L * 4);
     s.count = (int32_t *)take((size_t)(L + 1) * 4);
     s.first = (int32_t *)take((size_t)(L + 1) * 4);
+    s.grid = (int32_t *)s.keys_b;  // the tile sort leaves the second key buffer free
     s.cub_bytes = cub_bytes;
     s.cub_tmp = take(cub_bytes);
     if (w) *w = s;
@@ -1373,8 +1493,9 @@ extern "C" int fvgb_leaf_hash_insert(int32_t dtype, const void *rows, const int6
     LeafHash h;
     leaf_hash_layout(n, &h, align_ws(workspace));
     if (cudaMemsetAsync(h.table, 0xff, (size_t)h.cap * 8, s) != cudaSuccess ||
-        cudaMemsetAsync(stat, 0, 3 * 4, s) != cudaSuccess || cudaMemsetAsync(stat + 3, 0x80, 6 * 4, s) != cudaSuccess)
+        cudaMemsetAsync(h.mask, 0, (size_t)h.cap * 64, s) != cudaSuccess)
         return launch_status();
+    stat_init_kernel<<<(unsigned)ceil_div(num_grids + 9, 256), 256, 0, s>>>(stat, num_grids + 9);
     if (dtype < 0) launch_insert<int32_t, float>(rows, joffsets, num_grids, n, nullptr, nullptr, h, stat, s);
     else if (dtype == FVGB_F64) launch_insert<double, double>(rows, joffsets, num_grids, n, voxel_sizes, origins, h, stat, s);
     else if (dtype == FVGB_F16) launch_insert<__half, float>(rows, joffsets, num_grids, n, voxel_sizes, origins, h, stat, s);
@@ -1413,17 +1534,32 @@ extern "C" int fvgb_leaf_hash_finish(int64_t n, int32_t num_grids, int64_t num_l
     LeafSortWs w;
     leaf_sort_layout(num_leaves, &w, align_ws(workspace));
     const int64_t L = num_leaves;
-    if (cudaMemsetAsync(hash_slots, 0xff, sizeof(int32_t) * hash_capacity, s) != cudaSuccess) return launch_status();
-    leaf_bits_kernel<<<(unsigned)ceil_div(n, (int64_t)256 * kHashRows), 256, 0, s>>>(n, h);
     const int end_bit = order_key_end_bit(box_lo, box_hi);
     const int vb = end_bit > 9 ? end_bit - 9 : 0;
     const uint64_t low = (1ull << vb) - 1ull;
     int grid_bits = 0;
     while ((1 << grid_bits) < num_grids) ++grid_bits;
     const int bits = std::max(1, vb + grid_bits);
+    uint32_t *ka = reinterpret_cast<uint32_t *>(w.keys_a), *kb = reinterpret_cast<uint32_t *>(w.keys_b);
+    const unsigned warps = (unsigned)ceil_div(L, 8), ranks = (unsigned)ceil_div(L, 32);
+    if (L <= kTileLeaves) {
+        const unsigned tiles = (unsigned)ceil_div(L, (int64_t)kSortTile);
+        if (bits <= 32) {
+            leaf_tile_kernel<uint32_t><<<tiles, kSortTile, 0, s>>>(h, L, low, vb, ka, w.vals_a, hash_slots, hash_capacity);
+            leaf_rank_kernel<uint32_t><<<ranks, 256, 0, s>>>(h, (int32_t)L, ka, w.vals_a, w.vals_b, w.count, w.grid);
+        } else {
+            leaf_tile_kernel<uint64_t><<<tiles, kSortTile, 0, s>>>(h, L, low, vb, w.keys_a, w.vals_a, hash_slots,
+                                                                  hash_capacity);
+            leaf_rank_kernel<uint64_t><<<ranks, 256, 0, s>>>(h, (int32_t)L, w.keys_a, w.vals_a, w.vals_b, w.count, w.grid);
+        }
+        leaf_scan_kernel<<<1, kScanThreads, 0, s>>>((int32_t)L, w.count, w.grid, num_grids, w.first, out_joffsets);
+        leaf_emit_kernel<<<warps, 256, 0, s>>>(h, L, w.vals_b, w.first, out_ijk, leaves, hash_slots, hash_capacity);
+        count_launches(4);
+        return launch_status();
+    }
+    if (cudaMemsetAsync(hash_slots, 0xff, sizeof(int32_t) * hash_capacity, s) != cudaSuccess) return launch_status();
     size_t tb = w.cub_bytes;
     if (bits <= 32) {
-        uint32_t *ka = reinterpret_cast<uint32_t *>(w.keys_a), *kb = reinterpret_cast<uint32_t *>(w.keys_b);
         leaf_sort_keys_kernel<uint32_t><<<blocks_for(L), kThreads, 0, s>>>(h, L, low, vb, ka, w.vals_a);
         cub::DeviceRadixSort::SortPairs(w.cub_tmp, tb, ka, kb, w.vals_a, w.vals_b, (int)L, 0, bits, s);
     } else {
@@ -1433,11 +1569,10 @@ extern "C" int fvgb_leaf_hash_finish(int64_t n, int32_t num_grids, int64_t num_l
     leaf_counts_kernel<<<blocks_for(L + 1), kThreads, 0, s>>>(h, L, w.vals_b, w.count);
     tb = w.cub_bytes;
     cub::DeviceScan::ExclusiveSum(w.cub_tmp, tb, w.count, w.first, (int)L + 1, s);
-    leaf_emit_kernel<<<(unsigned)ceil_div(L, 8), 256, 0, s>>>(h, L, w.vals_b, w.first, out_ijk, leaves, hash_slots,
-                                                              hash_capacity);
+    leaf_emit_kernel<<<warps, 256, 0, s>>>(h, L, w.vals_b, w.first, out_ijk, leaves, hash_slots, hash_capacity);
     leaf_offsets_kernel<<<(unsigned)ceil_div(num_grids + 1, kThreads), kThreads, 0, s>>>(leaves, w.first, L, num_grids,
                                                                                          out_joffsets);
-    count_launches(5);
+    count_launches(4);
     return launch_status();
 }
 
@@ -1476,12 +1611,11 @@ extern "C" int fvgb_coarse_grid_index(const FvgbGrid *fine, const int32_t factor
     cudaStream_t s = as_stream(stream);
     CoarseHash h;
     coarse_hash_layout(nl, &h, align_ws(workspace));
-    if (cudaMemsetAsync(h.table, 0xff, (size_t)h.cap * 8, s) != cudaSuccess ||
-        cudaMemsetAsync(h.found, 0, 4, s) != cudaSuccess ||
-        cudaMemsetAsync(hash_slots, 0xff, sizeof(int32_t) * hash_capacity, s) != cudaSuccess)
+    if (cudaMemsetAsync(h.table, 0xff, (size_t)(reinterpret_cast<char *>(h.found + 1) - reinterpret_cast<char *>(h.table)),
+                        s) != cudaSuccess)
         return launch_status();
     coarse_insert_kernel<<<blocks_for(nl), kThreads, 0, s>>>(fine->leaves, nl, shv, low_mask, vb, h);
-    coarse_or_kernel<<<(unsigned)ceil_div(nl, 8), 256, 0, s>>>(fine->leaves, nl, shv, h);
+    coarse_or_kernel<<<(unsigned)ceil_div(nl, 8), 256, 0, s>>>(fine->leaves, nl, shv, h, hash_slots, hash_capacity);
     const unsigned ranks = (unsigned)ceil_div(nl, (int64_t)(kRankThreads / kRankSplit));
     if (bits <= 32) coarse_rank_kernel<uint32_t><<<ranks, kRankThreads, 0, s>>>(h);
     else coarse_rank_kernel<uint64_t><<<ranks, kRankThreads, 0, s>>>(h);

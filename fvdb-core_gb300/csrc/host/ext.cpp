@@ -189,15 +189,15 @@ GridPtr build_by_leaf_hash(int32_t dtype, const void *rows, const Tensor &joff, 
     size_t wsb = 0;
     check_status(fvgb_leaf_hash_workspace(n, &wsb), "grid build (workspace)");
     Tensor ws = workspace(wsb, dev);
-    Tensor stat = torch::empty({10}, i32);
+    Tensor stat = torch::empty({B + 9}, i32);
     check_status(fvgb_leaf_hash_insert(dtype, rows, joff.data_ptr<int64_t>(), (int32_t)B, n, vsd, ord,
                                        stat.data_ptr<int32_t>(), ws.data_ptr(), ws.numel(), s),
                  "grid build (leaves)");
-    int64_t *h = pinned_meta(dev.index(), std::max<size_t>(8, (size_t)B + 1));
-    TORCH_CHECK(cudaMemcpyAsync(h, stat.data_ptr<int32_t>(), 9 * sizeof(int32_t), cudaMemcpyDeviceToHost, cs) ==
+    int64_t *h = pinned_meta(dev.index(), (size_t)(B + 10) / 2);
+    TORCH_CHECK(cudaMemcpyAsync(h, stat.data_ptr<int32_t>(), (B + 9) * sizeof(int32_t), cudaMemcpyDeviceToHost, cs) ==
                         cudaSuccess &&
                     cudaStreamSynchronize(cs) == cudaSuccess,
-                "grid build: reading the leaf count failed");
+                "grid build: reading the counts failed");
     const int32_t *st = reinterpret_cast<const int32_t *>(h);
     if (st[2]) return nullptr;
     TORCH_CHECK_VALUE(st[1] == 0, "voxel coordinates must lie in [-2^20, 2^20) and inside their bounds");
@@ -209,7 +209,12 @@ GridPtr build_by_leaf_hash(int32_t dtype, const void *rows, const Tensor &joff, 
         g->box_hi[a] = st[6 + a];
     }
     g->cap = next_pow2(2 * g->L);
-    Tensor out_ijk = torch::empty({std::min<int64_t>(n, 512 * g->L), 3}, i32);
+    g->joffsets_host = torch::empty({B + 1}, torch::kInt64);
+    int64_t *jh = g->joffsets_host.data_ptr<int64_t>();
+    jh[0] = 0;
+    for (int64_t b = 0; b < B; ++b) jh[b + 1] = jh[b] + st[9 + b];
+    g->N = jh[B];
+    g->ijk = torch::empty({g->N, 3}, i32);
     g->joffsets = torch::empty({B + 1}, torch::dtype(torch::kInt64).device(dev));
     g->leaves = torch::empty({g->L * (int64_t)sizeof(FvgbLeaf)}, torch::dtype(torch::kUInt8).device(dev));
     g->hash = torch::empty({g->cap}, i32);
@@ -217,17 +222,10 @@ GridPtr build_by_leaf_hash(int32_t dtype, const void *rows, const Tensor &joff, 
     check_status(fvgb_leaf_hash_finish_workspace(g->L, &fb), "grid build (workspace)");
     Tensor fws = workspace(fb, dev);
     check_status(fvgb_leaf_hash_finish(n, (int32_t)B, g->L, g->box_lo, g->box_hi, ws.data_ptr(), ws.numel(),
-                                       out_ijk.data_ptr<int32_t>(), g->joffsets.data_ptr<int64_t>(),
+                                       g->ijk.data_ptr<int32_t>(), g->joffsets.data_ptr<int64_t>(),
                                        reinterpret_cast<FvgbLeaf *>(g->leaves.data_ptr<uint8_t>()),
                                        g->hash.data_ptr<int32_t>(), g->cap, fws.data_ptr(), fws.numel(), s),
                  "grid build (index)");
-    TORCH_CHECK(cudaMemcpyAsync(h, g->joffsets.data_ptr<int64_t>(), (B + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost,
-                                cs) == cudaSuccess &&
-                    cudaStreamSynchronize(cs) == cudaSuccess,
-                "grid build: reading the counts failed");
-    g->joffsets_host = torch::from_blob(h, {B + 1}, torch::kInt64).clone();
-    g->N = h[B];
-    g->ijk = out_ijk.narrow(0, 0, g->N);
     g->ready = std::make_shared<at::cuda::CUDAEvent>();
     g->ready->record(at::cuda::getCurrentCUDAStream(dev.index()));
     return g;
@@ -420,9 +418,6 @@ GridPtr build_coarse_by_leaves(const GridPtr &g, const Vec3 &f, const int32_t lo
         c10::cuda::CUDAStreamGuard sg(side);
         pb->out_ijk = torch::empty({std::max<int64_t>(g->N, 1), 3}, i32);
         pb->meta = torch::empty({B + 4}, torch::dtype(torch::kInt64).device(dev));
-        TORCH_CHECK(cudaMemsetAsync(pb->meta.data_ptr<int64_t>(), 0, (B + 4) * sizeof(int64_t), side.stream()) ==
-                        cudaSuccess,
-                    "coarse grid: clearing the counts failed");
         size_t wsb = 0;
         FvgbGrid fv = g->view();
         cudaStream_t cs = side.stream();
@@ -441,6 +436,8 @@ GridPtr build_coarse_by_leaves(const GridPtr &g, const Vec3 &f, const int32_t lo
         }
         if (!pb->leaves.defined()) {
             pb->leaf_ids = torch::empty({std::max<int64_t>(g->N, 1)}, i32);
+            TORCH_CHECK(cudaMemsetAsync(pb->meta.data_ptr<int64_t>(), 0, (B + 4) * sizeof(int64_t), cs) == cudaSuccess,
+                        "coarse grid: clearing the counts failed");
             check_status(fvgb_coarse_grid_workspace(g->L, &wsb), "coarse grid (workspace)");
             Tensor ws = workspace(wsb, dev);
             check_status(fvgb_coarse_grid_build(&fv, f.v, lo, hi, pb->out_ijk.data_ptr<int32_t>(),

@@ -121,11 +121,11 @@ int fvgb_ijk_sort_unique_in_box(const int32_t *ijk, const int64_t *joffsets, int
  * and voxel lists): the same grid as fvgb_ijk_sort_unique + fvgb_grid_leaf_scan +
  * fvgb_grid_index_build without sorting the rows.  num_grids <= 1023.
  *   insert: rows are ijk (dtype -1, int32) or points (FVGB_F32 / F64 / F16 / BF16, voxelised with
- *   voxel_sizes / origins as fvgb_points_to_ijk does).  stat (device int32 [9]): leaves, error word
- *   (FVGB_ERANGE), overflow (more than one leaf per eight rows: the caller sorts instead), then the
- *   largest -x, -y, -z, x, y, z.  The caller reads it and allocates.
+ *   voxel_sizes / origins as fvgb_points_to_ijk does).  stat (device int32 [9 + num_grids]): leaves,
+ *   error word (FVGB_ERANGE), overflow (more than one leaf per eight rows: the caller sorts instead),
+ *   the largest -x, -y, -z, x, y, z, then the voxels of each grid.  The caller reads it and allocates.
  *   finish: with the insert's workspace, the leaf count and the bounding box it reported: out_ijk
- *   (min(n, 512 num_leaves) rows), out_joffsets [num_grids + 1], the leaf table and the leaf hash
+ *   (a row per voxel), out_joffsets [num_grids + 1], the leaf table and the leaf hash
  *   (hash_capacity a power of two >= 2 num_leaves).
  * Replaces dispatchCreateNanoGridFromPoints / FromIJK (BuildGridFromPoints.cu:27-130,
  * BuildGridFromIjk.cu:26-83). */
@@ -177,7 +177,7 @@ int fvgb_coarse_grid_build(const FvgbGrid *fine, const int32_t factor[3], const 
                            int32_t *out_ijk, int64_t *meta, int32_t *leaf_ids, void *workspace, size_t workspace_bytes,
                            fvgb_stream_t stream);
 /* The same coarse grid with its index, for up to 49,152 fine leaves: ijk, meta (offsets, coarse leaves,
- * voxels; meta[num_grids + 3] is not written), leaf table [num_fine_leaves entries of room] and leaf
+ * voxels, 0), leaf table [num_fine_leaves entries of room] and leaf
  * hash (hash_capacity a power of two >= 2 num_fine_leaves).  Found through a hash table and ordered by
  * counting instead of sorting; FVGB_EINVAL where the grid is larger (fvgb_coarse_grid_build serves
  * it).  No counterpart in the reference. */

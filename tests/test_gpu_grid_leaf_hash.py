@@ -94,3 +94,25 @@ def test_out_of_range_rows_are_refused(cuda_device):
     ijk[1234, 1] = 1 << 20
     with pytest.raises(ValueError):
         fvdb.GridBatch.from_ijk(torch.from_numpy(ijk).to(cuda_device))
+
+
+@pytest.mark.parametrize("leaves", [511, 513, 65536, 65537])
+def test_leaf_counts(cuda_device, leaves):
+    """Edges of the leaf sort's tiles and its largest size (the radix sort serves more): distinct leaves
+    in three grids, one of them empty, at least nine rows per leaf."""
+    import fvdb
+
+    rng = np.random.default_rng(leaves)
+    n = max(N, 9 * leaves)
+    side = 48
+    cell = rng.permutation(side**3)[:leaves]
+    origin = 8 * np.stack([cell // side**2 - 20, cell // side % side - 7, cell % side], 1)
+    which = np.concatenate([np.arange(leaves), rng.integers(0, leaves, n - leaves)])
+    ijk = (origin[which] + rng.integers(0, 8, (n, 3))).astype(np.int32)
+    grid_of = np.sort(which % 2) * 2  # grids 0 and 2
+    ijk = ijk[np.argsort(which % 2, kind="stable")]
+    off = np.searchsorted(grid_of, np.arange(4)).astype(np.int64)
+    grid = fvdb.GridBatch.from_ijk(fvdb.JaggedTensor.from_data_and_offsets(
+        torch.from_numpy(ijk).to(cuda_device), torch.from_numpy(off).to(cuda_device)))
+    assert grid._impl.total_leaf_nodes == leaves
+    _check(grid, ijk, off)
