@@ -98,7 +98,7 @@ struct FwdArgs {
     int32_t *err;
     int32_t stages;
     int64_t n_tiles;
-    int32_t direct_store;  // 1: output rows contiguous (ldy == cout, cout % 8 == 0): one bulk store per tile
+    int32_t direct_store;  // 1: output rows contiguous (ldy == cout, cout % 8 == 0): one bulk store per staged row
     // width of the epilogue's own stores where direct_store is off: 2 = 32 bytes (cout, ldy multiples
     // of 16, y 32-byte aligned), 1 = 16 bytes (multiples of 8, y 16-byte aligned), 0 = one element
     int32_t vec_store;
@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_tc_fwd_kernel(FwdArgs a) {
                 } else {
                     // each thread stores its own row: one whole 32-byte sector per instruction.  With
                     // 2-byte stores a 256-channel tile took 32,768 partial-sector writes and the
-                    // epilogue, not the contraction, set the kernel's pace (4.3M rows, 128->256 FP8:
+                    // epilogue, not the contraction, set the kernel's pace (5.1M rows, 128->256 FP8:
                     // 12.7 ms with 2-byte stores, 4.0 ms with these)
                     uint16_t *yrow = reinterpret_cast<uint16_t *>(a.y) + yrow_i * a.ldy + c0;
                     if (a.vec_store == 2) {

@@ -796,7 +796,7 @@ std::optional<RowOrder> built_row_order(const PackPtr &p, bool transposed) {
 }
 
 // The row order for a tensor-core contraction once it is worth building: building it costs about
-// 0.19 ms for 1.08M rows x 27 (a sort and a permuted copy of the map), so the first tensor-core
+// 0.12 ms for 1.27M rows x 27 (a sort and a permuted copy of the map), so the first tensor-core
 // contraction over a map runs in index order and the order serves the second and later ones
 // (training re-uses every map for forward and data gradient).  The CUDA-core forms use the order
 // from the first call on large maps: it saves them far more than it costs (C2 layer 1 FP32:
@@ -804,10 +804,10 @@ std::optional<RowOrder> built_row_order(const PackPtr &p, bool transposed) {
 // Two kinds of map take the order at the first tensor-core contraction too:
 //   * the transposed map of a convolution whose stride covers its kernel: a row has at most one
 //     entry, an index-order tile multiplies all K offsets for it (2^3 stride 2, 256->128 BF16,
-//     1.08M rows: 1.13 ms in index order, 0.31 ms ordered plus 0.06 ms for the order);
+//     1.27M rows: 1.13 ms in index order, 0.31 ms ordered plus 0.06 ms for the order);
 //   * wide layers (row bytes times output channels of 128 x 256 and more), where a skipped offset
-//     saves more than its share of the sort: 128->256 FP8, 4.3M rows: 4.0 ms in index order, 2.7 ms
-//     ordered plus 0.6 ms for the order; 64->64 BF16 saves less than the order costs.
+//     saves more than its share of the sort: 128->256 FP8, 5.1M rows: 4.0 ms in index order, 2.6 ms
+//     ordered plus 0.42 ms for the order; 64->64 BF16 saves less than the order costs.
 // Below 2^14 rows the order's seven launches cost more than any of this.
 // A contraction that announces another over the same map (reuse) counts as reused.
 std::optional<RowOrder> pack_row_order_if_reused(PackPtr p, bool transposed, int64_t row_bytes, int64_t cout,
@@ -977,7 +977,7 @@ void check_device_errors(const torch::Device &dev) {
 // Features the tcgen05 contraction takes: BF16 or FP16 rows of whole, 16-byte aligned 16-byte pieces
 // (channels a multiple of 8) and at most 256 output channels.  Rows that do not fill their MMAs are
 // padded with zeros in shared memory, which costs far less than the CUDA cores: 24->40->40 FP16, 3^3
-// and 2^3 on 50k voxels: 297 us and 50 us of conversions to FP32 and back on the CUDA cores, 47 us
+// and 2^3 on 76k voxels: 297 us and 50 us of conversions to FP32 and back on the CUDA cores, 47 us
 // here; every other 16-bit shape keeps the CUDA-core form.
 bool use_tensor_cores(const Tensor &x, int64_t cin, int64_t cout) {
     return (x.scalar_type() == torch::kBFloat16 || x.scalar_type() == torch::kFloat16) && cin % 8 == 0 && cout <= 256 &&
@@ -1478,7 +1478,7 @@ GridPtr grid_subdivided(const GridPtr &g, const std::vector<int64_t> &f, const s
 Tensor flat2d(const Tensor &t) { return t.reshape({t.size(0), -1}).contiguous(); }
 
 // Window map of a pooling pair (fvgb_window_map) where the leaf-by-leaf map kernel serves it, which
-// takes windows of up to 32 voxels (2^3 stride 2, 0.29M coarse voxels: 17 us; larger windows are
+// takes windows of up to 32 voxels (2^3 stride 2, 0.36M coarse voxels: 18 us; larger windows are
 // cheaper looked up by the pooling kernels themselves).  Lives for one call: 4 bytes per window
 // position.
 std::optional<Tensor> window_map(const GridPtr &fine, const GridPtr &coarse, const Vec3 &w, const Vec3 &st) {
