@@ -612,10 +612,8 @@ struct PackInfo {
     std::optional<bool> gs_use_me;
     int64_t split_mask_num = 1;
     bool training_built = false;
-    // tile plans of the forward (0) / transposed (1) map per feature row size in bytes, and how
-    // often each was asked for
+    // tile plans of the forward (0) / transposed (1) map per feature row size in bytes
     std::map<std::pair<int, int32_t>, Tensor> plans;
-    std::map<std::pair<int, int32_t>, int> plan_requests;
     // contraction row order of the forward (0) / transposed (1) map: rows sorted by occupancy
     // mask (padded with -1), the map's rows in that order and the per-tile masks of that order;
     // and how often a tensor-core contraction asked for it
@@ -734,18 +732,6 @@ std::optional<Tensor> pack_tile_mask(PackPtr p, bool transposed) {
     return p->tile_mask_t;
 }
 
-// Whether a contraction may run over a tile plan (fvgb_conv_fwd_tc_planned) instead of over the
-// map directly (fvgb_conv_fwd_tc_bias).  A reused map with 4 <= K <= 32 runs over its row order
-// instead (faster still), so plans serve the small kernels (K < 4) only.  Measured on GB300 (1.08M surface voxels, 3x3x3): the
-// planned kernel is faster for rows shorter than 128 bytes (32->64 BF16: 0.31 vs 0.37 ms) and
-// slower for 128-byte rows (64->64 BF16: 0.73 vs 0.6 ms), where assembling the A operand in
-// tensor memory costs more than the gathers it saves; so plans serve short rows only.
-bool use_plan(int32_t dtype, int64_t K, int64_t cin, int64_t cout, int64_t elem) {
-    return cin * elem < 128 && fvgb_tc_plan_supported(dtype, (int32_t)K, (int32_t)cin, (int32_t)cout) == FVGB_OK;
-}
-
-std::optional<Tensor> pack_plan(PackPtr p, bool transposed, int32_t row_bytes);
-
 // Row order of a map for the contractions (fvgb_kmap_row_order): rows sorted by occupancy mask so
 // that a 128-row tile's rows share their offsets and the per-tile mask skips more of the
 // reduction (3x3x3 on the C2 sphere shells: 25.2 -> 16.9 active offsets per tile; a stride-2
@@ -821,21 +807,12 @@ std::optional<RowOrder> pack_row_order_if_reused(PackPtr p, bool transposed, int
     return pack_row_order(p, transposed);
 }
 
-// The plan of a map and row size once it is worth building: building one costs about 0.7x a
-// contraction over the map (0.26 ms for 1.08M rows x 27), and a contraction over it saves about
-// 0.2x, so the first contraction on a (map, row size) runs unplanned and the plan is built at the
-// second and reused by every later one (layers that share a kernel map, training iterations on a
-// cached map).
-std::optional<Tensor> pack_plan_if_reused(PackPtr p, bool transposed, int32_t row_bytes) {
-    const auto key = std::make_pair(transposed ? 1 : 0, row_bytes);
-    if (p->plans.count(key)) return p->plans[key];
-    if (++p->plan_requests[key] < 2) return std::nullopt;
-    return pack_plan(p, transposed, row_bytes);
-}
-
 // Tile plan (staging schedule of the planned tensor-core kernel) of the forward map
 // (transposed=false) or of the transposed map, for feature rows of row_bytes bytes; built once
-// per pack and row size.  nullopt where the planned kernel does not take the shape.
+// per pack and row size, for callers of fvgb_conv_fwd_tc_planned.  Contractions here do not use it:
+// with asynchronous gathers the direct kernel is the faster one on every shape that it takes (1.31M
+// rows, 32->64 BF16, GB300: 3 offsets 161 us against 198 and 157 for the plan; 27 offsets, 1.08M rows,
+// 264 us against 320 and 265).  nullopt where the planned kernel does not take the shape.
 std::optional<Tensor> pack_plan(PackPtr p, bool transposed, int32_t row_bytes) {
     resolve_pack(p);
     if (p->K > 32) return std::nullopt;
@@ -1103,22 +1080,9 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
         if (bias) b32 = bias->to(torch::kFloat32).contiguous();
         if (out_scale) s32 = out_scale->to(torch::kFloat32).contiguous();
         const float *sp = out_scale ? s32.data_ptr<float>() : nullptr;
-        // a map used again runs over its row order (measured faster than a tile plan: C2 layer 1,
-        // 32->64: 0.30 ms ordered, 0.32 ms planned, 0.365 ms in index order); the tile plan serves
-        // maps that have no row order (K < 4 or K > 32)
+        // a map contracted more than once runs over its row order (C2 layer 1, 32->64: 0.22 ms ordered,
+        // 0.26 ms in index order)
         const auto order = pack ? pack_row_order_if_reused(pack, map_t, cin * 2, cout, reuse) : std::nullopt;
-        std::optional<Tensor> plan;
-        if (pack && K < 4 && dt == FVGB_BF16 && use_plan(FVGB_BF16, K, cin, cout, 2))
-            plan = pack_plan_if_reused(pack, map_t, (int32_t)(cin * 2));
-        if (plan) {
-            check_status(fvgb_conv_fwd_tc_planned(FVGB_BF16, x.data_ptr(), x.size(0), (int32_t)cin, x.stride(0),
-                                                  plan->data_ptr(), n_out, (int32_t)K, packed.data_ptr(),
-                                                  (int32_t)cout, y.data_ptr(), y.stride(0), sp,
-                                                  bias ? b32.data_ptr<float>() : nullptr, relu ? 1 : 0,
-                                                  device_error_flag(x.device()).data_ptr<int32_t>(), s),
-                         "sparse conv forward (tensor cores)");
-            return y;
-        }
         const Tensor &m_used = order ? order->map : map;
         // the index order's tile masks are made only where no row order stands in for them
         const std::optional<Tensor> mask = order ? std::optional<Tensor>(order->mask) : pack ? pack_tile_mask(pack, map_t)
@@ -1387,16 +1351,6 @@ std::vector<Tensor> conv_forward_fp8(const Tensor &x, const Tensor &weights, Pac
     const Tensor &map = transposed ? pack_kmap_t(p) : pack_kmap(p);
     Tensor sw = s_w.contiguous();
     const auto order = pack_row_order_if_reused(p, transposed, cin, cout, false);
-    std::optional<Tensor> plan;
-    if (K < 4 && use_plan(FVGB_E4M3, K, cin, cout, 1)) plan = pack_plan_if_reused(p, transposed, (int32_t)cin);
-    if (plan) {
-        check_status(fvgb_conv_fwd_tc_planned(FVGB_E4M3, x8.data_ptr(), x8.size(0), (int32_t)cin, cin, plan->data_ptr(),
-                                              n_rows, (int32_t)K, packed.data_ptr(), (int32_t)cout, y.data_ptr(),
-                                              y.stride(0), sw.data_ptr<float>(), bp, relu ? 1 : 0,
-                                              device_error_flag(x.device()).data_ptr<int32_t>(), s),
-                     "sparse conv forward (fp8 tensor cores)");
-        return {y, s_x, s_w};
-    }
     const std::optional<Tensor> tmo = order ? std::optional<Tensor>(order->mask) : pack_tile_mask(p, transposed);
     check_status(fvgb_conv_fwd_tc_rows(FVGB_E4M3, x8.data_ptr(), x8.size(0), (int32_t)cin, cin,
                                        (order ? order->map : map).data_ptr<int32_t>(), n_rows, (int32_t)K,
