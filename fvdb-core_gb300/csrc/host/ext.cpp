@@ -120,10 +120,16 @@ struct GridImpl {
         Tensor meta_host;             // pinned int64 [B + 4]
         Tensor out_ijk, leaf_ids, meta;
         Tensor leaves, hash;          // an indexed build (fvgb_coarse_grid_index): room for the fine leaves
-        // the counts' copy into meta_host must land before the pinned block can be reused
+        // The build reads the fine grid's leaf table on the build stream, which the allocator knows
+        // nothing of: the fine grid stays until the counts, and so the build, are done.
+        std::shared_ptr<GridImpl> fine;
+        c10::cuda::CUDAStream build, caller;  // the build's stream and that of the call that asked for it
+        PendingBuild(c10::cuda::CUDAStream build, c10::cuda::CUDAStream caller) : build(build), caller(caller) {}
+        // nothing of the build runs any more when its buffers, the pinned block and the fine grid go
         ~PendingBuild() {
             try {
-                counted.synchronize();
+                if (counted.isCreated()) counted.synchronize();
+                else build.synchronize();
             } catch (...) {
             }
         }
@@ -403,7 +409,8 @@ GridPtr build_coarse_by_leaves(const GridPtr &g, const Vec3 &f, const int32_t lo
     // The build runs on the library's build stream once the fine grid is complete (its ready
     // event), so it does not wait for work queued on the caller's stream (e.g. the previous
     // step's convolutions); the host reads its counts only when the coarse grid is first used.
-    // Buffers are allocated for the build stream and handed to the using stream by resolve().
+    // Buffers are allocated for the build stream; resolve() hands them to the caller's stream and to
+    // the one that first uses the grid.
     auto main = at::cuda::getCurrentCUDAStream(dev.index());
     auto side = build_stream(dev.index());
     if (g->ready) g->ready->block(side);
@@ -412,7 +419,8 @@ GridPtr build_coarse_by_leaves(const GridPtr &g, const Vec3 &f, const int32_t lo
         e.record(main);
         e.block(side);
     }
-    auto pb = std::make_unique<GridImpl::PendingBuild>();
+    auto pb = std::make_unique<GridImpl::PendingBuild>(side, main);
+    pb->fine = g;
     pb->meta_host = torch::empty({B + 4}, torch::dtype(torch::kInt64).pinned_memory(true));
     {
         c10::cuda::CUDAStreamGuard sg(side);
@@ -475,9 +483,14 @@ void GridImpl::resolve() const {
     self->ijk = P.out_ijk.narrow(0, 0, self->N);
     auto main = at::cuda::getCurrentCUDAStream(dev.index());
     P.counted.block(main);  // what uses the grid follows its build on the device
-    // the buffers, allocated for the build stream, live on in the stream that uses the grid
+    // the buffers, allocated for the build stream, live on in the stream that asked for the grid and in
+    // the one that uses it first
+    const auto caller = P.caller;
     for (const Tensor &t : {P.out_ijk, P.meta, P.leaves, P.hash, P.leaf_ids})
-        if (t.defined()) t.record_stream(main);
+        if (t.defined()) {
+            t.record_stream(main);
+            if (caller != main) t.record_stream(caller);
+        }
     if (P.leaves.defined()) {
         self->cap = P.hash.size(0);
         self->leaves = P.leaves.narrow(0, 0, self->L * (int64_t)sizeof(FvgbLeaf));
@@ -490,9 +503,14 @@ void GridImpl::resolve() const {
         self->hash = torch::empty({self->cap}, i32);
         FvgbGrid v = self->view_unchecked();
         check_status(fvgb_grid_index_build(&v, P.leaf_ids.data_ptr<int32_t>(), main.stream()), "coarse grid (index)");
+        if (caller != main) {
+            self->leaves.record_stream(caller);
+            self->hash.record_stream(caller);
+        }
     }
     self->ready = std::make_shared<at::cuda::CUDAEvent>();
     self->ready->record(main);
+    if (caller != main && !P.leaves.defined()) self->ready->synchronize();  // the caller's stream may come next
     self->pending.reset();
     self->is_pending.store(false, std::memory_order_release);
 }
