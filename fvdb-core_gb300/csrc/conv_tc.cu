@@ -309,6 +309,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv_tc_wgrad_kernel(const __gr
     const int64_t all_tiles = (a.n_out + kTileM - 1) / kTileM;
     const int64_t n_tiles = (all_tiles - blockIdx.y + gridDim.y - 1) / gridDim.y;
     auto tile_of = [&](int64_t t) { return (int64_t)blockIdx.y + t * gridDim.y; };
+    const bool release = ROWS || a.stage_map;  // the gather warps read the tile buffers and release them
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) {
@@ -320,7 +321,10 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv_tc_wgrad_kernel(const __gr
             // with dy, or (ROWS) with the row numbers on mfull
             mbar_init(&tfull[b], ROWS ? kWgGatherWarps * 32 : 1);
             mbar_init(&mfull[b], 1);
-            mbar_init(&tempty[b], 1 + kWgGatherWarps);  // the tile's last MMA commit + each gather warp
+            // the tile's last MMA commit + each gather warp where the gather warps read the buffers too.
+            // Without map rows or row numbers in them (K > 32) they run ahead of the loader, and an
+            // arrival of theirs would count for a tile that the MMAs have yet to read.
+            mbar_init(&tempty[b], 1 + (release ? kWgGatherWarps : 0));
         }
         mbar_init(accum, 1);
         *abort = 0;
@@ -429,7 +433,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv_tc_wgrad_kernel(const __gr
             }
             // the tile's map rows were read into registers: release its buffers (with the MMA)
             __syncwarp();
-            if (lane == 0) mbar_arrive(&tempty[b]);
+            if (release && lane == 0) mbar_arrive(&tempty[b]);
             ++i;
         }
         cp_async_wait_all();
