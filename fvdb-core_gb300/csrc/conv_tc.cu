@@ -660,6 +660,11 @@ int conv_wgrad(bool f16, const void *x, int64_t n_x, int32_t c_in, int64_t ldx, 
                 record_message("cuTensorMapEncodeTiled is not available from the CUDA driver");
                 return FVGB_ECUDA;
             }
+            // A host thread that has made no runtime call yet (the backward thread, where the weight
+            // gradient alone is asked for and its buffers come from the caching allocator) has no
+            // current context, and the driver's encoder answers that with an error.
+            int dev = 0;
+            if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return launch_status();
             const cuuint64_t gdim[2] = {(cuuint64_t)c_out, (cuuint64_t)n_out};
             const cuuint64_t gstride[1] = {(cuuint64_t)lddy * 2};
             const cuuint32_t box[2] = {64, (cuuint32_t)kTileM};
