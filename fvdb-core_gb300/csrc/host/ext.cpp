@@ -1012,7 +1012,10 @@ std::mutex g_derived_mu;
 std::list<DerivedEntry> g_derived;  // most recently used first
 constexpr size_t kDerivedMax = 64;
 
+// Tensors made in inference mode have no version counter to tell their changes by: nothing derived
+// from one is kept.
 std::optional<Tensor> derived_get(const Tensor &src, int tag) {
+    if (src.is_inference()) return std::nullopt;
     const DerivedKey k = derived_key(src, tag);
     std::lock_guard<std::mutex> lock(g_derived_mu);
     for (auto it = g_derived.begin(); it != g_derived.end();) {
@@ -1031,6 +1034,7 @@ std::optional<Tensor> derived_get(const Tensor &src, int tag) {
 }
 
 void derived_put(const Tensor &src, int tag, const Tensor &value) {
+    if (src.is_inference()) return;
     DerivedEntry e{derived_key(src, tag), c10::weak_intrusive_ptr<c10::StorageImpl>(src.storage().getWeakStorageImpl()),
                    value};
     std::lock_guard<std::mutex> lock(g_derived_mu);
@@ -1040,6 +1044,19 @@ void derived_put(const Tensor &src, int tag, const Tensor &value) {
     });
     g_derived.push_front(std::move(e));
     while (g_derived.size() > kDerivedMax) g_derived.pop_back();
+}
+
+// The [K, Cin, Cout] weights of a 5-D weight tensor (see derived_get).  The cached copy serves every
+// later call, also one that saves it for a backward pass: it is an ordinary tensor whatever mode the
+// first call ran in.
+Tensor kio_weights(const Tensor &weights, bool transposed, int64_t cin, int64_t cout) {
+    if (auto c = derived_get(weights, transposed)) return *c;
+    c10::InferenceMode ordinary(false);
+    torch::NoGradGuard no_grad;
+    Tensor w = (transposed ? weights.permute({4, 3, 2, 0, 1}) : weights.permute({4, 3, 2, 1, 0})).reshape({-1, cin, cout});
+    // a copy is worth keeping; a view is free to make again (and must not pin the weights)
+    if (!w.is_alias_of(weights)) derived_put(weights, transposed, w);
+    return w;
 }
 
 // A stride-1 map of a grid onto itself with odd kernel extents: offset k has its mirror image at
@@ -1233,33 +1250,18 @@ std::vector<Tensor> conv_forward(const Tensor &x, const Tensor &weights, PackPtr
     TORCH_CHECK_VALUE(K0 == p->ks.v[0] && K1 == p->ks.v[1] && K2 == p->ks.v[2],
                       "kernel spatial shape must match the kernel map's kernel_size");
     int64_t cin, cout;
-    Tensor Wkio;
     if (!transposed) {
         TORCH_CHECK_VALUE(x.size(0) == n_src, "The number of input features must match the number of voxels");
         TORCH_CHECK_VALUE(weights.size(1) == x.size(1), "Expected input channels of kernels (", weights.size(1),
                           ") to equal input channels of features: ", x.size(1));
         cout = weights.size(0);
         cin = weights.size(1);
-        if (auto c = derived_get(weights, 0)) {
-            Wkio = *c;
-        } else {
-            Wkio = weights.permute({4, 3, 2, 1, 0}).reshape({-1, cin, cout});
-            // a copy is worth keeping; a view is free to make again (and must not pin the weights)
-            if (!Wkio.is_alias_of(weights)) derived_put(weights, 0, Wkio);
-        }
     } else {
         TORCH_CHECK_VALUE(x.size(0) == n_tgt, "The number of input features must match the number of voxels");
         TORCH_CHECK_VALUE(weights.size(0) == x.size(1), "Expected input channels of kernels (", weights.size(0),
                           ") to equal input channels of features: ", x.size(1));
         cin = weights.size(0);
         cout = weights.size(1);
-        if (auto c = derived_get(weights, 1)) {
-            Wkio = *c;
-        } else {
-            Wkio = weights.permute({4, 3, 2, 0, 1}).reshape({-1, cin, cout});
-            // a copy is worth keeping; a view is free to make again (and must not pin the weights)
-            if (!Wkio.is_alias_of(weights)) derived_put(weights, 1, Wkio);
-        }
     }
     if (bias) {
         TORCH_CHECK_VALUE(bias->dim() == 1 && bias->size(0) == cout, "bias must have shape (", cout, ",)");
@@ -1273,6 +1275,7 @@ std::vector<Tensor> conv_forward(const Tensor &x, const Tensor &weights, PackPtr
     const bool mirror = transposed && self_mirrored(p);  // the map itself stands in for its transposed one
     const bool map_t = transposed && !mirror;
     const int64_t n_out = transposed ? n_src : n_tgt;
+    const Tensor Wkio = kio_weights(weights, transposed, cin, cout);
     if (n_out == 0) return {torch::empty({0, cout}, x.options()), Wkio};
     Tensor y = gather_gemm(x, map_t ? pack_kmap_t(p) : pack_kmap(p), n_out, Wkio, false, bias,
                            p, map_t, relu, out_scale, mirror, has_backward && self_mirrored(p));
