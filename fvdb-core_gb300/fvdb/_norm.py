@@ -49,13 +49,16 @@ class GroupNormFunction(torch.autograd.Function):
         w = None if weight is None else weight.to(acc).contiguous()
         b = None if bias is None else bias.to(acc).contiguous()
         y, mean, rstd = _lib.load().group_norm_forward(x, joffsets, groups, w, b, eps)
-        ctx.save_for_backward(x, weight, bias, joffsets, mean, rstd)
-        ctx.groups, ctx.eps = groups, eps
+        ctx.save_for_backward(x, weight, bias, mean, rstd)
+        # the grid's own offsets, which carry no gradient; a grid built in inference mode has an
+        # inference tensor there, which cannot be saved
+        ctx.joffsets, ctx.groups, ctx.eps = joffsets, groups, eps
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        x, weight, bias, joffsets, mean, rstd = ctx.saved_tensors
+        x, weight, bias, mean, rstd = ctx.saved_tensors
+        joffsets = ctx.joffsets
         if torch.is_grad_enabled():  # create_graph: a gradient that can be differentiated again
             need = [t for t, n in zip((x, weight, bias), ctx.needs_input_grad) if n]
             counts = joffsets[1:] - joffsets[:-1]

@@ -83,3 +83,20 @@ def test_halo_convolution(cuda_device, dtype):
     y = grid.sparse_conv_halo(grid.jagged_like(x), w).jdata
     (dw,) = torch.autograd.grad(y, w, torch.ones_like(y))
     assert torch.equal(a, b) and torch.equal(y.detach(), b) and torch.isfinite(dw).all()
+
+
+@pytest.mark.parametrize("create_graph", [False, True])
+def test_group_norm_trains_on_a_grid_built_in_inference_mode(cuda_device, create_graph):
+    import fvdb
+    import fvdb.nn as fvnn
+
+    with torch.inference_mode():
+        grid = _grid(fvdb, cuda_device)
+        assert grid.joffsets.is_inference()
+    plain = _grid(fvdb, cuda_device)
+    net = fvnn.GroupNorm(4, 16).to(cuda_device)
+    x = torch.randn(grid.total_voxels, 16, device=cuda_device, requires_grad=True)
+    got, want = ([*torch.autograd.grad(net(fvnn.VDBTensor(g, x)).data.jdata.square().sum(),
+                                       [x, net.weight, net.bias], create_graph=create_graph)] for g in (grid, plain))
+    for a, b in zip(got, want):
+        torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-5)
