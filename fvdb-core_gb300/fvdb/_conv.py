@@ -13,7 +13,7 @@ from __future__ import annotations
 import torch
 
 from . import _lib
-from ._dispatch import plain_cuda, wants_grad
+from ._dispatch import has_memory, plain_cuda, wants_grad
 
 
 class SparseConvFunction(torch.autograd.Function):
@@ -47,7 +47,8 @@ class SparseConvFunction(torch.autograd.Function):
         # gradient = column sum of dy, accumulated in at least FP32 (FP64 stays FP64)
         y = ctx.saved_tensors[2] if ctx.relu else None
         dx = dw = db = None
-        if torch.is_grad_enabled():  # create_graph: operations that record their own gradient
+        if torch.is_grad_enabled() or not has_memory(grad_out):
+            # create_graph or batched gradients: operations that record their own gradient and batch
             if ctx.relu:
                 grad_out = grad_out * (y > 0)
             if need_db:

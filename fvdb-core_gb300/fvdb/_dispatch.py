@@ -20,3 +20,10 @@ def plain_cuda(*tensors) -> bool:
 def wants_grad(*tensors) -> bool:
     """Whether autograd would record an operation on these tensors."""
     return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
+
+
+def has_memory(t: torch.Tensor) -> bool:
+    """Whether a kernel can read the tensor: not so for the batched gradients of
+    autograd.grad(is_grads_batched=True) and of torch.func.vmap over a backward pass, which look like
+    ordinary tensors to the checks above (and reach a backward function with no transform active)."""
+    return torch._C._has_storage(t)

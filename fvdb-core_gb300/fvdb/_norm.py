@@ -6,7 +6,7 @@ from __future__ import annotations
 import torch
 
 from . import _lib
-from ._dispatch import plain_cuda
+from ._dispatch import has_memory, plain_cuda
 
 _DTYPES = (torch.float32, torch.float64, torch.bfloat16, torch.float16)
 
@@ -59,12 +59,14 @@ class GroupNormFunction(torch.autograd.Function):
     def backward(ctx, dy):
         x, weight, bias, mean, rstd = ctx.saved_tensors
         joffsets = ctx.joffsets
-        if torch.is_grad_enabled():  # create_graph: a gradient that can be differentiated again
+        create_graph = torch.is_grad_enabled()
+        if create_graph or not has_memory(dy):  # a gradient to differentiate again, or one per batch entry
             need = [t for t, n in zip((x, weight, bias), ctx.needs_input_grad) if n]
             counts = joffsets[1:] - joffsets[:-1]
             jidx = torch.repeat_interleave(torch.arange(counts.numel(), device=x.device), counts)
-            y = group_norm_composed(x, jidx, counts.numel(), ctx.groups, ctx.eps, weight, bias)
-            g = iter(torch.autograd.grad(y, need, dy, create_graph=True))
+            with torch.enable_grad():
+                y = group_norm_composed(x, jidx, counts.numel(), ctx.groups, ctx.eps, weight, bias)
+            g = iter(torch.autograd.grad(y, need, dy, create_graph=create_graph))
             return (*(next(g) if n else None for n in ctx.needs_input_grad[:3]), None, None, None)
         w = None if weight is None else weight.to(mean.dtype).contiguous()
         dx, dw, db = _lib.load().group_norm_backward(dy, x, joffsets, ctx.groups, w, mean, rstd, ctx.needs_input_grad[0])
