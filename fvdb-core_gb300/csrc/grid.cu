@@ -1110,18 +1110,21 @@ extern "C" int fvgb_coarse_grid_build(const FvgbGrid *fine, const int32_t factor
 // 7.9M points, 1.31M voxels, 22k leaves in four grids: voxelise, sort, unique and index took 1.9 ms,
 // 0.20 ms here, bound by the random reads of the table and the masks.  The table has room for
 // rows / 8 leaves at three quarters full; an input with more (fewer than eight rows per leaf) raises
-// `overflow` and is left to the sort.
+// `overflow` and is left to the sort, which takes the bounding box from here (the rows' own: it is
+// complete whatever the table's state) in place of a pass and a host read of its own.
 namespace fvgb {
 namespace {
 
 constexpr uint64_t kEmptyLeaf = ~0ull;
 constexpr int kHashRows = 4;      // rows per thread (more cost occupancy: 169 us with 8, 151 with 2, 132 with 4)
 constexpr int kHashProbes = 512;  // a full neighbourhood of the table counts as overflow
+constexpr int kTakenCounters = 64;  // CTAs count the slots they take on a line of their share of these
 constexpr int kHashMaxGrids = 1023;  // the grid index takes the key's top 10 bits (all ones: the empty slot)
 
 struct LeafHash {
     uint64_t *table;    // [cap] leaf keys, kEmptyLeaf where free
     uint64_t *mask;     // [cap][8] voxels of the slot's leaf, cleared with the pass
+    int32_t *taken;     // [kTakenCounters][32] slots taken, cleared with the masks before them
     uint64_t *keys;     // [max_leaves] key of each leaf, in insertion order
     uint32_t *leaf_slot;  // [max_leaves] its slot
     uint32_t cap;
@@ -1140,6 +1143,7 @@ size_t leaf_hash_layout(int64_t n, LeafHash *w, char *base) {
     h.cap = (uint32_t)((int64_t)h.max_leaves / 3 * 4 + 4);
     h.table = (uint64_t *)take((size_t)h.cap * 8);
     h.mask = (uint64_t *)take((size_t)h.cap * 64);
+    h.taken = (int32_t *)take((size_t)kTakenCounters * 32 * 4);
     h.keys = (uint64_t *)take((size_t)h.max_leaves * 8);
     h.leaf_slot = (uint32_t *)take((size_t)h.max_leaves * 4);
     if (w) *w = h;
@@ -1154,30 +1158,39 @@ __device__ __forceinline__ uint32_t leaf_home(const LeafHash &h, uint64_t key) {
     return __umulhi((uint32_t)(m >> 32), h.cap);
 }
 
-// The slot of a leaf, from slot s on.  stat: [0] leaves, [1] error word, [2] overflow, [3..5] largest
-// -x, -y, -z, [6..8] largest x, y, z, [9..] voxels of each grid
-__device__ __forceinline__ uint32_t insert_leaf(uint64_t *table, uint64_t *keys, uint32_t *leaf_slot, uint32_t cap,
-                                              int32_t max_leaves, uint64_t key, uint32_t s, int32_t *stat) {
-    for (int probe = 0; probe < kHashProbes; ++probe) {
-        uint64_t k = *reinterpret_cast<volatile uint64_t *>(table + s);
+// The slot of a leaf, from slot s on, or kNoSlot where the table is too full for the input.  `made`: this
+// thread took the slot.  stat: [0] leaves, [1] error word, [2] overflow, [3..5] largest -x, -y, -z, [6..8]
+// largest x, y, z, [9..] voxels of each grid.
+// An input with too many leaves fills the table in the first wave of CTAs, before any of them ends and
+// adds up its leaves, and probes of a full table are as long as they may be (1.05M scattered rows: 1.6 ms).
+// So the CTAs count slots as they take them, each on one of kTakenCounters lines; whoever brings a line
+// past its share of max_leaves, and every 1/16 of that further, adds them all up.  Lines that are all
+// below that leave the table below 80 % full.  The others look at the overflow word before each insertion
+// but the first and in long probes.
+constexpr uint32_t kNoSlot = ~0u;
+__device__ __forceinline__ uint32_t insert_leaf(const LeafHash &h, uint64_t key, uint32_t s, int32_t *stat, bool &made) {
+    for (int probe = 1; probe <= kHashProbes; ++probe) {
+        uint64_t k = *reinterpret_cast<volatile uint64_t *>(h.table + s);
         if (k == kEmptyLeaf) {
-            k = atomicCAS(reinterpret_cast<unsigned long long *>(table + s), kEmptyLeaf, key);
+            k = atomicCAS(reinterpret_cast<unsigned long long *>(h.table + s), kEmptyLeaf, key);
             if (k == kEmptyLeaf) {  // this thread's leaf
-                const int32_t id = atomicAdd(stat, 1);
-                if (id < max_leaves) {
-                    keys[id] = key;
-                    leaf_slot[id] = s;
-                } else {
-                    stat[2] = 1;
+                const int32_t share = h.max_leaves / kTakenCounters, step = (share + 15) / 16;
+                const int32_t past = atomicAdd(h.taken + (blockIdx.x % kTakenCounters) * 32, 1) - share;
+                if (past >= 0 && past % step == 0) {
+                    int32_t n = 0;
+                    for (int c = 0; c < kTakenCounters; ++c) n += *reinterpret_cast<volatile int32_t *>(h.taken + c * 32);
+                    if (n > h.max_leaves) stat[2] = 1;
                 }
+                made = true;
                 return s;
             }
         }
         if (k == key) return s;
-        s = s + 1 < cap ? s + 1 : 0;
+        s = s + 1 < h.cap ? s + 1 : 0;
+        if (probe % 16 == 0 && *reinterpret_cast<volatile int32_t *>(stat + 2)) return kNoSlot;
     }
     stat[2] = 1;
-    return s;
+    return kNoSlot;
 }
 
 __global__ void stat_init_kernel(int32_t *stat, int32_t n) {
@@ -1193,13 +1206,12 @@ __global__ void __launch_bounds__(256) leaf_insert_kernel(const P *__restrict__ 
                                                           int32_t *__restrict__ stat) {
     constexpr bool kPoints = !std::is_same<P, int32_t>::value;
     __shared__ T fac[6];
-    __shared__ int32_t sb[2], full, box[7][8];
+    __shared__ int32_t sb[2], full, first_id, made_by[8], box[7][8];
     const int64_t base = (int64_t)blockIdx.x * 256 * kHashRows;
     const int64_t last = min(n, base + 256 * kHashRows) - 1;
     if (threadIdx.x < 2) sb[threadIdx.x] = batch_of(joff, B, threadIdx.x == 0 ? base : last);
     if (threadIdx.x == 2) full = *reinterpret_cast<volatile int32_t *>(stat + 2);
     __syncthreads();
-    if (full) return;  // the input is left to the sort
     if (kPoints) {
         if (threadIdx.x < 3) {
             const double w = vs[3 * sb[0] + threadIdx.x], o = org[3 * sb[0] + threadIdx.x];
@@ -1237,39 +1249,56 @@ __global__ void __launch_bounds__(256) leaf_insert_kernel(const P *__restrict__ 
             lim[3 + a] = max(lim[3 + a], c[q][a]);
         }
     }
-    // Every step's accesses for all rows go out together: the first probe, which finds most leaves, the
-    // mask words, and the updates, whose results are looked at last (one after another each update's
-    // wait added up: 200 us for 7.9M points, 132 us).
-    uint64_t key[kHashRows], word[kHashRows];
-    uint32_t slot[kHashRows], bit[kHashRows];
-#pragma unroll
-    for (int q = 0; q < kHashRows; ++q) {
-        const int64_t i = min(base + q * 256 + threadIdx.x, last);
-        const int32_t b = sb[0] == sb[1] ? sb[0] : batch_of(joff, B, i);
-        const uint64_t k = order_key(c[q][0], c[q][1], c[q][2]);
-        bit[q] = (uint32_t)(k & 511);
-        key[q] = ((uint64_t)b << 54) | (k >> 9);
-        slot[q] = leaf_home(h, key[q]);
-        word[q] = __ldcg(h.table + slot[q]);
-    }
-#pragma unroll
-    for (int q = 0; q < kHashRows; ++q)
-        if (word[q] != key[q]) slot[q] = insert_leaf(h.table, h.keys, h.leaf_slot, h.cap, h.max_leaves, key[q], slot[q], stat);
-#pragma unroll
-    for (int q = 0; q < kHashRows; ++q)
-        word[q] = __ldcg(h.mask + (size_t)slot[q] * 8 + (bit[q] >> 6));
-#pragma unroll
-    for (int q = 0; q < kHashRows; ++q) {
-        const uint64_t m = 1ull << (bit[q] & 63);
-        if (!(word[q] & m))  // most rows of a dense cloud have nothing to set
-            word[q] = atomicOr(reinterpret_cast<unsigned long long *>(h.mask + (size_t)slot[q] * 8 + (bit[q] >> 6)), m);
-    }
     int32_t fresh = 0;  // voxels this thread set
+    uint32_t mine = 0;  // rows whose leaf this thread brought into the table
+    uint64_t key[kHashRows];
+    uint32_t slot[kHashRows];
+    if (!full) {  // else the input is left to the sort, which wants the bounding box alone
+        bool lost = false;
+        // Every step's accesses for all rows go out together: the first probe, which finds most leaves, the
+        // mask words, and the updates, whose results are looked at last (one after another each update's
+        // wait added up: 200 us for 7.9M points, 132 us).
+        uint64_t word[kHashRows];
+        uint32_t bit[kHashRows];
 #pragma unroll
-    for (int q = 0; q < kHashRows; ++q) {
-        if (word[q] >> (bit[q] & 63) & 1) continue;
-        if (sb[0] == sb[1]) ++fresh;
-        else atomicAdd(stat + 9 + (int32_t)(key[q] >> 54), 1);
+        for (int q = 0; q < kHashRows; ++q) {
+            const int64_t i = min(base + q * 256 + threadIdx.x, last);
+            const int32_t b = sb[0] == sb[1] ? sb[0] : batch_of(joff, B, i);
+            const uint64_t k = order_key(c[q][0], c[q][1], c[q][2]);
+            bit[q] = (uint32_t)(k & 511);
+            key[q] = ((uint64_t)b << 54) | (k >> 9);
+            slot[q] = leaf_home(h, key[q]);
+            word[q] = __ldcg(h.table + slot[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < kHashRows; ++q) {
+            if (word[q] == key[q] || lost) continue;
+            if (q > 0 && *reinterpret_cast<volatile int32_t *>(stat + 2)) {
+                lost = true;
+                continue;
+            }
+            bool made = false;
+            slot[q] = insert_leaf(h, key[q], slot[q], stat, made);
+            if (made) mine |= 1u << q;
+            lost = slot[q] == kNoSlot;
+        }
+#pragma unroll
+        for (int q = 0; q < kHashRows; ++q) {
+            if (lost) slot[q] = 0;  // the masks no longer matter
+            word[q] = __ldcg(h.mask + (size_t)slot[q] * 8 + (bit[q] >> 6));
+        }
+#pragma unroll
+        for (int q = 0; q < kHashRows; ++q) {
+            const uint64_t m = 1ull << (bit[q] & 63);
+            if (!(word[q] & m))  // most rows of a dense cloud have nothing to set
+                word[q] = atomicOr(reinterpret_cast<unsigned long long *>(h.mask + (size_t)slot[q] * 8 + (bit[q] >> 6)), m);
+        }
+#pragma unroll
+        for (int q = 0; q < kHashRows; ++q) {
+            if (word[q] >> (bit[q] & 63) & 1) continue;
+            if (sb[0] == sb[1]) ++fresh;
+            else atomicAdd(stat + 9 + (int32_t)(key[q] >> 54), 1);
+        }
     }
     if (!range) stat[1] = FVGB_ERANGE;
     // the bounding box, once per CTA: every update reads one address (a read per warp, 31k warps on
@@ -1281,7 +1310,39 @@ __global__ void __launch_bounds__(256) leaf_insert_kernel(const P *__restrict__ 
     }
     fresh = __reduce_add_sync(0xffffffffu, fresh);
     if ((threadIdx.x & 31) == 0) box[6][threadIdx.x >> 5] = fresh;
-    __syncthreads();
+    // leaves are numbered by the CTA: one update of the count for all of its own (one per leaf, all on one
+    // address, took 5 ns each: 0.9 ms for 175k leaves)
+    if (__syncthreads_or(mine != 0)) {
+        int32_t at = __popc(mine);
+        const int32_t own = at;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t v = __shfl_up_sync(0xffffffffu, at, o);
+            if ((threadIdx.x & 31) >= o) at += v;
+        }
+        if ((threadIdx.x & 31) == 31) made_by[threadIdx.x >> 5] = at;
+        __syncthreads();
+        int32_t before = 0, total = 0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+            if (w < (int)(threadIdx.x >> 5)) before += made_by[w];
+            total += made_by[w];
+        }
+        if (threadIdx.x == 0) first_id = atomicAdd(stat, total);
+        __syncthreads();
+        int32_t id = first_id + before + at - own;
+#pragma unroll
+        for (int q = 0; q < kHashRows; ++q) {
+            if (!(mine >> q & 1)) continue;
+            if (id < h.max_leaves) {
+                h.keys[id] = key[q];
+                h.leaf_slot[id] = slot[q];
+            } else {
+                stat[2] = 1;
+            }
+            ++id;
+        }
+    }
     if (threadIdx.x < 6) {
         int32_t v = box[threadIdx.x][0];
 #pragma unroll
@@ -1493,7 +1554,8 @@ extern "C" int fvgb_leaf_hash_insert(int32_t dtype, const void *rows, const int6
     LeafHash h;
     leaf_hash_layout(n, &h, align_ws(workspace));
     if (cudaMemsetAsync(h.table, 0xff, (size_t)h.cap * 8, s) != cudaSuccess ||
-        cudaMemsetAsync(h.mask, 0, (size_t)h.cap * 64, s) != cudaSuccess)
+        cudaMemsetAsync(h.mask, 0, (size_t)(reinterpret_cast<char *>(h.taken + kTakenCounters * 32) - reinterpret_cast<char *>(h.mask)),
+                        s) != cudaSuccess)
         return launch_status();
     stat_init_kernel<<<(unsigned)ceil_div(num_grids + 9, 256), 256, 0, s>>>(stat, num_grids + 9);
     if (dtype < 0) launch_insert<int32_t, float>(rows, joffsets, num_grids, n, nullptr, nullptr, h, stat, s);

@@ -15,6 +15,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <atomic>
 #include <list>
 #include <map>
@@ -173,10 +174,15 @@ Tensor per_grid_vec(const Tensor &t, int64_t B, const char *name) {
     return v.contiguous().clone();
 }
 
-// The grid of n rows (ijk for dtype -1, else points with device voxel_sizes / origins) through the
-// leaf hash, or null where the input has too few rows per leaf for it (the caller sorts).  From
-// kLeafHashRows rows on: below it the build is a dozen launches of a few microseconds either way and
-// the sort's single count read is the cheaper one.
+// Builds g from n rows (ijk for dtype -1, else points with device voxel sizes / origins vsd / ord) through
+// the leaf hash.  False where the input has too few rows per leaf for it: the caller sorts, inside the rows'
+// bounding box box[0..2], box[3..5]; that and g's transforms are set in any case. 
+// From kLeafHashRows rows on, where the sort reads the rows' bounding box first: the insertion measures it
+// too, so an input left to the sort pays little for the attempt (scattered rows: 0.3M 454 us before the
+// hash, 475 with it; 4.2M 1590 and 1613; six rows per leaf, 4.2M: 948 and 1029; points, whose conversion
+// got shorter: 4.2M 2226 and 1711).  Below the line the sort reads no box and the attempt is lost: 1k
+// scattered rows 263 us sorted, 317 with it; 65k 398 and 413; 0.25M 430 and 476.  Surfaces gain on both
+// sides of the line (65k rows: 385 us sorted, 158 hashed; 0.3M: 430 and 171).
 constexpr int64_t kLeafHashRows = (int64_t)1 << 18;
 constexpr int64_t kLeafHashGrids = 1023;
 
@@ -185,8 +191,8 @@ void fill_transforms(GridImpl &g, const Tensor &vs, const Tensor &org) {
     g.origins = per_grid_vec(org, g.B, "origins");
 }
 
-GridPtr build_by_leaf_hash(int32_t dtype, const void *rows, const Tensor &joff, int64_t n, const double *vsd,
-                           const double *ord) {
+bool build_by_leaf_hash(GridImpl &g, int32_t dtype, const void *rows, const Tensor &joff, int64_t n, const Tensor &vs,
+                        const Tensor &org, const double *vsd, const double *ord, int32_t box[6]) {
     auto dev = joff.device();
     const int64_t B = joff.size(0) - 1;
     auto s = cur_stream();
@@ -199,49 +205,51 @@ GridPtr build_by_leaf_hash(int32_t dtype, const void *rows, const Tensor &joff, 
     check_status(fvgb_leaf_hash_insert(dtype, rows, joff.data_ptr<int64_t>(), (int32_t)B, n, vsd, ord,
                                        stat.data_ptr<int32_t>(), ws.data_ptr(), ws.numel(), s),
                  "grid build (leaves)");
+    g.B = B;
+    fill_transforms(g, vs, org);  // while the rows are inserted
     int64_t *h = pinned_meta(dev.index(), (size_t)(B + 10) / 2);
     TORCH_CHECK(cudaMemcpyAsync(h, stat.data_ptr<int32_t>(), (B + 9) * sizeof(int32_t), cudaMemcpyDeviceToHost, cs) ==
                         cudaSuccess &&
                     cudaStreamSynchronize(cs) == cudaSuccess,
                 "grid build: reading the counts failed");
     const int32_t *st = reinterpret_cast<const int32_t *>(h);
-    if (st[2]) return nullptr;
     TORCH_CHECK_VALUE(st[1] == 0, "voxel coordinates must lie in [-2^20, 2^20) and inside their bounds");
-    auto g = std::make_shared<GridImpl>();
-    g->B = B;
-    g->L = st[0];
     for (int a = 0; a < 3; ++a) {
-        g->box_lo[a] = -st[3 + a];
-        g->box_hi[a] = st[6 + a];
+        box[a] = -st[3 + a];
+        box[3 + a] = st[6 + a];
     }
-    g->cap = next_pow2(2 * g->L);
-    g->joffsets_host = torch::empty({B + 1}, torch::kInt64);
-    int64_t *jh = g->joffsets_host.data_ptr<int64_t>();
+    if (st[2]) return false;
+    g.L = st[0];
+    std::copy(box, box + 3, g.box_lo);
+    std::copy(box + 3, box + 6, g.box_hi);
+    g.cap = next_pow2(2 * g.L);
+    g.joffsets_host = torch::empty({B + 1}, torch::kInt64);
+    int64_t *jh = g.joffsets_host.data_ptr<int64_t>();
     jh[0] = 0;
     for (int64_t b = 0; b < B; ++b) jh[b + 1] = jh[b] + st[9 + b];
-    g->N = jh[B];
-    g->ijk = torch::empty({g->N, 3}, i32);
-    g->joffsets = torch::empty({B + 1}, torch::dtype(torch::kInt64).device(dev));
-    g->leaves = torch::empty({g->L * (int64_t)sizeof(FvgbLeaf)}, torch::dtype(torch::kUInt8).device(dev));
-    g->hash = torch::empty({g->cap}, i32);
+    g.N = jh[B];
+    g.ijk = torch::empty({g.N, 3}, i32);
+    g.joffsets = torch::empty({B + 1}, torch::dtype(torch::kInt64).device(dev));
+    g.leaves = torch::empty({g.L * (int64_t)sizeof(FvgbLeaf)}, torch::dtype(torch::kUInt8).device(dev));
+    g.hash = torch::empty({g.cap}, i32);
     size_t fb = 0;
-    check_status(fvgb_leaf_hash_finish_workspace(g->L, &fb), "grid build (workspace)");
+    check_status(fvgb_leaf_hash_finish_workspace(g.L, &fb), "grid build (workspace)");
     Tensor fws = workspace(fb, dev);
-    check_status(fvgb_leaf_hash_finish(n, (int32_t)B, g->L, g->box_lo, g->box_hi, ws.data_ptr(), ws.numel(),
-                                       g->ijk.data_ptr<int32_t>(), g->joffsets.data_ptr<int64_t>(),
-                                       reinterpret_cast<FvgbLeaf *>(g->leaves.data_ptr<uint8_t>()),
-                                       g->hash.data_ptr<int32_t>(), g->cap, fws.data_ptr(), fws.numel(), s),
+    check_status(fvgb_leaf_hash_finish(n, (int32_t)B, g.L, g.box_lo, g.box_hi, ws.data_ptr(), ws.numel(),
+                                       g.ijk.data_ptr<int32_t>(), g.joffsets.data_ptr<int64_t>(),
+                                       reinterpret_cast<FvgbLeaf *>(g.leaves.data_ptr<uint8_t>()),
+                                       g.hash.data_ptr<int32_t>(), g.cap, fws.data_ptr(), fws.numel(), s),
                  "grid build (index)");
-    g->ready = std::make_shared<at::cuda::CUDAEvent>();
-    g->ready->record(at::cuda::getCurrentCUDAStream(dev.index()));
-    return g;
+    g.ready = std::make_shared<at::cuda::CUDAEvent>();
+    g.ready->record(at::cuda::getCurrentCUDAStream(dev.index()));
+    return true;
 }
 
 // Sorted-unique voxels in index order + leaf table + hash (one host sync for the counts and the
 // bounding box).  box_lo/box_hi (optional): bounds the caller knows for ijk, which shorten the
 // sort to the order-key bits that can differ.
 GridPtr build_grid(const Tensor &ijk_in, const Tensor &joff_in, const Tensor &vs, const Tensor &org,
-                   const int32_t *box_lo = nullptr, const int32_t *box_hi = nullptr, bool leaf_hash = true) {
+                   const int32_t *box_lo = nullptr, const int32_t *box_hi = nullptr) {
     TORCH_CHECK(ijk_in.is_cuda(), "fvdb_gb300 grids live on CUDA devices");
     c10::cuda::CUDAGuard guard(ijk_in.device());
     auto dev = ijk_in.device();
@@ -252,19 +260,20 @@ GridPtr build_grid(const Tensor &ijk_in, const Tensor &joff_in, const Tensor &vs
     const int64_t B = joff.size(0) - 1;
     TORCH_CHECK_VALUE(B >= 1, "a grid batch needs at least one grid");
     const int64_t n = ijk.size(0);
-    if (!(box_lo && box_hi) && leaf_hash && n >= kLeafHashRows && B <= kLeafHashGrids)
-        if (GridPtr h = build_by_leaf_hash(-1, ijk.data_ptr<int32_t>(), joff, n, nullptr, nullptr)) {
-            fill_transforms(*h, vs, org);
-            return h;
-        }
     auto g = std::make_shared<GridImpl>();
-    g->B = B;
-    fill_transforms(*g, vs, org);
+    int32_t box[6];
+    if (!(box_lo && box_hi) && n >= kLeafHashRows && B <= kLeafHashGrids) {
+        if (build_by_leaf_hash(*g, -1, ijk.data_ptr<int32_t>(), joff, n, vs, org, nullptr, nullptr, box)) return g;
+        box_lo = box;
+        box_hi = box + 3;
+    } else {
+        g->B = B;
+        fill_transforms(*g, vs, org);
+    }
     auto i32 = torch::dtype(torch::kInt32).device(dev);
     // Large inputs without known bounds: read their bounding box first (one small reduction and
     // one read) so the radix sort covers only the order-key bits that vary (3 of 8 passes for
     // coordinates in [0, 256)^3).  Small inputs sort the full key instead of paying the read.
-    int32_t mlo[3], mhi[3];
     if (!(box_lo && box_hi) && n >= (int64_t)1 << 18) {
         Tensor bx = torch::cat({std::get<0>(ijk.min(0)), std::get<0>(ijk.max(0))}).to(torch::kInt64);
         int64_t *hb = pinned_meta(dev.index(), 6);
@@ -274,11 +283,11 @@ GridPtr build_grid(const Tensor &ijk_in, const Tensor &joff_in, const Tensor &vs
                         cudaStreamSynchronize(cs) == cudaSuccess,
                     "grid build: reading the bounds failed");
         for (int a = 0; a < 3; ++a) {
-            mlo[a] = (int32_t)hb[a];
-            mhi[a] = (int32_t)hb[3 + a];
+            box[a] = (int32_t)hb[a];
+            box[3 + a] = (int32_t)hb[3 + a];
         }
-        box_lo = mlo;
-        box_hi = mhi;
+        box_lo = box;
+        box_hi = box + 3;
     }
     Tensor out_ijk = torch::empty({std::max<int64_t>(n, 1), 3}, i32);
     // device metadata read back in one copy: [0, B] voxel offsets, B+1 leaf count, B+2 voxel
@@ -364,18 +373,19 @@ GridPtr grid_from_points(const Tensor &points, const Tensor &joffsets, const Ten
     Tensor vsb = per_grid_vec(vs, B, "voxel_sizes"), orb = per_grid_vec(org, B, "origins");
     Tensor vsd = vsb.to(points.device()), ord = orb.to(points.device());
     const bool hashed = p.size(0) >= kLeafHashRows && B <= kLeafHashGrids;
-    if (hashed)
-        if (GridPtr g = build_by_leaf_hash(fvgb_dtype(p), p.data_ptr(), joff, p.size(0), vsd.data_ptr<double>(),
-                                           ord.data_ptr<double>())) {
-            fill_transforms(*g, vsb, orb);
+    int32_t box[6];
+    if (hashed) {
+        auto g = std::make_shared<GridImpl>();
+        if (build_by_leaf_hash(*g, fvgb_dtype(p), p.data_ptr(), joff, p.size(0), vsb, orb, vsd.data_ptr<double>(),
+                               ord.data_ptr<double>(), box))
             return g;
-        }
+    }
     Tensor ijk = torch::empty({p.size(0), 3}, torch::dtype(torch::kInt32).device(points.device()));
     check_status(fvgb_points_to_ijk(fvgb_dtype(p), p.data_ptr(), joff.data_ptr<int64_t>(), (int32_t)B, p.size(0),
                                     vsd.data_ptr<double>(), ord.data_ptr<double>(), ijk.data_ptr<int32_t>(),
                                     cur_stream()),
                  "points to ijk");
-    return build_grid(ijk, joff, vsb, orb, nullptr, nullptr, !hashed);
+    return hashed ? build_grid(ijk, joff, vsb, orb, box, box + 3) : build_grid(ijk, joff, vsb, orb);
 }
 
 // Coarse grid floor(ijk / f) of a grid, built leaf by leaf (fvgb_coarse_grid_build: one sort

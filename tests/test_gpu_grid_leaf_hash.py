@@ -116,3 +116,35 @@ def test_leaf_counts(cuda_device, leaves):
         torch.from_numpy(ijk).to(cuda_device), torch.from_numpy(off).to(cuda_device)))
     assert grid._impl.total_leaf_nodes == leaves
     _check(grid, ijk, off)
+
+
+@pytest.mark.parametrize("rows_per_leaf", [1.0, 5.0, 7.9, 8.1, 10.0])
+def test_inputs_near_and_past_the_table_size(cuda_device, rows_per_leaf):
+    """Rows in random order: the table overflows, or nearly, while every CTA is still inserting; the sort
+    that takes over works inside the bounding box that the insertion measured."""
+    import fvdb
+
+    n = N + 70001
+    leaves = int(n / rows_per_leaf)
+    rng = np.random.default_rng(leaves)
+    side = 80
+    cell = rng.permutation(side**3)[:leaves]
+    origin = 8 * np.stack([cell // side**2 - 60, cell // side % side - 33, cell % side + 11], 1)
+    which = np.concatenate([np.arange(leaves), rng.integers(0, leaves, n - leaves)])
+    ijk = (origin[rng.permutation(which)] + rng.integers(0, 8, (n, 3))).astype(np.int32)
+    off = np.array([0, n // 3, n // 3, n], dtype=np.int64)
+    grid = fvdb.GridBatch.from_ijk(fvdb.JaggedTensor.from_data_and_offsets(
+        torch.from_numpy(ijk).to(cuda_device), torch.from_numpy(off).to(cuda_device)))
+    _check(grid, ijk, off)
+    # the coarse grid's keys cover the fine grid's box
+    assert np.array_equal(grid.conv_grid(2, 2).ijk.jdata.cpu().numpy(), orc.grid_from_ijk(ijk >> 1, off)[0])
+
+
+@pytest.mark.parametrize("at", [0, -1])
+def test_out_of_range_rows_among_too_many_leaves_are_refused(cuda_device, at):
+    import fvdb
+
+    ijk = np.random.default_rng(5).integers(-(1 << 13), 1 << 13, (8 * N, 3)).astype(np.int32)
+    ijk[at, 2] = -(1 << 20) - 1
+    with pytest.raises(ValueError):
+        fvdb.GridBatch.from_ijk(torch.from_numpy(ijk).to(cuda_device))
