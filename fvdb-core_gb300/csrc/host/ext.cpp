@@ -1462,18 +1462,34 @@ GridPtr grid_subdivided(const GridPtr &g, const std::vector<int64_t> &f, const s
 
 Tensor flat2d(const Tensor &t) { return t.reshape({t.size(0), -1}).contiguous(); }
 
-// Window map of a pooling pair (fvgb_window_map) where the leaf-by-leaf map kernel serves it, which
-// takes windows of up to 32 voxels (2^3 stride 2, 0.36M coarse voxels: 18 us; larger windows are
-// cheaper looked up by the pooling kernels themselves).  Lives for one call: 4 bytes per window
-// position.
-std::optional<Tensor> window_map(const GridPtr &fine, const GridPtr &coarse, const Vec3 &w, const Vec3 &st) {
+// Window map of a pooling pair (fvgb_window_map): built leaf by leaf for windows of up to 32 voxels, 4
+// bytes per window position, for one call.  Null where the kernels look the windows up themselves:
+//   * fewer than `lookups` window positions in all, where the map's launch and allocation cost more than
+//     the lookups (see the callers);
+//   * fewer than 8 voxels per coarse leaf: the map is built by a warp per leaf (1.05M voxels, 2^3 windows,
+//     64 BF16 channels: one voxel per leaf 325 us looked up, 1424 over a map; 8 per leaf 266 and 267; 31
+//     per leaf 260 and 187);
+//   * no memory for it.
+std::optional<Tensor> window_map(const GridPtr &fine, const GridPtr &coarse, const Vec3 &w, const Vec3 &st, int64_t lookups) {
     const int64_t W = (int64_t)w.v[0] * w.v[1] * w.v[2];
     if (W > 32 || fine->N == 0 || coarse->N == 0 || fine->B != coarse->B) return std::nullopt;
-    Tensor map = torch::empty({coarse->N, W}, torch::dtype(torch::kInt32).device(fine->device()));
+    if (coarse->N * W < lookups || coarse->N < 8 * coarse->L) return std::nullopt;
+    Tensor map;
+    try {
+        map = torch::empty({coarse->N, W}, torch::dtype(torch::kInt32).device(fine->device()));
+    } catch (const c10::OutOfMemoryError &) {
+        return std::nullopt;
+    }
     FvgbGrid fv = fine->view(), cv = coarse->view();
     check_status(fvgb_window_map(&fv, &cv, w.v, st.v, map.data_ptr<int32_t>(), cur_stream()), "window map");
     return map;
 }
+
+// The line for sums and maxima over windows.  0.10M coarse voxels of surfaces, 64 BF16 channels, 2^3
+// windows (0.8M positions): 39 us looked up, 42 over a map; 3^3 at stride 2 (2.7M): 102 and 61; 0.35M, 2^3
+// (2.8M): 91 and 81.  In dense blocks lookups find their leaf in the cache: 0.26M coarse voxels, 2^3
+// (2.1M): 74 and 89; 3^3 at stride 3 (2.1M): 100 and 117; at stride 2 (7.1M): 282 and 156.
+int64_t reduce_lookups(const GridPtr &coarse) { return (int64_t)1 << (coarse->N > 256 * coarse->L ? 22 : 21); }
 constexpr int32_t kWindowSum = 2;  // mode of fvgb_pool_forward_map that sums the window rows
 
 // y [coarse N, C] = max / average pooling of x [fine N, *] (mode FVGB_POOL_MAX / FVGB_POOL_AVG)
@@ -1498,7 +1514,7 @@ Tensor pool_forward(int32_t mode, const GridPtr &fine, const GridPtr &coarse, co
     Tensor y = torch::empty({coarse->N, std::max<int64_t>(C, 1)}, x.options());
     if (C > 0 && coarse->N > 0) {
         FvgbGrid fv = fine->view(), cv = coarse->view();
-        if (auto map = window_map(fine, coarse, p, st))
+        if (auto map = window_map(fine, coarse, p, st, reduce_lookups(coarse)))
             check_status(fvgb_pool_forward_map(mode, fvgb_dtype(x), map->data_ptr<int32_t>(), coarse->N, (int32_t)map->size(1),
                                                xf.data_ptr(), C, (int32_t)C, y.data_ptr(), C, cur_stream()),
                          mode == FVGB_POOL_MAX ? "max_pool" : "avg_pool");
@@ -1524,8 +1540,14 @@ Tensor pool_backward(int32_t mode, const GridPtr &fine, const GridPtr &coarse, c
     auto s = cur_stream();
     if (C == 0 || fine->N == 0) return torch::zeros_like(x);
     if (mode == FVGB_POOL_MAX && st.v[0] >= p.v[0] && st.v[1] >= p.v[1] && st.v[2] >= p.v[2]) {
-        // windows that do not overlap: every row is written once, without a buffer to add into
-        if (auto map = window_map(fine, coarse, p, st)) {
+        // windows that do not overlap: every row is written once, without a buffer to add into; in 16
+        // bits that buffer is FP32 and converted, so the map pays from 0.8M positions on (64 BF16
+        // channels, dense 96^3, 2^3 windows: 176 us with the buffer, 114 over a map; 0.27M of surfaces the
+        // same), else from 2.1M for 2^3 (32 FP32 channels, surfaces, 2.8M: 194 and 129; dense 96^3, 0.9M:
+        // 100 and 106) and 4.2M for larger windows (4.2M 158 and 145; dense, 2.1M: 146 and 195)
+        const bool large = (int64_t)p.v[0] * p.v[1] * p.v[2] > 8;
+        const int64_t lookups = x.element_size() == 2 ? (int64_t)3 << 18 : (int64_t)1 << (large ? 22 : 21);
+        if (auto map = window_map(fine, coarse, p, st, lookups)) {
             Tensor dx = torch::zeros({fine->N, C}, x.options());
             check_status(fvgb_maxpool_backward_map(fvgb_dtype(x), map->data_ptr<int32_t>(), coarse->N,
                                                    (int32_t)map->size(1), xf.data_ptr(), C, (int32_t)C, df.data_ptr(), C,
@@ -1673,7 +1695,7 @@ Tensor upsample_backward(const GridPtr &coarse, const GridPtr &fine, const std::
     Tensor dx = torch::empty({coarse->N, std::max<int64_t>(C, 1)}, x.options());
     if (C > 0 && coarse->N > 0) {
         FvgbGrid fv = fine->view(), cv = coarse->view();
-        if (auto map = window_map(fine, coarse, f, f))
+        if (auto map = window_map(fine, coarse, f, f, reduce_lookups(coarse)))
             check_status(fvgb_pool_forward_map(kWindowSum, fvgb_dtype(x), map->data_ptr<int32_t>(), coarse->N,
                                                (int32_t)map->size(1), df.data_ptr(), C, (int32_t)C, dx.data_ptr(), C,
                                                cur_stream()),

@@ -91,10 +91,13 @@ struct Groups {
 constexpr int kGroupThreads = 256;
 constexpr int kGroupSmem = 32 * 1024;
 
-Groups groups_for(int32_t vecs, int W) {
+// lookups: the group's lanes also share one leaf-hash lookup per window entry, so a narrow row gets lanes
+// for those (0.02M voxels, one channel, 4^3 windows: 89 us a call with one lane per voxel).
+Groups groups_for(int32_t vecs, int W, bool lookups = false) {
     Groups g;
     g.gs = 0;
-    while ((1 << g.gs) < vecs && g.gs < 5) ++g.gs;
+    const int lanes = lookups && W > vecs ? W : vecs;
+    while ((1 << g.gs) < lanes && g.gs < 5) ++g.gs;
     while (g.gs < 5 && (size_t)(kGroupThreads >> g.gs) * W * 4 > kGroupSmem) ++g.gs;
     g.W = W;
     g.smem = (size_t)(kGroupThreads >> g.gs) * W * 4;
@@ -186,6 +189,39 @@ __global__ void __launch_bounds__(kGroupThreads, 4) window_reduce_kernel(FvgbGri
 #pragma unroll
         for (int e = 0; e < V; ++e) o.v[e] = SCALE ? mul_in<T>(Num<T>::from(acc[e]), avg) : Num<T>::from(acc[e]);
         st_vec<T, V>(y + c * ldy + ch, o);
+    }
+}
+
+// The same by lookups for windows of more than kGroupWindow positions: a warp per coarse voxel, a lookup
+// per lane, then a channel per lane.  The lookups set the pace here, and 32 registers let the SM hold twice
+// the warps of window_reduce_kernel (1.19M surface voxels, 3^3 windows at stride 3, 32 FP32 channels: 188
+// us with that kernel, 112 with this; 2^3 windows, 0.35M coarse: 78 with that, 145 with this).
+constexpr int kGroupWindow = 8;
+template <typename T, bool MAX, bool SCALE>
+__global__ void __launch_bounds__(kPoolWarps * 32) window_lookup_kernel(FvgbGrid fine, FvgbGrid coarse, int3 pf, int3 st,
+                                                                        const T *__restrict__ x, int64_t ldx, int32_t C,
+                                                                        T *__restrict__ y, int64_t ldy, double avg) {
+    using A = typename Num<T>::Acc;
+    __shared__ int32_t widx[kPoolWarps][kMaxWindow];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int W = pf.x * pf.y * pf.z;
+    for (int64_t c = (int64_t)blockIdx.x * kPoolWarps + warp; c < coarse.num_voxels; c += (int64_t)gridDim.x * kPoolWarps) {
+        const int32_t b = batch_of(coarse.voxel_offsets, coarse.num_grids, c);
+        const int3 base = make_int3(coarse.ijk[3 * c] * st.x, coarse.ijk[3 * c + 1] * st.y, coarse.ijk[3 * c + 2] * st.z);
+        window_indices(fine, b, base, pf, widx[warp], lane, 32);
+        for (int ch = lane; ch < C; ch += 32) {
+            A acc = MAX ? (A)(-INFINITY) : (A)0;
+            for (int w = 0; w < W; ++w) {
+                const int32_t f = widx[warp][w];
+                if (f < 0) continue;
+                const A v = Num<T>::to(x[(int64_t)f * ldx + ch]);
+                if constexpr (!MAX) acc = acc + v;
+                else if constexpr (sizeof(A) == 8) acc = fmax(v, acc);
+                else acc = fmaxf(v, acc);
+            }
+            y[c * ldy + ch] = SCALE ? mul_in<T>(Num<T>::from(acc), avg) : Num<T>::from(acc);
+        }
+        __syncwarp();
     }
 }
 
@@ -442,9 +478,22 @@ struct PoolFwd {
     static void run(int mode, const Windows &w, const void *x, int64_t ldx, int32_t C, void *y, int64_t ldy,
                     cudaStream_t s) {
         const double avg = 1.0 / (double)w.W;
+        if (!w.map && w.W > kGroupWindow) {
+            const unsigned blocks = pool_blocks(w.n_coarse);
+            if (mode == FVGB_POOL_MAX)
+                window_lookup_kernel<T, true, false><<<blocks, kPoolWarps * 32, 0, s>>>(w.fine, w.coarse, w.pf, w.st, (const T *)x,
+                                                                                     ldx, C, (T *)y, ldy, avg);
+            else if (mode == FVGB_POOL_AVG)
+                window_lookup_kernel<T, false, true><<<blocks, kPoolWarps * 32, 0, s>>>(w.fine, w.coarse, w.pf, w.st, (const T *)x,
+                                                                                     ldx, C, (T *)y, ldy, avg);
+            else
+                window_lookup_kernel<T, false, false><<<blocks, kPoolWarps * 32, 0, s>>>(w.fine, w.coarse, w.pf, w.st, (const T *)x,
+                                                                                      ldx, C, (T *)y, ldy, avg);
+            return;
+        }
         by_width<T>(whole_vectors<T>(C, {x, y}, {ldx, ldy}), [&](auto v) {
             constexpr int V = decltype(v)::value;
-            const Groups g = groups_for(C / V, w.W);
+            const Groups g = groups_for(C / V, w.W, !w.map);
             const unsigned blocks = group_blocks(w.n_coarse, g);
             if (mode == FVGB_POOL_MAX)
                 window_reduce_kernel<T, V, true, false><<<blocks, kGroupThreads, g.smem, s>>>(
@@ -487,7 +536,7 @@ struct AvgPoolBwd {
         const int W = (int)(ceil_div(pf.x, st.x) * ceil_div(pf.y, st.y) * ceil_div(pf.z, st.z));
         by_width<T>(whole_vectors<T>(C, {dy, dx}, {lddy, lddx}), [&](auto w) {
             constexpr int V = decltype(w)::value;
-            const Groups g = groups_for(C / V, W);
+            const Groups g = groups_for(C / V, W, true);
             avgpool_bwd_kernel<T, V><<<group_blocks(f.num_voxels, g), kGroupThreads, g.smem, s>>>(
                 f, c, pf, st, g, C, (const T *)dy, lddy, (T *)dx, lddx, avg);
         });
