@@ -1084,12 +1084,13 @@ bool self_mirrored(const PackPtr &p) {
 // mirror: W in reverse offset order (see self_mirrored).  reuse: the caller will contract over this
 // map again (training: the data gradient), so a large map gets its row order at once.
 // bias (optional, [cout]): added in the tensor-core epilogue, else after the contraction.
-// pack / map_t (optional): the pack info that owns `map` and whether `map` is its transposed map;
-// with them, shapes the planned kernel takes run over the pack's cached tile plan.
+// pack / map_t (optional): the pack info that owns `map` and whether `map` is its transposed map; its row
+// order or tile masks are used with it.  keep_packed: the packed weight image is kept for later calls with
+// the same weights.
 Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tensor &Wkio, bool transpose_w,
                    const std::optional<Tensor> &bias = std::nullopt, PackPtr pack = nullptr, bool map_t = false,
                    bool relu = false, const std::optional<Tensor> &out_scale = std::nullopt, bool mirror = false,
-                   bool reuse = false) {
+                   bool reuse = false, bool keep_packed = true) {
     c10::cuda::CUDAGuard guard(x.device());
     const int64_t K = map.size(1);
     const int64_t cin = transpose_w ? Wkio.size(2) : Wkio.size(1);
@@ -1107,7 +1108,8 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
     auto s = cur_stream();
     if (use_tensor_cores(x, cin, cout)) {
         const int tag = (transpose_w ? 3 : 2) + (mirror ? 2 : 0);
-        const bool same_type = Wkio.scalar_type() == x.scalar_type();  // the cached images are of the weights' own type
+        // the cached images are of the weights' own type
+        const bool same_type = keep_packed && Wkio.scalar_type() == x.scalar_type();
         std::optional<Tensor> cached = same_type ? derived_get(Wkio, tag) : std::nullopt;
         Tensor packed;
         if (cached && cached->device() == x.device()) {
@@ -1571,12 +1573,11 @@ Tensor pool_backward(int32_t mode, const GridPtr &fine, const GridPtr &coarse, c
     return dx.reshape(x.sizes());
 }
 
-// A kernel map of the grid onto itself for one halo call, where the tensor cores take the features
-// (or, for the weight gradient, where they are FP32): the leaf kernels below contract on CUDA cores.
-// The map lives for the call only.  Dense 96^3, 32->64 BF16 (GB300): the leaf kernel takes 2.9 ms
-// per direction and 15 ms for the weight gradient, the map 0.08 ms, a contraction over it 0.4 ms and
-// the weight gradient 0.2 ms.  Null where the map does not fit in memory (108 bytes per voxel):
-// the leaf kernels need none.
+// Halo convolutions run over a kernel map of the grid onto itself that lives for the call (108 bytes per
+// voxel), on the contraction kernels, or without a map on the leaf kernels, which contract on CUDA cores.
+// Dense 96^3, 32->64 BF16 (GB300): the leaf kernel takes 2.9 ms per direction and 15 ms for the weight
+// gradient, the map 0.08 ms, a contraction over it 0.4 ms and the weight gradient 0.2 ms.
+// Null where the map does not fit in memory.
 PackPtr halo_map(const GridPtr &g) {
     try {
         PackPtr p = make_pack({3, 3, 3}, {1, 1, 1}, g, std::nullopt);
@@ -1587,9 +1588,30 @@ PackPtr halo_map(const GridPtr &g) {
     }
 }
 
+// Which of the two a call takes; tests ask for one of them (kLeaf, kMap).
+enum HaloRoute : int64_t { kByRule = 0, kLeaf = 1, kMap = 2 };
+
+// The rule's lines.  The map's launches cost about 80 us however small the grid; the leaf kernels' time
+// grows with the channels' product, the leaves and the voxels.  A contraction alone, BF16, leaf kernel and map
+// (us, calls among others): 16->16 23k voxels in 437 leaves 67 and 83, 57k in 1114 under 80 each, 111k of
+// a dense block 81 and 76; 16->32 11k voxels 71 and 81, 23k faster over the map; 32->32 0.4k voxels 79 and
+// 113, 2.3k 84 and 86 (136 and 110 alone); 32->64 0.4k 146 and 139.  With the weight gradient: 16->16
+// 2.3k voxels 134 and 171, 5.7k 173 and 175 (234 and 186 alone); 32->32 0.4k 140 and 185, 2.3k 174 and 175;
+// 32->64 0.4k 210 and 182.  The FP32 weight gradient has its lines at the same places (16->16 2.3k 135 and 155,
+// 5.7k 174 and 151; 24->24 2.3k 173 and 157).
+bool halo_contraction_by_map(const GridPtr &g, int64_t channels) {
+    if (channels >= 2048) return true;
+    if (channels > 512) return g->N >= 2048;
+    if (channels > 256) return g->N >= 16384 || g->L >= 400;
+    return g->N >= 49152 || g->L >= 800;
+}
+bool halo_wgrad_by_map(const GridPtr &g, int64_t channels) {
+    return channels >= 2048 || g->N >= (channels > 512 ? 2048 : 4096);
+}
+
 // Stride-1 3^3 convolution over the grid: y = sum_k x[v + d_k] W[k] for W [27, Cin, Cout] (mirror:
 // the data gradient, W[26-k]^T with W in the forward's layout); `map` (optional) from halo_map.
-Tensor halo_conv_over(const GridPtr &g, const Tensor &x, const Tensor &w, bool mirror, PackPtr map) {
+Tensor halo_conv_over(const GridPtr &g, const Tensor &x, const Tensor &w, bool mirror, PackPtr map, int64_t route) {
     R(g);
     c10::cuda::CUDAGuard guard(g->device());
     TORCH_CHECK_VALUE(x.dim() == 2 && x.size(0) == g->N, "features must have shape (num_voxels, channels)");
@@ -1598,11 +1620,18 @@ Tensor halo_conv_over(const GridPtr &g, const Tensor &x, const Tensor &w, bool m
     const int64_t cin = x.size(1), cout = mirror ? w.size(1) : w.size(2);
     TORCH_CHECK_VALUE((mirror ? w.size(2) : w.size(1)) == cin, "halo weights do not match the feature channels");
     Tensor xc = x.contiguous(), wc = w.contiguous();
-    if (g->N > 0 && cin > 0 && cout > 0 && use_tensor_cores(xc, cin, cout)) {
+    if (g->N > 0 && cin > 0 && cout > 0 && use_tensor_cores(xc, cin, cout) && route != kLeaf &&
+        (map || route == kMap || halo_contraction_by_map(g, cin * cout))) {
         if (!map) map = halo_map(g);
-        if (map)
-            return gather_gemm(xc, pack_kmap(map), g->N, wc, mirror, std::nullopt, map, false,
-                               false, std::nullopt, mirror);
+        if (map) {
+            try {
+                // the weights are a tensor of this call: what is derived from them serves no other
+                return gather_gemm(xc, pack_kmap(map), g->N, wc, mirror, std::nullopt, map, false, false, std::nullopt, mirror,
+                                   false, false);
+            } catch (const c10::OutOfMemoryError &) {
+                map = nullptr;  // the leaf kernels need the output alone
+            }
+        }
     }
     Tensor y = torch::empty({g->N, cout}, x.options());
     if (g->N > 0 && cin > 0 && cout > 0) {
@@ -1616,12 +1645,17 @@ Tensor halo_conv_over(const GridPtr &g, const Tensor &x, const Tensor &w, bool m
     return y;
 }
 
-Tensor halo_conv(const GridPtr &g, const Tensor &x, const Tensor &w, bool mirror) {
-    return halo_conv_over(g, x, w, mirror, nullptr);
+Tensor halo_conv(const GridPtr &g, const Tensor &x, const Tensor &w, bool mirror, int64_t route) {
+    return halo_conv_over(g, x, w, mirror, nullptr, route);
+}
+
+// Whether the contraction's weight gradient takes these operands.
+bool halo_wgrad_takes(const Tensor &x, int64_t cin, int64_t cout) {
+    return x.scalar_type() == torch::kFloat32 || (use_tensor_cores(x, cin, cout) && cin <= 128 && cout % 8 == 0);
 }
 
 // dW [27, Cin, Cout] = sum_v x[v + d_k]^T dy[v] (fixed-order FP64 sum of per-chunk partials)
-Tensor halo_wgrad_over(const GridPtr &g, const Tensor &x, const Tensor &dy, PackPtr map) {
+Tensor halo_wgrad_over(const GridPtr &g, const Tensor &x, const Tensor &dy, PackPtr map, int64_t route) {
     R(g);
     c10::cuda::CUDAGuard guard(g->device());
     TORCH_CHECK_VALUE(x.dim() == 2 && dy.dim() == 2 && x.size(0) == g->N && dy.size(0) == g->N,
@@ -1630,10 +1664,16 @@ Tensor halo_wgrad_over(const GridPtr &g, const Tensor &x, const Tensor &dy, Pack
     const int64_t cin = x.size(1), cout = dy.size(1);
     Tensor dw = torch::empty({27, cin, cout}, x.options());
     if (cin == 0 || cout == 0) return dw;
-    const bool by_map = x.scalar_type() == torch::kFloat32 || (use_tensor_cores(xc, cin, cout) && cin <= 128 && cout % 8 == 0);
-    if (g->N > 0 && by_map) {
+    if (g->N > 0 && halo_wgrad_takes(xc, cin, cout) && route != kLeaf &&
+        (map || route == kMap || halo_wgrad_by_map(g, cin * cout))) {
         if (!map) map = halo_map(g);
-        if (map) return gather_wgrad(xc, pack_kmap(map), g->N, dc, 27, map, false);
+        if (map) {
+            try {
+                return gather_wgrad(xc, pack_kmap(map), g->N, dc, 27, map, false);
+            } catch (const c10::OutOfMemoryError &) {
+                map = nullptr;
+            }
+        }
     }
     FvgbGrid v = g->view();
     size_t wsb = 0;
@@ -1646,7 +1686,9 @@ Tensor halo_wgrad_over(const GridPtr &g, const Tensor &x, const Tensor &dy, Pack
     return dw;
 }
 
-Tensor halo_wgrad(const GridPtr &g, const Tensor &x, const Tensor &dy) { return halo_wgrad_over(g, x, dy, nullptr); }
+Tensor halo_wgrad(const GridPtr &g, const Tensor &x, const Tensor &dy, int64_t route) {
+    return halo_wgrad_over(g, x, dy, nullptr, route);
+}
 
 // (dx, dW) of one halo convolution; both gradients contract over one map
 std::vector<Tensor> halo_backward(const GridPtr &g, const Tensor &x, const Tensor &w, const Tensor &dy, bool need_dx,
@@ -1656,10 +1698,13 @@ std::vector<Tensor> halo_backward(const GridPtr &g, const Tensor &x, const Tenso
     const bool tensor_cores = x.dim() == 2 && dy.dim() == 2 && g->N > 0 && x.size(1) > 0 && dy.size(1) > 0 &&
                               use_tensor_cores(x.contiguous(), x.size(1), dy.size(1)) &&
                               use_tensor_cores(dy, dy.size(1), x.size(1));
-    PackPtr map = tensor_cores && need_dx && need_dw ? halo_map(g) : nullptr;
+    PackPtr map = tensor_cores && need_dx && need_dw && halo_wgrad_takes(x.contiguous(), x.size(1), dy.size(1)) &&
+                          halo_wgrad_by_map(g, x.size(1) * dy.size(1))
+                      ? halo_map(g)
+                      : nullptr;
     Tensor dx, dw;
-    if (need_dx) dx = halo_conv_over(g, dy, w, true, map);
-    if (need_dw) dw = halo_wgrad_over(g, x, dy, map);
+    if (need_dx) dx = halo_conv_over(g, dy, w, true, map, kByRule);
+    if (need_dw) dw = halo_wgrad_over(g, x, dy, map, kByRule);
     return {dx, dw};
 }
 
@@ -1874,8 +1919,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("check_device_errors", [](const torch::Device &d) { check_device_errors(d); },
           py::call_guard<py::gil_scoped_release>());
     m.def("conv_backward", &conv_backward, py::call_guard<py::gil_scoped_release>());
-    m.def("halo_conv", &halo_conv, py::call_guard<py::gil_scoped_release>());
-    m.def("halo_wgrad", &halo_wgrad, py::call_guard<py::gil_scoped_release>());
+    m.def("halo_conv", &halo_conv, py::arg("grid"), py::arg("features"), py::arg("weights"), py::arg("mirror"),
+          py::arg("route") = (int64_t)kByRule, py::call_guard<py::gil_scoped_release>());
+    m.def("halo_wgrad", &halo_wgrad, py::arg("grid"), py::arg("features"), py::arg("grad"),
+          py::arg("route") = (int64_t)kByRule, py::call_guard<py::gil_scoped_release>());
+    m.attr("HALO_LEAF") = (int64_t)kLeaf;
+    m.attr("HALO_MAP") = (int64_t)kMap;
     m.def("halo_backward", &halo_backward, py::call_guard<py::gil_scoped_release>());
     m.def("fold_batch_norm", &fold_batch_norm);
     m.def("fold_bias", &fold_bias);

@@ -1,9 +1,9 @@
 """Autograd Function of the leaf-halo convolution (GridBatch.sparse_conv_halo).
 
 Forward, data gradient and weight gradient run in the C++ extension (halo_conv /
-halo_wgrad): 16-bit features (and the FP32 weight gradient) over a kernel map that lives for the
-call, on the contraction kernels; the rest on the leaf kernels of csrc/halo.cu, with no map.  The
-weight layout and the backward follow the reference's autograd body
+halo_wgrad): 16-bit features (and the FP32 weight gradient) from a size on over a kernel map that lives
+for the call, on the contraction kernels; the rest, and every call that the map has no memory for, on
+the leaf kernels of csrc/halo.cu, with no map.  The weight layout and the backward follow the reference's autograd body
 (src/fvdb/detail/autograd/SparseConvolutionHalo.cpp:17-86): weights [O, I, 3, 3, 3] become
 [3, 3, 3, I, O] (offset k = 9 K2 + 3 K1 + K0, K2 on ijk axis 0); the data gradient is the same
 convolution of the output gradient with the mirrored, transposed weights; the weight gradient

@@ -166,12 +166,13 @@ class GridBatch:
         """Stride-1 3x3x3 convolution of `input` (one feature row per voxel) over this grid, with
         the reference's arguments, checks and error types (GridBatch.cpp:776-793,
         autograd/SparseConvolutionHalo.cpp:17-86).  16-bit features run over a stride-1 3^3
-        kernel map that lives for the call, on the tensor cores; FP32 and FP64 (and every type
-        where that map does not fit in memory) without a map: a CTA per leaf stages the leaf's
-        10^3 halo (through the leaf hash) in shared memory and convolves its active voxels.  x, y,
-        z offsets meet weight dims 4, 3, 2 (K2, K1, K0), the kernel map's convention, so the
-        result equals sparse_conv_3d over the grid's stride-1 3^3 map up to summation order.  `variant` picks one of the reference's halo kernels and is
-        accepted for compatibility (there is one implementation)."""
+        kernel map that lives for the call, on the tensor cores, unless the call is small; FP32 and
+        FP64 (and every type where that map does not fit in memory) without a map: a CTA per leaf
+        stages the leaf's 10^3 halo (through the leaf hash) in shared memory and convolves its
+        active voxels.  x, y, z offsets meet weight dims 4, 3, 2 (K2, K1, K0), the kernel map's
+        convention, so the result equals sparse_conv_3d over the grid's stride-1 3^3 map up to
+        summation order.  `variant` picks one of the reference's halo kernels and is accepted for
+        compatibility (there is one implementation)."""
         if not isinstance(input, JaggedTensor):
             raise TypeError("input must be a JaggedTensor")
         data = input.jdata

@@ -95,8 +95,10 @@ def test_group_norm_trains_on_a_grid_built_in_inference_mode(cuda_device, create
         assert grid.joffsets.is_inference()
     plain = _grid(fvdb, cuda_device)
     net = fvnn.GroupNorm(4, 16).to(cuda_device)
-    x = torch.randn(grid.total_voxels, 16, device=cuda_device, requires_grad=True)
-    got, want = ([*torch.autograd.grad(net(fvnn.VDBTensor(g, x)).data.jdata.square().sum(),
-                                       [x, net.weight, net.bias], create_graph=create_graph)] for g in (grid, plain))
-    for a, b in zip(got, want):
-        torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-5)
+    g = torch.Generator().manual_seed(4)
+    x = torch.randn(grid.total_voxels, 16, generator=g).to(cuda_device).requires_grad_(True)
+    dy = torch.randn(grid.total_voxels, 16, generator=g).to(cuda_device)
+    got, want = (torch.autograd.grad(net(fvnn.VDBTensor(v, x)).data.jdata, [x, net.weight, net.bias], dy,
+                                     create_graph=create_graph) for v in (grid, plain))
+    for a, b in zip(got, want):  # the composed operations' sums differ from run to run by FP32 rounding
+        assert float((a - b).norm() / b.norm()) <= 1e-4
