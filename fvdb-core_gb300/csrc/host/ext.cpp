@@ -644,7 +644,7 @@ struct PackInfo {
     std::map<std::pair<int, int32_t>, Tensor> plans;
     // contraction row order of the forward (0) / transposed (1) map: rows sorted by occupancy
     // mask (padded with -1), the map's rows in that order and the per-tile masks of that order;
-    // and how often a tensor-core contraction asked for it
+    // and how often a tensor-core contraction asked for it (1: also the mirrored forward map)
     std::optional<Tensor> order_rows[2], order_mask[2], order_map[2];
     int order_requests[2] = {0, 0};
 };
@@ -764,7 +764,7 @@ std::optional<Tensor> pack_tile_mask(PackPtr p, bool transposed) {
 // that a 128-row tile's rows share their offsets and the per-tile mask skips more of the
 // reduction (3x3x3 on the C2 sphere shells: 25.2 -> 16.9 active offsets per tile; a stride-2
 // transposed map, one valid offset of 8 per row: 8 -> ~1).  Built once per pack and direction,
-// for 4 <= K <= 32: {rows, tile masks, the map in that order}.
+// for 4 <= K <= 32 and where memory allows: {rows, tile masks, the map in that order}.
 struct RowOrder {
     Tensor rows, mask, map;
 };
@@ -777,12 +777,17 @@ std::optional<RowOrder> pack_row_order(PackPtr p, bool transposed) {
         const Tensor &m = transposed ? pack_kmap_t(p) : pack_kmap(p);
         const int64_t n = transposed ? p->src->N : p->tgt->N;
         const int64_t tiles = std::max<int64_t>((n + 127) / 128, 1);
-        Tensor rows = torch::empty({tiles * 128}, m.options());
-        Tensor tmask = torch::zeros({tiles}, m.options());
-        Tensor smap = torch::empty({tiles * 128, (int64_t)p->K}, m.options());
+        Tensor rows, tmask, smap, ws;
         size_t wsb = 0;
         check_status(fvgb_kmap_row_order_workspace(n, p->K, &wsb), "row order workspace");
-        Tensor ws = workspace(wsb, m.device());
+        try {
+            rows = torch::empty({tiles * 128}, m.options());
+            tmask = torch::zeros({tiles}, m.options());
+            smap = torch::empty({tiles * 128, (int64_t)p->K}, m.options());
+            ws = workspace(wsb, m.device());
+        } catch (const c10::OutOfMemoryError &) {
+            return std::nullopt;  // a contraction runs in index order as well
+        }
         if (!transposed && p->row_mask.defined())
             check_status(fvgb_kmap_row_order_masked(
                              m.data_ptr<int32_t>(), reinterpret_cast<const uint32_t *>(p->row_mask.data_ptr<int32_t>()), n,
@@ -809,29 +814,40 @@ std::optional<RowOrder> built_row_order(const PackPtr &p, bool transposed) {
     return RowOrder{*p->order_rows[d], *p->order_mask[d], *p->order_map[d]};
 }
 
-// The row order for a tensor-core contraction once it is worth building: building it costs about
-// 0.12 ms for 1.27M rows x 27 (a sort and a permuted copy of the map), so the first tensor-core
-// contraction over a map runs in index order and the order serves the second and later ones
-// (training re-uses every map for forward and data gradient).  The CUDA-core forms use the order
-// from the first call on large maps: it saves them far more than it costs (C2 layer 1 FP32:
-// 3.1 -> 2.0 ms).
-// Two kinds of map take the order at the first tensor-core contraction too:
-//   * the transposed map of a convolution whose stride covers its kernel: a row has at most one
-//     entry, an index-order tile multiplies all K offsets for it (2^3 stride 2, 256->128 BF16,
-//     1.27M rows: 1.13 ms in index order, 0.31 ms ordered plus 0.06 ms for the order);
-//   * wide layers (row bytes times output channels of 128 x 256 and more), where a skipped offset
-//     saves more than its share of the sort: 128->256 FP8, 5.1M rows: 4.0 ms in index order, 2.6 ms
-//     ordered plus 0.42 ms for the order; 64->64 BF16 saves less than the order costs.
-// Below 2^14 rows the order's seven launches cost more than any of this.
-// A contraction that announces another over the same map (reuse) counts as reused.
-std::optional<RowOrder> pack_row_order_if_reused(PackPtr p, bool transposed, int64_t row_bytes, int64_t cout,
-                                                 bool reuse) {
+// The row order for a tensor-core contraction once it is worth building.  Building it takes about 75 us of
+// small kernels and 85 us per million rows (x 27: a sort and a permuted copy of the map), and it saves a share
+// of every contraction, so the first contraction over a map runs in index order and the order serves the
+// second and later ones.  The data gradient of a map of a grid onto itself (mirror) is counted apart, as
+// the transposed map's is: one training step over a small map needs no order (33k voxels of a dense block,
+// 64->64 BF16: 364 us a step with it, 276 with transposed maps and none).  The CUDA-core forms use the
+// order from the first call on large maps: it saves them far more than it costs (C2 layer 1 FP32: 3.1 -> 2.0
+// ms).  Three kinds of call take it at the first tensor-core contraction too (BF16, us a call among others,
+// in index order and with the order built):
+//   * the transposed map of a convolution whose stride covers its kernel: a row has at most one entry, an
+//     index-order tile multiplies all K offsets for it.  Pays from rows of 256 bytes and n row_bytes^2 =
+//     2^34 on: 256->128, 2^3 stride 2: 0.056M rows 85 and 103, 0.11M 125 and 102, 0.88M 713 and 295;
+//     128->128: 0.11M 86 and 105, 0.26M 161 and 144, 0.53M 264 and 198; 64->64 never: 0.53M 137 and 172,
+//     0.88M 204 and 241;
+//   * wide layers (row bytes times output channels of 128 x 256 and more) over other than dense blocks,
+//     whose tiles have all offsets anyhow: rows of 256 bytes and more from 2^18 rows on (128->128: 0.23M 312
+//     and 340, 0.53M 654 and 581; dense 0.88M 1147 and 1255), shorter ones from 655k on (64->256: 0.23M
+//     194 and 255, 0.53M 393 and 410; 128->256 FP8: 0.53M 589 and 620, 5.1M 4000 and 3020);
+//   * a contraction that announces another over the same map (reuse: training), from 2^16 rows on (64->64, a
+//     training step: 0.022M 347 and 372, 0.056M 328 and 331, 0.11M 329 and 323, 0.53M 826 and 754).
+std::optional<RowOrder> pack_row_order_if_reused(PackPtr p, bool transposed, int64_t row_bytes, int64_t cout, bool reuse,
+                                                 bool mirror = false) {
     const int d = transposed ? 1 : 0;
-    const bool one_entry = transposed && p->st.v[0] >= p->ks.v[0] && p->st.v[1] >= p->ks.v[1] && p->st.v[2] >= p->ks.v[2];
-    const bool wide = row_bytes * cout >= 128 * 256;
-    const int64_t n = transposed ? p->src->N : p->tgt->N;
-    if (!p->order_rows[d] && !((one_entry || wide || reuse) && n >= ((int64_t)1 << 14)) && ++p->order_requests[d] < 2)
-        return std::nullopt;
+    if (!p->order_rows[d]) {
+        const GridPtr &rows = transposed ? p->src : p->tgt;
+        const int64_t n = rows->N;
+        const bool one_entry =
+            transposed && p->st.v[0] >= p->ks.v[0] && p->st.v[1] >= p->ks.v[1] && p->st.v[2] >= p->ks.v[2];
+        bool at_once = reuse && n >= (int64_t)1 << 16;
+        if (one_entry) at_once |= row_bytes >= 256 && (double)n * row_bytes * row_bytes >= (double)((int64_t)1 << 34);
+        else if (row_bytes * cout >= 128 * 256 && n <= 256 * rows->L)
+            at_once |= n >= (row_bytes >= 256 ? (int64_t)1 << 18 : (int64_t)5 << 17);
+        if (!at_once && ++p->order_requests[transposed || mirror ? 1 : 0] < 2) return std::nullopt;
+    }
     return pack_row_order(p, transposed);
 }
 
@@ -1129,7 +1145,7 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
         const float *sp = out_scale ? s32.data_ptr<float>() : nullptr;
         // a map contracted more than once runs over its row order (C2 layer 1, 32->64: 0.22 ms ordered,
         // 0.26 ms in index order)
-        const auto order = pack ? pack_row_order_if_reused(pack, map_t, cin * 2, cout, reuse) : std::nullopt;
+        const auto order = pack ? pack_row_order_if_reused(pack, map_t, cin * 2, cout, reuse, mirror) : std::nullopt;
         const Tensor &m_used = order ? order->map : map;
         // the index order's tile masks are made only where no row order stands in for them
         const std::optional<Tensor> mask = order ? std::optional<Tensor>(order->mask) : pack ? pack_tile_mask(pack, map_t)
@@ -1148,7 +1164,7 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
         // build); small ones only once reused, where the build's launches would dominate
         const auto order = !pack ? std::nullopt
                                  : (n_out >= (int64_t)1 << 16 ? pack_row_order(pack, map_t)
-                                                              : pack_row_order_if_reused(pack, map_t, 0, 0, reuse));
+                                                              : pack_row_order_if_reused(pack, map_t, 0, 0, reuse, mirror));
         const Tensor &m_used = order ? order->map : map;
         // W^T laid out with its output channels contiguous (a few hundred KB): the kernel reads the
         // weights in whole vectors
@@ -1882,6 +1898,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
              py::arg("kernel_size"), py::arg("stride"), py::arg("source_grid"), py::arg("target_grid") = py::none())
         .def("kmap", [](PackPtr p) { return pack_kmap(p); })
         .def("kmap_t", [](PackPtr p) { return pack_kmap_t(p); })
+        .def("has_row_order", [](PackPtr p, bool transposed) { return p->order_rows[transposed ? 1 : 0].has_value(); },
+             py::arg("transposed") = false)
         .def("tile_mask", [](PackPtr p, bool transposed) { return pack_tile_mask(p, transposed); },
              py::arg("transposed") = false)
         .def("tile_plan", [](PackPtr p, bool transposed, int32_t row_bytes) { return pack_plan(p, transposed, row_bytes); },

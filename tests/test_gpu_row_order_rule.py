@@ -1,0 +1,80 @@
+"""When a contraction takes a map's row order: at the first use of a large map that will be used again, at
+the second use of any, and never where memory does not allow it; with the same outputs bit for bit."""
+
+import pytest
+import torch
+
+from tests.helpers import dense_ijk, random_sparse_ijk
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(dev, n, cin, cout, ks=3, st=1, dense=False, transposed=False):
+    import fvdb
+
+    ijk = dense_ijk((48, 48, (n + 2303) // 2304))[:n] if dense else random_sparse_ijk(n, 96, 5)
+    grid = fvdb.GridBatch.from_ijk(torch.from_numpy(ijk).to(dev))
+    pack, tgt = grid.sparse_conv_kernel_map(ks, st)
+    g = torch.Generator().manual_seed(n)
+    rows = tgt.total_voxels if transposed else grid.total_voxels
+    x = torch.randn(rows, cin, generator=g).to(dev, torch.bfloat16)
+    shape = (cin, cout) if transposed else (cout, cin)
+    w = (torch.randn(*shape, ks, ks, ks, generator=g) * 0.05).to(dev, torch.bfloat16)
+    return grid, pack, x, w
+
+
+def _step(pack, x, w):
+    xr, wr = x.clone().requires_grad_(True), w.clone().requires_grad_(True)
+    y = pack.sparse_conv_3d(xr, wr).jdata
+    return [y.detach(), *torch.autograd.grad(y, [xr, wr], torch.ones_like(y))]
+
+
+@pytest.mark.parametrize("n", [(1 << 16) - 1, 1 << 16])
+def test_training_step(cuda_device, n):
+    grid, pack, x, w = _case(cuda_device, n, 32, 64)
+    first = _step(pack, x, w)
+    assert pack._impl.has_row_order() == (n >= 1 << 16)
+    second = _step(pack, x, w)  # the map's second forward contraction
+    assert pack._impl.has_row_order()
+    assert torch.equal(first[0], second[0]) and torch.equal(first[1], second[1])
+    assert float((first[2].float() - second[2].float()).norm() / second[2].float().norm()) <= 2**-8 + 2e-5
+
+
+@pytest.mark.parametrize("n,cin,cout,dense,at_once", [
+    ((1 << 18) - 1, 128, 128, False, False), (1 << 18, 128, 128, False, True), (1 << 18, 64, 256, False, False),
+    (1 << 18, 128, 128, True, False), (1 << 18, 128, 64, False, False)])
+def test_wide_layers(cuda_device, n, cin, cout, dense, at_once):
+    grid, pack, x, w = _case(cuda_device, n, cin, cout, dense=dense)
+    a = pack.sparse_conv_3d(x, w).jdata
+    assert pack._impl.has_row_order() == at_once
+    b = pack.sparse_conv_3d(x, w).jdata
+    assert pack._impl.has_row_order() and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("n,cin,at_once", [(65535, 256, False), (65536, 256, True), (65536, 128, False), (200000, 64, False)])
+def test_transposed_maps_of_one_entry(cuda_device, n, cin, at_once):
+    grid, pack, x, w = _case(cuda_device, n, cin, 32, ks=2, st=2, transposed=True)
+    a = pack.sparse_transpose_conv_3d(x, w).jdata
+    assert pack._impl.has_row_order(True) == at_once
+    b = pack.sparse_transpose_conv_3d(x, w).jdata
+    assert pack._impl.has_row_order(True) and torch.equal(a, b)
+
+
+def test_without_memory_for_the_order(cuda_device):
+    import fvdb
+
+    grid = fvdb.GridBatch.from_ijk(torch.from_numpy(dense_ijk((128, 128, 96))).to(cuda_device))
+    pack, _ = grid.sparse_conv_kernel_map(3, 1)
+    x = torch.randn(grid.total_voxels, 16, device=cuda_device).bfloat16()
+    w = (torch.randn(16, 16, 3, 3, 3, device=cuda_device) * 0.05).bfloat16()
+    want = pack.sparse_conv_3d(x, w).jdata
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(cuda_device).total_memory
+    try:  # the output takes 50 MB, the order 170
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (80 << 20)) / total)
+        got = pack.sparse_conv_3d(x, w).jdata
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert torch.equal(got, want) and not pack._impl.has_row_order()
+    assert torch.equal(pack.sparse_conv_3d(x, w).jdata, want) and pack._impl.has_row_order()
