@@ -700,7 +700,8 @@ Tensor build_kmap(const GridPtr &src, const GridPtr &tgt, const Vec3 &ks, const 
     }
     TORCH_CHECK(ok, "kernel map build: clearing the padding failed");
     FvgbGrid s = src->view(), t = tgt->view();
-    bool cube3 = tm && row_mask && tgt->N > 0;
+    // the row masks come from the 3^3 kernel, which suits grids of at least two voxels per leaf
+    bool cube3 = tm && row_mask && tgt->N > 0 && tgt->N >= 2 * tgt->L;
     for (int a = 0; a < 3; ++a) cube3 = cube3 && ks.v[a] == 3 && st.v[a] == 1;
     if (cube3) {
         *row_mask = torch::empty({tgt->N}, kmap.options());

@@ -326,7 +326,11 @@ __global__ void __launch_bounds__(32 * kWarpLeaves) kmap_warp_kernel(KmapParams 
 // a surface: 112 us with kmap_warp_kernel<3>, 84 us here, 76 us where the grid maps onto itself and the
 // leaf's own voxels need no walk over its mask words; a dense 96^3 block 40 us.  The rows' occupancy,
 // at hand here, is written out for the row order (a pass over the map for it: 137 us at 5.1M rows).
+// A leaf costs the same however few voxels it has, so targets with fewer than kHaloVoxels voxels per leaf
+// keep kmap_warp_kernel: 1.05M voxels in as many leaves 2393 us there, 2624 here (onto another grid 1249
+// and 1493); 2.3 per leaf 1057 and 874; 0.2M, 2.2 per leaf 206 and 153.
 constexpr int kHaloLeaves = 4;  // target leaves (warps) per CTA
+constexpr int kHaloVoxels = 2;
 struct HaloWarp {
     int32_t idx[1000];
     int32_t rows[32 * 27];
@@ -653,8 +657,8 @@ int build_map(const FvgbGrid *src, const FvgbGrid *tgt, const int32_t ksize[3], 
     auto span = [](int32_t s, int32_t st, int32_t k) { return ((7 * s + st + k - 1) >> 3) - (st >> 3) + 1; };
     const int64_t W = (int64_t)span(p.S2, p.st2, p.K2) * span(p.S1, p.st1, p.K1) * span(p.S0, p.st0, p.K0);
     p.window = W <= kMaxWindow ? (int32_t)W : 0;
-    if (!nbsizes && ld == 27 && ksize[0] == 3 && ksize[1] == 3 && ksize[2] == 3 && stride[0] == 1 && stride[1] == 1 &&
-        stride[2] == 1 && start[0] == -1 && start[1] == -1 && start[2] == -1) {
+    if ((row_mask || tgt->num_voxels >= kHaloVoxels * tgt->num_leaves) && !nbsizes && ld == 27 && ksize[0] == 3 &&
+        ksize[1] == 3 && ksize[2] == 3 && stride[0] == 1 && stride[1] == 1 && stride[2] == 1 && start[0] == -1 && start[1] == -1 && start[2] == -1) {
         constexpr int smem = kHaloLeaves * (int)sizeof(HaloWarp);
         static_assert(smem <= 48 * 1024 && sizeof(HaloWarp) % 16 == 0, "halo tables of a CTA");
         kmap_halo3_kernel<<<(unsigned)ceil_div(tgt->num_leaves, (int64_t)kHaloLeaves), 32 * kHaloLeaves, smem,

@@ -211,3 +211,32 @@ def test_coordinate_range_is_checked(fvdb, cuda_device):
     bad = torch.tensor([[0, 0, 0], [1 << 21, 0, 0]], dtype=torch.int32, device=cuda_device)
     with pytest.raises(ValueError):
         fvdb.GridBatch.from_ijk(bad)
+
+
+@pytest.mark.parametrize("voxels_over", [-1, 0])
+@pytest.mark.parametrize("same", [True, False])
+def test_maps_of_one_and_two_voxels_per_leaf(cuda_device, voxels_over, same):
+    """3^3 maps on both sides of the rule that chooses their kernel (two voxels per target leaf), over
+    scattered leaves of which every second one touches the next; FP32 contractions over them, whose row
+    order starts from row masks where the kernel makes them."""
+    import fvdb
+
+    leaves = 700
+    rng = np.random.default_rng(3)
+    cell = rng.permutation(14**3)[:leaves]
+    origin = 8 * np.stack([cell // 196 - 6, cell // 14 % 14 - 3, cell % 14], 1)
+    a = np.concatenate([origin + [0, 7, 0], origin + [7, 0, 7]])[: 2 * leaves + voxels_over].astype(np.int32)
+    grid = fvdb.GridBatch.from_ijk(torch.from_numpy(a).to(cuda_device))
+    assert grid._impl.total_leaf_nodes == leaves and grid.total_voxels == 2 * leaves + voxels_over
+    src = grid if same else fvdb.GridBatch.from_ijk(torch.from_numpy(
+        np.concatenate([origin + [1, 6, 7], origin + [7, 1, 7], origin + [0, 0, 0]]).astype(np.int32)).to(cuda_device))
+    pack, _ = src.sparse_conv_kernel_map(3, 1, None if same else grid)
+    s, t = src.ijk.jdata.cpu().numpy(), grid.ijk.jdata.cpu().numpy()
+    want = orc.kernel_map(s, np.array([0, len(s)]), t, np.array([0, len(t)]), 3, 1)
+    assert np.array_equal(pack._impl.kmap()[: len(t)].cpu().numpy(), want)
+    x = torch.randn(len(s), 8, device=cuda_device, dtype=torch.float64)
+    w = torch.randn(8, 8, 3, 3, 3, device=cuda_device, dtype=torch.float64)
+    y_ref = orc.conv_forward_f64(x.cpu().numpy(), w.cpu().numpy(), want)
+    for _ in range(2):  # the second contraction runs over the row order
+        y = pack.sparse_conv_3d(x, w).jdata.cpu().numpy()
+        assert np.linalg.norm(y - y_ref) <= 1e-12 * np.linalg.norm(y_ref)
