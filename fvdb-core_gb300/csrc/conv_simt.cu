@@ -102,19 +102,27 @@ __global__ void __launch_bounds__((FM / 8) * (FN / 4)) conv_fwd_simt_kernel(cons
         const int64_t n_here = n_out - m0 < FM ? n_out - m0 : FM;
         const int32_t words = (int32_t)n_here * K;
         uint32_t mine = 0;
-        if (ldm == K) {
-            for (int e = tid; e < FM * K; e += NT) {
-                int32_t v = e < words ? map[m0 * K + e] : -1;
-                if (v >= n_x) v = -1;
-                tile_map[e] = v;
-                if (v >= 0) mine |= 1u << (e % K);
+        // kBatch entries in flight per thread (one at a time a tile waited fourteen times for its map: 1.05M
+        // scattered rows in row order, one offset per tile, 32->33 FP32: 484 us)
+        constexpr int kBatch = 8;
+        const int step = NT % K;  // of an entry's offset from one entry of a thread to its next
+        int k = tid % K;
+        for (int e0 = tid; e0 < FM * K; e0 += kBatch * NT) {
+            int32_t v[kBatch];
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) {
+                const int e = e0 + i * NT;
+                v[i] = e >= words ? -1 : ldm == K ? __ldg(map + m0 * K + e) : __ldg(map + (m0 + e / K) * ldm + e % K);
             }
-        } else {
-            for (int e = tid; e < FM * K; e += NT) {
-                int32_t v = e < words ? map[(m0 + e / K) * ldm + e % K] : -1;
-                if (v >= n_x) v = -1;
-                tile_map[e] = v;
-                if (v >= 0) mine |= 1u << (e % K);
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) {
+                const int e = e0 + i * NT;
+                if (e < FM * K) {
+                    tile_map[e] = v[i] < n_x ? v[i] : -1;
+                    if (v[i] >= 0 && v[i] < n_x) mine |= 1u << k;
+                }
+                k += step;
+                if (k >= K) k -= K;
             }
         }
         mine = __reduce_or_sync(0xffffffffu, mine);
@@ -259,7 +267,7 @@ __global__ void __launch_bounds__((FM / 8) * (FN / 4)) conv_fwd_simt_kernel(cons
     }
 }
 
-// Short rows: few output channels, or few rows (whose maps have no row order).  A lane group of
+// Short rows: few output channels, or few rows.  A lane group of
 // cout / 4 lanes owns one output row and walks that row's present entries only -- the tiles above
 // multiply an offset for all of their rows as soon as one row has it -- with the whole weight tensor
 // in shared memory.  Sums run over offsets, then channels, as in the tiles: the same results.
@@ -332,11 +340,16 @@ int launch_fwd_simt(const void *x, int64_t n_x, int32_t cin, int64_t ldx, const 
     constexpr int VW = 16 / sizeof(T);
     const bool vec = cin % VW == 0 && ldx % VW == 0 && wsco == 1 && cout % VW == 0 && wsk % VW == 0 && wsci % VW == 0 &&
                      (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
-    // the short-row kernel: 16 channels and fewer always (a 64-wide tile would be three quarters
-    // empty); up to 32 only below 2^16 rows, where tiles have no row order
+    // The short-row kernel: 16 channels and fewer always (a 64-wide tile would be three quarters empty; 16->16,
+    // 1.2M surface voxels: 1135 us in 64-wide tiles, 706; 0.9M of a dense block 1385 and 956).  Up to 32
+    // channels where rows and channels are few: it multiplies present entries only but reads every weight for
+    // four products, so it wins by more the fewer entries rows have, and loses on dense blocks.  16->32, us
+    // among other calls, in 32-wide tiles and here: dense blocks 8k rows 33 and 35, 16k 34 and 49, 33k 43 and
+    // 86; surfaces 9k 33 and 25, 22k 39 and 46, 56k 48 and 82; random voxels at 8 % 20k 31 and 18, 59k 36 and
+    // 37.  8->32: dense 16k 33 and 29, 33k 43 and 50, surfaces 56k 47 and 46, random 59k 36 and 23.
     const int64_t wbytes = (int64_t)K * cin * cout * sizeof(T);
     if (vec && cout % 4 == 0 && K <= 32 && wbytes <= kShortSmem &&
-        (cout <= 16 || (cout <= 32 && n_out < ((int64_t)1 << 16)))) {
+        (cout <= 16 || (cout <= 32 && n_out < ((int64_t)1 << 16) && (cin <= 8 || n_out * cin <= (int64_t)7 << 15)))) {
         int gs = 0;
         while ((4 << gs) < cout) ++gs;
         if (set_dynamic_smem(conv_fwd_short_kernel<T>, kShortSmem) != cudaSuccess) return launch_status();
