@@ -344,8 +344,20 @@ def run_alone(model: ConvStack, req: Request, device) -> tuple[torch.Tensor, tor
     x = torch.zeros((grid.total_voxels, req.features.shape[1]), dtype=req.features.dtype, device=device)
     x[idx] = feats
     y = model(grid, x)
-    # through pinned memory: a copy to pageable memory goes through the driver's staging buffers
-    # piece by piece (20 MB of results: 310 us)
-    out = [torch.empty(t.shape, dtype=t.dtype, pin_memory=True).copy_(t, non_blocking=True) for t in (y, grid.ijk.jdata)]
-    torch.cuda.current_stream(y.device).synchronize()
-    return out[0], out[1]
+    return _to_host(y), _to_host(grid.ijk.jdata)
+
+
+_STAGED_BYTES = 2 << 20
+
+
+def _to_host(t: torch.Tensor) -> torch.Tensor:
+    """A copy of t in ordinary host memory, the caller's to keep (page-locked results would take a new
+    page-locked block per kept request and hold it).  Larger ones come down through page-locked memory, whose
+    block is free again after the call (0.31M rows of 32 BF16 and their coordinates, results kept: 1450 us
+    page-locked, 1670 copied straight into ordinary memory, 490 staged; dropped: 143, 150 and 354); below
+    2 MB the second copy costs more than it saves when results are dropped (0.9 MB: 32 us, 62)."""
+    if t.numel() * t.element_size() < _STAGED_BYTES:
+        return t.cpu()
+    staged = torch.empty(t.shape, dtype=t.dtype, pin_memory=True).copy_(t, non_blocking=True)
+    torch.cuda.current_stream(t.device).synchronize()
+    return staged.clone()
