@@ -995,7 +995,7 @@ __global__ void __launch_bounds__(256) coarse_place_kernel(CoarseHash h, int32_t
     emit_leaf(h.cmask[c * 8 + (lane >> 2)], o.x, o.y, o.z, o.w, h.base[p], p, lane, out_ijk, leaves, slots, cap);
 }
 
-// 8 + 4 bytes per slot (2 to 4 slots per fine leaf) and 116 per fine leaf
+// 8 + 4 bytes per slot (2 to 4 slots per fine leaf) and 108 per fine leaf
 size_t coarse_hash_layout(int64_t nl, CoarseHash *w, char *base) {
     CoarseHash h;
     h.cap = 64;
@@ -1669,7 +1669,7 @@ extern "C" int fvgb_coarse_grid_index(const FvgbGrid *fine, const int32_t factor
     int grid_bits = 0;
     while ((1 << grid_bits) < fine->num_grids) ++grid_bits;
     const int bits = vb + grid_bits;
-    if (bits >= 64) return FVGB_EINVAL;  // a key of all ones is the table's free slot
+    if (bits >= 64) return FVGB_ERANGE;  // a key of all ones is the table's free slot
     cudaStream_t s = as_stream(stream);
     CoarseHash h;
     coarse_hash_layout(nl, &h, align_ws(workspace));

@@ -449,7 +449,7 @@ GridPtr build_coarse_by_leaves(const GridPtr &g, const Vec3 &f, const int32_t lo
                                                   pb->meta.data_ptr<int64_t>(),
                                                   reinterpret_cast<FvgbLeaf *>(pb->leaves.data_ptr<uint8_t>()),
                                                   pb->hash.data_ptr<int32_t>(), cap, ws.data_ptr(), ws.numel(), cs);
-            if (st == FVGB_EINVAL) pb->leaves = pb->hash = Tensor();  // keys too wide: the sort
+            if (st == FVGB_ERANGE) pb->leaves = pb->hash = Tensor();  // keys too wide: the sort
             else check_status(st, "coarse grid");
         }
         if (!pb->leaves.defined()) {

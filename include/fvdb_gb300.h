@@ -179,8 +179,9 @@ int fvgb_coarse_grid_build(const FvgbGrid *fine, const int32_t factor[3], const 
 /* The same coarse grid with its index, for up to 49,152 fine leaves: ijk, meta (offsets, coarse leaves,
  * voxels, 0), leaf table [num_fine_leaves entries of room] and leaf
  * hash (hash_capacity a power of two >= 2 num_fine_leaves).  Found through a hash table and ordered by
- * counting instead of sorting; FVGB_EINVAL where the grid is larger (fvgb_coarse_grid_build serves
- * it).  No counterpart in the reference. */
+ * counting instead of sorting; the workspace query returns FVGB_EINVAL where the grid is larger and the
+ * build FVGB_ERANGE where grids and box need keys of 64 bits (fvgb_coarse_grid_build serves both).  No
+ * counterpart in the reference. */
 int fvgb_coarse_grid_index_workspace(int64_t num_fine_leaves, size_t *bytes);
 int fvgb_coarse_grid_index(const FvgbGrid *fine, const int32_t factor[3], const int32_t box_lo[3],
                            const int32_t box_hi[3], int32_t *out_ijk, int64_t *meta, FvgbLeaf *leaves,

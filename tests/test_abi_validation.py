@@ -69,3 +69,32 @@ def test_probe_checks(lib):
     assert lib.fvgb_row_gather_probe(I32(0), P, I64(100), P, I32(64), I32(1), P, ctypes.byref(bytes_), None) == EINVAL
     assert lib.fvgb_ffma_probe(None, I64(10), I32(1), ctypes.byref(flops), None) == EINVAL
     assert lib.fvgb_ffma_probe(P, I64(10), I32(65), ctypes.byref(flops), None) == EINVAL
+
+
+class _Grid(ctypes.Structure):
+    _fields_ = [
+        ("num_grids", I32), ("reserved", I32), ("num_voxels", I64), ("num_leaves", I64), ("hash_capacity", I64),
+        ("voxel_offsets", ctypes.c_void_p), ("ijk", ctypes.c_void_p), ("leaves", ctypes.c_void_p),
+        ("hash_slots", ctypes.c_void_p),
+    ]
+
+
+def test_coarse_grid_index_tells_wide_keys_from_bad_arguments(lib):
+    ERANGE = 3
+    n = SZ(0)
+    assert lib.fvgb_coarse_grid_index_workspace(I64(49153), ctypes.byref(n)) == EINVAL
+    assert lib.fvgb_coarse_grid_index_workspace(I64(10), ctypes.byref(n)) == 0
+    lim = 1 << 20
+
+    def call(grids, factor, lo, hi, cap=64, bytes_=n.value):
+        g = _Grid(grids, 0, 10, 10, 64, 64, 64, 64, 64)
+        v = lambda t: (I32 * 3)(*t)
+        return lib.fvgb_coarse_grid_index(ctypes.byref(g), v(factor), v(lo), v(hi), P, P, P, P, I64(cap), P, SZ(bytes_), None)
+
+    whole = ((-lim,) * 3, (lim - 1,) * 3)
+    assert call(513, (2, 2, 2), *whole) == ERANGE  # 54 + 10 bits
+    assert call(1025, (2, 2, 2), *whole) == EINVAL
+    assert call(513, (2, 3, 2), *whole) == EINVAL
+    assert call(513, (2, 2, 2), whole[1], whole[0]) == EINVAL
+    assert call(513, (2, 2, 2), *whole, cap=63) == EINVAL
+    assert call(513, (2, 2, 2), *whole, bytes_=16) == 6  # FVGB_ENOSPACE

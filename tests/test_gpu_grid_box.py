@@ -136,3 +136,21 @@ def test_coarse_grid_leaf_counts(cuda_device, leaves, factor):
     coarse = grid.conv_grid(factor, factor)
     assert np.array_equal(coarse.ijk.jdata.cpu().numpy(), c_ijk)
     assert np.array_equal(coarse.joffsets.cpu().numpy(), c_off)
+
+
+def test_coarse_grids_whose_keys_need_64_bits(cuda_device):
+    """Many grids over the whole coordinate range: the coarse leaves' keys do not fit beside the grid index,
+    and the sort serves them."""
+    import fvdb
+
+    rng = np.random.default_rng(8)
+    lim = 1 << 20
+    parts = [rng.choice([-lim, -4097, -1, 0, 5, lim - 1], (4, 3)).astype(np.int32) for _ in range(520)]
+    grid = fvdb.GridBatch.from_ijk(fvdb.JaggedTensor([torch.from_numpy(p).to(cuda_device) for p in parts]))
+    ijk, off = grid.ijk.jdata.cpu().numpy(), grid.joffsets.cpu().numpy()
+    coarse = grid.conv_grid(2, 2)
+    from oracle import oracle as orc
+
+    want, want_off = orc.grid_from_ijk(ijk >> 1, off)
+    assert np.array_equal(coarse.ijk.jdata.cpu().numpy(), want)
+    assert np.array_equal(coarse.joffsets.cpu().numpy(), want_off)
