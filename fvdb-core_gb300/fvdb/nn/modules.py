@@ -120,7 +120,8 @@ class SparseConv3d(nn.Module):
         s, t = (v.detach().float() for v in out_affine)
         if self.bias is None:
             return s, t
-        if plain_cuda(s, t, self.bias) and _vectors(s, t) and _vectors(self.bias) and self.bias.shape == s.shape:
+        if (plain_cuda(s, t, self.bias) and _vectors(s, t) and _vectors(self.bias) and self.bias.shape == s.shape and
+                self.bias.device == s.device):
             return s, _lib.load().fold_bias(self.bias.detach(), s, t)
         return s, self.bias.detach().float() * s + t
 
