@@ -834,7 +834,9 @@ std::optional<RowOrder> built_row_order(const PackPtr &p, bool transposed) {
 //     and 340, 0.53M 654 and 581; dense 0.88M 1147 and 1255), shorter ones from 655k on (64->256: 0.23M
 //     194 and 255, 0.53M 393 and 410; 128->256 FP8: 0.53M 589 and 620, 5.1M 4000 and 3020);
 //   * a contraction that announces another over the same map (reuse: training), from 2^16 rows on (64->64, a
-//     training step: 0.022M 347 and 372, 0.056M 328 and 331, 0.11M 329 and 323, 0.53M 826 and 754).
+//     training step: 0.022M 347 and 372, 0.056M 328 and 331, 0.11M 329 and 323, 0.53M 826 and 754) and two
+//     voxels per leaf (0.2M scattered voxels, one per leaf, whose rows have themselves alone: 522 and 572;
+//     11 per leaf 395 and 332).
 std::optional<RowOrder> pack_row_order_if_reused(PackPtr p, bool transposed, int64_t row_bytes, int64_t cout, bool reuse,
                                                  bool mirror = false) {
     const int d = transposed ? 1 : 0;
@@ -843,7 +845,7 @@ std::optional<RowOrder> pack_row_order_if_reused(PackPtr p, bool transposed, int
         const int64_t n = rows->N;
         const bool one_entry =
             transposed && p->st.v[0] >= p->ks.v[0] && p->st.v[1] >= p->ks.v[1] && p->st.v[2] >= p->ks.v[2];
-        bool at_once = reuse && n >= (int64_t)1 << 16;
+        bool at_once = reuse && n >= (int64_t)1 << 16 && n >= 2 * rows->L;
         if (one_entry) at_once |= row_bytes >= 256 && (double)n * row_bytes * row_bytes >= (double)((int64_t)1 << 34);
         else if (row_bytes * cout >= 128 * 256 && n <= 256 * rows->L)
             at_once |= n >= (row_bytes >= 256 ? (int64_t)1 << 18 : (int64_t)5 << 17);

@@ -40,6 +40,23 @@ def test_training_step(cuda_device, n):
     assert float((first[2].float() - second[2].float()).norm() / second[2].float().norm()) <= 2**-8 + 2e-5
 
 
+def test_training_step_over_scattered_voxels(cuda_device):
+    import fvdb
+
+    g = torch.Generator().manual_seed(1)
+    ijk = torch.randint(-4000, 4000, (70000, 3), generator=g, dtype=torch.int32)
+    grid = fvdb.GridBatch.from_ijk(ijk.to(cuda_device))
+    assert 1 << 16 <= grid.total_voxels < 2 * grid._impl.total_leaf_nodes
+    pack, _ = grid.sparse_conv_kernel_map(3, 1)
+    x = torch.randn(grid.total_voxels, 32, generator=g).to(cuda_device, torch.bfloat16)
+    w = (torch.randn(64, 32, 3, 3, 3, generator=g) * 0.05).to(cuda_device, torch.bfloat16)
+    first = _step(pack, x, w)
+    assert not pack._impl.has_row_order()
+    second = _step(pack, x, w)
+    assert pack._impl.has_row_order()
+    assert torch.equal(first[0], second[0]) and torch.equal(first[1], second[1])
+
+
 @pytest.mark.parametrize("n,cin,cout,dense,at_once", [
     ((1 << 18) - 1, 128, 128, False, False), (1 << 18, 128, 128, False, True), (1 << 18, 64, 256, False, False),
     (1 << 18, 128, 128, True, False), (1 << 18, 128, 64, False, False)])
