@@ -1158,35 +1158,35 @@ __device__ __forceinline__ uint32_t leaf_home(const LeafHash &h, uint64_t key) {
     return __umulhi((uint32_t)(m >> 32), h.cap);
 }
 
-// The slot of a leaf, from slot s on, or kNoSlot where the table is too full for the input.  `made`: this
-// thread took the slot.  stat: [0] leaves, [1] error word, [2] overflow, [3..5] largest -x, -y, -z, [6..8]
+// The slot of a leaf, from slot s on, or kNoSlot where the table is too full for the input, with kMade set
+// where this thread took it.  stat: [0] leaves, [1] error word, [2] overflow, [3..5] largest -x, -y, -z, [6..8]
 // largest x, y, z, [9..] voxels of each grid.
 // An input with too many leaves fills the table in the first wave of CTAs, before any of them ends and
 // adds up its leaves, and probes of a full table are as long as they may be (1.05M scattered rows: 1.6 ms).
 // So the CTAs count slots as they take them, each on one of kTakenCounters lines; whoever brings a line
 // past its share of max_leaves, and every 1/16 of that further, adds them all up.  Lines that are all
-// below that leave the table below 80 % full.  The others look at the overflow word before each insertion
-// but the first and in long probes.
-constexpr uint32_t kNoSlot = ~0u;
-__device__ __forceinline__ uint32_t insert_leaf(const LeafHash &h, uint64_t key, uint32_t s, int32_t *stat, bool &made) {
+// below that leave the table below 80 % full.  The others look at the overflow word after each leaf that they
+// bring and in long probes.
+constexpr uint64_t kNoSlot = 0xffffffffu, kMade = 1ull << 32;
+__device__ __forceinline__ uint64_t insert_leaf(uint64_t *table, int32_t *taken, uint32_t cap, int32_t max_leaves, uint64_t key,
+                                             uint32_t s, int32_t *stat) {
     for (int probe = 1; probe <= kHashProbes; ++probe) {
-        uint64_t k = *reinterpret_cast<volatile uint64_t *>(h.table + s);
+        uint64_t k = *reinterpret_cast<volatile uint64_t *>(table + s);
         if (k == kEmptyLeaf) {
-            k = atomicCAS(reinterpret_cast<unsigned long long *>(h.table + s), kEmptyLeaf, key);
+            k = atomicCAS(reinterpret_cast<unsigned long long *>(table + s), kEmptyLeaf, key);
             if (k == kEmptyLeaf) {  // this thread's leaf
-                const int32_t share = h.max_leaves / kTakenCounters, step = (share + 15) / 16;
-                const int32_t past = atomicAdd(h.taken + (blockIdx.x % kTakenCounters) * 32, 1) - share;
+                const int32_t share = max_leaves / kTakenCounters, step = (share + 15) / 16;
+                const int32_t past = atomicAdd(taken + (blockIdx.x % kTakenCounters) * 32, 1) - share;
                 if (past >= 0 && past % step == 0) {
                     int32_t n = 0;
-                    for (int c = 0; c < kTakenCounters; ++c) n += *reinterpret_cast<volatile int32_t *>(h.taken + c * 32);
-                    if (n > h.max_leaves) stat[2] = 1;
+                    for (int c = 0; c < kTakenCounters; ++c) n += *reinterpret_cast<volatile int32_t *>(taken + c * 32);
+                    if (n > max_leaves) stat[2] = 1;
                 }
-                made = true;
-                return s;
+                return s | kMade;
             }
         }
         if (k == key) return s;
-        s = s + 1 < h.cap ? s + 1 : 0;
+        s = s + 1 < cap ? s + 1 : 0;
         if (probe % 16 == 0 && *reinterpret_cast<volatile int32_t *>(stat + 2)) return kNoSlot;
     }
     stat[2] = 1;
@@ -1200,17 +1200,21 @@ __global__ void stat_init_kernel(int32_t *stat, int32_t n) {
 
 // The pass over ijk rows (P = int32_t) or points (P = the points' type, voxelised in T).
 template <typename P, typename T>
-__global__ void __launch_bounds__(256) leaf_insert_kernel(const P *__restrict__ in, const int64_t *__restrict__ joff,
+__global__ void __launch_bounds__(256, 5) leaf_insert_kernel(const P *__restrict__ in, const int64_t *__restrict__ joff,
                                                           int32_t B, int64_t n, const double *__restrict__ vs,
                                                           const double *__restrict__ org, LeafHash h,
                                                           int32_t *__restrict__ stat) {
     constexpr bool kPoints = !std::is_same<P, int32_t>::value;
     __shared__ T fac[6];
-    __shared__ int32_t sb[2], full, first_id, made_by[8], box[7][8];
+    __shared__ int32_t sb[2], full, made, first_id, box[7][8];
+    __shared__ uint32_t made_slot[256 * kHashRows];  // slots that the CTA took
     const int64_t base = (int64_t)blockIdx.x * 256 * kHashRows;
     const int64_t last = min(n, base + 256 * kHashRows) - 1;
     if (threadIdx.x < 2) sb[threadIdx.x] = batch_of(joff, B, threadIdx.x == 0 ? base : last);
-    if (threadIdx.x == 2) full = *reinterpret_cast<volatile int32_t *>(stat + 2);
+    if (threadIdx.x == 2) {
+        full = *reinterpret_cast<volatile int32_t *>(stat + 2);
+        made = 0;
+    }
     __syncthreads();
     if (kPoints) {
         if (threadIdx.x < 3) {
@@ -1250,16 +1254,12 @@ __global__ void __launch_bounds__(256) leaf_insert_kernel(const P *__restrict__ 
         }
     }
     int32_t fresh = 0;  // voxels this thread set
-    uint32_t mine = 0;  // rows whose leaf this thread brought into the table
-    uint64_t key[kHashRows];
-    uint32_t slot[kHashRows];
+    uint64_t key[kHashRows], word[kHashRows];
+    uint32_t slot[kHashRows], bit[kHashRows];
     if (!full) {  // else the input is left to the sort, which wants the bounding box alone
-        bool lost = false;
         // Every step's accesses for all rows go out together: the first probe, which finds most leaves, the
         // mask words, and the updates, whose results are looked at last (one after another each update's
         // wait added up: 200 us for 7.9M points, 132 us).
-        uint64_t word[kHashRows];
-        uint32_t bit[kHashRows];
 #pragma unroll
         for (int q = 0; q < kHashRows; ++q) {
             const int64_t i = min(base + q * 256 + threadIdx.x, last);
@@ -1270,17 +1270,29 @@ __global__ void __launch_bounds__(256) leaf_insert_kernel(const P *__restrict__ 
             slot[q] = leaf_home(h, key[q]);
             word[q] = __ldcg(h.table + slot[q]);
         }
+    }
+    if (!range) stat[1] = FVGB_ERANGE;
+#pragma unroll
+    for (int e = 0; e < 6; ++e) {
+        const int32_t v = __reduce_max_sync(0xffffffffu, lim[e]);
+        if ((threadIdx.x & 31) == 0) box[e][threadIdx.x >> 5] = v;
+    }
+    if (!full) {
+        bool lost = false, took = false;
 #pragma unroll
         for (int q = 0; q < kHashRows; ++q) {
             if (word[q] == key[q] || lost) continue;
-            if (q > 0 && *reinterpret_cast<volatile int32_t *>(stat + 2)) {
+            // who brings one leaf after another may be in an input of too many (a look per row, all at one
+            // address, took 30 us of 7.9M points' first wave)
+            if (took && *reinterpret_cast<volatile int32_t *>(stat + 2)) {
                 lost = true;
                 continue;
             }
-            bool made = false;
-            slot[q] = insert_leaf(h, key[q], slot[q], stat, made);
-            if (made) mine |= 1u << q;
-            lost = slot[q] == kNoSlot;
+            const uint64_t at = insert_leaf(h.table, h.taken, h.cap, h.max_leaves, key[q], slot[q], stat);
+            slot[q] = (uint32_t)at;
+            took = at & kMade;
+            if (took) made_slot[atomicAdd(&made, 1)] = (uint32_t)at;
+            lost = at == kNoSlot;
         }
 #pragma unroll
         for (int q = 0; q < kHashRows; ++q) {
@@ -1300,49 +1312,27 @@ __global__ void __launch_bounds__(256) leaf_insert_kernel(const P *__restrict__ 
             else atomicAdd(stat + 9 + (int32_t)(key[q] >> 54), 1);
         }
     }
-    if (!range) stat[1] = FVGB_ERANGE;
-    // the bounding box, once per CTA: every update reads one address (a read per warp, 31k warps on
-    // 7.9M points, set the kernel's pace: 170 us against 102), and the new voxels of the CTA's grid
-#pragma unroll
-    for (int e = 0; e < 6; ++e) {
-        const int32_t v = __reduce_max_sync(0xffffffffu, lim[e]);
-        if ((threadIdx.x & 31) == 0) box[e][threadIdx.x >> 5] = v;
-    }
     fresh = __reduce_add_sync(0xffffffffu, fresh);
     if ((threadIdx.x & 31) == 0) box[6][threadIdx.x >> 5] = fresh;
+    __syncthreads();
     // leaves are numbered by the CTA: one update of the count for all of its own (one per leaf, all on one
     // address, took 5 ns each: 0.9 ms for 175k leaves)
-    if (__syncthreads_or(mine != 0)) {
-        int32_t at = __popc(mine);
-        const int32_t own = at;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int32_t v = __shfl_up_sync(0xffffffffu, at, o);
-            if ((threadIdx.x & 31) >= o) at += v;
-        }
-        if ((threadIdx.x & 31) == 31) made_by[threadIdx.x >> 5] = at;
+    const int32_t n_made = made;
+    if (n_made) {
+        if (threadIdx.x == 0) first_id = atomicAdd(stat, n_made);
         __syncthreads();
-        int32_t before = 0, total = 0;
-#pragma unroll
-        for (int w = 0; w < 8; ++w) {
-            if (w < (int)(threadIdx.x >> 5)) before += made_by[w];
-            total += made_by[w];
-        }
-        if (threadIdx.x == 0) first_id = atomicAdd(stat, total);
-        __syncthreads();
-        int32_t id = first_id + before + at - own;
-#pragma unroll
-        for (int q = 0; q < kHashRows; ++q) {
-            if (!(mine >> q & 1)) continue;
+        for (int32_t i = threadIdx.x; i < n_made; i += 256) {
+            const int32_t id = first_id + i;
             if (id < h.max_leaves) {
-                h.keys[id] = key[q];
-                h.leaf_slot[id] = slot[q];
+                h.keys[id] = __ldcg(h.table + made_slot[i]);
+                h.leaf_slot[id] = made_slot[i];
             } else {
                 stat[2] = 1;
             }
-            ++id;
         }
     }
+    // the bounding box, once per CTA: every update reads one address (a read per warp, 31k warps on
+    // 7.9M points, set the kernel's pace: 170 us against 102), and the new voxels of the CTA's grid
     if (threadIdx.x < 6) {
         int32_t v = box[threadIdx.x][0];
 #pragma unroll

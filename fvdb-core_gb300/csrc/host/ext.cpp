@@ -176,13 +176,13 @@ Tensor per_grid_vec(const Tensor &t, int64_t B, const char *name) {
 
 // Builds g from n rows (ijk for dtype -1, else points with device voxel sizes / origins vsd / ord) through
 // the leaf hash.  False where the input has too few rows per leaf for it: the caller sorts, inside the rows'
-// bounding box box[0..2], box[3..5]; that and g's transforms are set in any case. 
+// bounding box box[0..2], box[3..5]; that and g's transforms are set in any case.
 // From kLeafHashRows rows on, where the sort reads the rows' bounding box first: the insertion measures it
-// too, so an input left to the sort pays little for the attempt (scattered rows: 0.3M 454 us before the
-// hash, 475 with it; 4.2M 1590 and 1613; six rows per leaf, 4.2M: 948 and 1029; points, whose conversion
-// got shorter: 4.2M 2226 and 1711).  Below the line the sort reads no box and the attempt is lost: 1k
-// scattered rows 263 us sorted, 317 with it; 65k 398 and 413; 0.25M 430 and 476.  Surfaces gain on both
-// sides of the line (65k rows: 385 us sorted, 158 hashed; 0.3M: 430 and 171).
+// too, which pays for most of an attempt in vain (scattered rows: 0.26M 463 us without the hash, 484 with it;
+// 4.2M 1599 and 1663; six rows per leaf, 4.2M: 944 and 1045; points, whose conversion got shorter: 4.2M
+// 2234 and 1744).  Below the line the sort reads no box and the attempt is lost: 1k scattered rows 263 us
+// sorted, 317 with it; 65k 398 and 413; 0.25M 430 and 476.  Surfaces gain on both sides of the line (65k
+// rows: 385 us sorted, 158 hashed; 0.3M: 430 and 171; dense 96^3 384 and 189).
 constexpr int64_t kLeafHashRows = (int64_t)1 << 18;
 constexpr int64_t kLeafHashGrids = 1023;
 
