@@ -808,13 +808,6 @@ std::optional<RowOrder> pack_row_order(PackPtr p, bool transposed) {
     return RowOrder{*p->order_rows[d], *p->order_mask[d], *p->order_map[d]};
 }
 
-// The row order if some contraction has built it.
-std::optional<RowOrder> built_row_order(const PackPtr &p, bool transposed) {
-    const int d = transposed ? 1 : 0;
-    if (!p->order_rows[d]) return std::nullopt;
-    return RowOrder{*p->order_rows[d], *p->order_mask[d], *p->order_map[d]};
-}
-
 // The row order for a tensor-core contraction once it is worth building.  Building it takes about 75 us of
 // small kernels and 85 us per million rows (x 27: a sort and a permuted copy of the map), and it saves a share
 // of every contraction, so the first contraction over a map runs in index order and the order serves the
@@ -837,20 +830,20 @@ std::optional<RowOrder> built_row_order(const PackPtr &p, bool transposed) {
 //     training step: 0.022M 347 and 372, 0.056M 328 and 331, 0.11M 329 and 323, 0.53M 826 and 754) and two
 //     voxels per leaf (0.2M scattered voxels, one per leaf, whose rows have themselves alone: 522 and 572;
 //     11 per leaf 395 and 332).
+bool row_order_at_once(const PackPtr &p, bool transposed, int64_t row_bytes, int64_t cout, bool reuse) {
+    const GridPtr &rows = transposed ? p->src : p->tgt;
+    const int64_t n = rows->N;
+    if (reuse && n >= (int64_t)1 << 16 && n >= 2 * rows->L) return true;
+    if (transposed && p->st.v[0] >= p->ks.v[0] && p->st.v[1] >= p->ks.v[1] && p->st.v[2] >= p->ks.v[2])
+        return row_bytes >= 256 && (double)n * row_bytes * row_bytes >= (double)((int64_t)1 << 34);
+    return row_bytes * cout >= 128 * 256 && n <= 256 * rows->L &&
+           n >= (row_bytes >= 256 ? (int64_t)1 << 18 : (int64_t)5 << 17);
+}
 std::optional<RowOrder> pack_row_order_if_reused(PackPtr p, bool transposed, int64_t row_bytes, int64_t cout, bool reuse,
                                                  bool mirror = false) {
-    const int d = transposed ? 1 : 0;
-    if (!p->order_rows[d]) {
-        const GridPtr &rows = transposed ? p->src : p->tgt;
-        const int64_t n = rows->N;
-        const bool one_entry =
-            transposed && p->st.v[0] >= p->ks.v[0] && p->st.v[1] >= p->ks.v[1] && p->st.v[2] >= p->ks.v[2];
-        bool at_once = reuse && n >= (int64_t)1 << 16 && n >= 2 * rows->L;
-        if (one_entry) at_once |= row_bytes >= 256 && (double)n * row_bytes * row_bytes >= (double)((int64_t)1 << 34);
-        else if (row_bytes * cout >= 128 * 256 && n <= 256 * rows->L)
-            at_once |= n >= (row_bytes >= 256 ? (int64_t)1 << 18 : (int64_t)5 << 17);
-        if (!at_once && ++p->order_requests[transposed || mirror ? 1 : 0] < 2) return std::nullopt;
-    }
+    if (!p->order_rows[transposed ? 1 : 0] && !row_order_at_once(p, transposed, row_bytes, cout, reuse) &&
+        ++p->order_requests[transposed || mirror ? 1 : 0] < 2)
+        return std::nullopt;
     return pack_row_order(p, transposed);
 }
 
@@ -1209,10 +1202,13 @@ Tensor gather_gemm(const Tensor &x, const Tensor &map, int64_t n_out, const Tens
 }
 
 // dW[k] = sum_m x[map[m,k]]^T dy[m]   -> [K, Cin, Cout]
-// pack, map_t: the owner of `map`; the tensor-core form runs over the map's row order where some
-// contraction has built one.
+// pack, map_t: the owner of `map`; ordered: the tensor-core form runs over the map's row order.  The order
+// of the rows is the order of the sum, so unlike a contraction's the result depends on it in the last bits:
+// a caller decides by the call's own sizes and types, never by whether the order happens to be built.  64->64
+// BF16, index and row order: 20k surface voxels 68 us each, 0.10M 101 each, 1.29M 555 and 523; 0.69M random
+// voxels, 20 per leaf, 335 and 184.
 Tensor gather_wgrad(const Tensor &x, const Tensor &map, int64_t n_out, const Tensor &dy, int64_t K,
-                    PackPtr pack = nullptr, bool map_t = false) {
+                    PackPtr pack = nullptr, bool map_t = false, bool ordered = false) {
     c10::cuda::CUDAGuard guard(x.device());
     const int64_t cin = x.size(1), cout = dy.size(1);
     const auto dtype = x.scalar_type();
@@ -1228,7 +1224,7 @@ Tensor gather_wgrad(const Tensor &x, const Tensor &map, int64_t n_out, const Ten
         size_t wsb = 0;
         check_status(fvgb_tc_wgrad_16bit_workspace(n_out, (int32_t)K, (int32_t)cin, (int32_t)cout, &wsb), "wgrad workspace");
         Tensor ws = workspace(wsb, x.device());
-        const std::optional<RowOrder> order = pack ? built_row_order(pack, map_t) : std::nullopt;
+        const std::optional<RowOrder> order = ordered ? pack_row_order(pack, map_t) : std::nullopt;
         const std::optional<Tensor> mask = order ? std::optional<Tensor>(order->mask) : pack ? pack_tile_mask(pack, map_t)
                                                                                              : std::nullopt;
         const uint32_t *tm = mask ? reinterpret_cast<const uint32_t *>(mask->data_ptr<int32_t>()) : nullptr;
@@ -1313,14 +1309,16 @@ std::vector<Tensor> conv_forward(const Tensor &x, const Tensor &weights, PackPtr
     return {y, Wkio};
 }
 
-// Returns (dx, dW) with dW in the 5-D layout of the forward weights.
+// Returns (dx, dW) with dW in the 5-D layout of the forward weights.  announced: the forward's has_backward;
+// the weight gradient runs over the row order that such a forward pass has built at once.
 std::vector<Tensor> conv_backward(const Tensor &dy_in, const Tensor &x, const Tensor &Wkio, PackPtr p, bool transposed,
-                                  bool need_dx, bool need_dw) {
+                                  bool need_dx, bool need_dw, bool announced = false) {
     resolve_pack(p);
     Tensor dy = dy_in.contiguous();
     const int64_t K = Wkio.size(0), cin = Wkio.size(1), cout = Wkio.size(2);
     Tensor dx, dW;
     const bool mirror = self_mirrored(p);
+    const bool ordered = row_order_at_once(p, transposed && !mirror, cin * 2, cout, announced && mirror);
     if (!transposed) {
         // dgrad: dx[i] = sum_k dy[mapT[i,k]] W[k]^T ;  wgrad: dW[k] = sum_m x[map[m,k]]^T dy[m]
         if (need_dx && mirror)
@@ -1329,14 +1327,14 @@ std::vector<Tensor> conv_backward(const Tensor &dy_in, const Tensor &x, const Te
         else if (need_dx)
             dx = gather_gemm(dy, pack_kmap_t(p), p->src->N, Wkio, true, std::nullopt, p, true);
         if (need_dw)
-            dW = gather_wgrad(x, pack_kmap(p), p->tgt->N, dy, K, p, false);
+            dW = gather_wgrad(x, pack_kmap(p), p->tgt->N, dy, K, p, false, ordered);
     } else {
         if (need_dx)
             dx = gather_gemm(dy, pack_kmap(p), p->tgt->N, Wkio, true, std::nullopt, p, false);
         if (need_dw && mirror)
-            dW = gather_wgrad(x, pack_kmap(p), p->src->N, dy, K, p, false).flip(0);
+            dW = gather_wgrad(x, pack_kmap(p), p->src->N, dy, K, p, false, ordered).flip(0);
         else if (need_dw)
-            dW = gather_wgrad(x, pack_kmap_t(p), p->src->N, dy, K, p, true);
+            dW = gather_wgrad(x, pack_kmap_t(p), p->src->N, dy, K, p, true, ordered);
     }
     if (need_dw) {
         dW = dW.reshape({p->ks.v[2], p->ks.v[1], p->ks.v[0], cin, cout});
@@ -1939,7 +1937,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           py::call_guard<py::gil_scoped_release>());
     m.def("check_device_errors", [](const torch::Device &d) { check_device_errors(d); },
           py::call_guard<py::gil_scoped_release>());
-    m.def("conv_backward", &conv_backward, py::call_guard<py::gil_scoped_release>());
+    m.def("conv_backward", &conv_backward, py::arg("grad"), py::arg("features"), py::arg("weights_kio"), py::arg("pack"),
+          py::arg("transposed"), py::arg("need_dx"), py::arg("need_dw"), py::arg("has_backward") = false,
+          py::call_guard<py::gil_scoped_release>());
     m.def("halo_conv", &halo_conv, py::arg("grid"), py::arg("features"), py::arg("weights"), py::arg("mirror"),
           py::arg("route") = (int64_t)kByRule, py::call_guard<py::gil_scoped_release>());
     m.def("halo_wgrad", &halo_wgrad, py::arg("grid"), py::arg("features"), py::arg("grad"),

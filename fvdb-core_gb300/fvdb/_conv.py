@@ -22,7 +22,8 @@ class SparseConvFunction(torch.autograd.Function):
                 relu: bool = False, scale=None):
         C = _lib.load()
         # a data gradient to come reuses the kernel map (and may share its row order)
-        y, wkio = C.conv_forward(features, weights, pack_impl, transposed, bias, relu, scale, ctx.needs_input_grad[0])
+        ctx.announced = ctx.needs_input_grad[0]
+        y, wkio = C.conv_forward(features, weights, pack_impl, transposed, bias, relu, scale, ctx.announced)
         ctx.scaled = scale is not None
         if relu:
             ctx.save_for_backward(features, wkio, y)
@@ -56,7 +57,8 @@ class SparseConvFunction(torch.autograd.Function):
         else:
             grad_out, db = C.bias_relu_backward(grad_out, y, need_db)
         if need_dx or need_dw:
-            dx, dw = C.conv_backward(grad_out, features, wkio, ctx.pack_impl, ctx.transposed, need_dx, need_dw)
+            dx, dw = C.conv_backward(grad_out, features, wkio, ctx.pack_impl, ctx.transposed, need_dx, need_dw,
+                                     ctx.announced)
         if need_db:
             db = db.to(ctx.bias_dtype)
         return (dx if need_dx else None), (dw if need_dw else None), None, None, db, None, None
