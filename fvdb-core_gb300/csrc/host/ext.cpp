@@ -821,7 +821,9 @@ std::optional<RowOrder> pack_row_order(PackPtr p, bool transposed) {
 //     index-order tile multiplies all K offsets for it.  Pays from rows of 256 bytes and n row_bytes^2 =
 //     2^34 on: 256->128, 2^3 stride 2: 0.056M rows 85 and 103, 0.11M 125 and 102, 0.88M 713 and 295;
 //     128->128: 0.11M 86 and 105, 0.26M 161 and 144, 0.53M 264 and 198; 64->64 never: 0.53M 137 and 172,
-//     0.88M 204 and 241;
+//     0.88M 204 and 241.  In training the weight gradient runs over it too (64->64: 0.26M 76 and 58, 0.88M
+//     150 and 99, 1.29M 200 and 132): from 128 bytes and 2^33 on (a step 64->32: 0.62M 359 and 350, 1.26M 600
+//     and 548);
 //   * wide layers (row bytes times output channels of 128 x 256 and more) over other than dense blocks,
 //     whose tiles have all offsets anyhow: rows of 256 bytes and more from 2^18 rows on (128->128: 0.23M 312
 //     and 340, 0.53M 654 and 581; dense 0.88M 1147 and 1255), shorter ones from 655k on (64->256: 0.23M
@@ -830,12 +832,18 @@ std::optional<RowOrder> pack_row_order(PackPtr p, bool transposed) {
 //     training step: 0.022M 347 and 372, 0.056M 328 and 331, 0.11M 329 and 323, 0.53M 826 and 754) and two
 //     voxels per leaf (0.2M scattered voxels, one per leaf, whose rows have themselves alone: 522 and 572;
 //     11 per leaf 395 and 332).
+bool one_entry_transposed(const PackPtr &p) {
+    return p->st.v[0] >= p->ks.v[0] && p->st.v[1] >= p->ks.v[1] && p->st.v[2] >= p->ks.v[2];
+}
 bool row_order_at_once(const PackPtr &p, bool transposed, int64_t row_bytes, int64_t cout, bool reuse) {
     const GridPtr &rows = transposed ? p->src : p->tgt;
     const int64_t n = rows->N;
+    if (transposed && one_entry_transposed(p)) {
+        const double size = (double)n * row_bytes * row_bytes;
+        return (row_bytes >= 256 && size >= (double)((int64_t)1 << 34)) ||
+               (reuse && row_bytes >= 128 && size >= (double)((int64_t)1 << 33));
+    }
     if (reuse && n >= (int64_t)1 << 16 && n >= 2 * rows->L) return true;
-    if (transposed && p->st.v[0] >= p->ks.v[0] && p->st.v[1] >= p->ks.v[1] && p->st.v[2] >= p->ks.v[2])
-        return row_bytes >= 256 && (double)n * row_bytes * row_bytes >= (double)((int64_t)1 << 34);
     return row_bytes * cout >= 128 * 256 && n <= 256 * rows->L &&
            n >= (row_bytes >= 256 ? (int64_t)1 << 18 : (int64_t)5 << 17);
 }
@@ -1092,6 +1100,12 @@ bool self_mirrored(const PackPtr &p) {
     return r;
 }
 
+// Whether the backward pass of a convolution gains from the row order of its forward pass: the data gradient
+// over the forward map, or the weight gradient of a transposed map of one entry a row.
+bool reused_in_backward(const PackPtr &p, bool transposed) {
+    return self_mirrored(p) || (transposed && one_entry_transposed(p));
+}
+
 // y[m] = sum_k x[map[m,k]] W[k]   for the first n_out rows of map
 // mirror: W in reverse offset order (see self_mirrored).  reuse: the caller will contract over this
 // map again (training: the data gradient), so a large map gets its row order at once.
@@ -1304,8 +1318,8 @@ std::vector<Tensor> conv_forward(const Tensor &x, const Tensor &weights, PackPtr
     const int64_t n_out = transposed ? n_src : n_tgt;
     const Tensor Wkio = kio_weights(weights, transposed, cin, cout);
     if (n_out == 0) return {torch::empty({0, cout}, x.options()), Wkio};
-    Tensor y = gather_gemm(x, map_t ? pack_kmap_t(p) : pack_kmap(p), n_out, Wkio, false, bias,
-                           p, map_t, relu, out_scale, mirror, has_backward && self_mirrored(p));
+    Tensor y = gather_gemm(x, map_t ? pack_kmap_t(p) : pack_kmap(p), n_out, Wkio, false, bias, p, map_t, relu, out_scale,
+                           mirror, has_backward && reused_in_backward(p, transposed));
     return {y, Wkio};
 }
 
@@ -1318,7 +1332,8 @@ std::vector<Tensor> conv_backward(const Tensor &dy_in, const Tensor &x, const Te
     const int64_t K = Wkio.size(0), cin = Wkio.size(1), cout = Wkio.size(2);
     Tensor dx, dW;
     const bool mirror = self_mirrored(p);
-    const bool ordered = row_order_at_once(p, transposed && !mirror, cin * 2, cout, announced && mirror);
+    const bool ordered = row_order_at_once(p, transposed && !mirror, cin * 2, cout,
+                                           announced && reused_in_backward(p, transposed));
     if (!transposed) {
         // dgrad: dx[i] = sum_k dy[mapT[i,k]] W[k]^T ;  wgrad: dW[k] = sum_m x[map[m,k]]^T dy[m]
         if (need_dx && mirror)

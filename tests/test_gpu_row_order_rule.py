@@ -77,6 +77,19 @@ def test_transposed_maps_of_one_entry(cuda_device, n, cin, at_once):
     assert pack._impl.has_row_order(True) and torch.equal(a, b)
 
 
+@pytest.mark.parametrize("n,cin,at_once", [((1 << 19) - 1, 64, False), (1 << 19, 64, True), (1 << 19, 32, False)])
+def test_transposed_maps_of_one_entry_in_training(cuda_device, n, cin, at_once):
+    grid, pack, x, w = _case(cuda_device, n, cin, 32, ks=2, st=2, transposed=True)
+    grads = []
+    for use in range(2):
+        xr, wr = x.clone().requires_grad_(True), w.clone().requires_grad_(True)
+        y = pack.sparse_transpose_conv_3d(xr, wr).jdata
+        assert pack._impl.has_row_order(True) == (at_once or use == 1)
+        y.backward(torch.ones_like(y))
+        grads.append((y.detach(), xr.grad, wr.grad))
+    assert all(torch.equal(a, b) for a, b in zip(*grads))
+
+
 def test_without_memory_for_the_order(cuda_device):
     import fvdb
 
