@@ -1108,7 +1108,7 @@ extern "C" int fvgb_coarse_grid_build(const FvgbGrid *fine, const int32_t factor
 // with the leaf table and the leaf hash in the same kernel.  Leaves sorted by (grid, order key) and
 // voxels by bit is the order of the voxel sort, so the grid is identical to fvgb_ijk_sort_unique's.
 // 7.9M points, 1.31M voxels, 22k leaves in four grids: voxelise, sort, unique and index took 1.9 ms,
-// 0.20 ms here, bound by the random reads of the table and the masks.  The table has room for
+// 0.21 ms here, bound by the random reads of the table and the masks.  The table has room for
 // rows / 8 leaves at three quarters full; an input with more (fewer than eight rows per leaf) raises
 // `overflow` and is left to the sort, which takes the bounding box from here (the rows' own: it is
 // complete whatever the table's state) in place of a pass and a host read of its own.
@@ -1116,7 +1116,7 @@ namespace fvgb {
 namespace {
 
 constexpr uint64_t kEmptyLeaf = ~0ull;
-constexpr int kHashRows = 4;      // rows per thread (more cost occupancy: 169 us with 8, 151 with 2, 132 with 4)
+constexpr int kHashRows = 4;      // rows per thread (more cost occupancy: 169 us with 8, 151 with 2, 132 with 4, before slots were counted; now 139)
 constexpr int kHashProbes = 512;  // a full neighbourhood of the table counts as overflow
 constexpr int kTakenCounters = 64;  // CTAs count the slots they take on a line of their share of these
 constexpr int kHashMaxGrids = 1023;  // the grid index takes the key's top 10 bits (all ones: the empty slot)

@@ -658,7 +658,8 @@ int build_map(const FvgbGrid *src, const FvgbGrid *tgt, const int32_t ksize[3], 
     const int64_t W = (int64_t)span(p.S2, p.st2, p.K2) * span(p.S1, p.st1, p.K1) * span(p.S0, p.st0, p.K0);
     p.window = W <= kMaxWindow ? (int32_t)W : 0;
     if ((row_mask || tgt->num_voxels >= kHaloVoxels * tgt->num_leaves) && !nbsizes && ld == 27 && ksize[0] == 3 &&
-        ksize[1] == 3 && ksize[2] == 3 && stride[0] == 1 && stride[1] == 1 && stride[2] == 1 && start[0] == -1 && start[1] == -1 && start[2] == -1) {
+        ksize[1] == 3 && ksize[2] == 3 && stride[0] == 1 && stride[1] == 1 && stride[2] == 1 && start[0] == -1 &&
+        start[1] == -1 && start[2] == -1) {
         constexpr int smem = kHaloLeaves * (int)sizeof(HaloWarp);
         static_assert(smem <= 48 * 1024 && sizeof(HaloWarp) % 16 == 0, "halo tables of a CTA");
         kmap_halo3_kernel<<<(unsigned)ceil_div(tgt->num_leaves, (int64_t)kHaloLeaves), 32 * kHaloLeaves, smem,

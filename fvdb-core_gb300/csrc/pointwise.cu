@@ -2,7 +2,7 @@
 // output is not positive and sums the bias gradient in the same pass.
 //
 // Bound by HBM: reads dy (and y), writes the masked dy.  Two layers of 1.27M x 64 BF16, one with a
-// ReLU: a comparison, a mixed-type product and two column sums took 538 us, 141 us here.
+// ReLU: a comparison, a mixed-type product and two column sums took 538 us, 124 us here.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 

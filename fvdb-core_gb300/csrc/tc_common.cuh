@@ -138,12 +138,6 @@ __device__ __forceinline__ void cp_async_arrive_noinc(uint64_t *bar) {
 }
 
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-// Wait until at most N of this thread's committed cp.async groups are pending.
-template <int N>
-__device__ __forceinline__ void cp_async_wait_group() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
 
 // 1-D bulk async copy shared -> global (bulk async-group completion).
 __device__ __forceinline__ void bulk_s2g(void *dst, uint32_t src, uint32_t bytes) {
