@@ -611,7 +611,8 @@ def leg_c1(fvdb, dev, args) -> dict:
 
 def leg_halo(fvdb, grid, x, model, args) -> dict:
     """Layer 1 of the headline step (3^3, stride 1, 32 -> 64) through GridBatch.sparse_conv_halo
-    (leaf-halo kernels, no kernel map) beside the kernel-map path (map build included), BF16 and
+    (BF16 and the FP32 weight gradient over a map that lives for the call, the FP32 forward and data
+    gradient on the leaf-halo kernels) beside the kernel-map path (map build included), BF16 and
     FP32, forward and forward + backward; errors of each against FP64.  On the headline's
     sphere-shell grids and on a dense 96^3 block (every leaf full)."""
     dev = x.device

@@ -123,7 +123,8 @@ int fvgb_ijk_sort_unique_in_box(const int32_t *ijk, const int64_t *joffsets, int
  *   insert: rows are ijk (dtype -1, int32) or points (FVGB_F32 / F64 / F16 / BF16, voxelised with
  *   voxel_sizes / origins as fvgb_points_to_ijk does).  stat (device int32 [9 + num_grids]): leaves,
  *   error word (FVGB_ERANGE), overflow (more than one leaf per eight rows: the caller sorts instead),
- *   the largest -x, -y, -z, x, y, z, then the voxels of each grid.  The caller reads it and allocates.
+ *   the largest -x, -y, -z, x, y, z of all rows (complete on overflow too, for the sort in that box),
+ *   then the voxels of each grid (not on overflow).  The caller reads it and allocates.
  *   finish: with the insert's workspace, the leaf count and the bounding box it reported: out_ijk
  *   (a row per voxel), out_joffsets [num_grids + 1], the leaf table and the leaf hash
  *   (hash_capacity a power of two >= 2 num_leaves).
@@ -177,8 +178,8 @@ int fvgb_coarse_grid_build(const FvgbGrid *fine, const int32_t factor[3], const 
                            int32_t *out_ijk, int64_t *meta, int32_t *leaf_ids, void *workspace, size_t workspace_bytes,
                            fvgb_stream_t stream);
 /* The same coarse grid with its index, for up to 49,152 fine leaves: ijk, meta (offsets, coarse leaves,
- * voxels, 0), leaf table [num_fine_leaves entries of room] and leaf
- * hash (hash_capacity a power of two >= 2 num_fine_leaves).  Found through a hash table and ordered by
+ * voxels, 0), leaf table [num_fine_leaves entries of room] and leaf hash
+ * (hash_capacity a power of two >= 2 num_fine_leaves).  Found through a hash table and ordered by
  * counting instead of sorting; the workspace query returns FVGB_EINVAL where the grid is larger and the
  * build FVGB_ERANGE where grids and box need keys of 64 bits (fvgb_coarse_grid_build serves both).  No
  * counterpart in the reference. */
