@@ -184,6 +184,11 @@ class ContinuousBatcher:
         i = 0
         while i < len(pending) or not self.idle():
             now = self.clock()
+            if i < len(pending) and pending[i].arrival <= now < pending[i].arrival + poll_sleep and self.idle():
+                # an idle server takes requests that come within a poll interval as one batch, also when
+                # it happens to look between them (a launch costs far more than the wait)
+                time.sleep(pending[i].arrival + poll_sleep - now)
+                now = self.clock()
             while i < len(pending) and pending[i].arrival <= now:
                 self.submit(pending[i])
                 i += 1
